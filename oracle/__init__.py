@@ -49,11 +49,11 @@ _dp = ctypes.POINTER(ctypes.c_double)
 
 
 def build(with_reference: bool | None = None) -> None:
-    """Compiles the restatement, and the reference harness when the reference tree exists."""
+    """Compiles the restatement, and the reference harness when the reference tree holds its headers."""
     targets = ["oracle"]
     tree = reference_tree()
     if with_reference is None:
-        with_reference = bool(tree) and os.path.isdir(tree)
+        with_reference = bool(tree) and os.path.isfile(os.path.join(tree, "FIELD_UNIFORM_1D.h"))
     if with_reference:
         targets.append("ref")
     subprocess.run(["make", "-s", "-C", HERE] + targets + ([f"REF={tree}"] if tree else []), check=True)
