@@ -8,11 +8,21 @@
 // a single instance is the same launch with one queue entry.  Each step is captured once into a
 // CUDA graph (queue reset + step kernel) and replayed.
 //
+// A step is a serial chain of short phases on one SM, so what it costs is the number of its
+// phases and the latency of each.  Two representations keep both small:
+//   - Masks and levels are bit planes while a step runs (one bit per point, the point i at bit
+//     i & 31 of word (i >> 5) + 1).  A pass over a mask is a handful of shifts per 32-bit word in
+//     one phase, where a point-per-thread pass walks every point of the line.  Levels are
+//     bit-sliced (`nb` planes per level set) next to a plane of the finest-level points.
+//   - The transforms and the stages run over compact lists of active points (16-bit entries where
+//     the line allows it); the transform list is ordered by level, so that the points a level
+//     predicts and the coarser points it updates are each one contiguous range.
+//
 // Per-instance layout in the pool (w = Nx + 6, ghost ring 3): doubles q[3][w] (conserved),
 // qc[3][w] (stage-start copy), qt[3][w] (coarse-point flux derivatives of a stage), fl[3][w] (face
-// fluxes, face i+1/2 at point i), then w + 32 doubles holding the stage worklists of an instance
-// too large to stage in shared memory (2 (w + 32) indices); bytes mask[w] (bits 0..3 mask0..3,
-// 4 previous mask0, 5/6 work bits), then 16-byte aligned level[4][w].
+// fluxes, face i+1/2 at point i), then 2 (w + 32) doubles of list space; then the bit planes.
+// Bytes mask[w] (bits 0..3 mask0..3, 4 previous mask0; 5..7 set on the ghost ring), then 16-byte
+// aligned level[4][w]: the form in which masks and levels rest between launches.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -47,475 +57,758 @@ struct Inst1 {
 // BOUNDARY_CONDITION values of the generic manager (BOUNDARY_MANAGER_1D.h:4-13).
 constexpr int kBcPeriodic1 = -3, kBcExtrapolation1 = -2;
 
+// Threads per CTA of the step kernel at most.
+#ifndef AWCM_MAX_THREADS_1D
+#define AWCM_MAX_THREADS_1D 768
+#endif
+constexpr int kMaxThreads1 = AWCM_MAX_THREADS_1D;
+
 struct Pool {
     double* q;
     uint8_t* m;
     Weights W;
 };
 
-__device__ __forceinline__ double block_max(double v, double* red)
-{
-    v = warp_max(v);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    double r = 0;
-    const int nw = (blockDim.x + 31) >> 5;
-    for (int k = 0; k < nw; ++k) r = maxd(r, red[k]);
-    __syncthreads();
-    return r;
-}
+__host__ __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
-// Sums of four per-thread counts over the block (one shared-memory round for all four).
-__device__ __forceinline__ void block_sum4(unsigned (&v)[4], unsigned* red)
+// ---------------------------------------------------------------------------------- bit planes
+// Planes of an instance, in this order: mask0..mask3, the previous mask0 (mask_temp), two work
+// planes, the finest-level points of level0..level3, then the nb slices of level0, of level1, ..
+// The bits of a word outside the ghosted line are set in the mask planes: ComputeLevel reads a
+// mask as set there, and every other pass ands with the words' valid bits.
+enum Plane1 : int { kPlTemp = 4, kPlAux = 5, kPlStart = 6, kPlFine = 7, kPlLevel = 11 };
+// Slices of a level value: enough for 0..maxl and one more value, all ones, which stands for a level
+// outside that range (only set_levels can put one there; it rests in the bytes and is never used).
+__host__ __device__ __forceinline__ int level_bits(int maxl)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-    __syncthreads();
-    if (lane == 0)
-        for (int k = 0; k < 4; ++k) red[4 * warp + k] = v[k];
-    __syncthreads();
-    for (int k = 0; k < 4; ++k) {
-        unsigned r = 0;
-        for (int q = 0; q < nw; ++q) r += red[4 * q + k];
-        v[k] = r;
-    }
-    __syncthreads();
+    int b = 1;
+    while ((1 << b) - 1 <= maxl) ++b;
+    return b;
 }
-
-// Exclusive prefix of v over the threads of the block (thread order); *total = the block sum.
-__device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* red, unsigned* total)
+__host__ __device__ __forceinline__ int plane_words1(int nx) { return ((nx - 1 + kGhost + 32) >> 5) + 1; }
+__host__ __device__ __forceinline__ size_t plane_bytes1(int nx, int maxl)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
-    unsigned x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    __syncthreads();
-    if (lane == 31) red[warp] = x;
-    __syncthreads();
-    unsigned before = 0, all = 0;
-    for (int k = 0; k < nw; ++k) {
-        const unsigned r = red[k];
-        before += k < warp ? r : 0u;
-        all += r;
-    }
-    *total = all;
-    return before + x - v;
+    return align16(sizeof(uint32_t) * (size_t)(kPlLevel + 4 * level_bits(maxl)) * (size_t)plane_words1(nx));
 }
+// List space: two regions of 2 (w + 32) entries each (a stage's faces and points).
+__host__ __device__ __forceinline__ size_t list_entries1(int w) { return 2 * ((size_t)w + 32); }
+__host__ __device__ __forceinline__ bool short_lists(int w) { return w <= 0xffff; }
+__host__ __device__ __forceinline__ size_t entry_bytes(int w) { return short_lists(w) ? 2 : 4; }
 
-// The same over 64-bit values (three packed 21-bit counts); red holds one 64-bit word per warp.
-__device__ __forceinline__ unsigned long long block_exclusive_scan64(unsigned long long v, unsigned long long* red,
-                                                                     unsigned long long* total)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
-    unsigned long long x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    __syncthreads();
-    if (lane == 31) red[warp] = x;
-    __syncthreads();
-    unsigned long long before = 0, all = 0;
-    for (int k = 0; k < nw; ++k) {
-        const unsigned long long r = red[k];
-        before += k < warp ? r : 0ull;
-        all += r;
-    }
-    *total = all;
-    return before + x - v;
-}
-
-// Block-wide stream compaction of the indices lo..hi whose predicate holds into `list` (order
-// preserved).  Returns the count.  Each thread owns a contiguous chunk of the range: it counts its
-// hits, one block-wide exclusive scan gives its output offset, and it writes its hits in order
-// (two evaluations of the predicate, three barriers in all, whatever the range).
-template <class Pred>
-__device__ int block_compact(int lo, int hi, Pred pred, uint32_t* list, unsigned* red)
-{
-    const int n = hi - lo + 1;
-    const int per = (n + (int)blockDim.x - 1) / (int)blockDim.x;
-    const int a0 = lo + (int)threadIdx.x * per;
-    const int a1 = min(a0 + per, hi + 1);
-    unsigned cnt = 0;
-    for (int i = a0; i < a1; ++i) cnt += pred(i) ? 1u : 0u;
-    unsigned total;
-    unsigned off = block_exclusive_scan(cnt, red, &total);
-    for (int i = a0; i < a1; ++i)
-        if (pred(i)) list[off++] = (uint32_t)i;
-    __syncthreads();
-    return (int)total;
-}
-
-// Views of one instance for a step or a pass.  Pointers are generic: in the step kernel the mask
-// bytes, the levels and the density plane point into the CTA's shared memory (staged in and out
-// around the step), elsewhere into the instance's global buffers.
-struct Ctx {
-    const Inst1& I;
-    double* q;   // q[p*w + i + 3] (plane 0 is read through q0)
-    double* qc;
-    double* qt;
-    double* fl;
-    uint8_t* m;  // m[i + 3]
-    int8_t* lv;  // lv[l*w + i + 3]
-    const Weights& W;
-    int w, nx, N1, maxl;
-    double* q0;  // density plane: q0[i + 3]
-    __device__ double& Q(int p, int i) const { return (p == 0 ? q0 : q + p * w)[i + kGhost]; }
-    __device__ double& QT(int p, int i) const { return qt[p * w + i + kGhost]; }
-    __device__ double& QC(int p, int i) const { return qc[p * w + i + kGhost]; }
-    __device__ uint8_t& M(int i) const { return m[i + kGhost]; }
-    __device__ int8_t& L(int l, int i) const { return lv[l * w + i + kGhost]; }
-    __device__ bool bit(int i, int b) const { return (m[i + kGhost] >> b) & 1u; }
-    // Mask push; pushes off the ghosted line (only reachable from inconsistent user-set
-    // masks/levels, where the reference writes out of bounds) are dropped.
-    // atomicOr on the containing 32-bit word: no dependent round trip per push.
-    __device__ void set(int i, int b) const
-    {
-        if (i < -kGhost || i >= nx + kGhost) return;
-        const uintptr_t a = reinterpret_cast<uintptr_t>(m + i + kGhost);
-        atomicOr(reinterpret_cast<unsigned*>(a & ~(uintptr_t)3), 1u << (8 * (unsigned)(a & 3) + b));
-    }
-    // The push of the bits `bits` (one byte's worth) of point i in one atomicOr.
-    __device__ void set_bits(int i, unsigned bits) const
-    {
-        if (i < -kGhost || i >= nx + kGhost) return;
-        const uintptr_t a = reinterpret_cast<uintptr_t>(m + i + kGhost);
-        atomicOr(reinterpret_cast<unsigned*>(a & ~(uintptr_t)3), bits << (8 * (unsigned)(a & 3)));
-    }
-    // The same push on the n <= 8 consecutive points i0 .. i0+n-1: one atomicOr per 32-bit word.
-    __device__ void set_run(int i0, int n, int b) const
-    {
-        const int lo = i0 < -kGhost ? -kGhost : i0, hi = min(i0 + n - 1, nx + kGhost - 1);
-        if (lo > hi) return;
-        uintptr_t a = reinterpret_cast<uintptr_t>(m + lo + kGhost);
-        const uintptr_t e = reinterpret_cast<uintptr_t>(m + hi + kGhost);
-        while (a <= e) {
-            const uintptr_t wb = a & ~(uintptr_t)3;
-            const uintptr_t we = wb + 3 < e ? wb + 3 : e;
-            unsigned bits = 0;
-            for (uintptr_t x = a; x <= we; ++x) bits |= 1u << (8 * (unsigned)(x & 3) + b);
-            atomicOr(reinterpret_cast<unsigned*>(wb), bits);
-            a = we + 1;
-        }
-    }
-    __device__ int D(int lev) const { return 1 << (maxl - lev); }
-    __device__ double w_(int cnt, int k) const { return W.w[cnt][k + 1]; }
+// The per-CTA workspace: class counters of the ordered list, list counters, reductions.
+struct Work1 {
+    unsigned cls[32], run[32], off[33];  // counts, write positions, starts of the level classes
+    unsigned mask_cnt[4];                // |mask0..mask3|
+    unsigned n_face[4], n_fin[4];        // of mask0..mask2: needed faces, finest-level points
+    unsigned n_list[4][4];               // per mask: entries written so far (faces, finest, coarse points)
+    unsigned long long red[3][2][32];    // per reduction of the step: two maxima, one value per warp
 };
 
+// A list of points (stored as i + kGhost) with 16- or 32-bit entries.
+struct List {
+    void* p;
+    bool half;
+    __device__ __forceinline__ int get(unsigned e) const
+    {
+        return (half ? (int)static_cast<const uint16_t*>(p)[e] : (int)static_cast<const uint32_t*>(p)[e]) - kGhost;
+    }
+    __device__ __forceinline__ void put(unsigned e, int i) const
+    {
+        if (half) static_cast<uint16_t*>(p)[e] = (uint16_t)(i + kGhost);
+        else static_cast<uint32_t*>(p)[e] = (uint32_t)(i + kGhost);
+    }
+    __device__ __forceinline__ List at(size_t e) const
+    {
+        return List{half ? (void*)(static_cast<uint16_t*>(p) + e) : (void*)(static_cast<uint32_t*>(p) + e), half};
+    }
+};
+
+// Views of one instance for a step or a pass.  Pointers are generic: in the step kernel the bit
+// planes, the conserved planes and more point into the CTA's shared memory (staged in and out around
+// the steps, see Layout1), elsewhere into the instance's global buffers.
+struct Ctx {
+    const Inst1& I;
+    double *q0, *q1, *q2;   // conserved planes: q0[i + 3]
+    double *qc, *qt, *fl;   // stage-start copy, coarse derivatives, face fluxes: x[p*w + i + 3]
+    uint32_t* pl;           // bit planes
+    uint32_t *m0, *aux;     // planes of mask0 and of the first work plane (they change places)
+    uint8_t* ls;            // the two list regions in shared memory (cap entries each) ...
+    uint8_t* lg;            // ... and in global memory (list_entries1 entries each)
+    unsigned cap;
+    Work1* wk;
+    const Weights& W;
+    int w, nx, N1, maxl, nb, nw;
+
+    __device__ double& Q(int p, int i) const { return (p == 0 ? q0 : p == 1 ? q1 : q2)[i + kGhost]; }
+    __device__ double& QT(int p, int i) const { return qt[p * w + i + kGhost]; }
+    __device__ double& QC(int p, int i) const { return qc[p * w + i + kGhost]; }
+    __device__ uint32_t* plane(int k) const { return pl + (size_t)k * nw; }
+    __device__ uint32_t* mask(int k) const { return k == 0 ? m0 : plane(k); }
+    __device__ uint32_t* fine(int k) const { return plane(kPlFine + k); }
+    __device__ uint32_t* slice(int k, int b) const { return plane(kPlLevel + k * nb + b); }
+    __device__ static bool bit(const uint32_t* P, int i) { return (P[(i >> 5) + 1] >> (i & 31)) & 1u; }
+    __device__ int level(int k, int i) const
+    {
+        int v = 0;
+        for (int b = 0; b < nb; ++b) v |= (int)((slice(k, b)[(i >> 5) + 1] >> (i & 31)) & 1u) << b;
+        return v;
+    }
+    __device__ int no_level() const { return (1 << nb) - 1; }
+    // Bits of word x that are points lo .. N1 + hi_pad of the line.
+    __device__ uint32_t upto(int x, int last) const
+    {
+        const int r = last - 32 * (x - 1);
+        return r < 0 ? 0u : r >= 31 ? ~0u : (2u << r) - 1u;
+    }
+    __device__ uint32_t inside(int x) const { return x < 1 ? 0u : upto(x, N1); }  // points [0, N1]
+    // Word x of a mask, everything off the ghosted line set / masked to the points [0, N1].
+    __device__ uint32_t padded(const uint32_t* P, int x) const { return x < 0 || x >= nw ? ~0u : P[x]; }
+    __device__ uint32_t points(const uint32_t* P, int x) const { return x < 1 || x >= nw ? 0u : P[x] & upto(x, N1); }
+    __device__ int D(int lev) const { return 1 << (maxl - lev); }
+    __device__ double w_(int cnt, int k) const { return W.w[cnt][k + 1]; }
+    // One point into a plane; points off the ghosted line (only reachable from inconsistent user-set
+    // masks/levels, where the reference writes out of bounds) are dropped.
+    __device__ void push(uint32_t* P, int i) const
+    {
+        if (i < -kGhost || i > N1 + kGhost) return;
+        atomicOr(&P[(i >> 5) + 1], 1u << (i & 31));
+    }
+    // The points of word x of a plane, shifted by +s and by -s, into P (all on the line).
+    __device__ void push_shifted(uint32_t* P, int x, uint32_t v, int s) const
+    {
+        const int o = s >> 5, b = s & 31;
+        const uint32_t up = v << b, dn = v >> b;
+        if (up) atomicOr(&P[x + o], up);
+        if (dn) atomicOr(&P[x - o], dn);
+        if (b) {
+            const uint32_t up1 = v >> (32 - b), dn1 = v << (32 - b);
+            if (up1) atomicOr(&P[x + o + 1], up1);
+            if (dn1) atomicOr(&P[x - o - 1], dn1);
+        }
+    }
+    // The region r list of n entries: in shared memory where it fits.
+    __device__ List list(int r, size_t n) const
+    {
+        const size_t eb = entry_bytes(w);
+        return List{n <= cap ? ls + r * eb * cap : lg + r * eb * list_entries1(w), short_lists(w)};
+    }
+};
+
+// Bits of a word whose point index is an odd multiple of 2^t (t < 5).
+__device__ __forceinline__ uint32_t odd_bits(int t)
+{
+    return t == 0 ? 0xAAAAAAAAu : t == 1 ? 0x44444444u : t == 2 ? 0x10101010u : t == 3 ? 0x01000100u : 0x00010000u;
+}
+// (cur << s) with the top of the word below it shifted in, (cur >> s) with the bottom of the word above.
+__device__ __forceinline__ uint32_t shl(uint32_t below, uint32_t cur, int s) { return __funnelshift_l(below, cur, s); }
+__device__ __forceinline__ uint32_t shr(uint32_t cur, uint32_t above, int s) { return __funnelshift_r(cur, above, s); }
+
+// Maximum of non-negative doubles over the warp by their bit patterns (which order like the values).
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v)
+{
+    const unsigned hi = (unsigned)(v >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)v : 0u);
+    return ((unsigned long long)mh << 32) | ml;
+}
+__device__ __forceinline__ void reduce_put(Work1* wk, int slot, int which, double v)
+{
+    const unsigned long long m = warp_max_bits((unsigned long long)__double_as_longlong(v));
+    if ((threadIdx.x & 31) == 0) wk->red[slot][which][threadIdx.x >> 5] = m;
+}
+// After the barrier that follows every warp's reduce_put; all 32 lanes of the warp call it.
+__device__ __forceinline__ double reduce_get(const Work1* wk, int slot, int which)
+{
+    const int lane = threadIdx.x & 31, n = (blockDim.x + 31) >> 5;
+    return __longlong_as_double((long long)warp_max_bits(lane < n ? wk->red[slot][which][lane] : 0ull));
+}
+
+// ------------------------------------------------------------------ masks and levels, bytes <-> planes
+// One warp per word, one point per lane.
+__device__ void load_planes(const Ctx& c, const uint8_t* mb, const int8_t* lb)
+{
+    const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    for (int x = threadIdx.x >> 5; x < c.nw; x += nwarp) {
+        const int i = 32 * (x - 1) + lane;
+        const bool on = i >= -kGhost && i <= c.N1 + kGhost;
+        const unsigned v = on ? mb[i + kGhost] : 0x1fu;
+        for (int k = 0; k < 5; ++k) {
+            const uint32_t b = __ballot_sync(0xffffffffu, (v >> k) & 1u);
+            if (lane == 0) (k == kPlTemp ? c.plane(kPlTemp) : c.mask(k))[x] = b;
+        }
+        for (int k = 0; k < 4; ++k) {
+            const int l = on && i >= 0 && i <= c.N1 ? lb[k * c.w + i + kGhost] : 0;
+            const int s = l < 0 || l > c.maxl ? c.no_level() : l;
+            const uint32_t f = __ballot_sync(0xffffffffu, s == c.maxl);
+            if (lane == 0) c.fine(k)[x] = f;
+            for (int b = 0; b < c.nb; ++b) {
+                const uint32_t y = __ballot_sync(0xffffffffu, (s >> b) & 1);
+                if (lane == 0) c.slice(k, b)[x] = y;
+            }
+        }
+    }
+}
+// A level outside 0..maxl keeps its byte.
+__device__ void store_planes(const Ctx& c, uint8_t* mb, int8_t* lb)
+{
+    const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    for (int x = threadIdx.x >> 5; x < c.nw; x += nwarp) {
+        const int i = 32 * (x - 1) + lane;
+        if (i < -kGhost || i > c.N1 + kGhost) continue;
+        const bool ghost = i < 0 || i > c.N1;
+        unsigned v = ghost ? 0xe0u : 0u;
+        for (int k = 0; k < 4; ++k) v |= ((c.mask(k)[x] >> lane) & 1u) << k;
+        v |= ((c.plane(kPlTemp)[x] >> lane) & 1u) << kBitTemp;
+        mb[i + kGhost] = (uint8_t)v;
+        if (ghost) continue;
+        for (int k = 0; k < 4; ++k) {
+            int l = 0;
+            for (int b = 0; b < c.nb; ++b) l |= (int)((c.slice(k, b)[x] >> lane) & 1u) << b;
+            if (l != c.no_level()) lb[k * c.w + i + kGhost] = (int8_t)l;
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------ lists of points
+// The points of [0, N1] in plane P (and not in `without`), ordered by class: class 0 = the coarsest
+// grid's nodes, class l + 1 = the details of level l (i = odd 2^t is a detail of level
+// maxl-1-t).  wk->off[k] is the start of class k, off[maxl + 1] the length.  Order within a class
+// is free: the points of one class neither read nor write one another.  Three barriers.
+__device__ __forceinline__ int class_of(const Ctx& c, int t) { return t >= c.maxl ? 0 : c.maxl - t; }
+__device__ List order_points(const Ctx& c, int region, const uint32_t* P, const uint32_t* without = nullptr)
+{
+    Work1* wk = c.wk;
+    auto word = [&](int x) { return c.points(P, x) & (without ? ~without[x] : ~0u); };
+    for (int x = 1 + (int)threadIdx.x; x < c.nw; x += blockDim.x) {
+        const uint32_t v = word(x);
+        if (!v) continue;
+#pragma unroll
+        for (int t = 0; t < 5; ++t) {
+            const int n = __popc(v & odd_bits(t));
+            if (n) atomicAdd(&wk->cls[class_of(c, t)], (unsigned)n);
+        }
+        if (v & 1u) atomicAdd(&wk->cls[x == 1 ? 0 : class_of(c, 5 + __ffs(x - 1) - 1)], 1u);
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        const unsigned n = wk->cls[lane];
+        unsigned s = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += y;
+        }
+        wk->cls[lane] = 0;
+        wk->run[lane] = wk->off[lane] = s - n;
+        if (lane == 31) wk->off[32] = s;
+    }
+    __syncthreads();
+    const List L = c.list(region, wk->off[32]);
+    // a warp takes every nwarp-th word, so that neighbouring active words go to different warps,
+    // and expands its non-empty words one by one, a point per lane
+    const int wp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    for (int x0 = 1 + wp; x0 < c.nw; x0 += 32 * nwarp) {
+        const int xl = x0 + nwarp * lane;
+        const uint32_t mine = xl < c.nw ? word(xl) : 0u;
+        unsigned todo = __ballot_sync(0xffffffffu, mine != 0);
+        while (todo) {
+            const int j = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t v = __shfl_sync(0xffffffffu, mine, j);
+            const int x = x0 + nwarp * j;
+            const int t = lane ? __ffs(lane) - 1 : x == 1 ? 31 : 5 + __ffs(x - 1) - 1;
+            const uint32_t grp = v & (lane ? odd_bits(t) : 1u);
+            const bool on = (v >> lane) & 1u;
+            const int lead = grp ? __ffs(grp) - 1 : lane;
+            unsigned base = 0;
+            if (on && lane == lead) base = atomicAdd(&wk->run[class_of(c, t)], (unsigned)__popc(grp));
+            base = __shfl_sync(0xffffffffu, base, lead);
+            if (on) L.put(base + __popc(grp & ((1u << lane) - 1u)), 32 * (x - 1) + lane);
+        }
+    }
+    __syncthreads();
+    return L;
+}
+
+// The lists of one stage over mask k: needed faces f in [-1, N1] (face f+1/2 is needed when a
+// finest-level point of the mask lies on either side), then the finest-level points, then the
+// coarse points.  Their lengths are known from count_masks1.  No barrier: the caller's next one
+// publishes the lists; the positions wk->n_list[k] must be zero before.
+struct StageLists {
+    List faces, fin, crs;
+    int nf, nfin, ncrs;
+};
+__device__ __forceinline__ StageLists stage_lists(const Ctx& c, int k, int region)
+{
+    const Work1* wk = c.wk;
+    const unsigned n = wk->mask_cnt[k], nf = wk->n_face[k], nfin = wk->n_fin[k];
+    const List L = c.list(region, (size_t)nf + n);
+    return StageLists{L, L.at(nf), L.at(nf + nfin), (int)nf, (int)nfin, (int)(n - nfin)};
+}
+// Words x of the finest-level points of mask k and of the faces they need (bit i: face i+1/2).
+__device__ __forceinline__ uint32_t fine_word(const Ctx& c, int k, int x)
+{
+    return x < 1 || x >= c.nw ? 0u : c.points(c.mask(k), x) & c.fine(k)[x];
+}
+__device__ void build_stage_lists(const Ctx& c, int k, int region)
+{
+    const StageLists L = stage_lists(c, k, region);
+    unsigned* pos = c.wk->n_list[k];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    // words to warps as in order_points
+    for (int x0 = wp; x0 < c.nw; x0 += 32 * nwarp) {
+        const int xl = x0 + nwarp * lane;
+        uint32_t m = 0, f = 0, fa = 0;
+        if (xl < c.nw) {
+            m = c.points(c.mask(k), xl);
+            f = fine_word(c, k, xl);
+            fa = f | shr(f, fine_word(c, k, xl + 1), 1);
+        }
+        unsigned todo = __ballot_sync(0xffffffffu, (m | fa) != 0);
+        while (todo) {
+            const int j = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t mj = __shfl_sync(0xffffffffu, m, j), fj = __shfl_sync(0xffffffffu, f, j);
+            const uint32_t faj = __shfl_sync(0xffffffffu, fa, j), cj = mj & ~fj;
+            unsigned base = 0;
+            if (lane < 3) base = atomicAdd(&pos[lane], (unsigned)__popc(lane == 0 ? faj : lane == 1 ? fj : cj));
+            const unsigned bf = __shfl_sync(0xffffffffu, base, 0), bp = __shfl_sync(0xffffffffu, base, 1);
+            const unsigned bc = __shfl_sync(0xffffffffu, base, 2);
+            const int i = 32 * (x0 + nwarp * j - 1) + lane;
+            if ((faj >> lane) & 1u) L.faces.put(bf + __popc(faj & lt), i);
+            if ((fj >> lane) & 1u) L.fin.put(bp + __popc(fj & lt), i);
+            if ((cj >> lane) & 1u) L.crs.put(bc + __popc(cj & lt), i);
+        }
+    }
+}
+
 // ------------------------------------------------------------------ PrepareEuler building blocks
-// ForwardWaveletTransformEuler (Wavelet/WAVELET_1D.h:282-335).
-__device__ void fwt1(const Ctx& c)
+// ForwardWaveletTransformEuler (Wavelet/WAVELET_1D.h:282-335) over the points of mask0, listed by
+// order_points: level by level the details of the level, then the coarser points.
+__device__ void fwt1(const Ctx& c, const List& L)
 {
+    const unsigned* off = c.wk->off;
+    double* q = c.q0;
+    const double tol = c.I.tol;
     for (int lev = c.maxl - 1; lev >= 0; --lev) {
-        const int D = c.D(lev), h = D >> 1, nd = c.N1 / D;
-        for (int a = threadIdx.x; a < nd; a += blockDim.x) {
-            const int i = h + a * D;
-            if (!c.bit(i, 0)) continue;
-            int s, k;
-            predict_stencil(i, D, c.N1, s, k);
-            double v = c.Q(0, i);
-            for (int cnt = 0; cnt < 4; ++cnt) v -= c.w_(cnt, k) * c.Q(0, s + cnt * D);
-            v *= 0.5;
-            c.Q(0, i) = v;
-            if (absd(v) < c.I.tol) c.M(i) &= (uint8_t)~1u;
-        }
-        __syncthreads();
-        for (int a = threadIdx.x; a < nd - 1; a += blockDim.x) {
-            const int i = D + a * D;
-            if (!c.bit(i, 0)) continue;
-            int s, k;
-            update_stencil(i, D, c.N1, s, k);
-            double v = c.Q(0, i);
-            for (int cnt = 0; cnt < 4; ++cnt) v += c.w_(cnt, k) * c.Q(0, s + cnt * D);
-            c.Q(0, i) = v;
-        }
-        __syncthreads();
-    }
-}
-
-// InverseWaveletTransformEuler (Wavelet/WAVELET_1D.h:337-391).
-__device__ void iwt1(const Ctx& c, int b)
-{
-    for (int lev = 0; lev < c.maxl; ++lev) {
-        const int D = c.D(lev), h = D >> 1, nd = c.N1 / D;
-        for (int a = threadIdx.x; a < nd - 1; a += blockDim.x) {
-            const int i = D + a * D;
-            if (!c.bit(i, b)) {
-                c.Q(0, i) = 0;
-                continue;
-            }
-            int s, k;
-            update_stencil(i, D, c.N1, s, k);
-            double v = c.Q(0, i);
-            for (int cnt = 0; cnt < 4; ++cnt) v -= c.w_(cnt, k) * c.Q(0, s + cnt * D);
-            c.Q(0, i) = v;
-        }
-        __syncthreads();
-        for (int a = threadIdx.x; a < nd; a += blockDim.x) {
-            const int i = h + a * D;
-            if (!c.bit(i, b)) {
-                c.Q(0, i) = 0;
-                continue;
-            }
-            int s, k;
-            predict_stencil(i, D, c.N1, s, k);
-            double v = c.Q(0, i);
-            v *= 2;
-            for (int cnt = 0; cnt < 4; ++cnt) v += c.w_(cnt, k) * c.Q(0, s + cnt * D);
-            c.Q(0, i) = v;
-        }
-        __syncthreads();
-    }
-}
-
-// AWCM_MANAGER_1D::CheckReconstruction (Wavelet/AWCM_MANAGER_1D.h:45-71), fine to coarse.
-__device__ void cr1(const Ctx& c, int b)
-{
-    for (int lev = c.maxl - 1; lev >= 0; --lev) {
-        const int D = c.D(lev), h = D >> 1, nd = c.N1 / D;
-        for (int a = threadIdx.x; a < nd; a += blockDim.x) {
-            const int i = h + a * D;
-            if (!c.bit(i, b)) continue;
-            int s, k;
-            predict_stencil(i, D, c.N1, s, k);
-            for (int cnt = 0; cnt < 4; ++cnt) c.set(s + cnt * D, b);
-        }
-        __syncthreads();
-    }
-}
-
-// AWCM_MANAGER_1D::AddAdjacentZone (Wavelet/AWCM_MANAGER_1D.h:14-43): detail points whose `src`
-// bit is set mark their finer neighbours in `b` (and in `b2` too when it is given, in the same
-// atomic).  i = odd * 2^t is a detail of level maxl-1-t.
-__device__ void aaz1(const Ctx& c, int b, int src, int b2 = -1)
-{
-    const unsigned bits = (1u << b) | (b2 >= 0 ? 1u << b2 : 0u);
-    for (int i = 1 + threadIdx.x; i <= c.N1 - 1; i += blockDim.x) {
-        const int t = __ffs(i) - 1;
-        if (t >= c.maxl || !c.bit(i, src)) continue;
-        const int off = t == 0 ? 1 : (1 << (t - 1));
-        c.set_bits(i - off, bits);
-        c.set_bits(i + off, bits);
-    }
-    __syncthreads();
-}
-
-// BadingBoundary (AWCM_1D.h:73-80: mask0 set on the three points at each end, i < 3 and
-// i > N1 - 3), then mask0 copied into the copy bit on the points [0, N1], one word at a time.
-__device__ void band_copy1(const Ctx& c)
-{
-    unsigned* mw = reinterpret_cast<unsigned*>(c.m);
-    for (int wi = (kGhost >> 2) + (int)threadIdx.x; wi <= ((c.N1 + kGhost) >> 2); wi += blockDim.x) {
-        unsigned pts = 0, band = 0;  // bit 0 of the bytes of points [0, N1] / of the banded ones
-#pragma unroll
-        for (int L = 0; L < 4; ++L) {
-            const int i = 4 * wi + L - kGhost;
-            if (i < 0 || i > c.N1) continue;
-            pts |= 1u << (8 * L);
-            if (!(3 <= i && i <= c.N1 - 3)) band |= 1u << (8 * L);
-        }
-        const unsigned v0 = mw[wi], v = v0 | band;
-        const unsigned nv = (v & ~(pts << kBitCopy)) | ((v & pts) << kBitCopy);
-        if (nv != v0) mw[wi] = nv;
-    }
-    __syncthreads();
-}
-
-// AWCM_MANAGER_1D::AddPointForDifferentiation (Wavelet/AWCM_MANAGER_1D.h:73-107), reading the
-// copy bit and level set l.
-__device__ void apd1(const Ctx& c, int b, int l)
-{
-    for (int i = threadIdx.x; i <= c.N1; i += blockDim.x) {
-        if (!c.bit(i, kBitCopy)) continue;
-        const int lev = c.L(l, i);
         const int D = c.D(lev);
-        const int is = i - 2 * D, ie = i + 2 * D;
-        if (lev == c.maxl) {
-            c.set_run(i - 3, 7, b);
-        } else if (is <= 0) {
-            for (int cnt = 0; cnt < 6; ++cnt) c.set(cnt * D, b);
-        } else if (ie >= c.N1) {
-            for (int cnt = 0; cnt < 6; ++cnt) c.set(c.N1 - cnt * D, b);
-        } else {
-            for (int cnt = 0; cnt < 5; ++cnt) c.set(is + cnt * D, b);
-        }
-    }
-    __syncthreads();
-}
-
-__device__ __forceinline__ bool mask_or_ghost1(const Ctx& c, int i, int b)
-{
-    if (i < -kGhost || i >= c.nx + kGhost) return true;
-    return c.bit(i, b);
-}
-
-// AWCM_MANAGER_1D::ComputeLevel (Wavelet/AWCM_MANAGER_1D.h:109-133), with the optional copy
-// mask_{k+1} = mask_k of the own point.  One 32-bit mask word (four points) per iteration: the copy
-// is one word operation and the level search runs for the mask's points only.  The search reads
-// bit b of other bytes, which no thread changes here (the copy writes bit copy_to, and bit
-// copy_to2 too when it is given).
-__device__ void cl1(const Ctx& c, int l, int b, int copy_to, int copy_to2 = -1)
-{
-    unsigned* mw = reinterpret_cast<unsigned*>(c.m);
-    const int nw = (c.w + 3) >> 2;
-    for (int wi = threadIdx.x; wi < nw; wi += blockDim.x) {
-        const unsigned v = mw[wi];
-        unsigned lanes = 0;  // the bytes of the word that are points of the line (ghosts included)
+        for (unsigned e = off[lev + 1] + threadIdx.x; e < off[lev + 2]; e += blockDim.x) {
+            const int i = L.get(e);
+            int s, k;
+            predict_stencil(i, D, c.N1, s, k);
+            double v = q[i + kGhost];
 #pragma unroll
-        for (int L = 0; L < 4; ++L) {
-            const int i = 4 * wi + L - kGhost;
-            if (i > c.N1 + kGhost) continue;
-            lanes |= 1u << (8 * L);
-            if (i < 0 || i > c.N1) continue;  // ghost byte: only the copy (the reference copies whole fields)
-            if (i == 0 || i == c.N1) {
-                c.L(l, i) = (int8_t)c.maxl;
-            } else if (!((v >> (8 * L + b)) & 1u)) {
-                c.L(l, i) = 0;
-            } else {
-                int dx = 1;
-                for (int lev = c.maxl; lev >= 0; --lev) {
-                    if (mask_or_ghost1(c, i - dx, b) || mask_or_ghost1(c, i + dx, b)) {
-                        c.L(l, i) = (int8_t)lev;
-                        break;
-                    }
-                    dx *= 2;
+            for (int cnt = 0; cnt < 4; ++cnt) v -= c.w_(cnt, k) * q[s + cnt * D + kGhost];
+            v *= 0.5;
+            q[i + kGhost] = v;
+            if (absd(v) < tol) atomicAnd(&c.m0[(i >> 5) + 1], ~(1u << (i & 31)));
+        }
+        __syncthreads();
+        for (unsigned e = threadIdx.x; e < off[lev + 1]; e += blockDim.x) {
+            const int i = L.get(e);
+            if (i == 0 || i == c.N1) continue;
+            int s, k;
+            update_stencil(i, D, c.N1, s, k);
+            double v = q[i + kGhost];
+#pragma unroll
+            for (int cnt = 0; cnt < 4; ++cnt) v += c.w_(cnt, k) * q[s + cnt * D + kGhost];
+            q[i + kGhost] = v;
+        }
+        __syncthreads();
+    }
+}
+
+// InverseWaveletTransformEuler(q, mask3) and InterpolateEuler(q, mask_temp, mask3)
+// (Wavelet/WAVELET_1D.h:337-391, 393-431) over the points of mask3, listed by order_points.
+// The interpolation of level l's new points (mask3 without mask_temp) reads the momentum and
+// energy of coarser points, the transform the density: one phase does both.  The work mask that the
+// reference closes first adds nothing here, because mask3 is closed under CheckReconstruction: the
+// closure of a part of it lies inside it.
+// The reference also sets the density to 0 at the points outside mask3, each in its level's phase.
+// A level's update reads those points before that phase, and nothing reads them after it (the
+// stencils of mask3's points lie in mask3), so the caller zeroes them at the end, or not at all
+// where the residue removal does.
+__device__ void iwt_interp1(const Ctx& c, const List& L, bool interp)
+{
+    const unsigned* off = c.wk->off;
+    const uint32_t* temp = c.plane(kPlTemp);
+    double* q = c.q0;
+    for (int lev = 0; lev < c.maxl; ++lev) {
+        const int D = c.D(lev);
+        for (unsigned e = threadIdx.x; e < off[lev + 1]; e += blockDim.x) {
+            const int i = L.get(e);
+            if (i == 0 || i == c.N1) continue;
+            int s, k;
+            update_stencil(i, D, c.N1, s, k);
+            double v = q[i + kGhost];
+#pragma unroll
+            for (int cnt = 0; cnt < 4; ++cnt) v -= c.w_(cnt, k) * q[s + cnt * D + kGhost];
+            q[i + kGhost] = v;
+        }
+        __syncthreads();
+        for (unsigned e = off[lev + 1] + threadIdx.x; e < off[lev + 2]; e += blockDim.x) {
+            const int i = L.get(e);
+            int s, k;
+            predict_stencil(i, D, c.N1, s, k);
+            double v = q[i + kGhost];
+            v *= 2;
+#pragma unroll
+            for (int cnt = 0; cnt < 4; ++cnt) v += c.w_(cnt, k) * q[s + cnt * D + kGhost];
+            q[i + kGhost] = v;
+            if (interp && !Ctx::bit(temp, i)) {
+                double a = 0, b = 0;
+#pragma unroll
+                for (int cnt = 0; cnt < 4; ++cnt) {
+                    a += c.w_(cnt, k) * c.Q(1, s + cnt * D);
+                    b += c.w_(cnt, k) * c.Q(2, s + cnt * D);
+                }
+                c.Q(1, i) = a;
+                c.Q(2, i) = b;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// CheckReconstruction (Wavelet/AWCM_MANAGER_1D.h:45-71), the levels of spacing h = 1..16: every
+// detail of the mask marks its four coarse neighbours i -+ h, i -+ 3h (shifted one-sided at the
+// ends), fine to coarse.  A word's outcome depends on at most 93 points around it, so each thread
+// closes a window of six words in registers and keeps its own one: no barrier between the levels.
+// Words are closed in place: a neighbour read after its own closure only holds points that belong
+// to the closure anyway.
+__device__ void close_words(const Ctx& c, uint32_t* P)
+{
+    const int top = min(c.maxl, 5), xr = (c.N1 >> 5) + 1;
+    for (int x = 1 + (int)threadIdx.x; x < c.nw; x += blockDim.x) {
+        uint32_t W[6];
+        uint32_t any = 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) any |= W[k] = c.points(P, x - 3 + k);
+        if (!any) continue;
+        const bool edge = x <= 4 || x >= xr - 4;  // the window may hold an end's one-sided stencils
+#pragma unroll
+        for (int t = 0; t < 5; ++t) {
+            if (t >= top) break;
+            const int h = 1 << t;
+            uint32_t d[8];
+            d[0] = d[7] = 0;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) d[k + 1] = W[k] & odd_bits(t);
+            if (edge) {
+                // the first detail h marks 0, 2h, 4h and 6h, the last one N1-6h .. N1 likewise: the
+                // point beyond the ordinary stencil (which stays clear of the line's other side)
+                uint32_t lo = 0, hi = 0;
+                const int sl = 1 + (h >> 5), tl = 1 + ((6 * h) >> 5);
+                const int sr = ((c.N1 - h) >> 5) + 1, tr = ((c.N1 - 6 * h) >> 5) + 1;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    if (x - 3 + k == sl) lo |= (W[k] >> (h & 31)) & 1u;
+                    if (x - 3 + k == sr) hi |= (W[k] >> ((c.N1 - h) & 31)) & 1u;
+                }
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    if (x - 3 + k == tl) W[k] |= lo << ((6 * h) & 31);
+                    if (x - 3 + k == tr) W[k] |= hi << ((c.N1 - 6 * h) & 31);
                 }
             }
-        }
-        if (copy_to >= 0) {
-            unsigned nv = (v & ~(lanes << copy_to)) | (((v >> b) & lanes) << copy_to);
-            if (copy_to2 >= 0) nv = (nv & ~(lanes << copy_to2)) | (((v >> b) & lanes) << copy_to2);
-            if (nv != v) mw[wi] = nv;
-        }
-    }
-    __syncthreads();
-}
-
-// Copies bit `from` into bit `to` on the points [0, N1] (ghosts: [-3, N1+3]), a word at a time.
-__device__ void copy_bit1(const Ctx& c, int from, int to, bool ghosts)
-{
-    const int x0 = ghosts ? 0 : kGhost, x1 = ghosts ? c.N1 + 2 * kGhost : c.N1 + kGhost;  // byte range
-    unsigned* mw = reinterpret_cast<unsigned*>(c.m);
-    for (int wi = (x0 >> 2) + (int)threadIdx.x; wi <= (x1 >> 2); wi += blockDim.x) {
-        unsigned lanes = 0;
 #pragma unroll
-        for (int L = 0; L < 4; ++L) {
-            const int x = 4 * wi + L;
-            if (x >= x0 && x <= x1) lanes |= 1u << (8 * L);
-        }
-        const unsigned v = mw[wi];
-        const unsigned nv = (v & ~(lanes << to)) | (((v >> from) & lanes) << to);
-        if (nv != v) mw[wi] = nv;
-    }
-    __syncthreads();
-}
-
-// WAVELET_1D::InterpolateEuler(q, mra, from, to) (Wavelet/WAVELET_1D.h:393-431).
-__device__ void interp1(const Ctx& c, int from, int to)
-{
-    // work bit = to and not from, on the points [0, N1], a word at a time
-    unsigned* mw = reinterpret_cast<unsigned*>(c.m);
-    for (int wi = (kGhost >> 2) + (int)threadIdx.x; wi <= ((c.N1 + kGhost) >> 2); wi += blockDim.x) {
-        unsigned lanes = 0;
-#pragma unroll
-        for (int L = 0; L < 4; ++L) {
-            const int x = 4 * wi + L;
-            if (x >= kGhost && x <= c.N1 + kGhost) lanes |= 1u << (8 * L);
-        }
-        const unsigned v = mw[wi];
-        const unsigned on = (v >> to) & ~(v >> from) & lanes;
-        const unsigned nv = (v & ~(lanes << kBitInterp)) | (on << kBitInterp);
-        if (nv != v) mw[wi] = nv;
-    }
-    __syncthreads();
-    cr1(c, kBitInterp);
-    for (int lev = 0; lev < c.maxl; ++lev) {
-        const int D = c.D(lev), h = D >> 1, nd = c.N1 / D;
-        for (int a = threadIdx.x; a < nd; a += blockDim.x) {
-            const int i = h + a * D;
-            if (!c.bit(i, kBitInterp) || c.bit(i, from)) continue;
-            int s, k;
-            predict_stencil(i, D, c.N1, s, k);
-            for (int p = 1; p < 3; ++p) {
-                double v = 0;
-                for (int cnt = 0; cnt < 4; ++cnt) v += c.w_(cnt, k) * c.Q(p, s + cnt * D);
-                c.Q(p, i) = v;
+            for (int k = 0; k < 6; ++k) {
+                uint32_t o;
+                if (t < 4) {
+                    o = shl(d[k], d[k + 1], h) | shr(d[k + 1], d[k + 2], h) | shl(d[k], d[k + 1], 3 * h) |
+                        shr(d[k + 1], d[k + 2], 3 * h);
+                } else {
+                    // bit 16 of a word marks bit 0 of the words at 0, +1, +2 and -1
+                    o = (d[k + 1] | d[k] | (k > 0 ? d[k - 1] : 0u) | d[k + 2]) >> 16;
+                }
+                W[k] |= edge ? o & c.inside(x - 3 + k) : o;
             }
         }
+        const uint32_t own = W[3];
+        if (own & ~P[x]) P[x] |= own;
+    }
+}
+// The levels of spacing h >= 32, whose points are bit 0 of their words.  Levels of up to 128
+// details on one warp, with warp barriers between them; larger ones on the whole block.
+__device__ void close_coarse_level(const Ctx& c, uint32_t* P, int t, int first, int stride)
+{
+    const int h = 1 << t, D = 2 * h, nd = c.N1 / D;
+    for (int a = first; a < nd; a += stride) {
+        const int i = h + a * D;
+        if (!(P[(i >> 5) + 1] & 1u)) continue;
+        int s, k;
+        predict_stencil(i, D, c.N1, s, k);
+#pragma unroll
+        for (int cnt = 0; cnt < 4; ++cnt) {
+            uint32_t* y = &P[((s + cnt * D) >> 5) + 1];
+            if (!(*y & 1u)) atomicOr(y, 1u);
+        }
+    }
+}
+__device__ void close1(const Ctx& c, uint32_t* P)
+{
+    close_words(c, P);
+    __syncthreads();
+    int t = 5;
+    for (; t < c.maxl && (c.N1 >> (t + 1)) > 128; ++t) {
+        close_coarse_level(c, P, t, threadIdx.x, blockDim.x);
+        __syncthreads();
+    }
+    if (t < c.maxl) {
+        if (threadIdx.x < 32)
+            for (; t < c.maxl; ++t) {
+                close_coarse_level(c, P, t, threadIdx.x, 32);
+                __syncwarp();
+            }
         __syncthreads();
     }
 }
 
-// AWCM_1D::PrepareEuler (Wavelet/AWCM_1D.h:86-120).
-__device__ void prepare1(const Ctx& c)
+// AddAdjacentZone (Wavelet/AWCM_MANAGER_1D.h:14-43) of word x of the mask whose words word(y) gives
+// (points [0, N1] only): the points that the word's own and the neighbouring details mark.  A detail
+// i = odd 2^t marks i -+ max(1, 2^(t-1)).
+template <class Word>
+__device__ __forceinline__ uint32_t zone_word(const Ctx& c, int x, Word word)
 {
-    copy_bit1(c, 0, kBitTemp, true);
-    fwt1(c);
-    band_copy1(c);
-    aaz1(c, 0, kBitCopy);
-    cr1(c, 0);
-    for (int k = 1; k <= 3; ++k) {
-        // level_{k-1} of mask_{k-1}; mask_k = mask_{k-1}, and the copy bit too
-        cl1(c, k - 1, k - 1, k, kBitCopy);
-        // AddAdjacentZone(mask_k) reads bit k-1 (== mask_k before it) and marks bit k and the copy
-        // bit, so the copy bit is mask_k after it: the input of AddPointForDifferentiation
-        aaz1(c, k, k - 1, kBitCopy);
-        apd1(c, k, k - 1);            // AddPointForDifferentiation(mask_k, level_{k-1})
-        cr1(c, k);
+    uint32_t s = 0;
+    if (x >= 1) {
+        const uint32_t l = word(x - 1), v = word(x), r = word(x + 1);
+        if (l | v | r) {
+            const uint32_t p01 = odd_bits(0) | (c.maxl > 1 ? odd_bits(1) : 0u);
+            s |= shl(l & p01, v & p01, 1) | shr(v & p01, r & p01, 1);
+#pragma unroll
+            for (int t = 2; t < 5; ++t) {
+                if (t >= c.maxl) break;
+                const uint32_t p = odd_bits(t);
+                s |= shl(l & p, v & p, 1 << (t - 1)) | shr(v & p, r & p, 1 << (t - 1));
+            }
+            if (c.maxl > 5) s |= ((x & 1) ? r & 1u : v & 1u) << 16;  // i = odd 32: bit 0 of an even word
+        }
+        // t >= 6: point 32 m' is marked by 32 (m' -+ 2^z), z = ctz(m'), if that is an odd multiple of 2^(z+1)
+        const int m = x - 1;
+        if (m > 0) {
+            const int z = __ffs(m) - 1;
+            if (z + 6 < c.maxl) {
+                const int lo = m - (1 << z), hi = m + (1 << z);
+                if (((lo >> (z + 1)) & 1) && (word(lo + 1) & 1u)) s |= 1u;
+                if (((hi >> (z + 1)) & 1) && (word(hi + 1) & 1u)) s |= 1u;
+            }
+        }
     }
-    cl1(c, 3, 3, -1);
-    iwt1(c, 3);
-    interp1(c, kBitTemp, 3);
+    return s;
+}
+
+// BadingBoundary (AWCM_1D.h:73-80: mask0 set on the three points at each end, i < 3 and i > N1 - 3).
+__device__ __forceinline__ uint32_t band_word(const Ctx& c, int x)
+{
+    uint32_t b = x == 1 ? 7u : 0u;
+    for (int i = c.N1 - 2; i <= c.N1; ++i)
+        if ((i >> 5) + 1 == x) b |= 1u << (i & 31);
+    return b;
+}
+
+// ComputeLevel (Wavelet/AWCM_MANAGER_1D.h:109-133) of word x of mask M into level set k: the points
+// whose nearest neighbour in the mask is 2^j away get level maxl - j (the reference searches the
+// distances one by one; here each distance is one shift of the whole word).  Off the ghosted line
+// the mask reads as set.  A point without any such neighbour keeps its level.
+// f(j, set): the word's points of level maxl - j, for each level that has any.
+template <class F>
+__device__ __forceinline__ void level_word(const Ctx& c, int k, const uint32_t* M, int x, F&& f)
+{
+    const uint32_t in = c.inside(x);
+    uint32_t ends = x == 1 ? 1u : 0u;  // the two end points: the finest level, in the mask or not
+    if ((c.N1 >> 5) + 1 == x) ends |= 1u << (c.N1 & 31);
+    const uint32_t on = in ? M[x] & in : 0u;
+    uint32_t todo = on & ~ends, fine = ends & in;
+    uint32_t S[5];
+#pragma unroll
+    for (int b = 0; b < 5; ++b) S[b] = ((c.maxl >> b) & 1) ? fine : 0u;
+    if (todo) {
+        const uint32_t l = c.padded(M, x - 1), v = M[x], r = c.padded(M, x + 1);
+        for (int j = 0; j <= c.maxl && todo; ++j) {
+            uint32_t near;
+            if (j < 5) near = shl(l, v, 1 << j) | shr(v, r, 1 << j);
+            else near = c.padded(M, x - (1 << (j - 5))) | c.padded(M, x + (1 << (j - 5)));
+            const uint32_t got = todo & near;
+            if (!got) continue;
+            todo &= ~near;
+            const int lev = c.maxl - j;
+            if (j == 0) fine |= got;
+            else f(j, got);
+#pragma unroll
+            for (int b = 0; b < 5; ++b)
+                if ((lev >> b) & 1) S[b] |= got;
+        }
+        if (todo) {  // no neighbour found: the level stays as it was
+            uint32_t was[5];
+#pragma unroll
+            for (int b = 0; b < 5; ++b) was[b] = b < c.nb ? c.slice(k, b)[x] & todo : 0u;
+            fine |= c.fine(k)[x] & todo;
+            for (uint32_t u = todo & ~c.fine(k)[x]; u; u &= u - 1) {
+                const uint32_t one = u & (0u - u);
+                int lev = 0;
+#pragma unroll
+                for (int b = 0; b < 5; ++b) lev |= (was[b] & one) ? 1 << b : 0;
+                if (lev != c.no_level()) f(c.maxl - lev, one);
+            }
+#pragma unroll
+            for (int b = 0; b < 5; ++b) S[b] |= was[b];
+        }
+    }
+    if (fine & on) f(0, fine & on);
+    c.fine(k)[x] = fine;
+#pragma unroll
+    for (int b = 0; b < 5; ++b)
+        if (b < c.nb) c.slice(k, b)[x] = S[b];
+}
+
+// AddPointForDifferentiation (Wavelet/AWCM_MANAGER_1D.h:73-107) of the points `set` (points [0, N1])
+// of word x, all of level maxl - j, into P: the finest level marks i-3 .. i+3, a coarser one
+// the 5 points i-2D .. i+2D, or 6 points from the end it is near to.  own: the part that falls in
+// the word itself.
+__device__ __forceinline__ void stencil_push(const Ctx& c, uint32_t* P, int x, int j, uint32_t set, uint32_t& own)
+{
+    if (j == 0) {
+        const uint32_t up = (set >> 31) | (set >> 30) | (set >> 29), dn = (set << 31) | (set << 30) | (set << 29);
+        own |= set | (set << 1) | (set << 2) | (set << 3) | (set >> 1) | (set >> 2) | (set >> 3);
+        if (up) atomicOr(&P[x + 1], up);
+        if (dn) atomicOr(&P[x - 1], dn);
+        return;
+    }
+    const int D = 1 << j;
+    const uint32_t left = set & c.upto(x, 2 * D), right = set & ~left & ~c.upto(x, c.N1 - 2 * D - 1);
+    const uint32_t mid = set & ~left & ~right;
+    if (left)
+        for (int n = 0; n < 6; ++n) c.push(P, n * D);
+    if (right)
+        for (int n = 0; n < 6; ++n) c.push(P, c.N1 - n * D);
+    if (mid) {
+        own |= mid;
+        c.push_shifted(P, x, mid, D);
+        c.push_shifted(P, x, mid, 2 * D);
+    }
+}
+
+// ComputeLevel(level_{k-1}, mask_{k-1}), mask_k = mask_{k-1}, AddAdjacentZone(mask_k) (zone) and
+// AddPointForDifferentiation(mask_k, level_{k-1}) in one phase.  All of them read mask_{k-1} only
+// (the zone's points are not in it, so their level is 0), and mask_k (clear before) takes ORs.
+__device__ void next_mask1(const Ctx& c, int k, bool zone)
+{
+    const uint32_t* A = c.mask(k - 1);
+    uint32_t* B = c.plane(k);
+    auto pts = [&](int y) { return c.points(A, y); };
+    for (int x = threadIdx.x; x < c.nw; x += blockDim.x) {
+        const uint32_t a = A[x];  // ghosts and the bits off the line included
+        uint32_t own = a;
+        const uint32_t fresh = zone ? zone_word(c, x, pts) & ~a : 0u;
+        own |= fresh;
+        level_word(c, k - 1, A, x, [&](int j, uint32_t set) { stencil_push(c, B, x, j, set, own); });
+        if (fresh) stencil_push(c, B, x, c.maxl, fresh, own);
+        if (own) atomicOr(&B[x], own);
+    }
+    __syncthreads();
+}
+
+// ComputeLevel alone.
+__device__ void levels1(const Ctx& c, int k, const uint32_t* M)
+{
+    for (int x = threadIdx.x; x < c.nw; x += blockDim.x) level_word(c, k, M, x, [](int, uint32_t) {});
+}
+
+// Numbers of points of mask0..mask3 in [0, N1], and of the finest-level points and needed faces of
+// mask0..mask2, into the workspace (zero before); no barrier.
+__device__ void count_masks1(const Ctx& c)
+{
+    for (int x0 = 0; x0 < c.nw; x0 += blockDim.x) {
+        const int x = x0 + (int)threadIdx.x;
+        const bool head = (threadIdx.x & 31) == 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned n = __reduce_add_sync(0xffffffffu, x < c.nw ? __popc(c.points(c.mask(k), x)) : 0);
+            if (n && head) atomicAdd(&c.wk->mask_cnt[k], n);
+            if (k == 3) continue;
+            const uint32_t f = fine_word(c, k, x);
+            const uint32_t fa = x < c.nw ? f | shr(f, fine_word(c, k, x + 1), 1) : 0u;
+            const unsigned nn = __reduce_add_sync(0xffffffffu, __popc(f) | (__popc(fa) << 16));
+            if (nn && head) {
+                atomicAdd(&c.wk->n_fin[k], nn & 0xffffu);
+                atomicAdd(&c.wk->n_face[k], nn >> 16);
+            }
+        }
+    }
+}
+
+// The mask and level chain and the transforms of AWCM_1D::PrepareEuler (Wavelet/AWCM_1D.h:86-120),
+// or with euler false of AWCM_1D::Prepare (Wavelet/AWCM_1D.h:45-72: no mask_temp, no adjacent zones
+// on mask1..mask3, no interpolation).  Leaves the ordered list of mask3 in region 0 and the counts
+// of the masks, and does not zero the density outside mask3 (see iwt_interp1).  The start's mask0
+// is in kPlTemp (euler) or kPlStart.
+__device__ List prepare1(Ctx& c, bool euler)
+{
+    Work1* wk = c.wk;
+    uint32_t* start = c.plane(euler ? kPlTemp : kPlStart);
+    for (int x = threadIdx.x; x < c.nw; x += blockDim.x) {
+        start[x] = c.m0[x];
+        c.plane(1)[x] = c.plane(2)[x] = c.plane(3)[x] = 0;
+    }
+    if (threadIdx.x < 16) wk->n_list[threadIdx.x >> 2][threadIdx.x & 3] = 0;
+    if (threadIdx.x < 4) wk->mask_cnt[threadIdx.x] = wk->n_face[threadIdx.x] = wk->n_fin[threadIdx.x] = 0;
+    fwt1(c, order_points(c, 0, c.m0));
+    for (int k = 0; k <= 3; ++k) {
+        if (k == 0) {
+            // banding and AddAdjacentZone of mask0, into the other plane
+            const uint32_t* m = c.m0;
+            auto band = [&](int y) { return y < 1 || y >= c.nw ? 0u : (m[y] | band_word(c, y)) & c.inside(y); };
+            for (int x = threadIdx.x; x < c.nw; x += blockDim.x)
+                c.aux[x] = m[x] | band_word(c, x) | zone_word(c, x, band);
+            __syncthreads();
+            uint32_t* t = c.m0;
+            c.m0 = c.aux;
+            c.aux = t;
+        } else {
+            next_mask1(c, k, euler);
+        }
+        close1(c, c.mask(k));
+    }
+    levels1(c, 3, c.plane(3));
+    count_masks1(c);
+    const List L3 = order_points(c, 0, c.plane(3));
+    iwt_interp1(c, L3, euler);
+    return L3;
 }
 
 // --------------------------------------------------------------------------------- RK3 stages
-__device__ void bc1(const Ctx& c)
+// The ghost cell fill of one component p and distance g (1..3) at both ends.
+__device__ __forceinline__ void bc_cell1(const Ctx& c, int p, int g)
 {
-    if (threadIdx.x < 3 * kGhost) {
-        const int p = threadIdx.x / kGhost, g = threadIdx.x % kGhost + 1;
-        if (!c.I.bc_generic) {
-            // BOUNDARY_MANAGER::SetBoundaryCondition (Problems/1D/PROBLEM_SHOCKTUBE.h:86-107).
-            c.Q(p, -g) = c.Q(p, 0);
-            c.Q(p, c.N1 + g) = c.Q(p, c.N1);
-        } else {
-            // BOUNDARY_MANAGER_1D<T>::SetBoundaryCondition (BOUNDARY_MANAGER_1D.h:47-75): zero-order
-            // extrapolation or the periodic image (ghost -g <- N1-(g-1), N1+g <- g-1) by the
-            // condition of each ghost cell; other conditions leave it.
-            const int kl = c.I.bcg[g - 1], kr = c.I.bcg[kGhost + g - 1];
-            if (kl == kBcExtrapolation1) c.Q(p, -g) = c.Q(p, 0);
-            else if (kl == kBcPeriodic1) c.Q(p, -g) = c.Q(p, c.N1 - (g - 1));
-            if (kr == kBcExtrapolation1) c.Q(p, c.N1 + g) = c.Q(p, c.N1);
-            else if (kr == kBcPeriodic1) c.Q(p, c.N1 + g) = c.Q(p, g - 1);
-        }
+    if (!c.I.bc_generic) {
+        // BOUNDARY_MANAGER::SetBoundaryCondition (Problems/1D/PROBLEM_SHOCKTUBE.h:86-107).
+        c.Q(p, -g) = c.Q(p, 0);
+        c.Q(p, c.N1 + g) = c.Q(p, c.N1);
+    } else {
+        // BOUNDARY_MANAGER_1D<T>::SetBoundaryCondition (BOUNDARY_MANAGER_1D.h:47-75): zero-order
+        // extrapolation or the periodic image (ghost -g <- N1-(g-1), N1+g <- g-1) by the
+        // condition of each ghost cell; other conditions leave it.
+        const int kl = c.I.bcg[g - 1], kr = c.I.bcg[kGhost + g - 1];
+        if (kl == kBcExtrapolation1) c.Q(p, -g) = c.Q(p, 0);
+        else if (kl == kBcPeriodic1) c.Q(p, -g) = c.Q(p, c.N1 - (g - 1));
+        if (kr == kBcExtrapolation1) c.Q(p, c.N1 + g) = c.Q(p, c.N1);
+        else if (kr == kBcPeriodic1) c.Q(p, c.N1 + g) = c.Q(p, g - 1);
     }
-    __syncthreads();
+}
+__device__ __forceinline__ void bc1(const Ctx& c)
+{
+    if (threadIdx.x < 3 * kGhost) bc_cell1(c, threadIdx.x / kGhost, threadIdx.x % kGhost + 1);
 }
 
-// nf: set when a speed is NaN or infinite (NaN/Inf state, negative pressure or density).
-__device__ double lf_speed1(const Ctx& c, int b, int l, double* red, bool& nf)
+// |u| + c (main_1d_euler.cpp:67-95); nf: set when it is NaN or infinite (NaN/Inf state, negative
+// pressure or density).
+__device__ __forceinline__ double speed1(double q0, double q1, double q2, double gamma, bool& nf)
 {
-    // main_1d_euler.cpp:86-95: max |u|+c over the finest-level points of mask b.
-    double a = 0;
-    for (int i = threadIdx.x; i <= c.N1; i += blockDim.x) {
-        if (!c.bit(i, b) || c.L(l, i) != c.maxl) continue;
-        const double q0 = c.Q(0, i), q1 = c.Q(1, i), q2 = c.Q(2, i);
-        const double u = q1 / q0;
-        const double s = sound1(q0, q1, q2, c.I.gamma);
-        nf |= !isfinite(absd(u) + s);
-        a = maxd(a, absd(u) + s);
-    }
-    return block_max(a, red);
+    const double s = absd(q1 / q0) + sound1(q0, q1, q2, gamma);
+    nf |= !isfinite(s);
+    return s;
 }
 
 // Coarse-level flux derivative (AWCM_1D::DifferentiateEuler*, Wavelet/AWCM_1D.h:142-189) with the
@@ -548,229 +841,150 @@ __device__ void coarse_dF1(const Ctx& c, int i, int d, double* dF)
     }
 }
 
-// Lists of one stage, from one pass over the points: faces f in [-1, N1] (face f+1/2 is needed when a
-// finest-level point of the stage's mask lies on either side) into fl_list[0, nf), finest-level
-// points into pl[0, nfin), coarse points (valid level, derivative stencil inside the ghosted line)
-// into pl[cap - ncrs, cap).  copy_qc: also the stage-start copy QC of every mask1 point (the only
-// points whose QC stages 2 and 3 read; mask0 is inside mask1).  Each thread owns a contiguous
-// chunk of positions and keeps its hits as bit sets (chunks of up to 64 positions; longer chunks
-// evaluate again), one block scan of the three packed counts places them; order is preserved.
-struct StageLists {
-    int nf, nfin, ncrs;
-};
-// Stage class of a point whose mask bit is set: 1 finest level, 2 coarse point with its derivative
-// stencil inside the ghosted line, 0 neither (main_1d_euler.cpp:111-133).
-__device__ __forceinline__ int stage_class(const Ctx& c, int l, int i)
+// Spacing of the coarse point i in level set k, or 0: a level outside 0..maxl or a derivative
+// stencil that leaves the ghosted line (the point then keeps its value).
+__device__ __forceinline__ int coarse_spacing(const Ctx& c, int k, int i)
 {
-    const int lev = c.L(l, i);
-    if (lev == c.maxl) return 1;
-    if (lev < 0 || lev > c.maxl) return 0;
+    const int lev = c.level(k, i);
+    if (lev > c.maxl) return 0;
     const int d = c.D(lev);
-    return (i - 2 * d < -kGhost || i + 2 * d > c.N1 + kGhost) ? 0 : 2;
-}
-__device__ __forceinline__ bool fin_byte(const Ctx& c, int b, int l, int x)
-{
-    return x >= kGhost && x <= c.N1 + kGhost && ((c.m[x] >> b) & 1u) && c.L(l, x - kGhost) == c.maxl;
+    return (i - 2 * d < -kGhost || i + 2 * d > c.N1 + kGhost) ? 0 : d;
 }
 
-// Word-level form of stage_lists for instances whose per-thread share is at most 16 mask words:
-// each thread reads its run of 32-bit mask words (four points each), looks up levels for the
-// stage's points only, and keeps its hits as bit sets over the run.
-__device__ StageLists stage_lists_words(const Ctx& c, int b, int l, bool copy_qc, uint32_t* fl_list, uint32_t* pl,
-                                        int cap, unsigned long long* red, int w0, int w1)
+// One stage over mask k / level set k (main_1d_euler.cpp:97-245): kind 1..3 with k = 2, 1, 0.  Faces
+// are computed once (face i+1/2 is shared by points i and i+1; the reference evaluates it for
+// both, identically).  The faces and the coarse derivatives read the stage input Q and run in one
+// phase (the coarse derivatives are parked in qt); the point updates follow in a second phase, so Q
+// is never read after a point of this stage has been written and no copy of the stage input is
+// needed.  Beside the faces the next stage's lists are built.  The update of a finest-level point
+// of stages 1 and 2 also gives its speed: these points are exactly those of the next stage's
+// Lax-Friedrichs scan (main_1d_euler.cpp:86-95), whose maximum over the block comes from slot
+// `kind` of the reductions after the barrier that ends the stage.
+__device__ __forceinline__ void stage1(const Ctx& c, int scheme, int kind, double alpha, double dt, bool& nf)
 {
-    const int xlo = kGhost - 1, xhi = c.N1 + kGhost;  // faces x in [xlo, xhi], points x in [kGhost, xhi]
-    const unsigned* mw = reinterpret_cast<const unsigned*>(c.m);
-    const int base = 4 * w0;
-    unsigned long long mf = 0, mp = 0, mc = 0;
-    bool fprev = w0 < w1 && fin_byte(c, b, l, base - 1);
-    for (int wi = w0; wi < w1; ++wi) {
-        const unsigned v = mw[wi];
-#pragma unroll
-        for (int L = 0; L < 4; ++L) {
-            const int x = 4 * wi + L;
-            int k = 0;
-            if (x >= kGhost && x <= xhi) {
-                if ((v >> (8 * L + b)) & 1u) k = stage_class(c, l, x - kGhost);
-                if (copy_qc && ((v >> (8 * L + 1)) & 1u))
-                    for (int q = 0; q < 3; ++q) c.QC(q, x - kGhost) = c.Q(q, x - kGhost);
-            }
-            const unsigned long long bit = 1ull << (x - base);
-            if (k == 1) mp |= bit;
-            else if (k == 2) mc |= bit;
-            // face x - 1 needs a finest-level point at x - 1 or x
-            if (x - 1 >= base && x - 1 >= xlo && (fprev || k == 1)) mf |= bit >> 1;
-            fprev = k == 1;
-        }
-    }
-    if (w0 < w1) {
-        const int xl = 4 * w1 - 1;
-        if (xl >= xlo && xl <= xhi && (fprev || fin_byte(c, b, l, xl + 1))) mf |= 1ull << (xl - base);
-    }
-    constexpr unsigned long long M21 = (1ull << 21) - 1;
-    unsigned long long tot;
-    const unsigned long long off = block_exclusive_scan64(
-        (unsigned long long)__popcll(mf) | ((unsigned long long)__popcll(mp) << 21) | ((unsigned long long)__popcll(mc) << 42),
-        red, &tot);
-    StageLists o{(int)(tot & M21), (int)((tot >> 21) & M21), (int)((tot >> 42) & M21)};
-    unsigned of = (unsigned)(off & M21), op = (unsigned)((off >> 21) & M21), oc = (unsigned)((off >> 42) & M21);
-    uint32_t* crs = pl + cap - o.ncrs;
-    for (; mf; mf &= mf - 1) fl_list[of++] = (uint32_t)(base + __ffsll(mf) - 1 - kGhost);
-    for (; mp; mp &= mp - 1) pl[op++] = (uint32_t)(base + __ffsll(mp) - 1 - kGhost);
-    for (; mc; mc &= mc - 1) crs[oc++] = (uint32_t)(base + __ffsll(mc) - 1 - kGhost);
-    __syncthreads();
-    return o;
-}
-
-__device__ StageLists stage_lists(const Ctx& c, int b, int l, bool copy_qc, uint32_t* fl_list, uint32_t* pl, int cap,
-                                  unsigned long long* red)
-{
-    {
-        const int wlo = (kGhost - 1) >> 2, whi = (c.N1 + kGhost) >> 2;
-        const int pw = (whi - wlo + (int)blockDim.x) / (int)blockDim.x;
-        if (pw <= 16) {
-            const int w0 = wlo + (int)threadIdx.x * pw;
-            return stage_lists_words(c, b, l, copy_qc, fl_list, pl, cap, red, w0, min(w0 + pw, whi + 1));
-        }
-    }
-    const int lo = -1, hi = c.N1;
-    const int n = hi - lo + 1;
-    const int per = (n + (int)blockDim.x - 1) / (int)blockDim.x;
-    const int a0 = lo + (int)threadIdx.x * per;
-    const int a1 = min(a0 + per, hi + 1);
-    // 0: not a stage point, 1: finest-level point, 2: coarse point (main_1d_euler.cpp:111-133)
-    auto cls = [&](int i) -> int {
-        if (i < 0 || i > c.N1 || !c.bit(i, b)) return 0;
-        const int lev = c.L(l, i);
-        if (lev == c.maxl) return 1;
-        if (lev < 0 || lev > c.maxl) return 0;
-        const int d = c.D(lev);
-        return (i - 2 * d < -kGhost || i + 2 * d > c.N1 + kGhost) ? 0 : 2;
-    };
-    const bool bits = per <= 64;
-    unsigned long long mf = 0, mp = 0, mc = 0;
-    unsigned cf = 0, cp = 0, cc = 0;
-    int k_i = a0 < a1 ? cls(a0) : 0;
-    for (int i = a0; i < a1; ++i) {
-        const int k_n = cls(i + 1);
-        const unsigned long long bit = 1ull << ((i - a0) & 63);
-        if (k_i == 1 || k_n == 1) {
-            ++cf;
-            if (bits) mf |= bit;
-        }
-        if (k_i == 1) {
-            ++cp;
-            if (bits) mp |= bit;
-        } else if (k_i == 2) {
-            ++cc;
-            if (bits) mc |= bit;
-        }
-        if (copy_qc && i >= 0 && c.bit(i, 1))
-            for (int k = 0; k < 3; ++k) c.QC(k, i) = c.Q(k, i);
-        k_i = k_n;
-    }
-    constexpr unsigned long long M21 = (1ull << 21) - 1;
-    unsigned long long tot;
-    const unsigned long long off =
-        block_exclusive_scan64((unsigned long long)cf | ((unsigned long long)cp << 21) | ((unsigned long long)cc << 42),
-                               red, &tot);
-    StageLists o{(int)(tot & M21), (int)((tot >> 21) & M21), (int)((tot >> 42) & M21)};
-    unsigned of = (unsigned)(off & M21), op = (unsigned)((off >> 21) & M21), oc = (unsigned)((off >> 42) & M21);
-    uint32_t* crs = pl + cap - o.ncrs;
-    if (bits) {
-        for (; mf; mf &= mf - 1) fl_list[of++] = (uint32_t)(a0 + __ffsll(mf) - 1);
-        for (; mp; mp &= mp - 1) pl[op++] = (uint32_t)(a0 + __ffsll(mp) - 1);
-        for (; mc; mc &= mc - 1) crs[oc++] = (uint32_t)(a0 + __ffsll(mc) - 1);
-    } else {
-        k_i = a0 < a1 ? cls(a0) : 0;
-        for (int i = a0; i < a1; ++i) {
-            const int k_n = cls(i + 1);
-            if (k_i == 1 || k_n == 1) fl_list[of++] = (uint32_t)i;
-            if (k_i == 1) pl[op++] = (uint32_t)i;
-            else if (k_i == 2) crs[oc++] = (uint32_t)i;
-            k_i = k_n;
-        }
-    }
-    __syncthreads();
-    return o;
-}
-
-// One stage over mask bit b / level set l (main_1d_euler.cpp:97-245).  Faces are computed once
-// (face i+1/2 is shared by points i and i+1; the reference evaluates it for both, identically).
-// The faces and the coarse derivatives read the stage input Q and run in one phase (the coarse
-// derivatives are parked in qt); the point updates follow in a second phase, so Q is never read
-// after a point of this stage has been written and no copy of the stage input is needed.
-template <int SCHEME>
-__device__ void stage1(const Ctx& c, int b, int l, double alpha, double dt, int kind, uint32_t* list,
-                       unsigned long long* red)
-{
-    const int cap = c.w + 32;
-    uint32_t* pl = list + cap;
-    const StageLists L = stage_lists(c, b, l, kind == 1, list, pl, cap, red);
-    const uint32_t* crs = pl + cap - L.ncrs;
+    const int k = 3 - kind, region = kind == 2 ? 0 : 1;
+    const StageLists L = stage_lists(c, k, region);
+    if (kind < 3) build_stage_lists(c, k - 1, 1 - region);
     for (int e = threadIdx.x; e < L.nf + L.ncrs; e += blockDim.x) {
         if (e < L.nf) {
-            const int f = (int)list[e];
+            const int f = L.faces.get(e);
             double s[6][3];
 #pragma unroll
             for (int p = 0; p < 6; ++p)
 #pragma unroll
-                for (int k = 0; k < 3; ++k) s[p][k] = c.Q(k, f - 2 + p);
+                for (int q = 0; q < 3; ++q) s[p][q] = c.Q(q, f - 2 + p);
             double o[3];
-            face_flux_1d<SCHEME>(s, alpha, c.I.gamma, o);
+            if (scheme == kWeno5) face_flux_1d<kWeno5>(s, alpha, c.I.gamma, o);
+            else face_flux_1d<kWenoZ>(s, alpha, c.I.gamma, o);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) c.fl[k * c.w + f + kGhost] = o[k];
+            for (int q = 0; q < 3; ++q) c.fl[q * c.w + f + kGhost] = o[q];
         } else {
-            const int i = (int)crs[e - L.nf];
+            const int i = L.crs.get(e - L.nf), d = coarse_spacing(c, k, i);
+            if (!d) continue;
             double dF[3];
-            coarse_dF1(c, i, c.D(c.L(l, i)), dF);
+            coarse_dF1(c, i, d, dF);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) c.QT(k, i) = dF[k];
+            for (int q = 0; q < 3; ++q) c.QT(q, i) = dF[q];
         }
     }
     __syncthreads();
+    double fast = 0;
     for (int e = threadIdx.x; e < L.nfin + L.ncrs; e += blockDim.x) {
         int i, d;
         double dF[3];
         if (e < L.nfin) {
-            i = (int)pl[e];
+            i = L.fin.get(e);
             d = 1;
-            for (int k = 0; k < 3; ++k) dF[k] = c.fl[k * c.w + i + kGhost] - c.fl[k * c.w + i - 1 + kGhost];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) dF[q] = c.fl[q * c.w + i + kGhost] - c.fl[q * c.w + i - 1 + kGhost];
         } else {
-            i = (int)crs[e - L.nfin];
-            d = c.D(c.L(l, i));
-            for (int k = 0; k < 3; ++k) dF[k] = c.QT(k, i);
+            i = L.crs.get(e - L.nfin);
+            d = coarse_spacing(c, k, i);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) dF[q] = d ? c.QT(q, i) : 0.0;
         }
+        // the stage-start copy: stages 2 and 3 read it on mask1 only
+        const bool keep = kind == 1 && Ctx::bit(c.plane(1), i);
         const double sc = dt / (c.I.dx * d);
-        for (int k = 0; k < 3; ++k) {
-            double& Qv = c.Q(k, i);
-            if (kind == 1) Qv = Qv - sc * dF[k];
-            else if (kind == 2) Qv = 0.75 * c.QC(k, i) + 0.25 * (Qv - sc * dF[k]);
-            else Qv = (c.QC(k, i) + 2.0 * (Qv - sc * dF[k])) / 3.0;
+        double v[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const double x = c.Q(q, i), start = kind == 1 ? 0.0 : c.QC(q, i);
+            if (keep) c.QC(q, i) = x;
+            const double r = x - sc * dF[q];
+            v[q] = kind == 1 ? r : kind == 2 ? 0.75 * start + 0.25 * r : (start + 2.0 * r) / 3.0;
+        }
+        if (!d) continue;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) c.Q(q, i) = v[q];
+        if (kind < 3) {
+            if (e < L.nfin) fast = maxd(fast, speed1(v[0], v[1], v[2], c.I.gamma, nf));
+            if (!c.I.bc_generic && (i == 0 || i == c.N1)) {
+                // the transmissive ghosts of the next stage's input
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    for (int g = 1; g <= kGhost; ++g) c.Q(q, i == 0 ? -g : c.N1 + g) = v[q];
+            }
         }
     }
-    __syncthreads();
+    if (kind < 3) {
+        reduce_put(c.wk, kind, 0, fast);
+        __syncthreads();
+        if (c.I.bc_generic) {
+            bc1(c);
+            __syncthreads();
+        }
+    }
 }
 
-// One RK3 step of one instance on the context's buffers (q, stage copies, faces, mask bytes, levels).
-template <int SCHEME>
-__device__ void step_ctx(Inst1& I, const Ctx& c, uint32_t* list, double* dred, unsigned* ured)
+// RemoveResidue (AWCM_MANAGER_1D.h:135-157): the first np components to 0 at the points [0, N1] off
+// mask0; dense: all of them, else those that the step can have left a value at (the start's mask0
+// and mask3; before the step the values off its mask0 were zero).  A warp per word.
+__device__ void remove_residue1(const Ctx& c, const uint32_t* start, int np, bool dense)
 {
-    unsigned long long* red64 = reinterpret_cast<unsigned long long*>(ured);
-    prepare1(c);
-
-    // CFL (main_1d_euler.cpp:67-81)
-    double mv = 0;
-    bool nf = false;  // a NaN or infinite wave speed in the CFL or LF scans
-    for (int i = threadIdx.x; i <= c.N1; i += blockDim.x) {
-        if (!c.bit(i, 3)) continue;
-        const double q0 = c.Q(0, i), q1 = c.Q(1, i), q2 = c.Q(2, i);
-        const double s = sound1(q0, q1, q2, I.gamma);
-        const double u = q1 / q0;
-        nf |= !isfinite(absd(u) + s);
-        mv = maxd(mv, absd(u) + s);
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    for (int x0 = wp; x0 < c.nw; x0 += 32 * nwarp) {
+        const int xl = x0 + nwarp * lane;
+        const uint32_t z =
+            xl < c.nw ? c.inside(xl) & ~c.m0[xl] & (dense ? ~0u : start[xl] | c.plane(3)[xl]) : 0u;
+        unsigned todo = __ballot_sync(0xffffffffu, z != 0);
+        while (todo) {
+            const int j = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t zj = __shfl_sync(0xffffffffu, z, j);
+            const int i = 32 * (x0 + nwarp * j - 1) + lane;
+            if ((zj >> lane) & 1u)
+                for (int p = 0; p < np; ++p) c.Q(p, i) = 0;
+        }
     }
-    mv = block_max(mv, dred);
+}
+
+// The CFL step, the three stages and the residue removal after prepare1; L3: the list of mask3.
+// dense: values may lie off the start's mask0.
+__device__ __forceinline__ void stages1(Inst1& I, const Ctx& c, const List& L3, bool dense)
+{
+    Work1* wk = c.wk;
+    // CFL over mask3 (main_1d_euler.cpp:67-81) and the first stage's LF speed over its finest-level
+    // points; beside it the first fill of the ghosts and the first stage's lists
+    double mv = 0, a1 = 0;
+    bool nf = false;  // a NaN or infinite wave speed in the CFL or LF scans
+    bc1(c);
+    build_stage_lists(c, 2, 1);
+    {
+        const uint32_t* f3 = c.fine(3);
+        const unsigned n3 = wk->off[32];
+        for (unsigned e = threadIdx.x; e < n3; e += blockDim.x) {
+            const int i = L3.get(e);
+            const double s = speed1(c.Q(0, i), c.Q(1, i), c.Q(2, i), I.gamma, nf);
+            mv = maxd(mv, s);
+            if (Ctx::bit(f3, i)) a1 = maxd(a1, s);
+        }
+    }
+    reduce_put(wk, 0, 0, mv);
+    reduce_put(wk, 0, 1, a1);
+    __syncthreads();
+    mv = reduce_get(wk, 0, 0);
+    a1 = reduce_get(wk, 0, 1);
     double dt = I.cfl * I.dx / mv;
     if (I.dt_fixed > 0) dt = I.dt_fixed;
     int do_print = 0;
@@ -778,37 +992,21 @@ __device__ void step_ctx(Inst1& I, const Ctx& c, uint32_t* list, double* dred, u
         dt = I.t_end - I.t;
         do_print = 1;
     }
-    unsigned cnt[4] = {0, 0, 0, 0};
-    for (int i = threadIdx.x; i <= c.N1; i += blockDim.x) {
-        const unsigned v = c.M(i);
-        for (int k = 0; k < 4; ++k) cnt[k] += (v >> k) & 1u;
+    double alpha = a1;
+#pragma unroll 1
+    for (int kind = 1; kind <= 3; ++kind) {
+        if (threadIdx.x == 0) I.alpha[kind - 1] = alpha;
+        stage1(c, I.scheme, kind, alpha, dt, nf);
+        if (kind < 3) alpha = reduce_get(wk, kind, 0);
     }
-    block_sum4(cnt, ured);
-
-    bc1(c);
-    const double a1 = lf_speed1(c, 3, 3, dred, nf);
-    // the stage-start copy QC is taken inside stage 1's list pass
-    stage1<SCHEME>(c, 2, 2, a1, dt, 1, list, red64);
-    bc1(c);
-    const double a2 = lf_speed1(c, 2, 2, dred, nf);
-    stage1<SCHEME>(c, 1, 1, a2, dt, 2, list, red64);
-    bc1(c);
-    const double a3 = lf_speed1(c, 1, 1, dred, nf);
-    stage1<SCHEME>(c, 0, 0, a3, dt, 3, list, red64);
+    remove_residue1(c, c.plane(kPlTemp), 3, dense);
     const bool any_nf = __syncthreads_or(nf);
-    // RemoveResidue (AWCM_MANAGER_1D.h:135-157)
-    for (int i = threadIdx.x; i <= c.N1; i += blockDim.x)
-        if (!c.bit(i, 0)) c.Q(0, i) = c.Q(1, i) = c.Q(2, i) = 0;
-    __syncthreads();
     if (threadIdx.x == 0) {
         I.dt = dt;
         I.mv = mv;
-        I.alpha[0] = a1;
-        I.alpha[1] = a2;
-        I.alpha[2] = a3;
         I.do_print = do_print;
-        for (int k = 0; k < 4; ++k) I.mask_cnt[k] = cnt[k];
-        I.upd += cnt[0];
+        for (int k = 0; k < 4; ++k) I.mask_cnt[k] = wk->mask_cnt[k];
+        I.upd += wk->mask_cnt[0];
         I.steps += 1;
         I.t += dt;
         I.done = I.t >= I.t_end;
@@ -825,26 +1023,7 @@ __device__ void step_ctx(Inst1& I, const Ctx& c, uint32_t* list, double* dred, u
 // ------------------------------------------------------------------- scalar AWCM (advection)
 // The scalar path of Wavelet/main_1d_advect.cpp:48-224: one field q advected with unit speed at a
 // fixed dt, on the same masks and levels.  q lives in plane 0 of the instance's field; the stage
-// outputs q_2, q_1, q_0 in the three planes of the stage-start copy.
-
-// AWCM_1D::Prepare (Wavelet/AWCM_1D.h:45-72): WAVELET_1D::ForwardWaveletTransform
-// (WAVELET_1D.h:90-144, the arithmetic of the Euler form on its density), banding, then the
-// mask/level chain without PrepareEuler's adjacent zones on mask1..mask3, the inverse transform
-// (WAVELET_1D.h:146-196) and no interpolation of new points.
-__device__ void prepare1_scalar(const Ctx& c)
-{
-    fwt1(c);
-    band_copy1(c);
-    aaz1(c, 0, kBitCopy);
-    cr1(c, 0);
-    for (int k = 1; k <= 3; ++k) {
-        cl1(c, k - 1, k - 1, k, kBitCopy);  // level_{k-1} of mask_{k-1}; mask_k = the copy bit = mask_{k-1}
-        apd1(c, k, k - 1);                  // AddPointForDifferentiation(mask_k, level_{k-1})
-        cr1(c, k);
-    }
-    cl1(c, 3, 3, -1);
-    iwt1(c, 3);
-}
+// outputs q_2 and q_1 in the first two planes of the stage-start copy.
 
 // Coarse-level derivative of the field with the driver's branch selection (main_1d_advect.cpp:
 // 62-83): AWCM_1D::Differentiate and the 4-point DifferentiateAtLeftBoundary (Wavelet/AWCM_1D.h:
@@ -865,80 +1044,65 @@ __device__ double coarse_d1_scalar(const Ctx& c, const double* in, int i, int d)
     return kD02 * Q(i + 2 * d) + kD12 * Q(i + d) + kD22 * Q(i) + kD32 * Q(i - d) + kD2 * Q(i - 2 * d);
 }
 
-// One scalar stage (main_1d_advect.cpp:50-99, :100-155, :164-212): out = in (the whole line),
-// then at the points of mask b (level set l) out(i) -= dt (F_r - F_l) / (dx dx_) on the finest
-// level, F_r = WENO5::ReconstructRight(in(i-2..i+2)) (WENO.h:101-104; the face i+1/2 is shared by
-// points i and i+1, which the reference evaluates twice identically), or out(i) -= dt / (dx dx_)
-// dF below it; then the driver's ghost copies of the end points.
-__device__ void stage1_scalar(const Ctx& c, const double* in, double* out, int b, int l, double dt, uint32_t* list,
-                              unsigned* ured)
+// One scalar stage (main_1d_advect.cpp:50-99, :100-155, :164-212) over mask k (kind 1..3 with k =
+// 2, 1, 0): the stage output is the stage input off the mask and in - dt (F_r - F_l) / (dx dx_) on
+// the finest level, F_r = WENO5::ReconstructRight(in(i-2..i+2)) (WENO.h:101-104; the face i+1/2
+// is shared by points i and i+1, which the reference evaluates twice identically), or in - dt /
+// (dx dx_) dF below it, with the end points copied into the ghosts.  Only the points of the mask
+// and the ghosts are written: the next stage's stencils lie in this stage's mask.
+// Kind 2 then combines q_1 = 3/4 q + 1/4 q_1 (after q_1's ghost copies), kind 3 q = 1/3 q + 2/3 q_0.
+__device__ __forceinline__ void stage1_scalar(const Ctx& c, int kind, const double* in, double* out, double dt)
 {
-    for (int t = threadIdx.x; t < c.w; t += blockDim.x) out[t] = in[t];
-    __syncthreads();
-    auto fin = [&](int i) { return i >= 0 && i <= c.N1 && c.bit(i, b) && c.L(l, i) == c.maxl; };
-    const int nf = block_compact(-1, c.N1, [&](int f) { return fin(f) || fin(f + 1); }, list, ured);
-    for (int e = threadIdx.x; e < nf; e += blockDim.x) {
-        const int f = (int)list[e];
+    const int k = 3 - kind, region = kind == 2 ? 0 : 1;
+    const StageLists L = stage_lists(c, k, region);
+    if (kind < 3) build_stage_lists(c, k - 1, 1 - region);
+    for (int e = threadIdx.x; e < L.nf; e += blockDim.x) {
+        const int f = L.faces.get(e);
         const double* v = in + f + kGhost;
         c.fl[f + kGhost] = recon_left<kWeno5>(v[2], v[1], v[0], v[-1], v[-2]);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i <= c.N1; i += blockDim.x) {
-        if (!c.bit(i, b)) continue;
-        const int lev = c.L(l, i);
-        if (lev < 0 || lev > c.maxl) continue;
-        const int d = c.D(lev);
-        if (lev != c.maxl && (i - 2 * d < -kGhost || i + 2 * d > c.N1 + kGhost)) continue;
-        double& o = out[i + kGhost];
-        if (lev == c.maxl) o = o - dt * (c.fl[i + kGhost] - c.fl[i - 1 + kGhost]) / (c.I.dx * d);
-        else o = o - dt / (c.I.dx * d) * coarse_d1_scalar(c, in, i, d);
-    }
-    __syncthreads();
-    if (threadIdx.x < kGhost) {
-        const int g = threadIdx.x + 1;
-        out[kGhost - g] = out[kGhost];
-        out[kGhost + c.N1 + g] = out[kGhost + c.N1];
+    double* q = c.q0;
+    for (int e = threadIdx.x; e < L.nfin + L.ncrs; e += blockDim.x) {
+        const int i = e < L.nfin ? L.fin.get(e) : L.crs.get(e - L.nfin);
+        double r = in[i + kGhost];
+        if (e < L.nfin) {
+            r = r - dt * (c.fl[i + kGhost] - c.fl[i - 1 + kGhost]) / (c.I.dx * 1);
+        } else {
+            const int d = coarse_spacing(c, k, i);
+            if (d) r = r - dt / (c.I.dx * d) * coarse_d1_scalar(c, in, i, d);
+        }
+        if (kind < 3 && (i == 0 || i == c.N1))
+            for (int g = 1; g <= kGhost; ++g) out[(i == 0 ? -g : c.N1 + g) + kGhost] = r;
+        if (kind == 1) out[i + kGhost] = r;
+        else if (kind == 2) out[i + kGhost] = 0.75 * q[i + kGhost] + 0.25 * r;
+        else q[i + kGhost] = kC1_3 * q[i + kGhost] + kD1 * r;
     }
     __syncthreads();
 }
 
-// One pass of the scalar driver loop: Prepare, the three stages at dt = dt_fixed (the driver's
-// 0.5 dx is the caller's choice), the combinations q_1 = 3/4 q + 1/4 q_1 on mask1 (after q_1's
-// ghost copies) and q = 1/3 q + 2/3 q_0 on mask0, and PostProcess (RemoveResidue on mask0).  The
-// ghosts of q itself are never rewritten, as in the driver.
-__device__ void step_ctx_scalar(Inst1& I, const Ctx& c, uint32_t* list, unsigned* ured)
+// One pass of the scalar driver loop after prepare1: the three stages at dt = dt_fixed (the driver's
+// 0.5 dx is the caller's choice) with their combinations, and PostProcess (RemoveResidue on
+// mask0).  The ghosts of q itself are never rewritten, as in the driver.
+__device__ __forceinline__ void stages1_scalar(Inst1& I, const Ctx& c, bool dense)
 {
-    prepare1_scalar(c);
+    Work1* wk = c.wk;
     const double dt = I.dt_fixed;
-    unsigned cnt[4] = {0, 0, 0, 0};
-    for (int i = threadIdx.x; i <= c.N1; i += blockDim.x) {
-        const unsigned v = c.M(i);
-        for (int k = 0; k < 4; ++k) cnt[k] += (v >> k) & 1u;
-    }
-    block_sum4(cnt, ured);
-    double* q = c.q;
-    double* q2 = c.qc;
-    double* q1 = c.qc + c.w;
-    double* q0 = c.qc + 2 * c.w;
-    stage1_scalar(c, q, q2, 2, 2, dt, list, ured);
-    stage1_scalar(c, q2, q1, 1, 1, dt, list, ured);
-    for (int i = threadIdx.x; i <= c.N1; i += blockDim.x)
-        if (c.bit(i, 1)) q1[i + kGhost] = 0.75 * q[i + kGhost] + 0.25 * q1[i + kGhost];
+    build_stage_lists(c, 2, 1);
     __syncthreads();
-    stage1_scalar(c, q1, q0, 0, 0, dt, list, ured);
-    for (int i = threadIdx.x; i <= c.N1; i += blockDim.x)
-        if (c.bit(i, 0)) q[i + kGhost] = kC1_3 * q[i + kGhost] + kD1 * q0[i + kGhost];
-    __syncthreads();
-    for (int i = threadIdx.x; i <= c.N1; i += blockDim.x)
-        if (!c.bit(i, 0)) q[i + kGhost] = 0;
-    __syncthreads();
+    double* s2 = c.qc;
+    double* s1 = c.qc + c.w;
+#pragma unroll 1
+    for (int kind = 1; kind <= 3; ++kind)
+        stage1_scalar(c, kind, kind == 1 ? c.q0 : kind == 2 ? s2 : s1, kind == 1 ? s2 : s1, dt);
+    remove_residue1(c, c.plane(kPlStart), 1, dense);
     if (threadIdx.x == 0) {
         I.dt = dt;
         I.mv = 0;
         I.alpha[0] = I.alpha[1] = I.alpha[2] = 0;
         I.do_print = 0;
-        for (int k = 0; k < 4; ++k) I.mask_cnt[k] = cnt[k];
-        I.upd += cnt[0];
+        for (int k = 0; k < 4; ++k) I.mask_cnt[k] = wk->mask_cnt[k];
+        I.upd += wk->mask_cnt[0];
         I.steps += 1;
         I.t += dt;
         I.done = I.t >= I.t_end;
@@ -946,54 +1110,47 @@ __device__ void step_ctx_scalar(Inst1& I, const Ctx& c, uint32_t* list, unsigned
     __syncthreads();
 }
 
-// Byte offset of the level planes behind the mask bytes of an instance's state block.
-__host__ __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
-
-// The stage worklists of an instance of w ghosted points: faces, then finest and coarse points.
-__host__ __device__ __forceinline__ size_t list_bytes(int w) { return sizeof(uint32_t) * 2 * (size_t)(w + 32); }
-
-// What a step keeps in the CTA's shared memory (the rest stays in the instance's global buffers):
-// kStageAll: mask bytes, the four level planes, the three conserved planes and the worklists;
-// kStagePlanes: mask bytes and the three conserved planes (levels and worklists global, for an
-// instance too large for kStageAll: a Jmax-13 tube needs 205 KB this way against 303 KB);
-// kStageDensity: mask bytes, levels, the density plane and the worklists (the scalar path stages
-// no plane); kStageNone: nothing.
-enum StageLayout : int { kStageNone = 0, kStageDensity = 1, kStagePlanes = 2, kStageAll = 3 };
-__host__ __device__ __forceinline__ size_t stage_bytes(int layout, int w)
+// ------------------------------------------------------------------------------- one instance
+// Doubles a step keeps per point of the line: the conserved planes, and the stage-start copy, the
+// coarse derivatives and the face fluxes (one, two, none and one plane in the scalar path).
+// What an instance keeps in the CTA's shared memory, the fullest that fits:
+//   kInAll: the bit planes, every double above and the lists (lines of up to ~2000 points);
+//   kInField: the bit planes, the conserved planes and as much of the lists as fits beside them
+//     (an 8193-point tube: 28 KB of planes, 197 KB of field);
+//   kInDensity: the bit planes, the density (or the scalar field) and lists;
+//   kInPlanes: the bit planes and lists;  kInNone: lists.
+enum Tier1 : int { kInNone = 0, kInPlanes = 1, kInDensity = 2, kInField = 3, kInAll = 4 };
+struct Layout1 {
+    int tier;
+    unsigned cap;   // list entries per region
+    size_t bytes;   // shared memory it takes
+};
+__host__ __device__ __forceinline__ size_t tier_doubles(int tier, bool scalar)
 {
-    const size_t m = align16((size_t)w), l = align16((size_t)4 * w), d = sizeof(double) * (size_t)w;
-    switch (layout) {
-        case kStageAll: return m + l + 3 * d + list_bytes(w);
-        case kStagePlanes: return m + 3 * d;
-        case kStageDensity: return m + l + d + list_bytes(w);
+    switch (tier) {
+        case kInAll: return scalar ? 4 : 12;
+        case kInField: return scalar ? 1 : 3;
+        case kInDensity: return 1;
         default: return 0;
     }
 }
-// The fullest layout that fits `avail` bytes; pool_lists: the instance has worklist space in the
-// pool (the batch; the allocation-free step has none).
-__host__ __device__ __forceinline__ int pick_layout(int w, size_t avail, bool scalar, bool pool_lists)
+__host__ __device__ __forceinline__ Layout1 pick_layout(int nx, int maxl, size_t avail, bool scalar)
 {
-    if (!scalar && stage_bytes(kStageAll, w) <= avail) return kStageAll;
-    if (!scalar && pool_lists && stage_bytes(kStagePlanes, w) <= avail) return kStagePlanes;
-    if (stage_bytes(kStageDensity, w) <= avail) return kStageDensity;
-    return kStageNone;
-}
-// Shared memory of the allocation-free step (kStageDensity).
-__host__ __device__ __forceinline__ size_t step_smem_bytes(int w) { return stage_bytes(kStageDensity, w); }
-
-// Copy of n bytes by all threads of the block; 16-byte words where both ends allow it.
-__device__ __forceinline__ void block_copy_bytes(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src, int n)
-{
-    int head = 0;
-    if ((((uintptr_t)dst | (uintptr_t)src) & 15) == 0) {
-        const int nv = n >> 4;
-        for (int t = threadIdx.x; t < nv; t += blockDim.x)
-            reinterpret_cast<int4*>(dst)[t] = reinterpret_cast<const int4*>(src)[t];
-        head = nv << 4;
+    const int w = nx + 2 * kGhost;
+    const size_t full = list_entries1(w), eb = 2 * entry_bytes(w), np = plane_bytes1(nx, maxl);
+    const size_t least = full < 512 ? full : 512;
+    for (int tier = kInAll; tier >= kInNone; --tier) {
+        const size_t fixed = tier == kInNone ? 0 : np + align16(sizeof(double) * tier_doubles(tier, scalar) * (size_t)w);
+        if (tier != kInNone && fixed + eb * least > avail) continue;
+        size_t cap = (avail - fixed) / eb;
+        cap = cap < full ? cap : full;
+        cap &= ~(size_t)7;
+        return Layout1{tier, (unsigned)cap, fixed + eb * cap};
     }
-    for (int t = head + threadIdx.x; t < n; t += blockDim.x) dst[t] = src[t];
+    return Layout1{kInNone, 0, 0};
 }
 
+// Copy of n doubles by all threads of the block; 16-byte words where both ends allow it.
 __device__ __forceinline__ void block_copy_doubles(double* __restrict__ dst, const double* __restrict__ src, int n)
 {
     int head = 0;
@@ -1006,96 +1163,114 @@ __device__ __forceinline__ void block_copy_doubles(double* __restrict__ dst, con
     for (int t = head + threadIdx.x; t < n; t += blockDim.x) dst[t] = src[t];
 }
 
-// One RK3 step of an instance, with the part of its state that `layout` names staged in the CTA's
-// shared memory (smem: stage_bytes(layout, w) bytes): the ~100 level-sequential mask and transform
-// phases of PrepareEuler and the stages then run on shared memory, with one global round trip in
-// and one out per step.  q: the three conserved planes (global); qc, qt, fl: stage-start copy,
-// coarse derivatives, face fluxes; mg: w mask bytes, lg: four planes of w levels (global); glist:
-// worklist space in the pool (layouts that keep the worklists global).  One call site for every
-// layout keeps the step kernel's code to one copy of each scheme.
-// Up to nsteps RK3 steps of instance I (the caller has checked that it is not done), staged into
-// shared memory once around them; the steps stop when the instance is done.
-__device__ void step_inst(Inst1& I, double* q, double* qc, double* qt, double* fl, uint8_t* mg, int8_t* lg,
-                          const Weights& W, uint8_t* smem, int layout, uint32_t* glist, double* dred, unsigned* ured,
-                          int nsteps = 1)
+// The global buffers of one instance.
+struct Buffers1 {
+    double *q, *qc, *qt, *fl;
+    void* lists;        // 2 regions of list_entries1(w) entries
+    uint32_t* planes;   // bit planes of an instance too large for shared memory (else unused)
+    uint8_t* mask;
+    int8_t* level;
+};
+__device__ __forceinline__ Ctx make_ctx(const Inst1& I, const Buffers1& g, Work1* wk, const Weights& W)
 {
     const int w = I.nx + 2 * kGhost;
-    // the scalar path reads and writes its field planes directly; only its masks are staged
+    uint32_t* pl = g.planes;
+    const int nw = plane_words1(I.nx);
+    return Ctx{I, g.q, g.q + w, g.q + 2 * w, g.qc, g.qt, g.fl, pl, pl, pl + (size_t)kPlAux * nw, nullptr,
+               static_cast<uint8_t*>(g.lists), 0, wk, W, w, I.nx, I.nx - 1, I.maxl, level_bits(I.maxl), nw};
+}
+
+// Up to nsteps RK3 steps of instance I (the caller has checked that it is not done), staged into
+// shared memory once around them; the steps stop when the instance is done.
+__device__ void step_inst(Inst1& I, const Buffers1& g, const Weights& W, uint8_t* smem, size_t smem_bytes, Work1* wk,
+                          int nsteps)
+{
     const bool scalar = I.scheme == kScalarAdvection;
-    const bool st_lv = layout == kStageDensity || layout == kStageAll;
-    const bool st_q0 = layout == kStageDensity && !scalar;
-    const bool st_q = layout == kStagePlanes || layout == kStageAll;
-    uint8_t* ms = mg;
-    int8_t* ls = lg;
-    double* qp = q;   // plane p at qp + p w
-    double* q0 = q;   // plane 0
-    uint32_t* list = glist;
-    if (layout != kStageNone) {
-        uint8_t* p = smem;
-        ms = p;
-        p += align16((size_t)w);
-        if (st_lv) {
-            ls = reinterpret_cast<int8_t*>(p);
-            p += align16((size_t)4 * w);
+    const int w = I.nx + 2 * kGhost;
+    const Layout1 lay = pick_layout(I.nx, I.maxl, smem_bytes, scalar);
+    Ctx c = make_ctx(I, g, wk, W);
+    uint8_t* p = smem;
+    if (lay.tier >= kInPlanes) {
+        c.pl = c.m0 = reinterpret_cast<uint32_t*>(p);
+        c.aux = c.plane(kPlAux);
+        p += plane_bytes1(I.nx, I.maxl);
+        double* d = reinterpret_cast<double*>(p);
+        p += align16(sizeof(double) * tier_doubles(lay.tier, scalar) * (size_t)w);
+        const int np = lay.tier < kInDensity ? 0 : lay.tier == kInDensity || scalar ? 1 : 3;
+        if (np) block_copy_doubles(c.q0 = d, g.q, w);
+        if (np == 3) {
+            block_copy_doubles(c.q1 = d + w, g.q + w, w);
+            block_copy_doubles(c.q2 = d + 2 * w, g.q + 2 * w, w);
         }
-        if (layout == kStageDensity) {
-            if (st_q0) q0 = reinterpret_cast<double*>(p);
-            p += sizeof(double) * (size_t)w;
+        d += np * w;
+        if (lay.tier == kInAll) {
+            c.qc = d;
+            d += (scalar ? 2 : 3) * w;
+            if (!scalar) {
+                c.qt = d;
+                d += 3 * w;
+            }
+            c.fl = d;
         }
-        if (st_q) {
-            qp = q0 = reinterpret_cast<double*>(p);
-            p += 3 * sizeof(double) * (size_t)w;
-        }
-        if (st_lv) list = reinterpret_cast<uint32_t*>(p);
-        block_copy_bytes(ms, mg, w);
-        if (st_lv) block_copy_bytes(reinterpret_cast<uint8_t*>(ls), reinterpret_cast<const uint8_t*>(lg), 4 * w);
-        if (st_q0) block_copy_doubles(q0, q, w);
-        if (st_q) block_copy_doubles(qp, q, 3 * w);
-        __syncthreads();
     }
-    const Ctx c{I, qp, qc, qt, fl, ms, ls, W, w, I.nx, I.nx - 1, I.maxl, q0};
+    c.ls = p;
+    c.cap = lay.cap;
+    if (threadIdx.x < 32) wk->cls[threadIdx.x] = 0;
+    load_planes(c, g.mask, g.level);
+    __syncthreads();
+    // Between steps the field is zero off mask0 (RemoveResidue); a field or masks set from outside
+    // need not be, and then the first step removes the residue everywhere.
+    bool off = false;
+    for (int t = threadIdx.x; t < I.nx; t += blockDim.x)
+        if (!Ctx::bit(c.m0, t))
+            for (int k = 0; k < (scalar ? 1 : 3); ++k) off |= __double_as_longlong(c.Q(k, t)) != 0;
+    bool dense = __syncthreads_or(off);
     for (int s = 0; s < nsteps; ++s) {
         // the step's end (thread 0, then a block barrier) sets done at t_end or on an error
         if (s > 0 && *reinterpret_cast<volatile int*>(&I.done)) break;
-        if (scalar) step_ctx_scalar(I, c, list, ured);
-        else if (I.scheme == kWeno5) step_ctx<kWeno5>(I, c, list, dred, ured);
-        else step_ctx<kWenoZ>(I, c, list, dred, ured);
+        const List L3 = prepare1(c, !scalar);
+        if (scalar) stages1_scalar(I, c, dense);
+        else stages1(I, c, L3, dense);
+        dense = false;
     }
-    if (layout != kStageNone) {
-        block_copy_bytes(mg, ms, w);
-        if (st_lv) block_copy_bytes(reinterpret_cast<uint8_t*>(lg), reinterpret_cast<const uint8_t*>(ls), 4 * w);
-        if (st_q0) block_copy_doubles(q, q0, w);
-        if (st_q) block_copy_doubles(q, qp, 3 * w);
-        __syncthreads();
-    }
+    store_planes(c, g.mask, g.level);
+    if (c.q0 != g.q) block_copy_doubles(g.q, c.q0, w);
+    if (c.q1 != g.q + w) block_copy_doubles(g.q + w, c.q1, w);
+    if (c.q2 != g.q + 2 * w) block_copy_doubles(g.q + 2 * w, c.q2, w);
+    __syncthreads();
 }
 
-// Global views of instance I in the pool.
-__device__ __forceinline__ Ctx make_ctx(Inst1& I, const Pool& P)
+// Doubles of the list space and offset of the bit planes behind an instance's 12 planes.
+__host__ __device__ __forceinline__ size_t pool_list_doubles(int w) { return 2 * ((size_t)w + 32); }
+__host__ __device__ __forceinline__ size_t pool_doubles(int nx, int maxl)
 {
-    const int w = I.nx + 2 * kGhost;
+    const int w = nx + 2 * kGhost;
+    const size_t n = 12 * (size_t)w + pool_list_doubles(w) + (plane_bytes1(nx, maxl) + 7) / 8;
+    return (n + 31) & ~(size_t)31;
+}
+__device__ __forceinline__ Buffers1 pool_buffers(const Inst1& I, const Pool& P)
+{
+    const size_t w = (size_t)I.nx + 2 * kGhost;
     double* base = P.q + I.q_off;
     uint8_t* mb = P.m + I.m_off;
-    return Ctx{I, base, base + 3 * w, base + 6 * w, base + 9 * w, mb, (int8_t*)(mb + align16((size_t)w)), P.W,
-               w, I.nx, I.nx - 1, I.maxl, base};
+    return Buffers1{base, base + 3 * w, base + 6 * w, base + 9 * w, base + 12 * w,
+                    reinterpret_cast<uint32_t*>(base + 12 * w + pool_list_doubles((int)w)), mb, (int8_t*)(mb + align16(w))};
 }
 
 // nsteps RK3 steps of every queued instance (fewer for an instance that reaches t_end).  CTAs pull
 // queue slots until the queue is exhausted, and run each instance's steps back to back before
 // taking the next: nsteps = 1 is one step of the whole batch (the per-step graph); a large
 // nsteps runs every instance to its end in one launch, each CTA independently of the others.
-// smem_bytes: the launch's dynamic shared memory; an instance whose staged step does not fit in
-// it runs on its global buffers (its worklists in the pool too).
-// Up to 768 threads per CTA (80 registers a thread, some of the face computation spilled to L1):
-// a CTA advances one instance through ~150 block-barrier phases per step, latency-bound, so more
-// warps per instance pay for the spills (Jmax-13 tail step 0.312 -> 0.255 ms against 384 threads
-// and 162 registers; the step-synchronous batched whole run 3.48e7 -> 4.20e7 updates/s).
-__global__ void __launch_bounds__(768, 1) k_step1d(Inst1* insts, int n, const int* __restrict__ order, unsigned* queue, Pool P,
+// smem_bytes: the launch's dynamic shared memory.
+// What bounds it: the latency of the step's phases on one SM.  Against one point per thread on mask
+// bytes, the bit planes and lists took a step of one line from 99 to 94 us (1025 points, 512
+// threads) and from 555 to 312 us (15361 points, 768 threads, a line whose bytes and levels did
+// not fit in shared memory), and the 32769-point scalar line from 795 to 464 us.
+__global__ void __launch_bounds__(kMaxThreads1, 1) k_step1d(Inst1* insts, int n, const int* __restrict__ order, unsigned* queue, Pool P,
                          unsigned smem_bytes, int nsteps)
 {
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ double dred[32];
-    __shared__ __align__(8) unsigned ured[128];
+    __shared__ Work1 wk;
     __shared__ int cur;
     for (;;) {
         if (threadIdx.x == 0) cur = (int)atomicAdd(queue, 1u);
@@ -1107,51 +1282,121 @@ __global__ void __launch_bounds__(768, 1) k_step1d(Inst1* insts, int n, const in
         if (I.t >= I.t_end || I.err) {
             if (threadIdx.x == 0) I.done = 1;
         } else {
-            const int w = I.nx + 2 * kGhost;
-            double* base = P.q + I.q_off;
-            uint8_t* mb = P.m + I.m_off;
-            step_inst(I, base, base + 3 * w, base + 6 * w, base + 9 * w, mb, (int8_t*)(mb + align16((size_t)w)), P.W,
-                      smem, pick_layout(w, smem_bytes, I.scheme == kScalarAdvection, true),
-                      reinterpret_cast<uint32_t*>(base + 12 * (size_t)w), dred, ured, nsteps);
+            step_inst(I, pool_buffers(I, P), P.W, smem, smem_bytes, &wk, nsteps);
         }
         __syncthreads();
     }
 }
 
-// Single passes for the C-ABI manager surface (one CTA per instance).
+// Single passes for the C-ABI manager surface (one CTA per instance), on planes in global memory.
+// The inverse transform of any mask: unlike in the step the mask need not be closed, so points
+// outside it are zeroed in their level's own phase, as in the reference.
+__device__ void iwt_any1(const Ctx& c, const uint32_t* M)
+{
+    for (int lev = 0; lev < c.maxl; ++lev) {
+        const int D = c.D(lev), h = D >> 1, nd = c.N1 / D;
+        for (int ph = 0; ph < 2; ++ph) {
+            for (int a = threadIdx.x; a < (ph ? nd : nd - 1); a += blockDim.x) {
+                const int i = ph ? h + a * D : D + a * D;
+                double v = 0;
+                if (Ctx::bit(M, i)) {
+                    int s, k;
+                    if (ph) predict_stencil(i, D, c.N1, s, k);
+                    else update_stencil(i, D, c.N1, s, k);
+                    v = c.Q(0, i);
+                    if (ph) v *= 2;
+                    for (int cnt = 0; cnt < 4; ++cnt) {
+                        const double x = c.w_(cnt, k) * c.Q(0, s + cnt * D);
+                        v = ph ? v + x : v - x;
+                    }
+                }
+                c.Q(0, i) = v;
+            }
+            __syncthreads();
+        }
+    }
+}
+// InterpolateEuler(q, mra, from, to) (Wavelet/WAVELET_1D.h:393-431) for any two masks.
+__device__ void interp_any1(const Ctx& c, const uint32_t* from, const uint32_t* to)
+{
+    for (int x = threadIdx.x; x < c.nw; x += blockDim.x) c.aux[x] = c.points(to, x) & ~from[x];
+    __syncthreads();
+    close1(c, c.aux);
+    const List L = order_points(c, 0, c.aux, from);
+    const unsigned* off = c.wk->off;
+    for (int lev = 0; lev < c.maxl; ++lev) {
+        const int D = c.D(lev);
+        for (unsigned e = off[lev + 1] + threadIdx.x; e < off[lev + 2]; e += blockDim.x) {
+            const int i = L.get(e);
+            int s, k;
+            predict_stencil(i, D, c.N1, s, k);
+            for (int p = 1; p < 3; ++p) {
+                double v = 0;
+                for (int cnt = 0; cnt < 4; ++cnt) v += c.w_(cnt, k) * c.Q(p, s + cnt * D);
+                c.Q(p, i) = v;
+            }
+        }
+        __syncthreads();
+    }
+}
+// Density (or scalar field) to 0 at the interior points outside M (the inverse transform's zeros).
+__device__ void zero_off1(const Ctx& c, const uint32_t* M)
+{
+    for (int i = 1 + (int)threadIdx.x; i < c.N1; i += blockDim.x)
+        if (!Ctx::bit(M, i)) c.Q(0, i) = 0;
+}
+
 __global__ void k_pass1d(Inst1* insts, int inst, Pool P, int op, int bit, int level_id)
 {
+    __shared__ Work1 wk;
     Inst1& I = insts[inst];
-    const Ctx c = make_ctx(I, P);
+    const Buffers1 g = pool_buffers(I, P);
+    Ctx c = make_ctx(I, g, &wk, P.W);
+    if (threadIdx.x < 32) wk.cls[threadIdx.x] = 0;
+    load_planes(c, g.mask, g.level);
+    __syncthreads();
+    uint32_t* M = c.mask(bit);  // bit kBitTemp is plane kPlTemp
     switch (op) {
-        case 0:  // AddAdjacentZone
-            copy_bit1(c, bit, kBitCopy, true);
-            aaz1(c, bit, kBitCopy);
+        case 0: {  // AddAdjacentZone
+            for (int x = threadIdx.x; x < c.nw; x += blockDim.x)
+                c.aux[x] = M[x] | zone_word(c, x, [&](int y) { return c.points(M, y); });
+            __syncthreads();
+            for (int x = threadIdx.x; x < c.nw; x += blockDim.x) M[x] = c.aux[x];
             break;
-        case 1: cr1(c, bit); break;
-        case 2:
-            copy_bit1(c, bit, kBitCopy, true);
-            apd1(c, bit, level_id);
+        }
+        case 1: close1(c, M); break;
+        case 2: {  // AddPointForDifferentiation
+            for (int x = threadIdx.x; x < c.nw; x += blockDim.x) c.aux[x] = c.points(M, x);
+            __syncthreads();
+            for (int i = threadIdx.x; i <= c.N1; i += blockDim.x) {
+                const int lev = c.level(level_id, i), x = (i >> 5) + 1;
+                if (!Ctx::bit(c.aux, i) || lev > c.maxl) continue;
+                uint32_t own = 0;
+                stencil_push(c, M, x, c.maxl - lev, 1u << (i & 31), own);
+                if (own) atomicOr(&M[x], own);
+            }
             break;
-        case 3: cl1(c, level_id, bit, -1); break;
+        }
+        case 3: levels1(c, level_id, M); break;
         case 4:
             for (int i = threadIdx.x; i <= c.N1; i += blockDim.x)
-                if (!c.bit(i, bit)) c.Q(0, i) = c.Q(1, i) = c.Q(2, i) = 0;
+                if (!Ctx::bit(M, i)) c.Q(0, i) = c.Q(1, i) = c.Q(2, i) = 0;
             break;
         case 5:
-            for (int i = threadIdx.x; i <= c.N1; i += blockDim.x)
-                if (!(3 <= i && i <= c.N1 - 3)) c.set(i, bit);
+            for (int x = threadIdx.x; x < c.nw; x += blockDim.x) M[x] |= band_word(c, x);
             break;
         case 10:
-            if (I.scheme == kScalarAdvection) prepare1_scalar(c);
-            else prepare1(c);
+            prepare1(c, I.scheme != kScalarAdvection);
+            zero_off1(c, c.plane(3));
             break;
-        case 11: fwt1(c); break;
-        case 12: iwt1(c, bit); break;
-        case 13: interp1(c, bit, level_id); break;  // InterpolateEuler(from = bit, to = level_id as a bit)
+        case 11: fwt1(c, order_points(c, 0, c.m0)); break;
+        case 12: iwt_any1(c, M); break;
+        case 13: interp_any1(c, M, c.mask(level_id)); break;  // InterpolateEuler(from = bit, to = level_id as a bit)
         case 14: bc1(c); break;
         default: break;
     }
+    __syncthreads();
+    store_planes(c, g.mask, g.level);
 }
 
 // EULER_EQUATION_1D batch entry points (EULER_EQUATION.h:16-26, 42-47): n states of 3 doubles.
@@ -1229,8 +1474,7 @@ struct Batch1D {
             max_w = std::max(max_w, w);
             I.q_off = (long long)qo;
             I.m_off = (long long)mo;
-            qo += (size_t)12 * w + (size_t)(w + 32);
-            qo = (qo + 31) & ~(size_t)31;
+            qo += pool_doubles(I.nx, I.maxl);
             mo += align16((size_t)w) + (size_t)4 * w;  // mask bytes, then the levels 16-byte aligned
             mo = (mo + 255) & ~(size_t)255;
         }
@@ -1283,19 +1527,19 @@ struct Batch1D {
         return cudaMemcpy(host.data(), d_inst, sizeof(Inst1) * n, cudaMemcpyDeviceToHost);
     }
 
-    // Dynamic shared memory of the step kernel: the fullest staging layout of the largest instance
-    // that fits the per-CTA limit, else the limit (the largest instances then run on their global
-    // buffers, the smaller ones still staged).  Smaller instances take the fullest layout that fits.
+    // Dynamic shared memory of the step kernel: what the instance that can use most takes, within the
+    // share of the SM's shared memory that each of the CTAs resident on it can have.
     size_t smem_cap = 227 * 1024;
     size_t smem_bytes() const
     {
-        const size_t e = stage_bytes(pick_layout(max_w, smem_cap, false, true), max_w);
-        const size_t sc = stage_bytes(pick_layout(max_w, smem_cap, true, true), max_w);
-        const size_t b = std::max(e, sc);
-        return b ? b : smem_cap;
+        size_t b = 0;
+        for (const Inst1& I : host)
+            b = std::max(b, pick_layout(I.nx, I.maxl, smem_cap, I.scheme == kScalarAdvection).bytes);
+        return b;
     }
 
     // Launch shape: threads per CTA and CTAs per SM (0 = as many as fit).
+    size_t smem = 0;
     int set_launch(int threads, int ctas_per_sm)
     {
         if (threads < 64 || threads > 1024 || threads % 32) return kErrArg;
@@ -1305,12 +1549,21 @@ struct Batch1D {
             return kErrArg;
         }
         block = threads;
-        int sms = 148, occ = 1, optin = 0;
+        int sms = 148, occ = 1, optin = 227 * 1024, per_sm = 228 * 1024;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) == cudaSuccess && optin > 0)
-            smem_cap = (size_t)optin - 1024;  // leave room for the kernel's static shared arrays
-        cudaFuncSetAttribute(k_step1d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes());
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_step1d, block, smem_bytes());
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+        cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
+        // the CTAs that registers and threads allow on an SM, as far as the batch fills them
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_step1d, block, 0);
+        if (occ < 1) occ = 1;
+        if (ctas_per_sm > 0) occ = std::min(occ, ctas_per_sm);
+        occ = std::min(occ, (n + sms - 1) / sms);
+        // 1 KB of each CTA's shared memory is the system's
+        const int stat = (int)fa.sharedSizeBytes;
+        smem_cap = (size_t)std::min(optin - stat, per_sm / occ - 1024 - stat) & ~(size_t)15;
+        smem = smem_bytes();
+        cudaFuncSetAttribute(k_step1d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_step1d, block, smem);
         if (occ < 1) occ = 1;
         if (ctas_per_sm > 0) occ = std::min(occ, ctas_per_sm);
         grid = std::min(n, sms * occ);
@@ -1322,7 +1575,8 @@ struct Batch1D {
     void enq_step(int nsteps = 1)
     {
         cudaMemsetAsync(d_queue, 0, sizeof(unsigned), stream);
-        k_step1d<<<grid, block, smem_bytes(), stream>>>(d_inst, n, d_order, d_queue, P, (unsigned)smem_bytes(), nsteps);
+        cudaFuncSetAttribute(k_step1d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_step1d<<<grid, block, smem, stream>>>(d_inst, n, d_order, d_queue, P, (unsigned)smem, nsteps);
     }
 
     int build_graph()
@@ -1510,36 +1764,40 @@ struct Batch1D {
 
 // =========================================================================== allocation-free step
 // One RK3 step of a single 1D instance whose conserved field and mask/level state live in device
-// buffers the caller owns, with every other buffer the step needs -- the stage-start and stage-input
-// copies of the field, the face fluxes and the instance descriptor -- placed in the file-scope
-// array below instead of memory allocated per instance.  It is sized for instances of up to
-// kNoAllocMaxNx points (Jmax 13 with 17 coarse points): 9 x 8199 doubles plus a 256-byte
-// descriptor, about 577 KiB, which every GPU that loads this library holds until the process exits.
+// buffers the caller owns, with every other buffer the step needs -- the stage-start copy of the
+// field, the coarse derivatives, the face fluxes, the lists and the instance descriptor -- placed
+// in the file-scope array below (or in shared memory) instead of memory allocated per instance.  It
+// is sized for instances of up to kNoAllocMaxNx points (Jmax 13 with 17 coarse points): 9 planes
+// of 8199 doubles, two list regions of 16-bit entries and a 256-byte descriptor, about 641 KiB,
+// which every GPU that loads this library holds until the process exits.
+constexpr int kNoAllocThreads = 512;
+constexpr size_t kNoAllocSmem = (227 * 1024 - sizeof(Work1)) & ~(size_t)15;
 constexpr int kNoAllocMaxNx = 8193;
 constexpr int kNoAllocMaxW = kNoAllocMaxNx + 2 * kGhost;
 constexpr int kNoAllocHeader = 32;  // doubles reserved for the descriptor (Inst1 fits in 256 bytes)
-constexpr size_t kNoAllocDoubles = kNoAllocHeader + (size_t)9 * kNoAllocMaxW;
+constexpr size_t kNoAllocLists = (size_t)kNoAllocMaxW + 32;  // 4 (w + 32) entries of 2 bytes
+constexpr size_t kNoAllocDoubles = kNoAllocHeader + (size_t)9 * kNoAllocMaxW + kNoAllocLists;
 static_assert(sizeof(Inst1) <= kNoAllocHeader * sizeof(double), "descriptor does not fit the reserved header");
 
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles];
 
 namespace {
 
-// scratch: the device address of g_noalloc_scratch (resolved on the host once per device).
-__global__ void k_step1d_noalloc(Inst1 param, double* q, uint8_t* state, double* scratch, double* out, Weights W)
+// scratch: the device address of g_noalloc_scratch (resolved on the host once per device).  The
+// bit planes of 8193 points (28 KB) are always in shared memory.
+__global__ void __launch_bounds__(kNoAllocThreads, 1)
+    k_step1d_noalloc(Inst1 param, double* q, uint8_t* state, double* scratch, double* out, Weights W, unsigned smem_bytes)
 {
-    extern __shared__ __align__(16) uint8_t smem[];  // step_smem_bytes(w)
-    __shared__ double dred[32];
-    __shared__ __align__(8) unsigned ured[128];
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ Work1 wk;
     Inst1& I = *reinterpret_cast<Inst1*>(scratch);
     if (threadIdx.x == 0) I = param;  // the descriptor is rewritten by every call
     __syncthreads();
     const int w = param.nx + 2 * kGhost;
     double* qc = scratch + kNoAllocHeader;
-    double* qt = qc + 3 * w;
-    double* fl = qt + 3 * w;
+    const Buffers1 g{q, qc, qc + 3 * w, qc + 6 * w, qc + 9 * w, nullptr, state, (int8_t*)(state + w)};
     if (I.t < I.t_end) {
-        step_inst(I, q, qc, qt, fl, state, (int8_t*)(state + w), W, smem, kStageDensity, nullptr, dred, ured);
+        step_inst(I, g, W, smem, smem_bytes, &wk, 1);
     } else if (threadIdx.x == 0) {
         I.done = 1;
     }
@@ -1867,10 +2125,11 @@ int awcm1d_step_noalloc(int num_levels, int nx_coarse, double x_min, double x_ma
     I.cfl = cfl;
     I.t = t;
     I.t_end = t_end;
-    const int w = (int)nx + 2 * kGhost;
-    const size_t smem = step_smem_bytes(w);  // 172 KB at the 8193-point limit
+    // what fits beside the kernel's static shared memory
+    const unsigned smem = (unsigned)pick_layout((int)nx, num_levels - 1, kNoAllocSmem, false).bytes;
     AWCM_CUDA_TRY(cudaFuncSetAttribute(k_step1d_noalloc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_step1d_noalloc<<<1, 256, smem, (cudaStream_t)stream>>>(I, q_dev, state_dev, scratch, out_dev, make_weights());
+    k_step1d_noalloc<<<1, kNoAllocThreads, smem, (cudaStream_t)stream>>>(I, q_dev, state_dev, scratch, out_dev, make_weights(),
+                                                                         smem);
     AWCM_CUDA_TRY(cudaGetLastError());
     return kOk;
 }
