@@ -57,9 +57,12 @@ struct Inst1 {
 // BOUNDARY_CONDITION values of the generic manager (BOUNDARY_MANAGER_1D.h:4-13).
 constexpr int kBcPeriodic1 = -3, kBcExtrapolation1 = -2;
 
-// Threads per CTA of the step kernel at most.
+// Threads per CTA: a caller may ask for up to 768, the step kernel runs at most 512, with 128 registers
+// each.  At 768 threads and 80 registers it spills about 1.2 KB a thread in and around the faces, and
+// every phase pays: a 1025-point step took 92 us against 75 us.
+constexpr int kMaxLaunch1 = 768;
 #ifndef AWCM_MAX_THREADS_1D
-#define AWCM_MAX_THREADS_1D 768
+#define AWCM_MAX_THREADS_1D 512
 #endif
 constexpr int kMaxThreads1 = AWCM_MAX_THREADS_1D;
 
@@ -804,9 +807,15 @@ __device__ __forceinline__ void bc1(const Ctx& c)
 
 // |u| + c (main_1d_euler.cpp:67-95); nf: set when it is NaN or infinite (NaN/Inf state, negative
 // pressure or density).
+__device__ __noinline__ double speed1_any(double q0, double q1, double q2, double gamma)
+{
+    return absd(q1 / q0) + sound1(q0, q1, q2, gamma);
+}
 __device__ __forceinline__ double speed1(double q0, double q1, double q2, double gamma, bool& nf)
 {
-    const double s = absd(q1 / q0) + sound1(q0, q1, q2, gamma);
+    SharedDiv dv;
+    double s = awcm::speed1(dv, q0, q1, q2, gamma);
+    if (dv.bad) s = speed1_any(q0, q1, q2, gamma);
     nf |= !isfinite(s);
     return s;
 }
@@ -814,14 +823,15 @@ __device__ __forceinline__ double speed1(double q0, double q1, double q2, double
 // Coarse-level flux derivative (AWCM_1D::DifferentiateEuler*, Wavelet/AWCM_1D.h:142-189) with the
 // driver's branch selection (main_1d_euler.cpp:111-133); right-boundary forms mirror the left ones.
 // Reads the stage input Q, which no point update has touched yet when it runs.
-__device__ void coarse_dF1(const Ctx& c, int i, int d, double* dF)
+template <class DV>
+__device__ __forceinline__ void coarse_dF1(DV& dv, const double* q0, const double* q1, const double* q2, int iend, int i,
+                                           int d, double* dF)
 {
     const double g = 1.4;  // EULER_EQUATION_1D euler_eqn(1.4) in the reference helpers
     auto F = [&](int ii, double* f) {
-        const double s[3] = {c.Q(0, ii), c.Q(1, ii), c.Q(2, ii)};
-        flux1(s, g, f);
+        const double s[3] = {q0[ii + kGhost], q1[ii + kGhost], q2[ii + kGhost]};
+        flux1(dv, s, g, f);
     };
-    const int iend = c.N1;
     double a[3], b[3], e[3], f[3], h[3];
     if (i - 2 * d > 0 && i + 2 * d < iend) {
         F(i - 2 * d, a), F(i - d, b), F(i + d, e), F(i + 2 * d, f);
@@ -839,6 +849,38 @@ __device__ void coarse_dF1(const Ctx& c, int i, int d, double* dF)
         F(i + 2 * d, a), F(i + d, b), F(i, e), F(i - d, f), F(i - 2 * d, h);
         for (int p = 0; p < 3; ++p) dF[p] = kD02 * a[p] + kD12 * b[p] + kD22 * e[p] + kD32 * f[p] + kD2 * h[p];
     }
+}
+
+// A coarse point or a face whose operands are outside the range of SharedDiv, with IEEE divisions.
+__device__ __noinline__ void coarse_any1(const double* q0, const double* q1, const double* q2, int N1, int i, int d,
+                                         double* out, int w)
+{
+    IeeeDiv dv;
+    double dF[3];
+    coarse_dF1(dv, q0, q1, q2, N1, i, d, dF);
+    for (int k = 0; k < 3; ++k) out[k * w] = dF[k];
+}
+template <class DV>
+__device__ __forceinline__ void face1(DV& dv, const double* q0, const double* q1, const double* q2, int f, int scheme,
+                                      double alpha, double gamma, double* out, int w)
+{
+    double s[6][3], o[3];
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+        s[p][0] = q0[f - 2 + p + kGhost];
+        s[p][1] = q1[f - 2 + p + kGhost];
+        s[p][2] = q2[f - 2 + p + kGhost];
+    }
+    if (scheme == kWeno5) face_flux_1d<kWeno5>(dv, s, alpha, gamma, o);
+    else face_flux_1d<kWenoZ>(dv, s, alpha, gamma, o);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) out[k * w] = o[k];
+}
+__device__ __noinline__ void face_any1(const double* q0, const double* q1, const double* q2, int f, int scheme,
+                                       double alpha, double gamma, double* out, int w)
+{
+    IeeeDiv dv;
+    face1(dv, q0, q1, q2, f, scheme, alpha, gamma, out, w);
 }
 
 // Spacing of the coarse point i in level set k, or 0: a level outside 0..maxl or a derivative
@@ -868,23 +910,18 @@ __device__ __forceinline__ void stage1(const Ctx& c, int scheme, int kind, doubl
     for (int e = threadIdx.x; e < L.nf + L.ncrs; e += blockDim.x) {
         if (e < L.nf) {
             const int f = L.faces.get(e);
-            double s[6][3];
-#pragma unroll
-            for (int p = 0; p < 6; ++p)
-#pragma unroll
-                for (int q = 0; q < 3; ++q) s[p][q] = c.Q(q, f - 2 + p);
-            double o[3];
-            if (scheme == kWeno5) face_flux_1d<kWeno5>(s, alpha, c.I.gamma, o);
-            else face_flux_1d<kWenoZ>(s, alpha, c.I.gamma, o);
-#pragma unroll
-            for (int q = 0; q < 3; ++q) c.fl[q * c.w + f + kGhost] = o[q];
+            SharedDiv dv;
+            face1(dv, c.q0, c.q1, c.q2, f, scheme, alpha, c.I.gamma, c.fl + f + kGhost, c.w);
+            if (dv.bad) face_any1(c.q0, c.q1, c.q2, f, scheme, alpha, c.I.gamma, c.fl + f + kGhost, c.w);
         } else {
             const int i = L.crs.get(e - L.nf), d = coarse_spacing(c, k, i);
             if (!d) continue;
+            SharedDiv dv;
             double dF[3];
-            coarse_dF1(c, i, d, dF);
+            coarse_dF1(dv, c.q0, c.q1, c.q2, c.N1, i, d, dF);
 #pragma unroll
             for (int q = 0; q < 3; ++q) c.QT(q, i) = dF[q];
+            if (dv.bad) coarse_any1(c.q0, c.q1, c.q2, c.N1, i, d, c.qt + i + kGhost, c.w);
         }
     }
     __syncthreads();
@@ -918,7 +955,10 @@ __device__ __forceinline__ void stage1(const Ctx& c, int scheme, int kind, doubl
 #pragma unroll
         for (int q = 0; q < 3; ++q) c.Q(q, i) = v[q];
         if (kind < 3) {
-            if (e < L.nfin) fast = maxd(fast, speed1(v[0], v[1], v[2], c.I.gamma, nf));
+            if (e < L.nfin) {
+                const double s = speed1(v[0], v[1], v[2], c.I.gamma, nf);
+                if (s > fast) fast = s;
+            }
             if (!c.I.bc_generic && (i == 0 || i == c.N1)) {
                 // the transmissive ghosts of the next stage's input
 #pragma unroll
@@ -976,8 +1016,8 @@ __device__ __forceinline__ void stages1(Inst1& I, const Ctx& c, const List& L3, 
         for (unsigned e = threadIdx.x; e < n3; e += blockDim.x) {
             const int i = L3.get(e);
             const double s = speed1(c.Q(0, i), c.Q(1, i), c.Q(2, i), I.gamma, nf);
-            mv = maxd(mv, s);
-            if (Ctx::bit(f3, i)) a1 = maxd(a1, s);
+            if (s > mv) mv = s;  // a NaN speed is flagged and left out
+            if (s > a1 && Ctx::bit(f3, i)) a1 = s;
         }
     }
     reduce_put(wk, 0, 0, mv);
@@ -1263,9 +1303,10 @@ __device__ __forceinline__ Buffers1 pool_buffers(const Inst1& I, const Pool& P)
 // nsteps runs every instance to its end in one launch, each CTA independently of the others.
 // smem_bytes: the launch's dynamic shared memory.
 // What bounds it: the latency of the step's phases on one SM.  Against one point per thread on mask
-// bytes, the bit planes and lists took a step of one line from 99 to 94 us (1025 points, 512
-// threads) and from 555 to 312 us (15361 points, 768 threads, a line whose bytes and levels did
-// not fit in shared memory), and the 32769-point scalar line from 795 to 464 us.
+// bytes, the bit planes and lists took a step of one line from 99 to 94 us (1025 points) and from 555
+// to 312 us (15361 points, a line whose bytes and levels did not fit in shared memory), and the
+// 32769-point scalar line from 795 to 464 us.  Divisions by shared reciprocals, and 512 threads of
+// 128 registers instead of 768 of 80, then took 1025 points to 78 us and 15361 points to 247 us.
 __global__ void __launch_bounds__(kMaxThreads1, 1) k_step1d(Inst1* insts, int n, const int* __restrict__ order, unsigned* queue, Pool P,
                          unsigned smem_bytes, int nsteps)
 {
@@ -1406,7 +1447,8 @@ __global__ void k_euler1d_flux(const double* __restrict__ q, double* __restrict_
     if (t >= n) return;
     const double s[3] = {q[3 * t], q[3 * t + 1], q[3 * t + 2]};
     double o[3];
-    flux1(s, gamma, o);
+    IeeeDiv dv;
+    flux1(dv, s, gamma, o);
     for (int k = 0; k < 3; ++k) f[3 * t + k] = o[k];
 }
 
@@ -1509,11 +1551,7 @@ struct Batch1D {
         P.q = d_q;
         P.m = d_m;
         P.W = make_weights();
-        // Default width: measured alone, lines of up to ~1000 points step 2-3 % faster with 512
-        // threads, longer ones fastest with 768 (the batch's critical path is its longest line).
-        int nx_max = 0;
-        for (int k = 0; k < n; ++k) nx_max = std::max(nx_max, host[k].nx);
-        return set_launch(nx_max <= 1100 ? 512 : 768, 0);
+        return set_launch(kMaxThreads1, 0);
     }
 
     cudaError_t upload_inst()
@@ -1543,12 +1581,13 @@ struct Batch1D {
     int set_launch(int threads, int ctas_per_sm)
     {
         if (threads < 64 || threads > 1024 || threads % 32) return kErrArg;
-        cudaFuncAttributes fa{};
-        if (cudaFuncGetAttributes(&fa, k_step1d) == cudaSuccess && threads > fa.maxThreadsPerBlock) {
-            set_last_error("launch shape exceeds the step kernel's register budget", __FILE__, __LINE__);
+        if (threads > kMaxLaunch1) {
+            set_last_error("launch shape exceeds the step kernel's limit of 768 threads", __FILE__, __LINE__);
             return kErrArg;
         }
-        block = threads;
+        cudaFuncAttributes fa{};
+        AWCM_CUDA_TRY(cudaFuncGetAttributes(&fa, k_step1d));
+        block = std::min(threads, kMaxThreads1);
         int sms = 148, occ = 1, optin = 227 * 1024, per_sm = 228 * 1024;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);

@@ -1428,6 +1428,22 @@ __global__ void k_wt_bottom_y(Grid2 g, Field4 f, int part, const StepState* st)
 // `bit` (main_2d_euler(quad).cpp:86-104); with mv != null also the CFL speed
 // max (|u|+c)+(|v|+c) (:61-76).  A CTA covers 128 columns (one mask word of four points per
 // lane) x 32 rows (four per warp); empty words cost one load.  Maxima are order-independent.
+__device__ __noinline__ void speeds_any(double q0, double q1, double q2, double q3, double gamma, double* out)
+{
+    IeeeDiv dv;
+    const double q[4] = {q0, q1, q2, q3};
+    speeds2(dv, q, gamma, out[0], out[1]);
+}
+__device__ __forceinline__ void speeds(const double* q, double gamma, double& sx, double& sy)
+{
+    SharedDiv dv;
+    speeds2(dv, q, gamma, sx, sy);
+    if (dv.bad) {
+        double s[2];
+        speeds_any(q[0], q[1], q[2], q[3], gamma, s);
+        sx = s[0], sy = s[1];
+    }
+}
 constexpr int kAlphaRows = 4;
 __global__ void __launch_bounds__(256) k_alpha(Grid2 g, Field4 f, const uint8_t* __restrict__ m, int bit,
                                                double* ax, double* ay, double* mv, const StepState* st,
@@ -1456,9 +1472,8 @@ __global__ void __launch_bounds__(256) k_alpha(Grid2 g, Field4 f, const uint8_t*
                 if (!((hit >> (8 * L)) & 1u)) continue;
                 const size_t a = g.at(i0 + L, j);
                 const double q[4] = {f.p[0][a], f.p[1][a], f.p[2][a], f.p[3][a]};
-                const double c = sound2(q, g.gamma);
-                const double sx = absd(q[1] / q[0]) + c;
-                const double sy = absd(q[2] / q[0]) + c;
+                double sx, sy;
+                speeds(q, g.gamma, sx, sy);
                 nf |= !(isfinite(sx) && isfinite(sy));
                 sx_row = maxd(sx_row, sx);
                 cm[L] = maxd(cm[L], sy);
@@ -1512,9 +1527,8 @@ __device__ void alpha_list_run(const Grid2& g, Field4 f, const uint32_t* __restr
             const int i = (int)(idx % (uint32_t)g.pitch) - kGhost;
             j = (int)(idx / (uint32_t)g.pitch) - kGhost;
             const double q[4] = {f.p[0][idx], f.p[1][idx], f.p[2][idx], f.p[3][idx]};
-            const double c = sound2(q, g.gamma);
-            sx = absd(q[1] / q[0]) + c;
-            const double sy = absd(q[2] / q[0]) + c;
+            double sy;
+            speeds(q, g.gamma, sx, sy);
             nf |= !(isfinite(sx) && isfinite(sy));
             if (sy > 0) atomic_max_nonneg(&ay[i], sy);
         }
@@ -1770,11 +1784,38 @@ __global__ void __launch_bounds__(256) k_lists(Grid2 g, const uint8_t* __restric
 // --------------------------------------------------------------------------------- stage kernels
 // Face flux from the compacted face list: x faces (DIR 0) read cells i-2..i+3 of row j, y faces
 // (DIR 1) cells j-2..j+3 of column i (WENOZ_EULER_SOLVER_2D::ComputeFluxX/Y, WENOZ.h:236-320).
+// What bounds it: the FP64 pipe (2 cycles a warp instruction).  With divisions by shared reciprocals
+// (SharedDiv) a million faces take 120-126 us against 165 us with IEEE divisions.
 // CUSTOM false: the reference's WENO-Z parameters as compile-time constants (eps 1e-40, exact
 // |b0 - b2|); true: the instance's runtime parameters (the differentiable mode).
 #ifndef AWCM_FACE_MIN_CTAS
 #define AWCM_FACE_MIN_CTAS 4
 #endif
+template <int DIR, bool CUSTOM, class DV>
+__device__ __forceinline__ void face2(DV& dv, const Field4& f, long idx, long step, double al, double gamma, double eps,
+                                      double delta, const Field4& out)
+{
+    double s[6][4], o[4];
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+        const long a = idx + (p - 2) * step;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s[p][k] = f.p[k][a];
+    }
+    if (CUSTOM) face_flux_2d<DIR>(dv, s, al, gamma, o, eps, delta);
+    else face_flux_2d<DIR>(dv, s, al, gamma, o);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) out.p[k][idx] = o[k];
+}
+// A face whose operands are outside the range of SharedDiv, with IEEE divisions.
+template <int DIR, bool CUSTOM>
+__device__ __noinline__ void face_any2(Field4 f, long idx, long step, double al, double gamma, double eps, double delta,
+                                       Field4 out)
+{
+    IeeeDiv dv;
+    face2<DIR, CUSTOM>(dv, f, idx, step, al, gamma, eps, delta, out);
+}
+
 template <int DIR, bool CUSTOM>
 __global__ void __launch_bounds__(128, AWCM_FACE_MIN_CTAS)
     k_face(Grid2 g, Field4 f, Field4 out, const uint32_t* __restrict__ list, const unsigned* __restrict__ count,
@@ -1792,19 +1833,11 @@ __global__ void __launch_bounds__(128, AWCM_FACE_MIN_CTAS)
         const int ii = (int)(idx % (uint32_t)g.pitch) - kGhost;
         const int jj = (int)(idx / (uint32_t)g.pitch) - kGhost;
         const long step = DIR == 0 ? 1 : g.pitch;
-        double s[6][4];
-#pragma unroll
-        for (int p = 0; p < 6; ++p) {
-            const long a = (long)idx + (p - 2) * step;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) s[p][k] = f.p[k][a];
-        }
         const double al = DIR == 0 ? alpha[jj] : alpha[ii];
-        double o[4];
-        if (CUSTOM) face_flux_2d<DIR>(s, al, g.gamma, o, g.wz_eps, g.wz_delta);
-        else face_flux_2d<DIR>(s, al, g.gamma, o);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) out.p[k][idx] = o[k];
+        SharedDiv dv;
+        if (CUSTOM) dv.bad = !(g.wz_eps >= 1e-40 && g.wz_eps < 1e40 && g.wz_delta < 1e40);
+        face2<DIR, CUSTOM>(dv, f, idx, step, al, g.gamma, g.wz_eps, g.wz_delta, out);
+        if (dv.bad) face_any2<DIR, CUSTOM>(f, idx, step, al, g.gamma, g.wz_eps, g.wz_delta, out);
     }
 }
 
