@@ -80,6 +80,8 @@ __host__ __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) &
 // The bits of a word outside the ghosted line are set in the mask planes: ComputeLevel reads a
 // mask as set there, and every other pass ands with the words' valid bits.
 enum Plane1 : int { kPlTemp = 4, kPlAux = 5, kPlStart = 6, kPlFine = 7, kPlLevel = 11 };
+// Behind the planes: the points 32 m of a mask, packed again (see close1).
+__host__ __device__ __forceinline__ int coarse_words1(int nw) { return (nw + 31) / 32 + 2; }
 // Slices of a level value: enough for 0..maxl and one more value, all ones, which stands for a level
 // outside that range (only set_levels can put one there; it rests in the bytes and is never used).
 __host__ __device__ __forceinline__ int level_bits(int maxl)
@@ -91,7 +93,8 @@ __host__ __device__ __forceinline__ int level_bits(int maxl)
 __host__ __device__ __forceinline__ int plane_words1(int nx) { return ((nx - 1 + kGhost + 32) >> 5) + 1; }
 __host__ __device__ __forceinline__ size_t plane_bytes1(int nx, int maxl)
 {
-    return align16(sizeof(uint32_t) * (size_t)(kPlLevel + 4 * level_bits(maxl)) * (size_t)plane_words1(nx));
+    const size_t nw = (size_t)plane_words1(nx);
+    return align16(sizeof(uint32_t) * ((size_t)(kPlLevel + 4 * level_bits(maxl)) * nw + coarse_words1((int)nw)));
 }
 // List space: two regions of 2 (w + 32) entries each (a stage's faces and points).
 __host__ __device__ __forceinline__ size_t list_entries1(int w) { return 2 * ((size_t)w + 32); }
@@ -100,6 +103,7 @@ __host__ __device__ __forceinline__ size_t entry_bytes(int w) { return short_lis
 
 // The per-CTA workspace: class counters of the ordered list, list counters, reductions.
 struct Work1 {
+    Inst1 inst;                          // the instance's descriptor while its steps run
     unsigned cls[32], run[32], off[33];  // counts, write positions, starts of the level classes
     unsigned mask_cnt[4];                // |mask0..mask3|
     unsigned n_face[4], n_fin[4];        // of mask0..mask2: needed faces, finest-level points
@@ -148,6 +152,7 @@ struct Ctx {
     __device__ uint32_t* plane(int k) const { return pl + (size_t)k * nw; }
     __device__ uint32_t* mask(int k) const { return k == 0 ? m0 : plane(k); }
     __device__ uint32_t* fine(int k) const { return plane(kPlFine + k); }
+    __device__ uint32_t* coarse() const { return plane(kPlLevel + 4 * nb); }
     __device__ uint32_t* slice(int k, int b) const { return plane(kPlLevel + k * nb + b); }
     __device__ static bool bit(const uint32_t* P, int i) { return (P[(i >> 5) + 1] >> (i & 31)) & 1u; }
     __device__ int level(int k, int i) const
@@ -281,18 +286,25 @@ __device__ List order_points(const Ctx& c, int region, const uint32_t* P, const 
 {
     Work1* wk = c.wk;
     auto word = [&](int x) { return c.points(P, x) & (without ? ~without[x] : ~0u); };
-    for (int x = 1 + (int)threadIdx.x; x < c.nw; x += blockDim.x) {
-        const uint32_t v = word(x);
-        if (!v) continue;
-#pragma unroll
-        for (int t = 0; t < 5; ++t) {
-            const int n = __popc(v & odd_bits(t));
-            if (n) atomicAdd(&wk->cls[class_of(c, t)], (unsigned)n);
-        }
-        if (v & 1u) atomicAdd(&wk->cls[x == 1 ? 0 : class_of(c, 5 + __ffs(x - 1) - 1)], 1u);
+    // a warp takes every nwarp-th word, so that neighbouring active words go to different warps.
+    // Points of odd multiples of 1 .. 16 are counted per warp: n0 and n1 hold the packed counts.
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    auto counts = [&](uint32_t v, unsigned& n) {
+        const unsigned a = __reduce_add_sync(0xffffffffu, (unsigned)__popc(v & odd_bits(0)) | (__popc(v & odd_bits(1)) << 10) |
+                                                              (__popc(v & odd_bits(2)) << 20));
+        const unsigned b = __reduce_add_sync(0xffffffffu, (unsigned)__popc(v & odd_bits(3)) | (__popc(v & odd_bits(4)) << 10));
+        n = lane == 0 ? a & 1023u : lane == 1 ? (a >> 10) & 1023u : lane == 2 ? a >> 20 : lane == 3 ? b & 1023u : b >> 10;
+        return (a | b) != 0;
+    };
+    auto class0 = [&](int x) { return x == 1 ? 0 : class_of(c, 5 + __ffs(x - 1) - 1); };  // of bit 0 of word x
+    for (int x0 = 1 + wp; x0 < c.nw; x0 += 32 * nwarp) {
+        const int x = x0 + nwarp * lane;
+        const uint32_t v = x < c.nw ? word(x) : 0u;
+        unsigned n;
+        if (counts(v, n) && lane < 5 && n) atomicAdd(&wk->cls[class_of(c, lane)], n);
+        if (v & 1u) atomicAdd(&wk->cls[class0(x)], 1u);
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31;
     if (threadIdx.x < 32) {
         const unsigned n = wk->cls[lane];
         unsigned s = n;
@@ -307,26 +319,24 @@ __device__ List order_points(const Ctx& c, int region, const uint32_t* P, const 
     }
     __syncthreads();
     const List L = c.list(region, wk->off[32]);
-    // a warp takes every nwarp-th word, so that neighbouring active words go to different warps,
-    // and expands its non-empty words one by one, a point per lane
-    const int wp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    // the warp reserves its ranges, then expands its non-empty words one by one, a point per lane
+    const int t = lane ? __ffs(lane) - 1 : 5;
+    const uint32_t group = lane ? odd_bits(t) : 0u;
     for (int x0 = 1 + wp; x0 < c.nw; x0 += 32 * nwarp) {
         const int xl = x0 + nwarp * lane;
         const uint32_t mine = xl < c.nw ? word(xl) : 0u;
-        unsigned todo = __ballot_sync(0xffffffffu, mine != 0);
+        if (mine & 1u) L.put(atomicAdd(&wk->run[class0(xl)], 1u), 32 * (xl - 1));
+        unsigned n, pos = 0;
+        if (!counts(mine, n)) continue;
+        if (lane < 5 && n) pos = atomicAdd(&wk->run[class_of(c, lane)], n);
+        pos = __shfl_sync(0xffffffffu, pos, t < 5 ? t : 0);  // the next position of this lane's group
+        unsigned todo = __ballot_sync(0xffffffffu, (mine & ~1u) != 0);
         while (todo) {
             const int j = __ffs(todo) - 1;
             todo &= todo - 1;
-            const uint32_t v = __shfl_sync(0xffffffffu, mine, j);
-            const int x = x0 + nwarp * j;
-            const int t = lane ? __ffs(lane) - 1 : x == 1 ? 31 : 5 + __ffs(x - 1) - 1;
-            const uint32_t grp = v & (lane ? odd_bits(t) : 1u);
-            const bool on = (v >> lane) & 1u;
-            const int lead = grp ? __ffs(grp) - 1 : lane;
-            unsigned base = 0;
-            if (on && lane == lead) base = atomicAdd(&wk->run[class_of(c, t)], (unsigned)__popc(grp));
-            base = __shfl_sync(0xffffffffu, base, lead);
-            if (on) L.put(base + __popc(grp & ((1u << lane) - 1u)), 32 * (x - 1) + lane);
+            const uint32_t v = __shfl_sync(0xffffffffu, mine, j) & group;
+            if ((v >> lane) & 1u) L.put(pos + __popc(v & ((1u << lane) - 1u)), 32 * (x0 + nwarp * j - 1) + lane);
+            pos += __popc(v);
         }
     }
     __syncthreads();
@@ -369,19 +379,25 @@ __device__ void build_stage_lists(const Ctx& c, int k, int region)
             fa = f | shr(f, fine_word(c, k, xl + 1), 1);
         }
         unsigned todo = __ballot_sync(0xffffffffu, (m | fa) != 0);
+        if (!todo) continue;
+        const unsigned nfa = __reduce_add_sync(0xffffffffu, __popc(fa));
+        const unsigned nfc = __reduce_add_sync(0xffffffffu, __popc(f) | (__popc(m & ~f) << 16));
+        unsigned base = 0;
+        if (lane < 3) base = atomicAdd(&pos[lane], lane == 0 ? nfa : lane == 1 ? nfc & 0xffffu : nfc >> 16);
+        unsigned bf = __shfl_sync(0xffffffffu, base, 0), bp = __shfl_sync(0xffffffffu, base, 1);
+        unsigned bc = __shfl_sync(0xffffffffu, base, 2);
         while (todo) {
             const int j = __ffs(todo) - 1;
             todo &= todo - 1;
             const uint32_t mj = __shfl_sync(0xffffffffu, m, j), fj = __shfl_sync(0xffffffffu, f, j);
             const uint32_t faj = __shfl_sync(0xffffffffu, fa, j), cj = mj & ~fj;
-            unsigned base = 0;
-            if (lane < 3) base = atomicAdd(&pos[lane], (unsigned)__popc(lane == 0 ? faj : lane == 1 ? fj : cj));
-            const unsigned bf = __shfl_sync(0xffffffffu, base, 0), bp = __shfl_sync(0xffffffffu, base, 1);
-            const unsigned bc = __shfl_sync(0xffffffffu, base, 2);
             const int i = 32 * (x0 + nwarp * j - 1) + lane;
             if ((faj >> lane) & 1u) L.faces.put(bf + __popc(faj & lt), i);
             if ((fj >> lane) & 1u) L.fin.put(bp + __popc(fj & lt), i);
             if ((cj >> lane) & 1u) L.crs.put(bc + __popc(cj & lt), i);
+            bf += __popc(faj);
+            bp += __popc(fj);
+            bc += __popc(cj);
         }
     }
 }
@@ -474,96 +490,113 @@ __device__ void iwt_interp1(const Ctx& c, const List& L, bool interp)
     }
 }
 
-// CheckReconstruction (Wavelet/AWCM_MANAGER_1D.h:45-71), the levels of spacing h = 1..16: every
-// detail of the mask marks its four coarse neighbours i -+ h, i -+ 3h (shifted one-sided at the
-// ends), fine to coarse.  A word's outcome depends on at most 93 points around it, so each thread
-// closes a window of six words in registers and keeps its own one: no barrier between the levels.
-// Words are closed in place: a neighbour read after its own closure only holds points that belong
-// to the closure anyway.
-__device__ void close_words(const Ctx& c, uint32_t* P)
+// CheckReconstruction (Wavelet/AWCM_MANAGER_1D.h:45-71) marks the four coarse neighbours i -+ h, i -+ 3h of
+// every detail i of spacing h, fine to coarse; at the ends, where the stencil of the first detail
+// h is that of the next one (0, 2h, 4h, 6h) and that of the last one N1 - h that of N1 - 3h.
+//
+// close_word: word x of a mask (words ld(y), points 0..n1) after the levels of spacing 1 .. 2^(top-1),
+// top <= 5.  The word's outcome depends on at most 93 points around it, so a thread closes a window of
+// six words in registers, without a barrier between the levels.  A neighbour read after its own
+// closure only holds points that belong to the closure anyway, so words are closed in place.
+template <class Load>
+__device__ __forceinline__ uint32_t close_word(Load ld, int x, int n1, int top)
 {
-    const int top = min(c.maxl, 5), xr = (c.N1 >> 5) + 1;
-    for (int x = 1 + (int)threadIdx.x; x < c.nw; x += blockDim.x) {
-        uint32_t W[6];
-        uint32_t any = 0;
+    uint32_t W[6], in[6];
+    uint32_t any = 0;
 #pragma unroll
-        for (int k = 0; k < 6; ++k) any |= W[k] = c.points(P, x - 3 + k);
-        if (!any) continue;
-        const bool edge = x <= 4 || x >= xr - 4;  // the window may hold an end's one-sided stencils
+    for (int k = 0; k < 6; ++k) {
+        const int r = n1 - 32 * (x - 4 + k);
+        in[k] = x - 3 + k < 1 || r < 0 ? 0u : r >= 31 ? ~0u : (2u << r) - 1u;
+        any |= W[k] = in[k] ? ld(x - 3 + k) & in[k] : 0u;
+    }
+    if (!any) return 0u;
+    const bool left = x <= 4, right = x + 2 >= (n1 >> 5) - 1;
 #pragma unroll
-        for (int t = 0; t < 5; ++t) {
-            if (t >= top) break;
-            const int h = 1 << t;
-            uint32_t d[8];
-            d[0] = d[7] = 0;
+    for (int t = 0; t < 5; ++t) {
+        if (t >= top) break;
+        const int h = 1 << t;
+        uint32_t d[8];
+        d[0] = d[7] = 0;
 #pragma unroll
-            for (int k = 0; k < 6; ++k) d[k + 1] = W[k] & odd_bits(t);
-            if (edge) {
-                // the first detail h marks 0, 2h, 4h and 6h, the last one N1-6h .. N1 likewise: the
-                // point beyond the ordinary stencil (which stays clear of the line's other side)
-                uint32_t lo = 0, hi = 0;
-                const int sl = 1 + (h >> 5), tl = 1 + ((6 * h) >> 5);
-                const int sr = ((c.N1 - h) >> 5) + 1, tr = ((c.N1 - 6 * h) >> 5) + 1;
+        for (int k = 0; k < 6; ++k) d[k + 1] = W[k] & odd_bits(t);
+        if (left) {
+            // the detail h (word 1) also as 3h (the same word, for h = 16 the next one)
 #pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    if (x - 3 + k == sl) lo |= (W[k] >> (h & 31)) & 1u;
-                    if (x - 3 + k == sr) hi |= (W[k] >> ((c.N1 - h) & 31)) & 1u;
+            for (int k = 0; k < 6; ++k)
+                if (x - 3 + k == 1) {
+                    const uint32_t b = d[k + 1] & (1u << h);
+                    if (t < 4) d[k + 1] |= b << ((2 * h) & 31);
+                    else if (k < 5) d[k + 2] |= b;
                 }
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    if (x - 3 + k == tl) W[k] |= lo << ((6 * h) & 31);
-                    if (x - 3 + k == tr) W[k] |= hi << ((c.N1 - 6 * h) & 31);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                uint32_t o;
-                if (t < 4) {
-                    o = shl(d[k], d[k + 1], h) | shr(d[k + 1], d[k + 2], h) | shl(d[k], d[k + 1], 3 * h) |
-                        shr(d[k + 1], d[k + 2], 3 * h);
-                } else {
-                    // bit 16 of a word marks bit 0 of the words at 0, +1, +2 and -1
-                    o = (d[k + 1] | d[k] | (k > 0 ? d[k - 1] : 0u) | d[k + 2]) >> 16;
-                }
-                W[k] |= edge ? o & c.inside(x - 3 + k) : o;
-            }
         }
-        const uint32_t own = W[3];
+        if (right) {
+            // the detail n1 - h also as n1 - 3h
+            const int a = n1 - h, b = n1 - 3 * h;
+            uint32_t on = 0;
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+                if (x - 3 + k == (a >> 5) + 1) on = (d[k + 1] >> (a & 31)) & 1u;
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+                if (x - 3 + k == (b >> 5) + 1) d[k + 1] |= on << (b & 31);
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            uint32_t o;
+            if (t < 4) {
+                o = shl(d[k], d[k + 1], h) | shr(d[k + 1], d[k + 2], h) | shl(d[k], d[k + 1], 3 * h) |
+                    shr(d[k + 1], d[k + 2], 3 * h);
+            } else {
+                // bit 16 of a word marks bit 0 of the words at 0, +1, +2 and -1
+                o = (d[k + 1] | d[k] | (k > 0 ? d[k - 1] : 0u) | d[k + 2]) >> 16;
+            }
+            W[k] |= o & in[k];
+        }
+    }
+    return W[3];
+}
+// The whole closure of plane P: the words of the five finest levels, then one warp packs the points
+// 32 m, closes them in the same way for the next five levels, and spreads the new ones back; levels
+// beyond those (lines of more than 4 2^10 points have few of them) go point by point.
+__device__ __forceinline__ void close1(const Ctx& c, uint32_t* P)
+{
+    const int top = min(c.maxl, 5);
+    for (int x = 1 + (int)threadIdx.x; x < c.nw; x += blockDim.x) {
+        const uint32_t own = close_word([&](int y) { return P[y]; }, x, c.N1, top);
         if (own & ~P[x]) P[x] |= own;
     }
-}
-// The levels of spacing h >= 32, whose points are bit 0 of their words.  Levels of up to 128
-// details on one warp, with warp barriers between them; larger ones on the whole block.
-__device__ void close_coarse_level(const Ctx& c, uint32_t* P, int t, int first, int stride)
-{
-    const int h = 1 << t, D = 2 * h, nd = c.N1 / D;
-    for (int a = first; a < nd; a += stride) {
-        const int i = h + a * D;
-        if (!(P[(i >> 5) + 1] & 1u)) continue;
-        int s, k;
-        predict_stencil(i, D, c.N1, s, k);
-#pragma unroll
-        for (int cnt = 0; cnt < 4; ++cnt) {
-            uint32_t* y = &P[((s + cnt * D) >> 5) + 1];
-            if (!(*y & 1u)) atomicOr(y, 1u);
-        }
-    }
-}
-__device__ void close1(const Ctx& c, uint32_t* P)
-{
-    close_words(c, P);
     __syncthreads();
-    int t = 5;
-    for (; t < c.maxl && (c.N1 >> (t + 1)) > 128; ++t) {
-        close_coarse_level(c, P, t, threadIdx.x, blockDim.x);
-        __syncthreads();
-    }
-    if (t < c.maxl) {
-        if (threadIdx.x < 32)
-            for (; t < c.maxl; ++t) {
-                close_coarse_level(c, P, t, threadIdx.x, 32);
+    if (c.maxl > 5) {
+        if (threadIdx.x < 32) {
+            const int lane = threadIdx.x, m1 = c.N1 >> 5, nc = (m1 >> 5) + 2;
+            uint32_t* C = c.coarse();
+            for (int y = 1; y < nc; ++y) {
+                const int m = 32 * (y - 1) + lane;
+                const uint32_t v = __ballot_sync(0xffffffffu, m <= m1 && (P[m + 1] & 1u));
+                if (lane == 0) C[y] = v;
+            }
+            __syncwarp();
+            for (int y0 = 1; y0 < nc; y0 += 32) {
+                const int y = y0 + lane;
+                const uint32_t was = y < nc ? C[y] : 0u;
+                const uint32_t own = y < nc ? close_word([&](int z) { return C[z]; }, y, m1, min(c.maxl - 5, 5)) : 0u;
+                for (uint32_t n = own & ~was; n; n &= n - 1) P[32 * (y - 1) + __ffs(n)] |= 1u;
+                if (y < nc) C[y] = was | own;
                 __syncwarp();
             }
+            for (int t = 10; t < c.maxl; ++t) {
+                const int h = 1 << t, D = 2 * h, nd = c.N1 / D;
+                for (int a = lane; a < nd; a += 32) {
+                    const int i = h + a * D;
+                    if (!(P[(i >> 5) + 1] & 1u)) continue;
+                    int s, k;
+                    predict_stencil(i, D, c.N1, s, k);
+#pragma unroll
+                    for (int cnt = 0; cnt < 4; ++cnt) atomicOr(&P[((s + cnt * D) >> 5) + 1], 1u);
+                }
+                __syncwarp();
+            }
+        }
         __syncthreads();
     }
 }
@@ -615,51 +648,52 @@ __device__ __forceinline__ uint32_t band_word(const Ctx& c, int x)
 // whose nearest neighbour in the mask is 2^j away get level maxl - j (the reference searches the
 // distances one by one; here each distance is one shift of the whole word).  Off the ghosted line
 // the mask reads as set.  A point without any such neighbour keeps its level.
-// f(j, set): the word's points of level maxl - j, for each level that has any.
-template <class F>
-__device__ __forceinline__ void level_word(const Ctx& c, int k, const uint32_t* M, int x, F&& f)
+// rest(j, set): called for each of those points, with its level maxl - j.
+__device__ __forceinline__ uint32_t end_bits(const Ctx& c, int x)
 {
-    const uint32_t in = c.inside(x);
-    uint32_t ends = x == 1 ? 1u : 0u;  // the two end points: the finest level, in the mask or not
-    if ((c.N1 >> 5) + 1 == x) ends |= 1u << (c.N1 & 31);
-    const uint32_t on = in ? M[x] & in : 0u;
-    uint32_t todo = on & ~ends, fine = ends & in;
+    return (x == 1 ? 1u : 0u) | ((c.N1 >> 5) + 1 == x ? 1u << (c.N1 & 31) : 0u);
+}
+// The points of word x (v, with its neighbours l and r) that have a neighbour in M at distance 2^j.
+__device__ __forceinline__ uint32_t near_word(const Ctx& c, const uint32_t* M, int x, uint32_t l, uint32_t v, uint32_t r, int j)
+{
+    if (j < 5) return shl(l, v, 1 << j) | shr(v, r, 1 << j);
+    return c.padded(M, x - (1 << (j - 5))) | c.padded(M, x + (1 << (j - 5)));
+}
+template <class F>
+__device__ __forceinline__ void level_word(const Ctx& c, int k, const uint32_t* M, int x, F&& rest)
+{
+    const uint32_t in = c.inside(x), ends = end_bits(c, x);  // the ends: the finest level, in the mask or not
+    uint32_t todo = in ? M[x] & in & ~ends : 0u, fine = ends;
     uint32_t S[5];
 #pragma unroll
     for (int b = 0; b < 5; ++b) S[b] = ((c.maxl >> b) & 1) ? fine : 0u;
     if (todo) {
         const uint32_t l = c.padded(M, x - 1), v = M[x], r = c.padded(M, x + 1);
         for (int j = 0; j <= c.maxl && todo; ++j) {
-            uint32_t near;
-            if (j < 5) near = shl(l, v, 1 << j) | shr(v, r, 1 << j);
-            else near = c.padded(M, x - (1 << (j - 5))) | c.padded(M, x + (1 << (j - 5)));
-            const uint32_t got = todo & near;
-            if (!got) continue;
-            todo &= ~near;
-            const int lev = c.maxl - j;
+            const uint32_t got = todo & near_word(c, M, x, l, v, r, j);
+            todo &= ~got;
             if (j == 0) fine |= got;
-            else f(j, got);
+            const int lev = c.maxl - j;
 #pragma unroll
             for (int b = 0; b < 5; ++b)
                 if ((lev >> b) & 1) S[b] |= got;
         }
         if (todo) {  // no neighbour found: the level stays as it was
-            uint32_t was[5];
-#pragma unroll
-            for (int b = 0; b < 5; ++b) was[b] = b < c.nb ? c.slice(k, b)[x] & todo : 0u;
-            fine |= c.fine(k)[x] & todo;
-            for (uint32_t u = todo & ~c.fine(k)[x]; u; u &= u - 1) {
+            const uint32_t old = c.fine(k)[x] & todo;
+            fine |= old;
+            for (uint32_t u = todo; u; u &= u - 1) {
                 const uint32_t one = u & (0u - u);
                 int lev = 0;
 #pragma unroll
-                for (int b = 0; b < 5; ++b) lev |= (was[b] & one) ? 1 << b : 0;
-                if (lev != c.no_level()) f(c.maxl - lev, one);
+                for (int b = 0; b < 5; ++b)
+                    if (b < c.nb && (c.slice(k, b)[x] & one)) {
+                        lev |= 1 << b;
+                        S[b] |= one;
+                    }
+                if (lev != c.no_level()) rest(c.maxl - lev, one);
             }
-#pragma unroll
-            for (int b = 0; b < 5; ++b) S[b] |= was[b];
         }
     }
-    if (fine & on) f(0, fine & on);
     c.fine(k)[x] = fine;
 #pragma unroll
     for (int b = 0; b < 5; ++b)
@@ -696,18 +730,42 @@ __device__ __forceinline__ void stencil_push(const Ctx& c, uint32_t* P, int x, i
 // ComputeLevel(level_{k-1}, mask_{k-1}), mask_k = mask_{k-1}, AddAdjacentZone(mask_k) (zone) and
 // AddPointForDifferentiation(mask_k, level_{k-1}) in one phase.  All of them read mask_{k-1} only
 // (the zone's points are not in it, so their level is 0), and mask_k (clear before) takes ORs.
+// A warp takes 32 words and one job at a time -- the points of one distance, the zone, or the level
+// planes -- so that the searches of the levels run side by side: as one chain per word they took
+// 4.7 us of a 1025-point step's phase.
 __device__ void next_mask1(const Ctx& c, int k, bool zone)
 {
     const uint32_t* A = c.mask(k - 1);
     uint32_t* B = c.plane(k);
     auto pts = [&](int y) { return c.points(A, y); };
-    for (int x = threadIdx.x; x < c.nw; x += blockDim.x) {
+    const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    const int nch = (c.nw + 31) >> 5, njobs = (c.maxl + 3) * nch;
+    for (int job = threadIdx.x >> 5; job < njobs; job += nwarp) {
+        const int j = job / nch, x = 32 * (job - j * nch) + lane;
+        if (x >= c.nw) continue;
         const uint32_t a = A[x];  // ghosts and the bits off the line included
-        uint32_t own = a;
-        const uint32_t fresh = zone ? zone_word(c, x, pts) & ~a : 0u;
-        own |= fresh;
-        level_word(c, k - 1, A, x, [&](int j, uint32_t set) { stencil_push(c, B, x, j, set, own); });
-        if (fresh) stencil_push(c, B, x, c.maxl, fresh, own);
+        uint32_t own = 0;
+        if (j <= c.maxl) {
+            const uint32_t ends = end_bits(c, x), on = a & c.inside(x);
+            uint32_t got = on & ~ends;
+            if (got) {
+                // the points with a neighbour 2^j away and none nearer
+                const uint32_t l = c.padded(A, x - 1), r = c.padded(A, x + 1);
+                for (int i = 0; i < j; ++i) got &= ~near_word(c, A, x, l, a, r, i);
+                if (got) got &= near_word(c, A, x, l, a, r, j);
+            }
+            if (j == 0) got |= ends & on;
+            if (got) stencil_push(c, B, x, j, got, own);
+        } else if (j == c.maxl + 1) {
+            own = a;
+            if (zone) {
+                const uint32_t fresh = zone_word(c, x, pts) & ~a;
+                own |= fresh;
+                if (fresh) stencil_push(c, B, x, c.maxl, fresh, own);
+            }
+        } else {
+            level_word(c, k - 1, A, x, [&](int jj, uint32_t set) { stencil_push(c, B, x, jj, set, own); });
+        }
         if (own) atomicOr(&B[x], own);
     }
     __syncthreads();
@@ -926,6 +984,7 @@ __device__ __forceinline__ void stage1(const Ctx& c, int scheme, int kind, doubl
     }
     __syncthreads();
     double fast = 0;
+    const double sc1 = dt / (c.I.dx * 1);
     for (int e = threadIdx.x; e < L.nfin + L.ncrs; e += blockDim.x) {
         int i, d;
         double dF[3];
@@ -942,7 +1001,8 @@ __device__ __forceinline__ void stage1(const Ctx& c, int scheme, int kind, doubl
         }
         // the stage-start copy: stages 2 and 3 read it on mask1 only
         const bool keep = kind == 1 && Ctx::bit(c.plane(1), i);
-        const double sc = dt / (c.I.dx * d);
+        // dt / (dx d): d is a power of two
+        const double sc = sc1 * __hiloint2double((1023 - (31 - __clz(d | 1))) << 20, 0);
         double v[3];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
@@ -1222,9 +1282,10 @@ __device__ __forceinline__ Ctx make_ctx(const Inst1& I, const Buffers1& g, Work1
 
 // Up to nsteps RK3 steps of instance I (the caller has checked that it is not done), staged into
 // shared memory once around them; the steps stop when the instance is done.
-__device__ void step_inst(Inst1& I, const Buffers1& g, const Weights& W, uint8_t* smem, size_t smem_bytes, Work1* wk,
-                          int nsteps)
+// Works on wk->inst (set by the caller, behind a barrier).
+__device__ void step_inst(const Buffers1& g, const Weights& W, uint8_t* smem, size_t smem_bytes, Work1* wk, int nsteps)
 {
+    Inst1& I = wk->inst;
     const bool scalar = I.scheme == kScalarAdvection;
     const int w = I.nx + 2 * kGhost;
     const Layout1 lay = pick_layout(I.nx, I.maxl, smem_bytes, scalar);
@@ -1323,7 +1384,13 @@ __global__ void __launch_bounds__(kMaxThreads1, 1) k_step1d(Inst1* insts, int n,
         if (I.t >= I.t_end || I.err) {
             if (threadIdx.x == 0) I.done = 1;
         } else {
-            step_inst(I, pool_buffers(I, P), P.W, smem, smem_bytes, &wk, nsteps);
+            static_assert(sizeof(Inst1) % 4 == 0, "copied by words");
+            constexpr int nword = sizeof(Inst1) / 4;
+            uint32_t *gl = reinterpret_cast<uint32_t*>(&I), *sh = reinterpret_cast<uint32_t*>(&wk.inst);
+            for (int t = threadIdx.x; t < nword; t += blockDim.x) sh[t] = gl[t];
+            __syncthreads();
+            step_inst(pool_buffers(wk.inst, P), P.W, smem, smem_bytes, &wk, nsteps);
+            for (int t = threadIdx.x; t < nword; t += blockDim.x) gl[t] = sh[t];
         }
         __syncthreads();
     }
@@ -1804,19 +1871,17 @@ struct Batch1D {
 // =========================================================================== allocation-free step
 // One RK3 step of a single 1D instance whose conserved field and mask/level state live in device
 // buffers the caller owns, with every other buffer the step needs -- the stage-start copy of the
-// field, the coarse derivatives, the face fluxes, the lists and the instance descriptor -- placed
-// in the file-scope array below (or in shared memory) instead of memory allocated per instance.  It
+// field, the coarse derivatives, the face fluxes and the lists -- placed in the file-scope array
+// below or in shared memory instead of memory allocated per instance.  It
 // is sized for instances of up to kNoAllocMaxNx points (Jmax 13 with 17 coarse points): 9 planes
-// of 8199 doubles, two list regions of 16-bit entries and a 256-byte descriptor, about 641 KiB,
+// of 8199 doubles and two list regions of 16-bit entries, about 641 KiB,
 // which every GPU that loads this library holds until the process exits.
 constexpr int kNoAllocThreads = 512;
 constexpr size_t kNoAllocSmem = (227 * 1024 - sizeof(Work1)) & ~(size_t)15;
 constexpr int kNoAllocMaxNx = 8193;
 constexpr int kNoAllocMaxW = kNoAllocMaxNx + 2 * kGhost;
-constexpr int kNoAllocHeader = 32;  // doubles reserved for the descriptor (Inst1 fits in 256 bytes)
 constexpr size_t kNoAllocLists = (size_t)kNoAllocMaxW + 32;  // 4 (w + 32) entries of 2 bytes
-constexpr size_t kNoAllocDoubles = kNoAllocHeader + (size_t)9 * kNoAllocMaxW + kNoAllocLists;
-static_assert(sizeof(Inst1) <= kNoAllocHeader * sizeof(double), "descriptor does not fit the reserved header");
+constexpr size_t kNoAllocDoubles = (size_t)9 * kNoAllocMaxW + kNoAllocLists;
 
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles];
 
@@ -1829,14 +1894,14 @@ __global__ void __launch_bounds__(kNoAllocThreads, 1)
 {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ Work1 wk;
-    Inst1& I = *reinterpret_cast<Inst1*>(scratch);
-    if (threadIdx.x == 0) I = param;  // the descriptor is rewritten by every call
+    Inst1& I = wk.inst;
+    if (threadIdx.x == 0) I = param;
     __syncthreads();
     const int w = param.nx + 2 * kGhost;
-    double* qc = scratch + kNoAllocHeader;
+    double* qc = scratch;
     const Buffers1 g{q, qc, qc + 3 * w, qc + 6 * w, qc + 9 * w, nullptr, state, (int8_t*)(state + w)};
     if (I.t < I.t_end) {
-        step_inst(I, g, W, smem, smem_bytes, &wk, 1);
+        step_inst(g, W, smem, smem_bytes, &wk, 1);
     } else if (threadIdx.x == 0) {
         I.done = 1;
     }
