@@ -80,8 +80,6 @@ __host__ __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) &
 // The bits of a word outside the ghosted line are set in the mask planes: ComputeLevel reads a
 // mask as set there, and every other pass ands with the words' valid bits.
 enum Plane1 : int { kPlTemp = 4, kPlAux = 5, kPlStart = 6, kPlFine = 7, kPlLevel = 11 };
-// Behind the planes: the points 32 m of a mask, packed again (see close1).
-__host__ __device__ __forceinline__ int coarse_words1(int nw) { return (nw + 31) / 32 + 2; }
 // Slices of a level value: enough for 0..maxl and one more value, all ones, which stands for a level
 // outside that range (only set_levels can put one there; it rests in the bytes and is never used).
 __host__ __device__ __forceinline__ int level_bits(int maxl)
@@ -93,8 +91,7 @@ __host__ __device__ __forceinline__ int level_bits(int maxl)
 __host__ __device__ __forceinline__ int plane_words1(int nx) { return ((nx - 1 + kGhost + 32) >> 5) + 1; }
 __host__ __device__ __forceinline__ size_t plane_bytes1(int nx, int maxl)
 {
-    const size_t nw = (size_t)plane_words1(nx);
-    return align16(sizeof(uint32_t) * ((size_t)(kPlLevel + 4 * level_bits(maxl)) * nw + coarse_words1((int)nw)));
+    return align16(sizeof(uint32_t) * (size_t)(kPlLevel + 4 * level_bits(maxl)) * (size_t)plane_words1(nx));
 }
 // List space: two regions of 2 (w + 32) entries each (a stage's faces and points).
 __host__ __device__ __forceinline__ size_t list_entries1(int w) { return 2 * ((size_t)w + 32); }
@@ -152,7 +149,6 @@ struct Ctx {
     __device__ uint32_t* plane(int k) const { return pl + (size_t)k * nw; }
     __device__ uint32_t* mask(int k) const { return k == 0 ? m0 : plane(k); }
     __device__ uint32_t* fine(int k) const { return plane(kPlFine + k); }
-    __device__ uint32_t* coarse() const { return plane(kPlLevel + 4 * nb); }
     __device__ uint32_t* slice(int k, int b) const { return plane(kPlLevel + k * nb + b); }
     __device__ static bool bit(const uint32_t* P, int i) { return (P[(i >> 5) + 1] >> (i & 31)) & 1u; }
     __device__ int level(int k, int i) const
@@ -180,19 +176,6 @@ struct Ctx {
     {
         if (i < -kGhost || i > N1 + kGhost) return;
         atomicOr(&P[(i >> 5) + 1], 1u << (i & 31));
-    }
-    // The points of word x of a plane, shifted by +s and by -s, into P (all on the line).
-    __device__ void push_shifted(uint32_t* P, int x, uint32_t v, int s) const
-    {
-        const int o = s >> 5, b = s & 31;
-        const uint32_t up = v << b, dn = v >> b;
-        if (up) atomicOr(&P[x + o], up);
-        if (dn) atomicOr(&P[x - o], dn);
-        if (b) {
-            const uint32_t up1 = v >> (32 - b), dn1 = v << (32 - b);
-            if (up1) atomicOr(&P[x + o + 1], up1);
-            if (dn1) atomicOr(&P[x - o - 1], dn1);
-        }
     }
     // The region r list of n entries: in shared memory where it fits.
     __device__ List list(int r, size_t n) const
@@ -403,37 +386,61 @@ __device__ void build_stage_lists(const Ctx& c, int k, int region)
 }
 
 // ------------------------------------------------------------------ PrepareEuler building blocks
+// One phase of a transform over the entries [lo, hi) of an ordered list, on spacing D: the details of
+// one level (predict) or the coarser points (update), forward or inverse.  temp: the inverse predict
+// also interpolates momentum and energy of the points outside it.
+// The weights away from the ends, -1/16 and 9/16 (make_weights gives them exactly).
+constexpr double kInnerW0 = -0.0625, kInnerW1 = 0.5625;
+enum Lift1 { kPredictF, kUpdateF, kUpdateI, kPredictI };
+template <int OP>
+__device__ __forceinline__ void lift1(const Ctx& c, const List& L, unsigned lo, unsigned hi, int D,
+                                      const uint32_t* temp = nullptr)
+{
+    constexpr bool predict = OP == kPredictF || OP == kPredictI;
+    const double tol = c.I.tol;
+    for (unsigned e = lo + threadIdx.x; e < hi; e += blockDim.x) {
+        const int i = L.get(e);
+        if (!predict && (i == 0 || i == c.N1)) continue;
+        int s, k;
+        if (predict) predict_stencil(i, D, c.N1, s, k);
+        else update_stencil(i, D, c.N1, s, k);
+        double* q = c.q0 + kGhost;
+        double v = q[i], w[4] = {kInnerW0, kInnerW1, kInnerW1, kInnerW0};
+        if (k != 1)
+#pragma unroll
+            for (int n = 0; n < 4; ++n) w[n] = c.w_(n, k);
+        if (OP == kPredictI) v *= 2;
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const double y = w[n] * q[s + n * D];
+            v = OP == kPredictF || OP == kUpdateI ? v - y : v + y;
+        }
+        if (OP == kPredictF) v *= 0.5;
+        q[i] = v;
+        if (OP == kPredictF && absd(v) < tol) atomicAnd(&c.m0[(i >> 5) + 1], ~(1u << (i & 31)));
+        if (OP == kPredictI && temp && !Ctx::bit(temp, i)) {
+            const double *a = c.q1 + kGhost, *b = c.q2 + kGhost;
+            double y = 0, z = 0;
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                y += w[n] * a[s + n * D];
+                z += w[n] * b[s + n * D];
+            }
+            c.q1[i + kGhost] = y;
+            c.q2[i + kGhost] = z;
+        }
+    }
+}
+
 // ForwardWaveletTransformEuler (Wavelet/WAVELET_1D.h:282-335) over the points of mask0, listed by
 // order_points: level by level the details of the level, then the coarser points.
 __device__ void fwt1(const Ctx& c, const List& L)
 {
     const unsigned* off = c.wk->off;
-    double* q = c.q0;
-    const double tol = c.I.tol;
     for (int lev = c.maxl - 1; lev >= 0; --lev) {
-        const int D = c.D(lev);
-        for (unsigned e = off[lev + 1] + threadIdx.x; e < off[lev + 2]; e += blockDim.x) {
-            const int i = L.get(e);
-            int s, k;
-            predict_stencil(i, D, c.N1, s, k);
-            double v = q[i + kGhost];
-#pragma unroll
-            for (int cnt = 0; cnt < 4; ++cnt) v -= c.w_(cnt, k) * q[s + cnt * D + kGhost];
-            v *= 0.5;
-            q[i + kGhost] = v;
-            if (absd(v) < tol) atomicAnd(&c.m0[(i >> 5) + 1], ~(1u << (i & 31)));
-        }
+        lift1<kPredictF>(c, L, off[lev + 1], off[lev + 2], c.D(lev));
         __syncthreads();
-        for (unsigned e = threadIdx.x; e < off[lev + 1]; e += blockDim.x) {
-            const int i = L.get(e);
-            if (i == 0 || i == c.N1) continue;
-            int s, k;
-            update_stencil(i, D, c.N1, s, k);
-            double v = q[i + kGhost];
-#pragma unroll
-            for (int cnt = 0; cnt < 4; ++cnt) v += c.w_(cnt, k) * q[s + cnt * D + kGhost];
-            q[i + kGhost] = v;
-        }
+        lift1<kUpdateF>(c, L, 0, off[lev + 1], c.D(lev));
         __syncthreads();
     }
 }
@@ -452,151 +459,94 @@ __device__ void iwt_interp1(const Ctx& c, const List& L, bool interp)
 {
     const unsigned* off = c.wk->off;
     const uint32_t* temp = c.plane(kPlTemp);
-    double* q = c.q0;
     for (int lev = 0; lev < c.maxl; ++lev) {
+        const unsigned lo = off[lev + 1], hi = off[lev + 2];
         const int D = c.D(lev);
-        for (unsigned e = threadIdx.x; e < off[lev + 1]; e += blockDim.x) {
-            const int i = L.get(e);
-            if (i == 0 || i == c.N1) continue;
-            int s, k;
-            update_stencil(i, D, c.N1, s, k);
-            double v = q[i + kGhost];
-#pragma unroll
-            for (int cnt = 0; cnt < 4; ++cnt) v -= c.w_(cnt, k) * q[s + cnt * D + kGhost];
-            q[i + kGhost] = v;
-        }
+        lift1<kUpdateI>(c, L, 0, lo, D);
         __syncthreads();
-        for (unsigned e = off[lev + 1] + threadIdx.x; e < off[lev + 2]; e += blockDim.x) {
-            const int i = L.get(e);
-            int s, k;
-            predict_stencil(i, D, c.N1, s, k);
-            double v = q[i + kGhost];
-            v *= 2;
-#pragma unroll
-            for (int cnt = 0; cnt < 4; ++cnt) v += c.w_(cnt, k) * q[s + cnt * D + kGhost];
-            q[i + kGhost] = v;
-            if (interp && !Ctx::bit(temp, i)) {
-                double a = 0, b = 0;
-#pragma unroll
-                for (int cnt = 0; cnt < 4; ++cnt) {
-                    a += c.w_(cnt, k) * c.Q(1, s + cnt * D);
-                    b += c.w_(cnt, k) * c.Q(2, s + cnt * D);
-                }
-                c.Q(1, i) = a;
-                c.Q(2, i) = b;
-            }
-        }
+        lift1<kPredictI>(c, L, lo, hi, D, interp ? temp : nullptr);
         __syncthreads();
     }
 }
 
-// CheckReconstruction (Wavelet/AWCM_MANAGER_1D.h:45-71) marks the four coarse neighbours i -+ h, i -+ 3h of
-// every detail i of spacing h, fine to coarse; at the ends, where the stencil of the first detail
-// h is that of the next one (0, 2h, 4h, 6h) and that of the last one N1 - h that of N1 - 3h.
-//
-// close_word: word x of a mask (words ld(y), points 0..n1) after the levels of spacing 1 .. 2^(top-1),
-// top <= 5.  The word's outcome depends on at most 93 points around it, so a thread closes a window of
-// six words in registers, without a barrier between the levels.  A neighbour read after its own
-// closure only holds points that belong to the closure anyway, so words are closed in place.
-template <class Load>
-__device__ __forceinline__ uint32_t close_word(Load ld, int x, int n1, int top)
+// CheckReconstruction (Wavelet/AWCM_MANAGER_1D.h:45-71): every detail i of spacing h = 2^t in the
+// mask marks its four coarse neighbours i -+ h, i -+ 3h, fine to coarse.  At the ends the stencil of
+// the first detail h is that of the next one (0, 2h, 4h, 6h), and that of the last one N1 - h that of
+// N1 - 3h, so those two count twice.  A level up to h = 16 is a few shifts of each word and its
+// neighbours, and five levels reach at most 93 points: a warp holds 32 consecutive words, one per
+// lane, takes the neighbours by shuffles through all five levels without a barrier, and keeps the 26
+// words in the middle (three words of margin on either side).  A word that another warp has closed
+// already only holds points that belong to the closure anyway, so words are closed in place.
+// (One window of six words per thread took 2.7 us a mask of 1025 points with the coarse levels, a
+// block barrier per level the same.)  The levels above are bit 0 of their words: up to 128 details on
+// one warp, more on the whole block.
+__device__ __forceinline__ void close_words(const Ctx& c, uint32_t* P)
 {
-    uint32_t W[6], in[6];
-    uint32_t any = 0;
+    constexpr int kKeep = 26, kMargin = 3;
+    const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5, top = min(c.maxl, 5);
+    for (int x0 = 1 + (int)(threadIdx.x >> 5) * kKeep; x0 < c.nw; x0 += nwarp * kKeep) {
+        const int x = x0 - kMargin + lane;
+        const uint32_t in = x < c.nw ? c.inside(x) : 0u;
+        uint32_t v = in ? P[x] & in : 0u;
+        if (!__any_sync(0xffffffffu, v != 0)) continue;
+        const uint32_t was = v;
+        const int rl = c.N1 - 32 * (x - 1);  // bit of the last point, counted from this word
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const int r = n1 - 32 * (x - 4 + k);
-        in[k] = x - 3 + k < 1 || r < 0 ? 0u : r >= 31 ? ~0u : (2u << r) - 1u;
-        any |= W[k] = in[k] ? ld(x - 3 + k) & in[k] : 0u;
-    }
-    if (!any) return 0u;
-    const bool left = x <= 4, right = x + 2 >= (n1 >> 5) - 1;
-#pragma unroll
-    for (int t = 0; t < 5; ++t) {
-        if (t >= top) break;
-        const int h = 1 << t;
-        uint32_t d[8];
-        d[0] = d[7] = 0;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) d[k + 1] = W[k] & odd_bits(t);
-        if (left) {
-            // the detail h (word 1) also as 3h (the same word, for h = 16 the next one)
-#pragma unroll
-            for (int k = 0; k < 6; ++k)
-                if (x - 3 + k == 1) {
-                    const uint32_t b = d[k + 1] & (1u << h);
-                    if (t < 4) d[k + 1] |= b << ((2 * h) & 31);
-                    else if (k < 5) d[k + 2] |= b;
-                }
-        }
-        if (right) {
-            // the detail n1 - h also as n1 - 3h
-            const int a = n1 - h, b = n1 - 3 * h;
-            uint32_t on = 0;
-#pragma unroll
-            for (int k = 0; k < 6; ++k)
-                if (x - 3 + k == (a >> 5) + 1) on = (d[k + 1] >> (a & 31)) & 1u;
-#pragma unroll
-            for (int k = 0; k < 6; ++k)
-                if (x - 3 + k == (b >> 5) + 1) d[k + 1] |= on << (b & 31);
-        }
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            uint32_t o;
+        for (int t = 0; t < 5; ++t) {
+            if (t >= top) break;
+            const int h = 1 << t;
+            uint32_t d = v & odd_bits(t);
+            // the detail h (in word 1) also as 3h, for h = 16 in the next word
             if (t < 4) {
-                o = shl(d[k], d[k + 1], h) | shr(d[k + 1], d[k + 2], h) | shl(d[k], d[k + 1], 3 * h) |
-                    shr(d[k + 1], d[k + 2], 3 * h);
+                if (x == 1) d |= (d & (1u << h)) << (2 * h);
+            } else {
+                const uint32_t b = __shfl_up_sync(0xffffffffu, d, 1);
+                if (x == 2) d |= b;
+            }
+            // the detail N1 - h also as N1 - 3h, in the same word or the one below
+            {
+                const int s = rl - h;
+                const uint32_t e = s >= 0 && s < 32 ? d & (1u << s) : 0u;
+                const uint32_t f = __shfl_down_sync(0xffffffffu, e, 1);
+                d |= t < 4 ? shr(e, f, 2 * h) : f;
+            }
+            const uint32_t l = __shfl_up_sync(0xffffffffu, d, 1), r = __shfl_down_sync(0xffffffffu, d, 1);
+            if (t < 4) {
+                v |= (shl(l, d, h) | shr(d, r, h) | shl(l, d, 3 * h) | shr(d, r, 3 * h)) & in;
             } else {
                 // bit 16 of a word marks bit 0 of the words at 0, +1, +2 and -1
-                o = (d[k + 1] | d[k] | (k > 0 ? d[k - 1] : 0u) | d[k + 2]) >> 16;
+                const uint32_t ll = __shfl_up_sync(0xffffffffu, d, 2);
+                v |= ((l | d | r | ll) >> 16) & in;
             }
-            W[k] |= o & in[k];
         }
+        // (the shuffles' end lanes took their own words for their outer neighbours': margin only)
+        if (lane >= kMargin && lane < kMargin + kKeep && v != was) P[x] |= v;
     }
-    return W[3];
 }
-// The whole closure of plane P: the words of the five finest levels, then one warp packs the points
-// 32 m, closes them in the same way for the next five levels, and spreads the new ones back; levels
-// beyond those (lines of more than 4 2^10 points have few of them) go point by point.
+__device__ __forceinline__ void close_point(const Ctx& c, uint32_t* P, int t, int a)
+{
+    const int h = 1 << t, D = 2 * h, i = h + a * D;
+    if (!(P[(i >> 5) + 1] & 1u)) return;
+    int s, k;
+    predict_stencil(i, D, c.N1, s, k);
+#pragma unroll
+    for (int cnt = 0; cnt < 4; ++cnt) atomicOr(&P[((s + cnt * D) >> 5) + 1], 1u);
+}
 __device__ __forceinline__ void close1(const Ctx& c, uint32_t* P)
 {
-    const int top = min(c.maxl, 5);
-    for (int x = 1 + (int)threadIdx.x; x < c.nw; x += blockDim.x) {
-        const uint32_t own = close_word([&](int y) { return P[y]; }, x, c.N1, top);
-        if (own & ~P[x]) P[x] |= own;
-    }
+    close_words(c, P);
     __syncthreads();
-    if (c.maxl > 5) {
-        if (threadIdx.x < 32) {
-            const int lane = threadIdx.x, m1 = c.N1 >> 5, nc = (m1 >> 5) + 2;
-            uint32_t* C = c.coarse();
-            for (int y = 1; y < nc; ++y) {
-                const int m = 32 * (y - 1) + lane;
-                const uint32_t v = __ballot_sync(0xffffffffu, m <= m1 && (P[m + 1] & 1u));
-                if (lane == 0) C[y] = v;
-            }
-            __syncwarp();
-            for (int y0 = 1; y0 < nc; y0 += 32) {
-                const int y = y0 + lane;
-                const uint32_t was = y < nc ? C[y] : 0u;
-                const uint32_t own = y < nc ? close_word([&](int z) { return C[z]; }, y, m1, min(c.maxl - 5, 5)) : 0u;
-                for (uint32_t n = own & ~was; n; n &= n - 1) P[32 * (y - 1) + __ffs(n)] |= 1u;
-                if (y < nc) C[y] = was | own;
+    int t = 5;
+    for (; t < c.maxl && (c.N1 >> (t + 1)) > 128; ++t) {
+        for (int a = threadIdx.x; a < (c.N1 >> (t + 1)); a += blockDim.x) close_point(c, P, t, a);
+        __syncthreads();
+    }
+    if (t < c.maxl) {
+        if (threadIdx.x < 32)
+            for (; t < c.maxl; ++t) {
+                for (int a = threadIdx.x; a < (c.N1 >> (t + 1)); a += 32) close_point(c, P, t, a);
                 __syncwarp();
             }
-            for (int t = 10; t < c.maxl; ++t) {
-                const int h = 1 << t, D = 2 * h, nd = c.N1 / D;
-                for (int a = lane; a < nd; a += 32) {
-                    const int i = h + a * D;
-                    if (!(P[(i >> 5) + 1] & 1u)) continue;
-                    int s, k;
-                    predict_stencil(i, D, c.N1, s, k);
-#pragma unroll
-                    for (int cnt = 0; cnt < 4; ++cnt) atomicOr(&P[((s + cnt * D) >> 5) + 1], 1u);
-                }
-                __syncwarp();
-            }
-        }
         __syncthreads();
     }
 }
@@ -648,7 +598,7 @@ __device__ __forceinline__ uint32_t band_word(const Ctx& c, int x)
 // whose nearest neighbour in the mask is 2^j away get level maxl - j (the reference searches the
 // distances one by one; here each distance is one shift of the whole word).  Off the ghosted line
 // the mask reads as set.  A point without any such neighbour keeps its level.
-// rest(j, set): called for each of those points, with its level maxl - j.
+// f(j, set): called for those points with their levels maxl - j, and with `all` for every level's.
 __device__ __forceinline__ uint32_t end_bits(const Ctx& c, int x)
 {
     return (x == 1 ? 1u : 0u) | ((c.N1 >> 5) + 1 == x ? 1u << (c.N1 & 31) : 0u);
@@ -660,7 +610,7 @@ __device__ __forceinline__ uint32_t near_word(const Ctx& c, const uint32_t* M, i
     return c.padded(M, x - (1 << (j - 5))) | c.padded(M, x + (1 << (j - 5)));
 }
 template <class F>
-__device__ __forceinline__ void level_word(const Ctx& c, int k, const uint32_t* M, int x, F&& rest)
+__device__ __forceinline__ void level_word(const Ctx& c, int k, const uint32_t* M, int x, F&& f, bool all = false)
 {
     const uint32_t in = c.inside(x), ends = end_bits(c, x);  // the ends: the finest level, in the mask or not
     uint32_t todo = in ? M[x] & in & ~ends : 0u, fine = ends;
@@ -673,6 +623,7 @@ __device__ __forceinline__ void level_word(const Ctx& c, int k, const uint32_t* 
             const uint32_t got = todo & near_word(c, M, x, l, v, r, j);
             todo &= ~got;
             if (j == 0) fine |= got;
+            else if (all && got) f(j, got);
             const int lev = c.maxl - j;
 #pragma unroll
             for (int b = 0; b < 5; ++b)
@@ -690,10 +641,11 @@ __device__ __forceinline__ void level_word(const Ctx& c, int k, const uint32_t* 
                         lev |= 1 << b;
                         S[b] |= one;
                     }
-                if (lev != c.no_level()) rest(c.maxl - lev, one);
+                if (lev != c.no_level()) f(c.maxl - lev, one);
             }
         }
     }
+    if (all && in && (fine & M[x] & in)) f(0, fine & M[x] & in);
     c.fine(k)[x] = fine;
 #pragma unroll
     for (int b = 0; b < 5; ++b)
@@ -713,26 +665,52 @@ __device__ __forceinline__ void stencil_push(const Ctx& c, uint32_t* P, int x, i
         if (dn) atomicOr(&P[x - 1], dn);
         return;
     }
-    const int D = 1 << j;
-    const uint32_t left = set & c.upto(x, 2 * D), right = set & ~left & ~c.upto(x, c.N1 - 2 * D - 1);
-    const uint32_t mid = set & ~left & ~right;
-    if (left)
-        for (int n = 0; n < 6; ++n) c.push(P, n * D);
-    if (right)
-        for (int n = 0; n < 6; ++n) c.push(P, c.N1 - n * D);
-    if (mid) {
-        own |= mid;
-        c.push_shifted(P, x, mid, D);
-        c.push_shifted(P, x, mid, 2 * D);
+    const int D = 1 << j, i0 = 32 * (x - 1);
+    if (i0 <= 2 * D) {
+        const uint32_t left = set & c.upto(x, 2 * D);
+        if (left)
+            for (int n = 0; n < 6; ++n) c.push(P, n * D);
+        set &= ~left;
+    }
+    if (i0 + 31 >= c.N1 - 2 * D) {
+        const uint32_t right = set & ~c.upto(x, c.N1 - 2 * D - 1);
+        if (right)
+            for (int n = 0; n < 6; ++n) c.push(P, c.N1 - n * D);
+        set &= ~right;
+    }
+    if (!set) return;
+    own |= set;
+    if (j < 5) {
+        // within the word and its two neighbours (2 D = 32 is the whole word)
+        uint32_t up = set >> (32 - D), dn = set << (32 - D);
+        own |= (set << D) | (set >> D);
+        if (j < 4) {
+            own |= (set << (2 * D)) | (set >> (2 * D));
+            up |= set >> (32 - 2 * D);
+            dn |= set << (32 - 2 * D);
+        } else {
+            up |= set;
+            dn |= set;
+        }
+        if (up) atomicOr(&P[x + 1], up);
+        if (dn) atomicOr(&P[x - 1], dn);
+    } else {
+        const int o = D >> 5;
+        atomicOr(&P[x + o], set);
+        atomicOr(&P[x - o], set);
+        atomicOr(&P[x + 2 * o], set);
+        atomicOr(&P[x - 2 * o], set);
     }
 }
 
 // ComputeLevel(level_{k-1}, mask_{k-1}), mask_k = mask_{k-1}, AddAdjacentZone(mask_k) (zone) and
 // AddPointForDifferentiation(mask_k, level_{k-1}) in one phase.  All of them read mask_{k-1} only
 // (the zone's points are not in it, so their level is 0), and mask_k (clear before) takes ORs.
-// A warp takes 32 words and one job at a time -- the points of one distance, the zone, or the level
-// planes -- so that the searches of the levels run side by side: as one chain per word they took
-// 4.7 us of a 1025-point step's phase.
+// Lines of up to a few hundred points leave most warps idle at one word per thread.  There a warp takes
+// 32 words and one job at a time -- the points of one distance, the zone, or the level planes -- so that
+// the searches of the levels run side by side; each of them searches the nearer distances again, so
+// with more words a thread goes through its word's distances in turn.
+constexpr int kJobWords1 = 3;  // times 32 words
 __device__ void next_mask1(const Ctx& c, int k, bool zone)
 {
     const uint32_t* A = c.mask(k - 1);
@@ -740,6 +718,18 @@ __device__ void next_mask1(const Ctx& c, int k, bool zone)
     auto pts = [&](int y) { return c.points(A, y); };
     const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
     const int nch = (c.nw + 31) >> 5, njobs = (c.maxl + 3) * nch;
+    if (nch > kJobWords1) {
+        for (int x = threadIdx.x; x < c.nw; x += blockDim.x) {
+            const uint32_t a = A[x];
+            const uint32_t fresh = zone ? zone_word(c, x, pts) & ~a : 0u;
+            uint32_t own = a | fresh;
+            level_word(c, k - 1, A, x, [&](int j, uint32_t set) { stencil_push(c, B, x, j, set, own); }, true);
+            if (fresh) stencil_push(c, B, x, c.maxl, fresh, own);
+            if (own) atomicOr(&B[x], own);
+        }
+        __syncthreads();
+        return;
+    }
     for (int job = threadIdx.x >> 5; job < njobs; job += nwarp) {
         const int j = job / nch, x = 32 * (job - j * nch) + lane;
         if (x >= c.nw) continue;
