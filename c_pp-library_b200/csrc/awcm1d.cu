@@ -91,7 +91,8 @@ __host__ __device__ __forceinline__ int level_bits(int maxl)
 __host__ __device__ __forceinline__ int plane_words1(int nx) { return ((nx - 1 + kGhost + 32) >> 5) + 1; }
 __host__ __device__ __forceinline__ size_t plane_bytes1(int nx, int maxl)
 {
-    return align16(sizeof(uint32_t) * (size_t)(kPlLevel + 4 * level_bits(maxl)) * (size_t)plane_words1(nx));
+    // whole bank rows: the field follows in shared memory
+    return (sizeof(uint32_t) * (size_t)(kPlLevel + 4 * level_bits(maxl)) * (size_t)plane_words1(nx) + 127) & ~(size_t)127;
 }
 // List space: two regions of 2 (w + 32) entries each (a stage's faces and points).
 __host__ __device__ __forceinline__ size_t list_entries1(int w) { return 2 * ((size_t)w + 32); }
@@ -127,12 +128,27 @@ struct List {
     }
 };
 
+// Place of ghosted point x of a conserved plane in shared memory (mask m = 15; 0 in global memory: x
+// itself).  The points of a level are a power of two apart, so in a linear plane the 32 lanes of a
+// warp meet in one or a few of the 16 double-wide banks: every access of a level of spacing 16 or
+// more took 32 turns.  Exchanging the 16 places of a bank row by the higher bits of x spreads any
+// power-of-two stride over all banks.
+__device__ __forceinline__ int place(int x, int m) { return x ^ (((x >> 4) ^ (x >> 8) ^ (x >> 12)) & m); }
+struct Field1 {
+    double *q0, *q1, *q2;  // conserved planes
+    int m0, m12;           // place() masks of q0 and of q1, q2
+    __device__ __forceinline__ double& at(int p, int i) const
+    {
+        return p == 0 ? q0[place(i + kGhost, m0)] : (p == 1 ? q1 : q2)[place(i + kGhost, m12)];
+    }
+};
+
 // Views of one instance for a step or a pass.  Pointers are generic: in the step kernel the bit
 // planes, the conserved planes and more point into the CTA's shared memory (staged in and out around
 // the steps, see Layout1), elsewhere into the instance's global buffers.
 struct Ctx {
     const Inst1& I;
-    double *q0, *q1, *q2;   // conserved planes: q0[i + 3]
+    Field1 f;               // conserved planes
     double *qc, *qt, *fl;   // stage-start copy, coarse derivatives, face fluxes: x[p*w + i + 3]
     uint32_t* pl;           // bit planes
     uint32_t *m0, *aux;     // planes of mask0 and of the first work plane (they change places)
@@ -143,7 +159,7 @@ struct Ctx {
     const Weights& W;
     int w, nx, N1, maxl, nb, nw;
 
-    __device__ double& Q(int p, int i) const { return (p == 0 ? q0 : p == 1 ? q1 : q2)[i + kGhost]; }
+    __device__ double& Q(int p, int i) const { return f.at(p, i); }
     __device__ double& QT(int p, int i) const { return qt[p * w + i + kGhost]; }
     __device__ double& QC(int p, int i) const { return qc[p * w + i + kGhost]; }
     __device__ uint32_t* plane(int k) const { return pl + (size_t)k * nw; }
@@ -404,30 +420,28 @@ __device__ __forceinline__ void lift1(const Ctx& c, const List& L, unsigned lo, 
         int s, k;
         if (predict) predict_stencil(i, D, c.N1, s, k);
         else update_stencil(i, D, c.N1, s, k);
-        double* q = c.q0 + kGhost;
-        double v = q[i], w[4] = {kInnerW0, kInnerW1, kInnerW1, kInnerW0};
+        double v = c.Q(0, i), w[4] = {kInnerW0, kInnerW1, kInnerW1, kInnerW0};
         if (k != 1)
 #pragma unroll
             for (int n = 0; n < 4; ++n) w[n] = c.w_(n, k);
         if (OP == kPredictI) v *= 2;
 #pragma unroll
         for (int n = 0; n < 4; ++n) {
-            const double y = w[n] * q[s + n * D];
+            const double y = w[n] * c.Q(0, s + n * D);
             v = OP == kPredictF || OP == kUpdateI ? v - y : v + y;
         }
         if (OP == kPredictF) v *= 0.5;
-        q[i] = v;
+        c.Q(0, i) = v;
         if (OP == kPredictF && absd(v) < tol) atomicAnd(&c.m0[(i >> 5) + 1], ~(1u << (i & 31)));
         if (OP == kPredictI && temp && !Ctx::bit(temp, i)) {
-            const double *a = c.q1 + kGhost, *b = c.q2 + kGhost;
             double y = 0, z = 0;
 #pragma unroll
             for (int n = 0; n < 4; ++n) {
-                y += w[n] * a[s + n * D];
-                z += w[n] * b[s + n * D];
+                y += w[n] * c.Q(1, s + n * D);
+                z += w[n] * c.Q(2, s + n * D);
             }
-            c.q1[i + kGhost] = y;
-            c.q2[i + kGhost] = z;
+            c.Q(1, i) = y;
+            c.Q(2, i) = z;
         }
     }
 }
@@ -872,12 +886,11 @@ __device__ __forceinline__ double speed1(double q0, double q1, double q2, double
 // driver's branch selection (main_1d_euler.cpp:111-133); right-boundary forms mirror the left ones.
 // Reads the stage input Q, which no point update has touched yet when it runs.
 template <class DV>
-__device__ __forceinline__ void coarse_dF1(DV& dv, const double* q0, const double* q1, const double* q2, int iend, int i,
-                                           int d, double* dF)
+__device__ __forceinline__ void coarse_dF1(DV& dv, const Field1& q, int iend, int i, int d, double* dF)
 {
     const double g = 1.4;  // EULER_EQUATION_1D euler_eqn(1.4) in the reference helpers
     auto F = [&](int ii, double* f) {
-        const double s[3] = {q0[ii + kGhost], q1[ii + kGhost], q2[ii + kGhost]};
+        const double s[3] = {q.at(0, ii), q.at(1, ii), q.at(2, ii)};
         flux1(dv, s, g, f);
     };
     double a[3], b[3], e[3], f[3], h[3];
@@ -900,35 +913,31 @@ __device__ __forceinline__ void coarse_dF1(DV& dv, const double* q0, const doubl
 }
 
 // A coarse point or a face whose operands are outside the range of SharedDiv, with IEEE divisions.
-__device__ __noinline__ void coarse_any1(const double* q0, const double* q1, const double* q2, int N1, int i, int d,
-                                         double* out, int w)
+__device__ __noinline__ void coarse_any1(Field1 q, int N1, int i, int d, double* out, int w)
 {
     IeeeDiv dv;
     double dF[3];
-    coarse_dF1(dv, q0, q1, q2, N1, i, d, dF);
+    coarse_dF1(dv, q, N1, i, d, dF);
     for (int k = 0; k < 3; ++k) out[k * w] = dF[k];
 }
 template <class DV>
-__device__ __forceinline__ void face1(DV& dv, const double* q0, const double* q1, const double* q2, int f, int scheme,
-                                      double alpha, double gamma, double* out, int w)
+__device__ __forceinline__ void face1(DV& dv, const Field1& q, int f, int scheme, double alpha, double gamma, double* out,
+                                      int w)
 {
     double s[6][3], o[3];
 #pragma unroll
-    for (int p = 0; p < 6; ++p) {
-        s[p][0] = q0[f - 2 + p + kGhost];
-        s[p][1] = q1[f - 2 + p + kGhost];
-        s[p][2] = q2[f - 2 + p + kGhost];
-    }
+    for (int p = 0; p < 6; ++p)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s[p][k] = q.at(k, f - 2 + p);
     if (scheme == kWeno5) face_flux_1d<kWeno5>(dv, s, alpha, gamma, o);
     else face_flux_1d<kWenoZ>(dv, s, alpha, gamma, o);
 #pragma unroll
     for (int k = 0; k < 3; ++k) out[k * w] = o[k];
 }
-__device__ __noinline__ void face_any1(const double* q0, const double* q1, const double* q2, int f, int scheme,
-                                       double alpha, double gamma, double* out, int w)
+__device__ __noinline__ void face_any1(Field1 q, int f, int scheme, double alpha, double gamma, double* out, int w)
 {
     IeeeDiv dv;
-    face1(dv, q0, q1, q2, f, scheme, alpha, gamma, out, w);
+    face1(dv, q, f, scheme, alpha, gamma, out, w);
 }
 
 // Spacing of the coarse point i in level set k, or 0: a level outside 0..maxl or a derivative
@@ -959,17 +968,17 @@ __device__ __forceinline__ void stage1(const Ctx& c, int scheme, int kind, doubl
         if (e < L.nf) {
             const int f = L.faces.get(e);
             SharedDiv dv;
-            face1(dv, c.q0, c.q1, c.q2, f, scheme, alpha, c.I.gamma, c.fl + f + kGhost, c.w);
-            if (dv.bad) face_any1(c.q0, c.q1, c.q2, f, scheme, alpha, c.I.gamma, c.fl + f + kGhost, c.w);
+            face1(dv, c.f, f, scheme, alpha, c.I.gamma, c.fl + f + kGhost, c.w);
+            if (dv.bad) face_any1(c.f, f, scheme, alpha, c.I.gamma, c.fl + f + kGhost, c.w);
         } else {
             const int i = L.crs.get(e - L.nf), d = coarse_spacing(c, k, i);
             if (!d) continue;
             SharedDiv dv;
             double dF[3];
-            coarse_dF1(dv, c.q0, c.q1, c.q2, c.N1, i, d, dF);
+            coarse_dF1(dv, c.f, c.N1, i, d, dF);
 #pragma unroll
             for (int q = 0; q < 3; ++q) c.QT(q, i) = dF[q];
-            if (dv.bad) coarse_any1(c.q0, c.q1, c.q2, c.N1, i, d, c.qt + i + kGhost, c.w);
+            if (dv.bad) coarse_any1(c.f, c.N1, i, d, c.qt + i + kGhost, c.w);
         }
     }
     __syncthreads();
@@ -1122,9 +1131,9 @@ __device__ __forceinline__ void stages1(Inst1& I, const Ctx& c, const List& L3, 
 // no scalar overload of AWCM_1D (the driver does not compile as shipped); they take the 5-point
 // form of the vector counterpart, DifferentiateEulerAtLeftBoundary (AWCM_1D.h:174-185), with the
 // identity flux of unit-speed advection.
-__device__ double coarse_d1_scalar(const Ctx& c, const double* in, int i, int d)
+__device__ double coarse_d1_scalar(const Ctx& c, const double* in, int m, int i, int d)
 {
-    auto Q = [&](int ii) { return in[ii + kGhost]; };
+    auto Q = [&](int ii) { return in[place(ii + kGhost, m)]; };
     const int iend = c.N1;
     if (i - 2 * d > 0 && i + 2 * d < iend) return kD1 * (Q(i + d) - Q(i - d)) + kD2 * (Q(i + 2 * d) - Q(i - 2 * d));
     if (i - 2 * d < 0) return kD1 * (Q(i + d) - Q(i - d)) + kD2 * (Q(i + 2 * d) - Q(i - d));
@@ -1141,32 +1150,31 @@ __device__ double coarse_d1_scalar(const Ctx& c, const double* in, int i, int d)
 // (dx dx_) dF below it, with the end points copied into the ghosts.  Only the points of the mask
 // and the ghosts are written: the next stage's stencils lie in this stage's mask.
 // Kind 2 then combines q_1 = 3/4 q + 1/4 q_1 (after q_1's ghost copies), kind 3 q = 1/3 q + 2/3 q_0.
-__device__ __forceinline__ void stage1_scalar(const Ctx& c, int kind, const double* in, double* out, double dt)
+__device__ __forceinline__ void stage1_scalar(const Ctx& c, int kind, const double* in, int m, double* out, double dt)
 {
+    auto In = [&](int i) { return in[place(i + kGhost, m)]; };
     const int k = 3 - kind, region = kind == 2 ? 0 : 1;
     const StageLists L = stage_lists(c, k, region);
     if (kind < 3) build_stage_lists(c, k - 1, 1 - region);
     for (int e = threadIdx.x; e < L.nf; e += blockDim.x) {
         const int f = L.faces.get(e);
-        const double* v = in + f + kGhost;
-        c.fl[f + kGhost] = recon_left<kWeno5>(v[2], v[1], v[0], v[-1], v[-2]);
+        c.fl[f + kGhost] = recon_left<kWeno5>(In(f + 2), In(f + 1), In(f), In(f - 1), In(f - 2));
     }
     __syncthreads();
-    double* q = c.q0;
     for (int e = threadIdx.x; e < L.nfin + L.ncrs; e += blockDim.x) {
         const int i = e < L.nfin ? L.fin.get(e) : L.crs.get(e - L.nfin);
-        double r = in[i + kGhost];
+        double r = In(i);
         if (e < L.nfin) {
             r = r - dt * (c.fl[i + kGhost] - c.fl[i - 1 + kGhost]) / (c.I.dx * 1);
         } else {
             const int d = coarse_spacing(c, k, i);
-            if (d) r = r - dt / (c.I.dx * d) * coarse_d1_scalar(c, in, i, d);
+            if (d) r = r - dt / (c.I.dx * d) * coarse_d1_scalar(c, in, m, i, d);
         }
         if (kind < 3 && (i == 0 || i == c.N1))
             for (int g = 1; g <= kGhost; ++g) out[(i == 0 ? -g : c.N1 + g) + kGhost] = r;
         if (kind == 1) out[i + kGhost] = r;
-        else if (kind == 2) out[i + kGhost] = 0.75 * q[i + kGhost] + 0.25 * r;
-        else q[i + kGhost] = kC1_3 * q[i + kGhost] + kD1 * r;
+        else if (kind == 2) out[i + kGhost] = 0.75 * c.Q(0, i) + 0.25 * r;
+        else c.Q(0, i) = kC1_3 * c.Q(0, i) + kD1 * r;
     }
     __syncthreads();
 }
@@ -1184,7 +1192,7 @@ __device__ __forceinline__ void stages1_scalar(Inst1& I, const Ctx& c, bool dens
     double* s1 = c.qc + c.w;
 #pragma unroll 1
     for (int kind = 1; kind <= 3; ++kind)
-        stage1_scalar(c, kind, kind == 1 ? c.q0 : kind == 2 ? s2 : s1, kind == 1 ? s2 : s1, dt);
+        stage1_scalar(c, kind, kind == 1 ? c.f.q0 : kind == 2 ? s2 : s1, kind == 1 ? c.f.m0 : 0, kind == 1 ? s2 : s1, dt);
     remove_residue1(c, c.plane(kPlStart), 1, dense);
     if (threadIdx.x == 0) {
         I.dt = dt;
@@ -1215,12 +1223,16 @@ struct Layout1 {
     unsigned cap;   // list entries per region
     size_t bytes;   // shared memory it takes
 };
-__host__ __device__ __forceinline__ size_t tier_doubles(int tier, bool scalar)
+// Planes of the field are whole bank rows (16 doubles), see place().
+constexpr int kPlaceMask = 15;
+__host__ __device__ __forceinline__ int row_doubles(int w) { return (w + 15) & ~15; }
+__host__ __device__ __forceinline__ size_t tier_doubles(int tier, bool scalar, int w)
 {
+    const size_t ws = (size_t)row_doubles(w);
     switch (tier) {
-        case kInAll: return scalar ? 4 : 12;
-        case kInField: return scalar ? 1 : 3;
-        case kInDensity: return 1;
+        case kInAll: return scalar ? ws + 3 * (size_t)w : 3 * ws + 9 * (size_t)w;
+        case kInField: return scalar ? ws : 3 * ws;
+        case kInDensity: return ws;
         default: return 0;
     }
 }
@@ -1230,7 +1242,7 @@ __host__ __device__ __forceinline__ Layout1 pick_layout(int nx, int maxl, size_t
     const size_t full = list_entries1(w), eb = 2 * entry_bytes(w), np = plane_bytes1(nx, maxl);
     const size_t least = full < 512 ? full : 512;
     for (int tier = kInAll; tier >= kInNone; --tier) {
-        const size_t fixed = tier == kInNone ? 0 : np + align16(sizeof(double) * tier_doubles(tier, scalar) * (size_t)w);
+        const size_t fixed = tier == kInNone ? 0 : np + align16(sizeof(double) * tier_doubles(tier, scalar, w));
         if (tier != kInNone && fixed + eb * least > avail) continue;
         size_t cap = (avail - fixed) / eb;
         cap = cap < full ? cap : full;
@@ -1238,19 +1250,6 @@ __host__ __device__ __forceinline__ Layout1 pick_layout(int nx, int maxl, size_t
         return Layout1{tier, (unsigned)cap, fixed + eb * cap};
     }
     return Layout1{kInNone, 0, 0};
-}
-
-// Copy of n doubles by all threads of the block; 16-byte words where both ends allow it.
-__device__ __forceinline__ void block_copy_doubles(double* __restrict__ dst, const double* __restrict__ src, int n)
-{
-    int head = 0;
-    if ((((uintptr_t)dst | (uintptr_t)src) & 15) == 0) {
-        const int nv = n >> 1;
-        for (int t = threadIdx.x; t < nv; t += blockDim.x)
-            reinterpret_cast<double2*>(dst)[t] = reinterpret_cast<const double2*>(src)[t];
-        head = nv << 1;
-    }
-    for (int t = head + threadIdx.x; t < n; t += blockDim.x) dst[t] = src[t];
 }
 
 // The global buffers of one instance.
@@ -1266,7 +1265,7 @@ __device__ __forceinline__ Ctx make_ctx(const Inst1& I, const Buffers1& g, Work1
     const int w = I.nx + 2 * kGhost;
     uint32_t* pl = g.planes;
     const int nw = plane_words1(I.nx);
-    return Ctx{I, g.q, g.q + w, g.q + 2 * w, g.qc, g.qt, g.fl, pl, pl, pl + (size_t)kPlAux * nw, nullptr,
+    return Ctx{I, Field1{g.q, g.q + w, g.q + 2 * w, 0, 0}, g.qc, g.qt, g.fl, pl, pl, pl + (size_t)kPlAux * nw, nullptr,
                static_cast<uint8_t*>(g.lists), 0, wk, W, w, I.nx, I.nx - 1, I.maxl, level_bits(I.maxl), nw};
 }
 
@@ -1286,14 +1285,12 @@ __device__ void step_inst(const Buffers1& g, const Weights& W, uint8_t* smem, si
         c.aux = c.plane(kPlAux);
         p += plane_bytes1(I.nx, I.maxl);
         double* d = reinterpret_cast<double*>(p);
-        p += align16(sizeof(double) * tier_doubles(lay.tier, scalar) * (size_t)w);
-        const int np = lay.tier < kInDensity ? 0 : lay.tier == kInDensity || scalar ? 1 : 3;
-        if (np) block_copy_doubles(c.q0 = d, g.q, w);
-        if (np == 3) {
-            block_copy_doubles(c.q1 = d + w, g.q + w, w);
-            block_copy_doubles(c.q2 = d + 2 * w, g.q + 2 * w, w);
-        }
-        d += np * w;
+        p += align16(sizeof(double) * tier_doubles(lay.tier, scalar, w));
+        const int np = lay.tier < kInDensity ? 0 : lay.tier == kInDensity || scalar ? 1 : 3, ws = row_doubles(w);
+        for (int t = threadIdx.x; t < np * w; t += blockDim.x) d[t / w * ws + place(t % w, kPlaceMask)] = g.q[t];
+        if (np) c.f.q0 = d, c.f.m0 = kPlaceMask;
+        if (np == 3) c.f.q1 = d + ws, c.f.q2 = d + 2 * ws, c.f.m12 = kPlaceMask;
+        d += np * ws;
         if (lay.tier == kInAll) {
             c.qc = d;
             d += (scalar ? 2 : 3) * w;
@@ -1325,9 +1322,13 @@ __device__ void step_inst(const Buffers1& g, const Weights& W, uint8_t* smem, si
         dense = false;
     }
     store_planes(c, g.mask, g.level);
-    if (c.q0 != g.q) block_copy_doubles(g.q, c.q0, w);
-    if (c.q1 != g.q + w) block_copy_doubles(g.q + w, c.q1, w);
-    if (c.q2 != g.q + 2 * w) block_copy_doubles(g.q + 2 * w, c.q2, w);
+    for (int t = threadIdx.x; t < w; t += blockDim.x) {
+        if (c.f.m0) g.q[t] = c.f.q0[place(t, kPlaceMask)];
+        if (c.f.m12) {
+            g.q[w + t] = c.f.q1[place(t, kPlaceMask)];
+            g.q[2 * w + t] = c.f.q2[place(t, kPlaceMask)];
+        }
+    }
     __syncthreads();
 }
 
@@ -1361,7 +1362,7 @@ __device__ __forceinline__ Buffers1 pool_buffers(const Inst1& I, const Pool& P)
 __global__ void __launch_bounds__(kMaxThreads1, 1) k_step1d(Inst1* insts, int n, const int* __restrict__ order, unsigned* queue, Pool P,
                          unsigned smem_bytes, int nsteps)
 {
-    extern __shared__ __align__(16) uint8_t smem[];
+    extern __shared__ __align__(128) uint8_t smem[];
     __shared__ Work1 wk;
     __shared__ int cur;
     for (;;) {
@@ -1882,7 +1883,7 @@ namespace {
 __global__ void __launch_bounds__(kNoAllocThreads, 1)
     k_step1d_noalloc(Inst1 param, double* q, uint8_t* state, double* scratch, double* out, Weights W, unsigned smem_bytes)
 {
-    extern __shared__ __align__(16) uint8_t smem[];
+    extern __shared__ __align__(128) uint8_t smem[];
     __shared__ Work1 wk;
     Inst1& I = wk.inst;
     if (threadIdx.x == 0) I = param;
