@@ -594,8 +594,9 @@ __device__ __forceinline__ void interp_point(const Grid2& g, Field4 q, int i, in
         if (p >= p0) q.p[p][a] = out[p];
 }
 
+// work: the bit of the work mask (kBitInterp), or mask3 itself (see enq_interp_new).
 template <int PH>
-__device__ void ph_interp(const Grid2& g, Field4 q, const uint8_t* __restrict__ m, int lev, int from_bit, int p0,
+__device__ void ph_interp(const Grid2& g, Field4 q, const uint8_t* __restrict__ m, int lev, int work, int from_bit, int p0,
                           Span sp)
 {
     const int D = g.D(lev);
@@ -611,7 +612,7 @@ __device__ void ph_interp(const Grid2& g, Field4 q, const uint8_t* __restrict__ 
         }
         const size_t a = g.at(i, j);
         const unsigned mb = m[a];
-        if (!((mb >> kBitInterp) & 1u) || ((mb >> from_bit) & 1u)) continue;
+        if (!((mb >> work) & 1u) || ((mb >> from_bit) & 1u)) continue;
         interp_point(g, q, i, j, a, D, w, p0);
     }
 }
@@ -619,8 +620,8 @@ __device__ void ph_interp(const Grid2& g, Field4 q, const uint8_t* __restrict__ 
 // Row-scan form of ph_interp for the fine levels: PH 0 scans every row of the level (d1 on the
 // even ones, d2 on the odd ones), PH 1 only the odd rows (d3).
 template <int PH>
-__device__ void ph_interp_rows(const Grid2& g, Field4 q, const uint8_t* __restrict__ m, int lev, int from_bit, int p0,
-                               Span sp)
+__device__ void ph_interp_rows(const Grid2& g, Field4 q, const uint8_t* __restrict__ m, int lev, int work, int from_bit,
+                               int p0, Span sp)
 {
     const int D = g.D(lev), h = D >> 1;
     const int rows = PH == 0 ? 2 : 1;
@@ -629,12 +630,12 @@ __device__ void ph_interp_rows(const Grid2& g, Field4 q, const uint8_t* __restri
     const unsigned row0 = (unsigned)kGhost * ((unsigned)g.pitch / 4u);
     for (unsigned t = sp.t0; t < n; t += sp.stride) {
         // every row of the finest detail level (h = 1, PH 0): word t of the grid rows
-        if (PH == 0 && h == 1 && !((mp[row0 + t] >> kBitInterp) & kLaneBits)) continue;
+        if (PH == 0 && h == 1 && !((mp[row0 + t] >> work) & ~(mp[row0 + t] >> from_bit) & kLaneBits)) continue;
         int j, i0;
         unsigned wdx;
         const unsigned lanes = rowscan_word(g, lev, rows, t, j, i0, wdx);
         const unsigned v = mp[wdx];
-        unsigned hit = (v >> kBitInterp) & ~(v >> from_bit) & lane_bits(lanes);
+        unsigned hit = (v >> work) & ~(v >> from_bit) & lane_bits(lanes);
         while (hit) {
             const int L = (__ffs(hit) - 1) >> 3;
             hit &= hit - 1;
@@ -647,16 +648,14 @@ __device__ void ph_interp_rows(const Grid2& g, Field4 q, const uint8_t* __restri
 }
 
 // ------------------------------------------------------------------------------- dense mask passes
-// Bits 1..3 (mask1..mask3) of the four bytes of a mask word.
-constexpr unsigned kMask123 = (kLaneBits << 1) | (kLaneBits << 2) | (kLaneBits << 3);
-// Copies bit `from` into bit `to` on every byte; `clear` (lane-replicated bits) is cleared too.
-__device__ void ph_copy_bit_all(uint8_t* m, size_t n, int from, int to, Span sp, unsigned clear = 0)
+// Copies bit `from` into bit `to` on every byte.
+__device__ void ph_copy_bit_all(uint8_t* m, size_t n, int from, int to, Span sp)
 {
     unsigned* mw = reinterpret_cast<unsigned*>(m);
     const unsigned nw = (unsigned)(n / 4);
     for (unsigned w = sp.t0; w < nw; w += sp.stride) {
         const unsigned v = mw[w];
-        const unsigned nv = ((v & ~(kLaneBits << to)) | (((v >> from) & kLaneBits) << to)) & ~clear;
+        const unsigned nv = (v & ~(kLaneBits << to)) | (((v >> from) & kLaneBits) << to);
         if (nv != v) mw[w] = nv;
     }
 }
@@ -824,80 +823,6 @@ __device__ void ph_apd(const Grid2& g, uint8_t* m, const int8_t* lvl, int bit, i
     }
 }
 
-// ComputeLevel of mask k-1 into lvl, mask_k = mask_{k-1} and AddPointForDifferentiation(mask_k,
-// level_{k-1}) in one pass, for bit k cleared beforehand on every byte: the copy and the pushes
-// both only set bit k (atomic ORs), nothing in the pass reads bit k, bit k-1 does not change,
-// and each point's level is computed by the thread that then reads it.  The same results as
-// ph_cl followed by ph_apd.
-__device__ void ph_cl_apd(const Grid2& g, uint8_t* m, int8_t* lvl, int k, size_t plane, Span sp)
-{
-    const int NX = g.nx - 1, NY = g.ny - 1;
-    const int src = k - 1;
-    unsigned* mp = reinterpret_cast<unsigned*>(m);
-    unsigned* lp = reinterpret_cast<unsigned*>(lvl);
-    const unsigned nw = (unsigned)(plane / 4);
-    for (unsigned w = sp.t0; w < nw; w += sp.stride) {
-        const unsigned v = mp[w];
-        // most words hold no point of mask k-1 and no non-zero level: nothing to write or push
-        if (!((v >> src) & kLaneBits) && !lp[w]) continue;
-        const MaskWord mw = mask_word(g, w);
-        const unsigned G = grid_lanes(g, mw);
-        unsigned lv = 0;
-        if (G) {
-            const unsigned lv0 = lp[w];
-            lv = lv0;
-            const unsigned on = (v >> src) & kLaneBits;
-#pragma unroll
-            for (int L = 0; L < 4; ++L) {
-                if (!((G >> L) & 1u)) continue;
-                const unsigned sh = 8u * L;
-                if (!((on >> sh) & 1u)) {
-                    lv &= ~(0xffu << sh);
-                    continue;
-                }
-                const int i = mw.i0 + L, j = mw.j;
-                int dx = 1;
-                for (int lev = g.maxl; lev >= 0; --lev) {
-                    if (mask_or_ghost(g, m, i - dx, j, src) || mask_or_ghost(g, m, i + dx, j, src) ||
-                        mask_or_ghost(g, m, i, j - dx, src) || mask_or_ghost(g, m, i, j + dx, src)) {
-                        lv = (lv & ~(0xffu << sh)) | ((unsigned)(uint8_t)(int8_t)lev << sh);
-                        break;
-                    }
-                    dx *= 2;
-                }
-            }
-            if (lv != lv0) lp[w] = lv;
-        }
-        const unsigned cp = ((v >> src) & kLaneBits) << k;
-        if (cp) atomicOr(&mp[w], cp);
-        if (mw.j < 1 || mw.j > NY - 1) continue;
-        const unsigned I = lanes_in(mw.i0, 1, NX - 1);
-        unsigned hit = (v >> src) & lane_bits(I);
-        while (hit) {
-            const int L = (__ffs(hit) - 1) >> 3;
-            hit &= hit - 1;
-            const int i = mw.i0 + L, j = mw.j;
-            const int lev = (int)(int8_t)(uint8_t)(lv >> (8 * L));
-            if (lev == g.maxl) {
-                // i, j in [1, N-1]: the cross i-3..i+3, j-3..j+3 lies on the ghosted plane
-                push_run(g, m, i - 3, 7, 1, j, k);
-                for (int c = -3; c <= 3; ++c)
-                    if (c) push_bit_in(g, m, i, j + c, k);
-                continue;
-            }
-            const int D = g.D(lev);
-            int lo = -2, hi = 2;
-            if (i - 2 * D < 0) lo = -1;
-            else if (i + 2 * D > NX) hi = 1;
-            for (int c = lo; c <= hi; ++c) push_bit(g, m, i + D * c, j, k);
-            lo = -2, hi = 2;
-            if (j - 2 * D < 0) lo = -1;
-            else if (j + 2 * D > NY) hi = 1;
-            for (int c = lo; c <= hi; ++c) push_bit(g, m, i, j + D * c, k);
-        }
-    }
-}
-
 // Work mask of InterpolateEuler: `to` minus `from` over the grid points (ghost bits untouched);
 // to < 0 stands for every grid point (InterpolateAllGridEuler).
 __device__ void ph_interp_init(const Grid2& g, uint8_t* m, int from, int to, Span sp)
@@ -986,25 +911,25 @@ __global__ void k_cr_rows(Grid2 g, uint8_t* m, int lev, int bit, const StepState
     ph_cr_rows(g, m, lev, bit, grid_span());
 }
 template <int PH>
-__global__ void k_interp(Grid2 g, Field4 q, const uint8_t* m, int lev, int from_bit, int p0, const StepState* st)
+__global__ void k_interp(Grid2 g, Field4 q, const uint8_t* m, int lev, int work, int from_bit, int p0, const StepState* st)
 {
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
-    ph_interp<PH>(g, q, m, lev, from_bit, p0, grid_span());
+    ph_interp<PH>(g, q, m, lev, work, from_bit, p0, grid_span());
 }
 template <int PH>
-__global__ void k_interp_rows(Grid2 g, Field4 q, const uint8_t* m, int lev, int from_bit, int p0,
+__global__ void k_interp_rows(Grid2 g, Field4 q, const uint8_t* m, int lev, int work, int from_bit, int p0,
                               const StepState* st)
 {
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
-    ph_interp_rows<PH>(g, q, m, lev, from_bit, p0, grid_span());
+    ph_interp_rows<PH>(g, q, m, lev, work, from_bit, p0, grid_span());
 }
-__global__ void k_copy_bit_all(uint8_t* m, size_t n, int from, int to, const StepState* st, unsigned clear)
+__global__ void k_copy_bit_all(uint8_t* m, size_t n, int from, int to, const StepState* st)
 {
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
-    ph_copy_bit_all(m, n, from, to, grid_span(), clear);
+    ph_copy_bit_all(m, n, from, to, grid_span());
 }
 __global__ void k_band_copy(Grid2 g, uint8_t* m, int bit, int copy_to, const StepState* st)
 {
@@ -1030,25 +955,6 @@ __global__ void k_apd(Grid2 g, uint8_t* m, const int8_t* lvl, int bit, int src, 
     AWCM_SKIP_IF_DONE(st);
     ph_apd(g, m, lvl, bit, src, grid_span());
 }
-__global__ void k_cl_apd(Grid2 g, uint8_t* m, int8_t* lvl, int k, size_t plane, const StepState* st)
-{
-    pdl_begin();
-    AWCM_SKIP_IF_DONE(st);
-    ph_cl_apd(g, m, lvl, k, plane, grid_span());
-}
-// The coarsest level's first inverse-transform phase (CTAs [0, nb)) and the interpolation work mask
-// `to` minus `from` (the other CTAs) in one launch: the mask pass rewrites only the work bit.
-__global__ void k_iwt0_interp_init(Grid2 g, double* q, uint8_t* m, int lev, int to, int from, int sparse,
-                                   const StepState* st, unsigned nb)
-{
-    pdl_begin();
-    AWCM_SKIP_IF_DONE(st);
-    if (blockIdx.x < nb)
-        ph_iwt<0>(g, q, m, lev, to, !sparse || !st || st->full_zero,
-                  Span{blockIdx.x * blockDim.x + threadIdx.x, nb * blockDim.x});
-    else
-        ph_interp_init(g, m, from, to, Span{(blockIdx.x - nb) * blockDim.x + threadIdx.x, (gridDim.x - nb) * blockDim.x});
-}
 __global__ void k_interp_init(Grid2 g, uint8_t* m, int from, int to, const StepState* st)
 {
     pdl_begin();
@@ -1061,6 +967,427 @@ __global__ void k_remove_residue(Grid2 g, Field4 q, const uint8_t* m, int bit, i
     AWCM_SKIP_IF_DONE(st);
     const bool full = !sparse || (st && st->full_zero);
     ph_remove_residue(g, q, m, bit, full, grid_span());
+}
+
+// ---------------------------------------------------------------------------------- mask bit planes
+// The mask and level chain of PrepareEuler between the two transforms (banding, AddAdjacentZone,
+// CheckReconstruction, ComputeLevel, AddPointForDifferentiation: Wavelet/AWCM_2D.h:114-147) works on bit
+// planes, one bit per point: a pass is a few shifts per 32 points, and a point takes what its
+// neighbours push on it by reading them, where the byte form issues up to 19 atomics per active
+// detail.  A plane has the mask's byte layout (bit (i+3) & 31 of word (i+3) >> 5 of row j+3, pitch / 32
+// words a row), so a word is 32 aligned mask bytes.  Bits off the ghosted plane are set: ComputeLevel
+// reads a mask as set there.
+// live[k]: the points whose level_k byte may differ from 0 (all of them after a write from outside).
+struct Bits2 {
+    uint32_t* m[4];    // mask0..mask3
+    uint32_t* aux;     // mask0 before its adjacent zone
+    uint32_t* live[3];
+    int nwx;           // words per row
+};
+
+__device__ __forceinline__ uint32_t bshl(uint32_t below, uint32_t cur, int s) { return __funnelshift_l(below, cur, s); }
+__device__ __forceinline__ uint32_t bshr(uint32_t cur, uint32_t above, int s) { return __funnelshift_r(cur, above, s); }
+// Bits of word x whose column lies in [lo, hi].
+__device__ __forceinline__ uint32_t cols_in(int x, int lo, int hi)
+{
+    const int a = lo + kGhost - 32 * x, b = hi + kGhost - 32 * x;
+    if (a > 31 || b < 0 || b < a) return 0u;
+    const uint32_t up = b >= 31 ? ~0u : (2u << b) - 1u;
+    return a <= 0 ? up : up & (~0u << a);
+}
+// Bits of word x whose column is a multiple of 2^t, and an odd multiple of it.
+__device__ __forceinline__ uint32_t cols_mult(int x, int t)
+{
+    if (t >= 5) return (x & ((1 << (t - 5)) - 1)) == 0 ? 1u << kGhost : 0u;
+    const uint32_t p = t == 0 ? ~0u : t == 1 ? 0x55555555u : t == 2 ? 0x11111111u : t == 3 ? 0x01010101u : 0x00010001u;
+    return __funnelshift_l(p, p, kGhost);
+}
+__device__ __forceinline__ uint32_t cols_odd(int x, int t) { return cols_mult(x, t) & ~cols_mult(x, t + 1); }
+
+// One bit of each byte of 32 mask bytes as a bit word, and back.
+__device__ __forceinline__ uint32_t gather_bits(const uint32_t (&v)[8], int bit)
+{
+    uint32_t r = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) r |= ((((v[q] >> bit) & kLaneBits) * 0x01020408u) >> 24 & 15u) << (4 * q);
+    return r;
+}
+__device__ __forceinline__ uint32_t spread4(uint32_t bits) { return (bits & 15u) * 0x00204081u & kLaneBits; }
+__device__ __forceinline__ void load32(const uint8_t* p, uint32_t (&v)[8])
+{
+    const uint4 a = reinterpret_cast<const uint4*>(p)[0], b = reinterpret_cast<const uint4*>(p)[1];
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+
+// mask0 of the byte plane with the banding (see ph_band_copy) into aux; the other planes cleared.
+__device__ void bits_pack(const Grid2& g, const Bits2& B, const uint8_t* __restrict__ m, Span sp)
+{
+    const unsigned n = (unsigned)g.rows * (unsigned)B.nwx;
+    for (unsigned w = sp.t0; w < n; w += sp.stride) {
+        const int r = (int)(w / (unsigned)B.nwx), x = (int)w - r * B.nwx, j = r - kGhost;
+        uint32_t v[8];
+        load32(m + 32 * (size_t)w, v);
+        uint32_t b = gather_bits(v, 0);
+        if (j >= 0 && j < g.ny) {
+            uint32_t inner = j >= 2 && j <= g.ny - 3 ? cols_in(x, 2, g.nx - 3) : 0u;
+            if (g.bc_kind == AWCM_BC_WIND_TUNNEL) {
+                if (abs(j - g.wt_j) <= 2) inner &= ~cols_in(x, g.wt_i - 2, g.nx - 1);
+                if (j <= g.wt_j + 2) inner &= ~cols_in(x, g.wt_i - 2, g.wt_i + 2);
+            }
+            b |= cols_in(x, 0, g.nx - 1) & ~inner;
+        }
+        B.aux[w] = b | ~cols_in(x, -kGhost, g.nx - 1 + kGhost);
+        B.m[0][w] = B.m[1][w] = B.m[2][w] = B.m[3][w] = 0;
+    }
+}
+
+// The points `s` of word x of a row, shifted by +-d columns, into the row P (what falls off the row is
+// dropped); own: the part in word x itself.
+__device__ __forceinline__ void push_cols(uint32_t* P, int nwx, int x, uint32_t s, int d, bool lo, bool hi, uint32_t& own)
+{
+    if (d < 32) {
+        if (hi) {
+            own |= s << d;
+            const uint32_t up = s >> (32 - d);
+            if (up && x + 1 < nwx) atomicOr(&P[x + 1], up);
+        }
+        if (lo) {
+            own |= s >> d;
+            const uint32_t dn = s << (32 - d);
+            if (dn && x > 0) atomicOr(&P[x - 1], dn);
+        }
+        return;
+    }
+    const int o = d >> 5;
+    if (hi && x + o < nwx) atomicOr(&P[x + o], s);
+    if (lo && x - o >= 0) atomicOr(&P[x - o], s);
+}
+
+// AddAdjacentZone (see ph_aaz) of aux into mask0 (clear before).
+__device__ void bits_zone(const Grid2& g, const Bits2& B, Span sp)
+{
+    const int NX = g.nx - 1, NY = g.ny - 1, nwx = B.nwx;
+    const unsigned n = (unsigned)g.rows * (unsigned)nwx;
+    for (unsigned w = sp.t0; w < n; w += sp.stride) {
+        const uint32_t a = B.aux[w];
+        if (!a) continue;
+        const int r = (int)(w / (unsigned)nwx), x = (int)w - r * nwx, j = r - kGhost;
+        uint32_t own = a;
+        const uint32_t d = j >= 0 && j <= NY ? a & cols_in(x, 0, NX) : 0u;
+        if (d) {
+            uint32_t *M = B.m[0], *row = M + (size_t)r * nwx;
+            auto push = [&](uint32_t s, int t) {
+                const int h = 1 << t, q = t ? h >> 1 : 0;
+                push_cols(row, nwx, x, s, h, true, true, own);
+                atomicOr(&row[x - h * nwx], s);
+                atomicOr(&row[x + h * nwx], s);
+                if (q) {
+                    push_cols(row, nwx, x, s, q, true, true, own);
+                    atomicOr(&row[x - q * nwx], s);
+                    atomicOr(&row[x + q * nwx], s);
+                }
+            };
+            const int tj = j == 0 ? 64 : __ffs(j) - 1;
+            if (j != 0 && j != NY)
+                for (int t = 0; t < tj && t < g.maxl; ++t) {
+                    const uint32_t s = d & cols_odd(x, t);
+                    if (s) push(s, t);
+                }
+            if (tj < g.maxl) {
+                const uint32_t s = d & cols_mult(x, tj) & cols_in(x, 1, NX - 1);
+                if (s) push(s, tj);
+            }
+        }
+        atomicOr(&B.m[0][w], own);
+    }
+}
+
+// CheckReconstruction (AWCM_MANAGER_2D.h:63-158, see ph_cr) of the level of spacing h = 2^t.  Rows j =
+// 0, h, 2h .. are base + (j >> sh) nwx (base: row 0).  Up to h = 16 it is a gather:
+//   an odd row takes, on its even columns, the columns -+h, -+3h of its own d3 points;
+//   an even row takes from the odd rows -+h, -+3h their d3 points (marking d1 points there) and d2 points
+//   (marking c points), and on its even columns the columns -+h, -+3h of those d3 points and of its own
+//   d1 points.
+// At the ends the stencil of the first detail h is that of the detail 3h, and likewise at the other end,
+// so the first one counts as both.  A warp takes consecutive words of a row (two words of margin on the
+// left, one on the right; short rows several to a warp), so a word's neighbours come by shuffles.
+// A row's thread writes points of the row that no other thread of the pass reads, or (d1, d2 points
+// set by a d3 point) whose marks lie among those of the d3 point.
+// The coarser levels, whose columns are one bit of every (h / 32)-th word, push point by point.
+constexpr int kCloseKeep = 29, kCloseLeft = 2;
+__host__ __device__ __forceinline__ int close_rows_per_warp(int nwx) { return nwx <= 32 ? 32 / nwx : 1; }
+__host__ __device__ __forceinline__ long close_warps(long nr, int nwx)
+{
+    if (nwx > 32) return nr * ((nwx + kCloseKeep - 1) / kCloseKeep);
+    return (nr + close_rows_per_warp(nwx) - 1) / close_rows_per_warp(nwx);
+}
+__device__ void bits_close_level(const Grid2& g, uint32_t* base, int sh, int nwx, int t, Span sp)
+{
+    const int h = 1 << t, NX = g.nx - 1, NY = g.ny - 1;
+    if (t >= 5) {
+        const unsigned nc = (unsigned)(NX >> t) + 1u, n = ((unsigned)(NY >> t) + 1u) * nc;
+        for (unsigned u = sp.t0; u < n; u += sp.stride) {
+            const unsigned b = u / nc, a = u - b * nc;
+            const bool io = a & 1u, jo = b & 1u;
+            const int i = (int)a << t, j = (int)b << t, D = 2 * h;
+            if (!io && (!jo || i == 0 || i == NX)) continue;
+            if (!jo && (j == 0 || j == NY)) continue;
+            if (!((base[(size_t)(j >> sh) * nwx + (i >> 5)] >> kGhost) & 1u)) continue;
+            auto put = [&](int ii, int jj) { atomicOr(&base[(size_t)(jj >> sh) * nwx + (ii >> 5)], 1u << kGhost); };
+            int is = 0, js = 0, k;
+            if (io) predict_stencil(i, D, NX, is, k);
+            if (jo) predict_stencil(j, D, NY, js, k);
+            for (int c = 0; c < 4; ++c) {
+                if (io) put(is + c * D, j);
+                if (jo) put(i, js + c * D);
+                if (io && jo)
+                    for (int e = 0; e < 4; ++e) put(is + c * D, js + e * D);
+            }
+        }
+        return;
+    }
+    const int nr = (NY >> t) + 1, lane = threadIdx.x & 31;
+    const int rpw = close_rows_per_warp(nwx), chunks = nwx > 32 ? (nwx + kCloseKeep - 1) / kCloseKeep : 1;
+    const int fa = h + kGhost, fb = 3 * h + kGhost, la = NX - h + kGhost;
+    const unsigned n = (unsigned)close_warps(nr, nwx);
+    for (unsigned it = sp.t0 >> 5; it < n; it += sp.stride >> 5) {
+        int rr, x;
+        bool keep;
+        if (nwx <= 32) {
+            const int sub = lane / nwx;
+            x = lane - sub * nwx;
+            rr = (int)it * rpw + sub;
+            keep = sub < rpw && rr < nr;
+        } else {
+            rr = (int)(it / (unsigned)chunks);
+            x = ((int)it - rr * chunks) * kCloseKeep - kCloseLeft + lane;
+            keep = lane >= kCloseLeft && lane < kCloseLeft + kCloseKeep;
+        }
+        const bool on = x >= 0 && x < nwx && rr < nr && (nwx > 32 || keep);
+        const int j = rr << t;
+        const bool odd_row = rr & 1;
+        uint32_t* R = base + (size_t)(j >> sh) * nwx + x;
+        uint32_t own = 0, v = 0;  // this word; the rows around it (even rows)
+        if (on) {
+            own = *R;
+            if (!odd_row) {
+                const long st = (long)(h >> sh) * nwx;
+#pragma unroll
+                for (int k = -3; k <= 3; k += 2)
+                    if (j + k * h > 0 && j + k * h < NY) v |= R[k * st];
+                if (j == 6 * h) v |= R[-5 * st];
+                if (j == NY - 6 * h) v |= R[5 * st];
+            }
+        }
+        const uint32_t in = on ? cols_in(x, 0, NX) : 0u;
+        const bool own_details = odd_row || (j != 0 && j != NY);
+        uint32_t d = (v | (own_details ? own : 0u)) & cols_odd(x, t) & in;
+        if (t < 4) {
+            if (x == 0) d |= ((d >> fa) & 1u) << fb;
+        } else {
+            const uint32_t p = __shfl_up_sync(0xffffffffu, d, 1);
+            if (x == 1) d |= p & (1u << fa);  // fb is bit fa of word 1
+        }
+        {
+            const uint32_t e = x == la >> 5 ? d & (1u << (la & 31)) : 0u;
+            uint32_t f = __shfl_down_sync(0xffffffffu, e, 1);
+            if (x == nwx - 1) f = 0;
+            d |= t < 4 ? bshr(e, f, 2 * h) : f;
+        }
+        uint32_t l = __shfl_up_sync(0xffffffffu, d, 1), r = __shfl_down_sync(0xffffffffu, d, 1);
+        if (x == 0) l = 0;
+        if (x == nwx - 1) r = 0;
+        uint32_t mark;
+        if (t < 4) {
+            mark = bshl(l, d, h) | bshr(d, r, h) | bshl(l, d, 3 * h) | bshr(d, r, 3 * h);
+        } else {
+            // column 32 x' + 16 marks 32 x' - 32, 32 x', +32 and +64
+            uint32_t ll = __shfl_up_sync(0xffffffffu, d, 2);
+            if (x < 2) ll = 0;
+            mark = (ll | l | d | r) >> 16;
+        }
+        mark &= cols_mult(x, t + 1);
+        // the d3 and d2 points around (d2 points do not include the two end columns)
+        mark |= v & cols_mult(x, t) & cols_in(x, 1, NX - 1);
+        mark &= in;
+        if (keep && on && (mark & ~own)) *R = own | mark;
+    }
+}
+
+// Word x of row r of M, everything off the plane set.
+__device__ __forceinline__ uint32_t padded2(const Grid2& g, const uint32_t* M, int nwx, int r, int x)
+{
+    return r < 0 || r >= g.rows || x < 0 || x >= nwx ? ~0u : M[(size_t)r * nwx + x];
+}
+
+// ComputeLevel(level_{k-1}, mask_{k-1}), mask_k = mask_{k-1} and AddPointForDifferentiation(mask_k,
+// level_{k-1}) (see ph_cl, ph_apd) into mask_k (clear before).  A distance of the level search is one shift of
+// the word's row and a word of two other rows.
+__device__ void bits_next(const Grid2& g, const Bits2& B, int8_t* lvl, int k, Span sp)
+{
+    const int NX = g.nx - 1, NY = g.ny - 1, nwx = B.nwx;
+    const uint32_t* A = B.m[k - 1];
+    uint32_t* M = B.m[k];
+    const unsigned n = (unsigned)g.rows * (unsigned)nwx;
+    for (unsigned w = sp.t0; w < n; w += sp.stride) {
+        const uint32_t a = A[w], was = B.live[k - 1][w];
+        if (!(a | was)) continue;
+        const int r = (int)(w / (unsigned)nwx), x = (int)w - r * nwx, j = r - kGhost;
+        const uint32_t in = j >= 0 && j <= NY ? cols_in(x, 0, NX) : 0u;
+        const uint32_t on = a & in;
+        uint32_t own = a;
+        if (on | (was & in)) {
+            uint32_t lev4[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            const uint32_t mid = j >= 1 && j <= NY - 1 ? cols_in(x, 1, NX - 1) : 0u;
+            uint32_t* row = M + (size_t)r * nwx;
+            // the points `s` of level maxl - e: their level bytes, and their stencils into mask_k
+            auto take = [&](uint32_t s, int e) {
+                const uint32_t lev = (uint32_t)(g.maxl - e);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) lev4[q] |= spread4(s >> (4 * q)) * lev;
+                s &= mid;
+                if (!s) return;
+                if (e == 0) {
+                    own |= (s << 1) | (s << 2) | (s << 3) | (s >> 1) | (s >> 2) | (s >> 3);
+                    const uint32_t up = (s >> 31) | (s >> 30) | (s >> 29), dn = (s << 31) | (s << 30) | (s << 29);
+                    if (up && x + 1 < nwx) atomicOr(&row[x + 1], up);
+                    if (dn && x > 0) atomicOr(&row[x - 1], dn);
+#pragma unroll
+                    for (int c = 1; c <= 3; ++c) {
+                        atomicOr(&row[x - c * nwx], s);
+                        atomicOr(&row[x + c * nwx], s);
+                    }
+                    return;
+                }
+                const int D = 1 << e;
+                const uint32_t left = s & cols_in(x, 0, 2 * D - 1), right = s & ~left & cols_in(x, NX - 2 * D + 1, NX);
+                push_cols(row, nwx, x, s, D, true, true, own);
+                push_cols(row, nwx, x, s & ~left, 2 * D, true, false, own);
+                push_cols(row, nwx, x, s & ~right, 2 * D, false, true, own);
+                const int lo = j - 2 * D < 0 ? -1 : -2, hi = lo == -2 && j + 2 * D > NY ? 1 : 2;
+                for (int c = lo; c <= hi; ++c) {
+                    const int rr = r + c * D;
+                    if (c && rr >= 0 && rr < g.rows) atomicOr(&M[(size_t)rr * nwx + x], s);
+                }
+            };
+            uint32_t todo = on;
+            if (todo) {
+                const uint32_t l = padded2(g, A, nwx, r, x - 1), rt = padded2(g, A, nwx, r, x + 1);
+                for (int e = 0; e <= g.maxl && todo; ++e) {
+                    const int d = 1 << e;
+                    uint32_t near = padded2(g, A, nwx, r - d, x) | padded2(g, A, nwx, r + d, x);
+                    if (e < 5) near |= bshl(l, a, d) | bshr(a, rt, d);
+                    else near |= padded2(g, A, nwx, r, x - (d >> 5)) | padded2(g, A, nwx, r, x + (d >> 5));
+                    const uint32_t got = todo & near;
+                    todo &= ~got;
+                    if (got) take(got, e);
+                }
+            }
+            int8_t* lp = lvl + 32 * (size_t)w;
+            for (uint32_t u = todo; u; u &= u - 1) {  // no neighbour found: the level stays as it was
+                const int b = __ffs(u) - 1, lev = lp[b];
+                if (lev >= 0 && lev <= g.maxl) take(1u << b, g.maxl - lev);
+                else lev4[b >> 2] |= (uint32_t)(uint8_t)lev << (8 * (b & 3));
+            }
+            uint32_t* lw = reinterpret_cast<uint32_t*>(lp);
+            if (in == ~0u) {
+                reinterpret_cast<uint4*>(lw)[0] = make_uint4(lev4[0], lev4[1], lev4[2], lev4[3]);
+                reinterpret_cast<uint4*>(lw)[1] = make_uint4(lev4[4], lev4[5], lev4[6], lev4[7]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const uint32_t keep = ~(spread4(in >> (4 * q)) * 255u);  // ghosts keep theirs
+                    if (keep != ~0u) lw[q] = (lw[q] & keep) | lev4[q];
+                }
+            }
+            B.live[k - 1][w] = on;
+        } else if (was) {
+            B.live[k - 1][w] = 0;
+        }
+        if (own) atomicOr(&M[w], own);
+    }
+}
+
+// The planes mask0..mask3 back into the byte plane (its other bits stay).
+__device__ void bits_unpack(const Grid2& g, const Bits2& B, uint8_t* m, Span sp)
+{
+    const unsigned n = (unsigned)g.rows * (unsigned)B.nwx;
+    for (unsigned w = sp.t0; w < n; w += sp.stride) {
+        uint32_t v[8], o[8];
+        load32(m + 32 * (size_t)w, v);
+        const uint32_t b[4] = {B.m[0][w], B.m[1][w], B.m[2][w], B.m[3][w]};
+        uint32_t diff = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            o[q] = v[q] & 0xf0f0f0f0u;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) o[q] |= spread4(b[k] >> (4 * q)) << k;
+            diff |= o[q] ^ v[q];
+        }
+        if (!diff) continue;
+        uint4* p = reinterpret_cast<uint4*>(m + 32 * (size_t)w);
+        p[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        p[1] = make_uint4(o[4], o[5], o[6], o[7]);
+    }
+}
+
+__global__ void k_bits_pack(Grid2 g, Bits2 B, const uint8_t* m, const StepState* st)
+{
+    pdl_begin();
+    if (st && st->done) return;
+    bits_pack(g, B, m, grid_span());
+}
+__global__ void k_bits_zone(Grid2 g, Bits2 B, const StepState* st)
+{
+    pdl_begin();
+    if (st && st->done) return;
+    bits_zone(g, B, grid_span());
+}
+__global__ void k_bits_close(Grid2 g, uint32_t* M, int nwx, int t, const StepState* st)
+{
+    pdl_begin();
+    if (st && st->done) return;
+    bits_close_level(g, M + (size_t)kGhost * nwx, 0, nwx, t, grid_span());
+}
+__global__ void k_bits_next(Grid2 g, Bits2 B, int8_t* lvl, int k, const StepState* st)
+{
+    pdl_begin();
+    if (st && st->done) return;
+    bits_next(g, B, lvl, k, grid_span());
+}
+__global__ void k_bits_unpack(Grid2 g, Bits2 B, uint8_t* m, const StepState* st)
+{
+    pdl_begin();
+    if (st && st->done) return;
+    bits_unpack(g, B, m, grid_span());
+}
+constexpr int kBitsThreads = 1024;
+// The whole chain of a small grid in one CTA, its planes in shared memory: no launch per pass.
+__global__ void __launch_bounds__(kBitsThreads) k_bits_all(Grid2 g, Bits2 B, uint8_t* m, int8_t* l0, int8_t* l1, int8_t* l2,
+                                                           const StepState* st)
+{
+    extern __shared__ uint32_t rows_sm[];
+    pdl_begin();
+    if (st && st->done) return;
+    const size_t n = (size_t)g.rows * B.nwx;
+    B.aux = rows_sm;
+    for (int k = 0; k < 4; ++k) B.m[k] = rows_sm + (k + 1) * n;
+    const Span sp{threadIdx.x, blockDim.x};
+    bits_pack(g, B, m, sp);
+    __syncthreads();
+    bits_zone(g, B, sp);
+    __syncthreads();
+    for (int k = 0; k <= 3; ++k) {
+        if (k) {
+            bits_next(g, B, k == 1 ? l0 : k == 2 ? l1 : l2, k, sp);
+            __syncthreads();
+        }
+        for (int t = 0; t < g.maxl; ++t) {
+            bits_close_level(g, B.m[k] + (size_t)kGhost * B.nwx, 0, B.nwx, t, sp);
+            __syncthreads();
+        }
+    }
+    bits_unpack(g, B, m, sp);
 }
 
 // ------------------------------------------------------------------- persistent PrepareEuler
@@ -1174,9 +1501,9 @@ __global__ void __launch_bounds__(kPrepThreads, 1) k_prepare(PrepArgs A)
         SYNC_OR_LEAVE;
     }
     for (int lev = 0; lev < g.maxl; ++lev) {
-        ph_interp<0>(g, A.q, A.m, lev, kBitTemp, 1, sp);
+        ph_interp<0>(g, A.q, A.m, lev, kBitInterp, kBitTemp, 1, sp);
         SYNC_OR_LEAVE;
-        ph_interp<1>(g, A.q, A.m, lev, kBitTemp, 1, sp);
+        ph_interp<1>(g, A.q, A.m, lev, kBitInterp, kBitTemp, 1, sp);
         if (lev + 1 < g.maxl) SYNC_OR_LEAVE;
     }
 #undef SYNC_OR_LEAVE
@@ -2187,6 +2514,8 @@ struct Solver2D {
     double* ay[kStages] = {};
     StepState* st = nullptr;
     uint32_t* lists[kNumLists] = {};
+    Bits2 bits{};
+    uint32_t* bits_mem = nullptr;
     void* staging = nullptr;
     size_t staging_bytes = 0;
     int8_t* bcf_dev = nullptr;  // BOUNDARY_CONDITION plane of the generic manager
@@ -2251,10 +2580,15 @@ struct Solver2D {
     template <typename... P, typename... A>
     void launch(void (*kern)(P...), dim3 grid, dim3 block, A&&... args)
     {
+        launch_smem(kern, grid, block, 0, std::forward<A>(args)...);
+    }
+    template <typename... P, typename... A>
+    void launch_smem(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A&&... args)
+    {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = grid;
         cfg.blockDim = block;
-        cfg.dynamicSmemBytes = 0;
+        cfg.dynamicSmemBytes = smem;
         cfg.stream = cur ? cur : stream;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -2283,6 +2617,7 @@ struct Solver2D {
             fr(lvl[k]);
         }
         fr(m);
+        fr(bits_mem);
         for (int s = 0; s < kStages; ++s) {
             fr(ax[s]);
             fr(ay[s]);
@@ -2367,6 +2702,13 @@ struct Solver2D {
             AWCM_CUDA_TRY(cudaMemsetAsync(fy.p[k], 0, plane * sizeof(double), stream));
         }
         AWCM_CUDA_TRY(cudaMalloc(&m, plane));
+        bits.nwx = g.pitch / 32;
+        AWCM_CUDA_TRY(cudaMalloc(&bits_mem, 8 * bit_words() * sizeof(uint32_t)));
+        for (int k = 0; k < 4; ++k) bits.m[k] = bits_mem + k * bit_words();
+        bits.aux = bits_mem + 4 * bit_words();
+        for (int k = 0; k < 3; ++k) bits.live[k] = bits_mem + (5 + k) * bit_words();
+        mark_levels();
+        AWCM_CUDA_TRY(cudaFuncSetAttribute(k_bits_all, cudaFuncAttributeMaxDynamicSharedMemorySize, kBitsSmem));
         for (int s = 0; s < kStages; ++s) {
             AWCM_CUDA_TRY(cudaMalloc(&ax[s], sizeof(double) * g.ny));
             AWCM_CUDA_TRY(cudaMalloc(&ay[s], sizeof(double) * g.nx));
@@ -2473,6 +2815,7 @@ struct Solver2D {
         if (rc) return rc;
         AWCM_CUDA_TRY(cudaMemcpyAsync(staging, host, 4 * n * sizeof(int), cudaMemcpyHostToDevice, stream));
         launch(k_levels_in, blocks_for((long)n, 256), 256, g, (const int*)staging, lvl[0], lvl[1], lvl[2], lvl[3]);
+        mark_levels();
         AWCM_CUDA_TRY(cudaGetLastError());
         AWCM_CUDA_TRY(cudaStreamSynchronize(stream));
         return kOk;
@@ -2489,6 +2832,10 @@ struct Solver2D {
         AWCM_CUDA_TRY(cudaStreamSynchronize(stream));
         return kOk;
     }
+
+    size_t bit_words() const { return plane / 32; }
+    // After the level planes were written by anything but the step's mask chain: it rewrites all of them.
+    void mark_levels() { cudaMemsetAsync(bits.live[0], 0xff, 3 * bit_words() * sizeof(uint32_t), stream); }
 
     void mark_full_zero()
     {
@@ -2554,22 +2901,14 @@ struct Solver2D {
         }
     }
 
-    // init_from >= 0: the first launch also builds the work mask of the interpolation that follows
-    // (ph_interp_init from init_from to bit), which the inverse transform does not read.
     // sparse: in PrepareEuler (mask_temp = the starting mask0), see ph_iwt.
-    void enq_iwt(int bit, const StepState* s, int init_from = -1, bool sparse = false)
+    void enq_iwt(int bit, const StepState* s, bool sparse = false)
     {
         const int sp = sparse ? 1 : 0;
         for (int lev = 0; lev < g.maxl; ++lev) {
             const Band b3 = band_of(g, lev, 2), b1 = band_of(g, lev, 0), b2 = band_of(g, lev, 1), bc = band_of(g, lev, 3);
-            if (lev == 0 && init_from >= 0) {
-                const unsigned nb = pb((long)bc.cx * bc.cy);
-                launch(k_iwt0_interp_init, nb + pb(words()), 256, g, q.p[0], m, lev, bit, init_from, sp, s, nb);
-                after("k_iwt0_interp_init");
-            } else {
-                launch(k_iwt<0>, pb((long)bc.cx * bc.cy), 256, g, q.p[0], m, lev, bit, sp, s);
-                after("k_iwt<0>");
-            }
+            launch(k_iwt<0>, pb((long)bc.cx * bc.cy), 256, g, q.p[0], m, lev, bit, sp, s);
+            after("k_iwt<0>");
             launch(k_iwt<1>, pb((long)b1.cx * b1.cy + (long)b2.cx * b2.cy), 256, g, q.p[0], m, lev, bit, sp, s);
             after("k_iwt<1>");
             launch(k_iwt<2>, pb((long)b3.cx * b3.cy), 256, g, q.p[0], m, lev, bit, sp, s);
@@ -2578,34 +2917,75 @@ struct Solver2D {
         }
     }
 
-    // init_done: the work mask was built by the inverse transform's first launch.
-    void enq_interp(int from, int to, const StepState* s, int p0 = 1, bool init_done = false)
+    void enq_interp(int from, int to, const StepState* s, int p0 = 1)
     {
-        if (!init_done) {
-            launch(k_interp_init, pb(words()), 256, g, m, from, to, s);
-            after("k_interp_init");
-            launches += 1;
-        }
+        launch(k_interp_init, pb(words()), 256, g, m, from, to, s);
+        after("k_interp_init");
+        launches += 1;
         enq_cr(kBitInterp, s);
+        enq_interp_levels(kBitInterp, from, s, p0);
+    }
+    // PrepareEuler's interpolation, mask_temp to mask3: its work mask, mask3 without mask_temp closed under
+    // CheckReconstruction, marks no further point, because mask3 itself is closed: the points to
+    // interpolate are those of mask3 outside mask_temp.
+    void enq_interp_new(const StepState* s) { enq_interp_levels(3, kBitTemp, s, 1); }
+    void enq_interp_levels(int work, int from, const StepState* s, int p0)
+    {
         for (int lev = 0; lev < g.maxl; ++lev) {
             if (row_scan(lev)) {
-                launch(k_interp_rows<0>, pb(rowscan_threads(lev, 2)), 256, g, q, m, lev, from, p0, s);
+                launch(k_interp_rows<0>, pb(rowscan_threads(lev, 2)), 256, g, q, m, lev, work, from, p0, s);
                 after("k_interp_rows<0>");
-                launch(k_interp_rows<1>, pb(rowscan_threads(lev, 1)), 256, g, q, m, lev, from, p0, s);
+                launch(k_interp_rows<1>, pb(rowscan_threads(lev, 1)), 256, g, q, m, lev, work, from, p0, s);
                 after("k_interp_rows<1>");
             } else {
-                launch(k_interp<0>, pb(band_count(lev, 0) + band_count(lev, 1)), 256, g, q, m, lev, from, p0, s);
+                launch(k_interp<0>, pb(band_count(lev, 0) + band_count(lev, 1)), 256, g, q, m, lev, work, from, p0, s);
                 after("k_interp<0>");
-                launch(k_interp<1>, pb(band_count(lev, 2)), 256, g, q, m, lev, from, p0, s);
+                launch(k_interp<1>, pb(band_count(lev, 2)), 256, g, q, m, lev, work, from, p0, s);
                 after("k_interp<1>");
             }
             launches += 2;
         }
     }
 
+    // The mask and level chain on bit planes, from the forward transform's mask0 to mask0..mask3 and
+    // level0..level2.  Grids of up to kBitsOne words a plane (128 x 129 points and the like) in one launch of one
+    // CTA; larger ones a launch per pass.
+    static constexpr long kBitsOne = 4096;
+    static constexpr int kBitsSmem = 200 * 1024;
+    void enq_masks(const StepState* s)
+    {
+        const long n = (long)bit_words();
+        if (n <= kBitsOne) {
+            launch_smem(k_bits_all, 1, kBitsThreads, 5 * n * sizeof(uint32_t), g, bits, m, lvl[0], lvl[1], lvl[2], s);
+            after("k_bits_all");
+            launches += 1;
+            return;
+        }
+        launch(k_bits_pack, pb(n), 256, g, bits, m, s);
+        after("k_bits_pack");
+        launch(k_bits_zone, pb(n), 256, g, bits, s);
+        after("k_bits_zone");
+        for (int k = 0; k <= 3; ++k) {
+            if (k) {
+                launch(k_bits_next, pb(n), 256, g, bits, lvl[k - 1], k, s);
+                after("k_bits_next");
+            }
+            for (int t = 0; t < g.maxl; ++t) {
+                const long rows = (((long)g.ny - 1) >> t) + 1;
+                const long threads = t < 5 ? 32 * close_warps(rows, bits.nwx) : rows * (((g.nx - 1) >> t) + 1);
+                launch(k_bits_close, pb(threads), 256, g, bits.m[k], bits.nwx, t, s);
+                after("k_bits_close");
+            }
+            launches += (k ? 1 : 0) + g.maxl;
+        }
+        launch(k_bits_unpack, pb(n), 256, g, bits, m, s);
+        after("k_bits_unpack");
+        launches += 3;
+    }
+
     void enq_aaz(int bit, const StepState* s)
     {
-        launch(k_copy_bit_all, pb(words()), 256, m, plane, bit, kBitCopy, s, 0u);
+        launch(k_copy_bit_all, pb(words()), 256, m, plane, bit, kBitCopy, s);
         after("k_copy_bit_all");
         launch(k_aaz, pb(words()), 256, g, m, bit, kBitCopy, s);
         after("k_aaz");
@@ -2667,56 +3047,38 @@ struct Solver2D {
             if (lists) enq_lists(0);
             return;
         }
-        // mask_temp = mask0; also clears mask1..3, which the merged ComputeLevel +
-        // AddPointForDifferentiation passes below rebuild by ORs
-        if (!scalar) launch(k_copy_bit_all, pb(words()), 256, m, plane, 0, kBitTemp, s, kMask123);
-        after("k_copy_bit_all");
-        launches += 1;
-        enq_fwt(s, !scalar);
-        launch(k_band_copy, pb(words()), 256, g, m, 0, kBitCopy, s);
-        after("k_band_copy");
-        launch(k_aaz, pb(words()), 256, g, m, 0, kBitCopy, s);
-        after("k_aaz");
-        launches += 2;
-        enq_cr(0, s);
-        for (int k = 1; k <= 3; ++k) {
-            if (!scalar) {
-                launch(k_cl_apd, pb(words()), 256, g, m, lvl[k - 1], k, plane, s);
-                after("k_cl_apd");
-                launches += 1;
-            } else {
-                launch(k_cl, pb(words()), 256, g, m, lvl[k - 1], k - 1, k, plane, s);
-                after("k_cl");
-                launch(k_apd, pb(words()), 256, g, m, lvl[k - 1], k, k - 1, s);
-                after("k_apd");
-                launches += 2;
-            }
-            enq_cr(k, s);
+        // mask_temp = mask0
+        if (!scalar) {
+            launch(k_copy_bit_all, pb(words()), 256, m, plane, 0, kBitTemp, s);
+            after("k_copy_bit_all");
+            launches += 1;
         }
+        enq_fwt(s, !scalar);
+        enq_masks(s);
         // AWCM_2D::Prepare (the scalar form, Wavelet/AWCM_2D.h:52-79) ends with the inverse transform
         if (scalar) {
             enq_iwt(3, s);
             if (lists) enq_lists(0);
         } else if (!fork_ok()) {
-            enq_iwt(3, s, kBitTemp, true);
-            enq_interp(kBitTemp, 3, s, 1, true);
+            enq_iwt(3, s, true);
+            enq_interp_new(s);
             if (lists) enq_lists(0);
         } else {
             // The inverse transform writes the density only and reads mask3; the interpolation
-            // reads and writes components 1..3 and the interpolation work bit; the worklist build
+            // reads mask3 and mask_temp and reads and writes components 1..3; the worklist build
             // reads the mask bits 0..3 and the level planes and writes the lists: disjoint, so the
             // three run as parallel branches of the graph.
             cudaEventRecord(ev_fork, stream);
             cudaStreamWaitEvent(side, ev_fork, 0);
             if (lists) cudaStreamWaitEvent(side2, ev_fork, 0);
             cur = side;
-            enq_interp(kBitTemp, 3, s, 1, false);
+            enq_interp_new(s);
             if (lists) {
                 cur = side2;
                 enq_lists(0);
             }
             cur = nullptr;
-            enq_iwt(3, s, -1, true);
+            enq_iwt(3, s, true);
             join(side, ev_join);
             if (lists) join(side2, ev_join2);
         }
@@ -3240,10 +3602,13 @@ struct Solver2D {
             case 0: enq_aaz(b, nullptr); break;
             case 1: enq_cr(b, nullptr); break;
             case 2:
-                launch(k_copy_bit_all, pb(words()), 256, m, plane, b, kBitCopy, nullptr, 0u);
+                launch(k_copy_bit_all, pb(words()), 256, m, plane, b, kBitCopy, nullptr);
                 launch(k_apd, pb(words()), 256, g, m, lvl[level_id], b, kBitCopy, nullptr);
                 break;
-            case 3: launch(k_cl, pb(words()), 256, g, m, lvl[level_id], b, -1, plane, nullptr); break;
+            case 3:
+                launch(k_cl, pb(words()), 256, g, m, lvl[level_id], b, -1, plane, nullptr);
+                mark_levels();
+                break;
             case 4: launch(k_remove_residue, pb(words()), 256, g, q, m, b, 0, nullptr); break;
             case 5: launch(k_band_copy, pb(words()), 256, g, m, b, -1, nullptr); break;
             default: return kErrArg;
@@ -3892,6 +4257,7 @@ int awcm2d_set_prepare_mode(awcm2d_t h, int mode)
     AWCM_H(h);
     if (mode != 0 && mode != 1) return awcm::kErrArg;
     h->s.prep_mode = mode;
+    h->s.mark_levels();  // the persistent kernel writes the level planes itself
     if (h->s.graph) cudaGraphExecDestroy(h->s.graph);
     h->s.graph = nullptr;
     return awcm::kOk;
