@@ -872,6 +872,11 @@ __device__ void ph_remove_residue(const Grid2& g, Field4 q, const uint8_t* m, in
 }
 
 // ------------------------------------------------------------------------ standalone kernels
+#ifndef AWCM_COARSE_POINTS
+#define AWCM_COARSE_POINTS 1024
+#endif
+constexpr int kCoarseThreads = 1024;
+constexpr long kCoarsePoints = AWCM_COARSE_POINTS;
 #define AWCM_SKIP_IF_DONE(st) \
     if ((st) && (st)->done) return
 
@@ -909,6 +914,50 @@ __global__ void k_cr_rows(Grid2 g, uint8_t* m, int lev, int bit, const StepState
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
     ph_cr_rows(g, m, lev, bit, grid_span());
+}
+// The coarse levels top, top-1 .. 0 (0 .. top) of a transform in one CTA: a level of a few thousand points
+// takes about as long there as its launch does.
+__global__ void __launch_bounds__(kCoarseThreads) k_fwt_coarse(Grid2 g, double* q, double* tb, uint8_t* m, int top, int idle,
+                                                              const StepState* st)
+{
+    pdl_begin();
+    AWCM_SKIP_IF_DONE(st);
+    const Span sp{threadIdx.x, blockDim.x};
+    for (int lev = top; lev >= 0; --lev) {
+        ph_fwt_a(g, q, tb, m, lev, st->tol, idle != 0, sp);
+        __syncthreads();
+        ph_fwt_b(g, q, tb, m, lev, idle != 0, sp);
+        __syncthreads();
+    }
+}
+__global__ void __launch_bounds__(kCoarseThreads) k_iwt_coarse(Grid2 g, double* q, const uint8_t* m, int top, int bit, int sparse,
+                                                              const StepState* st)
+{
+    pdl_begin();
+    AWCM_SKIP_IF_DONE(st);
+    const bool zero_all = !sparse || !st || st->full_zero;
+    const Span sp{threadIdx.x, blockDim.x};
+    for (int lev = 0; lev <= top; ++lev) {
+        ph_iwt<0>(g, q, m, lev, bit, zero_all, sp);
+        __syncthreads();
+        ph_iwt<1>(g, q, m, lev, bit, zero_all, sp);
+        __syncthreads();
+        ph_iwt<2>(g, q, m, lev, bit, zero_all, sp);
+        __syncthreads();
+    }
+}
+__global__ void __launch_bounds__(kCoarseThreads) k_interp_coarse(Grid2 g, Field4 q, const uint8_t* m, int top, int work,
+                                                                 int from_bit, int p0, const StepState* st)
+{
+    pdl_begin();
+    AWCM_SKIP_IF_DONE(st);
+    const Span sp{threadIdx.x, blockDim.x};
+    for (int lev = 0; lev <= top; ++lev) {
+        ph_interp<0>(g, q, m, lev, work, from_bit, p0, sp);
+        __syncthreads();
+        ph_interp<1>(g, q, m, lev, work, from_bit, p0, sp);
+        __syncthreads();
+    }
 }
 template <int PH>
 __global__ void k_interp(Grid2 g, Field4 q, const uint8_t* m, int lev, int work, int from_bit, int p0, const StepState* st)
@@ -2858,6 +2907,14 @@ struct Solver2D {
         const Band b = band_of(g, lev, which);
         return (long)b.cx * b.cy;
     }
+    // The finest of the coarse levels that share one launch (-1: none; one level alone gains nothing; the
+    // finest level has its own form).
+    int coarse_top() const
+    {
+        int top = -1;
+        while (top + 2 < g.maxl && details(top + 1) <= kCoarsePoints) ++top;
+        return top;
+    }
     long details(int lev) const { return band_count(lev, 0) + band_count(lev, 1) + band_count(lev, 2); }
 
     // Fine levels (point spacing <= kRowScanMaxH) scan mask words row by row and skip empty words;
@@ -2891,7 +2948,8 @@ struct Solver2D {
     void enq_fwt(const StepState* s, bool idle = false)
     {
         const int id = idle ? 1 : 0;
-        for (int lev = g.maxl - 1; lev >= 0; --lev) {
+        const int top = coarse_top();
+        for (int lev = g.maxl - 1; lev > top; --lev) {
             launch(k_fwt_a, pb(details(lev)), 256, g, q.p[0], fx.p[0], m, lev, id, s);
             after("k_fwt_a");
             const long nb = band_count(lev, 3) + band_count(lev, 0) + band_count(lev, 1);
@@ -2899,13 +2957,23 @@ struct Solver2D {
             after("k_fwt_b");
             launches += 2;
         }
+        if (top >= 0) {
+            launch(k_fwt_coarse, 1, kCoarseThreads, g, q.p[0], fx.p[0], m, top, id, s);
+            after("k_fwt_coarse");
+            launches += 1;
+        }
     }
 
     // sparse: in PrepareEuler (mask_temp = the starting mask0), see ph_iwt.
     void enq_iwt(int bit, const StepState* s, bool sparse = false)
     {
-        const int sp = sparse ? 1 : 0;
-        for (int lev = 0; lev < g.maxl; ++lev) {
+        const int sp = sparse ? 1 : 0, top = coarse_top();
+        if (top >= 0) {
+            launch(k_iwt_coarse, 1, kCoarseThreads, g, q.p[0], m, top, bit, sp, s);
+            after("k_iwt_coarse");
+            launches += 1;
+        }
+        for (int lev = top + 1; lev < g.maxl; ++lev) {
             const Band b3 = band_of(g, lev, 2), b1 = band_of(g, lev, 0), b2 = band_of(g, lev, 1), bc = band_of(g, lev, 3);
             launch(k_iwt<0>, pb((long)bc.cx * bc.cy), 256, g, q.p[0], m, lev, bit, sp, s);
             after("k_iwt<0>");
@@ -2931,7 +2999,13 @@ struct Solver2D {
     void enq_interp_new(const StepState* s) { enq_interp_levels(3, kBitTemp, s, 1); }
     void enq_interp_levels(int work, int from, const StepState* s, int p0)
     {
-        for (int lev = 0; lev < g.maxl; ++lev) {
+        const int top = coarse_top();
+        if (top >= 0) {
+            launch(k_interp_coarse, 1, kCoarseThreads, g, q, m, top, work, from, p0, s);
+            after("k_interp_coarse");
+            launches += 1;
+        }
+        for (int lev = top + 1; lev < g.maxl; ++lev) {
             if (row_scan(lev)) {
                 launch(k_interp_rows<0>, pb(rowscan_threads(lev, 2)), 256, g, q, m, lev, work, from, p0, s);
                 after("k_interp_rows<0>");
