@@ -871,6 +871,22 @@ __device__ void ph_remove_residue(const Grid2& g, Field4 q, const uint8_t* m, in
     }
 }
 
+// Start of a step: whether there is one to take, and the reset of its device-side scalars.  keep_lists:
+// the step reuses the worklists (and mask counts) of the previous one (frozen masks).
+__device__ __forceinline__ bool step_done(const StepState* st) { return st->t >= st->t_end || st->error; }
+__device__ __forceinline__ void begin_step(StepState* st, bool done, int keep_lists)
+{
+    st->done = done ? 1 : 0;
+    if (done) return;
+    st->bar[0] = 0;
+    st->bar_err = 0;
+    st->nonfinite = 0;
+    st->mv = 0;
+    if (keep_lists) return;
+    for (int k = 0; k < 4 * kStages; ++k) st->cnt[k] = 0;
+    for (int k = 0; k < 4; ++k) st->mask_cnt[k] = 0;
+}
+
 // ------------------------------------------------------------------------ standalone kernels
 #ifndef AWCM_COARSE_POINTS
 #define AWCM_COARSE_POINTS 1024
@@ -973,6 +989,15 @@ __global__ void k_interp_rows(Grid2 g, Field4 q, const uint8_t* m, int lev, int 
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
     ph_interp_rows<PH>(g, q, m, lev, work, from_bit, p0, grid_span());
+}
+// The first launch of an Euler step: k_begin's bookkeeping by its first thread, and mask_temp = mask0.
+// Nothing in it reads what the bookkeeping writes.
+__global__ void k_begin_copy(uint8_t* m, size_t n, int from, int to, StepState* st)
+{
+    pdl_begin();
+    const bool done = step_done(st);
+    if (blockIdx.x == 0 && threadIdx.x == 0) begin_step(st, done, 0);
+    if (!done) ph_copy_bit_all(m, n, from, to, grid_span());
 }
 __global__ void k_copy_bit_all(uint8_t* m, size_t n, int from, int to, const StepState* st)
 {
@@ -1802,8 +1827,7 @@ __global__ void k_wt_bottom_y(Grid2 g, Field4 f, int part, const StepState* st)
 // ------------------------------------------------------------------------- CFL and LF reductions
 // Per-row alpha_x[j] = max |u|+c and per-column alpha_y[i] = max |v|+c over the points of mask
 // `bit` (main_2d_euler(quad).cpp:86-104); with mv != null also the CFL speed
-// max (|u|+c)+(|v|+c) (:61-76).  A CTA covers 128 columns (one mask word of four points per
-// lane) x 32 rows (four per warp); empty words cost one load.  Maxima are order-independent.
+// max (|u|+c)+(|v|+c) (:61-76).  Maxima are order-independent.
 __device__ __noinline__ void speeds_any(double q0, double q1, double q2, double q3, double gamma, double* out)
 {
     IeeeDiv dv;
@@ -1820,60 +1844,66 @@ __device__ __forceinline__ void speeds(const double* q, double gamma, double& sx
         sx = s[0], sy = s[1];
     }
 }
-constexpr int kAlphaRows = 4;
-__global__ void __launch_bounds__(256) k_alpha(Grid2 g, Field4 f, const uint8_t* __restrict__ m, int bit,
+// Maximum of non-negative doubles over the warp by their bit patterns (NaN: the largest).
+__device__ __forceinline__ double warp_max_nonneg(double v)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const unsigned hi = (unsigned)(b >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)b : 0u);
+    return __hiloint2double((int)mh, (int)ml);
+}
+// A warp covers 32 columns x `rows` rows, one point per lane and row: a point is a chain of divisions and a
+// square root (~0.4 us), so its rows are few -- one to eight, as many as keep the launch at some 16 CTAs an
+// SM (with four points a lane and four rows a warp the scan of 641x385 points took 14.6 us, of 2049^2 23.3).
+// The masks of all rows are loaded before the first is looked at.
+constexpr int kAlphaMaxRows = 8;
+__global__ void __launch_bounds__(256) k_alpha(Grid2 g, Field4 f, const uint8_t* __restrict__ m, int bit, int rows,
                                                double* ax, double* ay, double* mv, const StepState* st,
                                                int* nonfinite)
 {
     pdl_begin();
-    if (st && st->done) return;
-    __shared__ double col[8][128];
+    const int done = st ? st->done : 0;
+    __shared__ double col[8][32];
     __shared__ double cfl[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned wpr = (unsigned)g.pitch / 4u;  // mask words per plane row
-    const unsigned wi = blockIdx.x * 32u + lane;
-    const int i0 = 4 * (int)wi - kGhost;
-    const unsigned* mp = reinterpret_cast<const unsigned*>(m);
-    double cm[4] = {0, 0, 0, 0};
-    double vmax = 0;
-    bool nf = false;  // a NaN or infinite speed (NaN/Inf state, negative pressure or density)
-    for (int r = 0; r < kAlphaRows; ++r) {
-        const int j = (int)blockIdx.y * (8 * kAlphaRows) + warp * kAlphaRows + r;
-        double sx_row = 0;
-        if (j < g.ny && wi < wpr) {
-            const unsigned lanes = lanes_in(i0, 0, g.nx - 1);
-            const unsigned hit = (mp[(size_t)(j + kGhost) * wpr + wi] >> bit) & lane_bits(lanes);
+    const int i = 32 * (int)blockIdx.x - kGhost + lane;  // the pitch is a multiple of 32
+    const int j0 = ((int)blockIdx.y * 8 + warp) * rows;
+    unsigned on = 0;  // bit r: the point of row j0 + r is in the mask
 #pragma unroll
-            for (int L = 0; L < 4; ++L) {
-                if (!((hit >> (8 * L)) & 1u)) continue;
-                const size_t a = g.at(i0 + L, j);
-                const double q[4] = {f.p[0][a], f.p[1][a], f.p[2][a], f.p[3][a]};
-                double sx, sy;
-                speeds(q, g.gamma, sx, sy);
-                nf |= !(isfinite(sx) && isfinite(sy));
-                sx_row = maxd(sx_row, sx);
-                cm[L] = maxd(cm[L], sy);
-                vmax = maxd(vmax, sx + sy);
-            }
+    for (int r = 0; r < kAlphaMaxRows; ++r)
+        if (r < rows && j0 + r < g.ny && i >= 0 && i < g.nx) on |= ((unsigned)(m[g.at(i, j0 + r)] >> bit) & 1u) << r;
+    if (done) return;
+    double cm = 0, vmax = 0;
+    bool nf = false;  // a NaN or infinite speed (NaN/Inf state, negative pressure or density)
+    for (unsigned todo = __reduce_or_sync(0xffffffffu, on); todo; todo &= todo - 1) {
+        const int r = __ffs(todo) - 1;
+        double sx = 0, sy = 0;
+        if ((on >> r) & 1u) {
+            const size_t a = g.at(i, j0 + r);
+            const double q[4] = {f.p[0][a], f.p[1][a], f.p[2][a], f.p[3][a]};
+            speeds(q, g.gamma, sx, sy);
+            nf |= !(isfinite(sx) && isfinite(sy));
+            if (!(sx >= 0)) sx = 0;  // NaN: flagged, left out
+            if (!(sy >= 0)) sy = 0;
+            cm = maxd(cm, sy);
+            vmax = maxd(vmax, sx + sy);
         }
-        const double rowmax = warp_max(sx_row);
-        if (ax && lane == 0 && j < g.ny && rowmax > 0) atomic_max_nonneg(&ax[j], rowmax);
+        const double rowmax = warp_max_nonneg(sx);
+        if (ax && lane == 0 && rowmax > 0) atomic_max_nonneg(&ax[j0 + r], rowmax);
     }
     if (nonfinite && __any_sync(0xffffffffu, nf) && lane == 0) atomicOr(nonfinite, 1);
-#pragma unroll
-    for (int L = 0; L < 4; ++L) col[warp][4 * lane + L] = cm[L];
-    vmax = warp_max(vmax);
+    col[warp][lane] = cm;
+    vmax = warp_max_nonneg(vmax);
     if (lane == 0) cfl[warp] = vmax;
     __syncthreads();
-    if (threadIdx.x < 128) {
-        double c = col[0][threadIdx.x];
-        for (int y = 1; y < 8; ++y) c = maxd(c, col[y][threadIdx.x]);
-        const int i = 4 * ((int)blockIdx.x * 32) - kGhost + (int)threadIdx.x;
+    if (threadIdx.x < 32) {
+        double c = col[0][lane];
+#pragma unroll
+        for (int y = 1; y < 8; ++y) c = maxd(c, col[y][lane]);
         if (ay && i >= 0 && i < g.nx && c > 0) atomic_max_nonneg(&ay[i], c);
-        if (mv && threadIdx.x == 0) {
-            double v = cfl[0];
-            for (int y = 1; y < 8; ++y) v = maxd(v, cfl[y]);
-            if (v > 0) atomic_max_nonneg(mv, v);
+        if (mv) {
+            const double v = warp_max_nonneg(lane < 8 ? cfl[lane] : 0.0);
+            if (lane == 0 && v > 0) atomic_max_nonneg(mv, v);
         }
     }
 }
@@ -1977,19 +2007,10 @@ __global__ void k_dt(Grid2 g, StepState* st)
     compute_dt(g, st);
 }
 
-// keep_lists: the step reuses the worklists (and mask counts) of the previous one (frozen masks).
 __global__ void k_begin(StepState* st, int keep_lists)
 {
     pdl_begin();
-    st->done = (st->t >= st->t_end || st->error) ? 1 : 0;
-    if (st->done) return;
-    st->bar[0] = 0;
-    st->bar_err = 0;
-    st->nonfinite = 0;
-    st->mv = 0;
-    if (keep_lists) return;
-    for (int k = 0; k < 4 * kStages; ++k) st->cnt[k] = 0;
-    for (int k = 0; k < 4; ++k) st->mask_cnt[k] = 0;
+    begin_step(st, step_done(st), keep_lists);
 }
 
 __global__ void k_copy4(Field4 dst, Field4 src, size_t n)
@@ -3091,11 +3112,17 @@ struct Solver2D {
         launches += 1;
     }
 
-    // lists: the step's worklists are built too (without dt), as soon as the masks and levels are
-    // final.
+    // Begins the step (k_begin or k_begin_copy) as well.  lists: the step's worklists are built too (without dt),
+    // as soon as the masks and levels are final.
     void enq_prepare(const StepState* s, bool lists = false)
     {
-        if (prep_mode == 0 && s == st && prep_blocks > 0) {
+        const bool persistent = prep_mode == 0 && s == st && prep_blocks > 0;
+        if (persistent || scalar) {
+            launch(k_begin, 1, 1, st, 0);
+            after("k_begin");
+            launches += 1;
+        }
+        if (persistent) {
             PrepArgs A;
             A.g = g;
             A.q = q;
@@ -3123,8 +3150,8 @@ struct Solver2D {
         }
         // mask_temp = mask0
         if (!scalar) {
-            launch(k_copy_bit_all, pb(words()), 256, m, plane, 0, kBitTemp, s);
-            after("k_copy_bit_all");
+            launch(k_begin_copy, pb(words()), 256, m, plane, 0, kBitTemp, st);
+            after("k_begin_copy");
             launches += 1;
         }
         enq_fwt(s, !scalar);
@@ -3174,8 +3201,10 @@ struct Solver2D {
     // zeroed by the boundary fill before this launch.
     void enq_alpha(Field4 f, int bit, int stage, bool with_cfl, double* axp = nullptr, double* ayp = nullptr)
     {
-        dim3 grid((unsigned)(g.pitch / 4 + 31) / 32, (unsigned)(g.ny + 8 * kAlphaRows - 1) / (8 * kAlphaRows));
-        launch(k_alpha, grid, 256, g, f, m, bit, axp ? axp : ax[stage], ayp ? ayp : ay[stage],
+        const long warps = (long)(g.pitch / 32) * g.ny;  // at one row a warp
+        const int rows = (int)std::min<long>(kAlphaMaxRows, std::max<long>(1, warps / (8L * 2 * face_blocks)));
+        dim3 grid((unsigned)(g.pitch / 32), (unsigned)(g.ny + 8 * rows - 1) / (8 * rows));
+        launch(k_alpha, grid, 256, g, f, m, bit, rows, axp ? axp : ax[stage], ayp ? ayp : ay[stage],
                with_cfl ? &st->mv : nullptr, st, with_cfl ? &st->nonfinite : nullptr);
         after("k_alpha");
         launches += 1;
@@ -3273,9 +3302,6 @@ struct Solver2D {
     {
         launches = 0;
         mark();
-        launch(k_begin, 1, 1, st, 0);
-        after("k_begin");
-        launches += 1;
         // the worklists (and the zeroing of stage 2/3's speed accumulators) are built beside the
         // last PrepareEuler passes; dt is computed by the first stage's y-face launch
         enq_prepare(st, true);
@@ -3356,8 +3382,6 @@ struct Solver2D {
     void enq_step_scalar()
     {
         launches = 0;
-        launch(k_begin, 1, 1, st, 0);
-        launches += 1;
         enq_prepare(st);
         enq_bc(alias(q.p[0]), st);
         launch(k_dt, 1, 1, g, st);
@@ -3576,7 +3600,6 @@ struct Solver2D {
     {
         int rc = write_params(tol, 0, 0, 1, 0);
         if (rc) return rc;
-        launch(k_begin, 1, 1, st, 0);
         enq_prepare(st);
         AWCM_CUDA_TRY(cudaGetLastError());
         AWCM_CUDA_TRY(cudaStreamSynchronize(stream));
