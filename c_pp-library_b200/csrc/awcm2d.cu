@@ -1056,8 +1056,16 @@ struct Bits2 {
     uint32_t* m[4];    // mask0..mask3
     uint32_t* aux;     // mask0 before its adjacent zone
     uint32_t* live[3];
-    int nwx;           // words per row
+    int nwx;            // words per row
+    unsigned nwx_inv;   // ceil(2^32 / nwx) where that divides every word's index exactly, else 0
+    int rpw, chunks;    // close_rows_per_warp, warps per row of a longer one
+    unsigned chunks_inv;
 };
+// u / d by the reciprocal inv = ceil(2^32 / d) (0: by division).  Exact while u (inv d - 2^32) < 2^32.
+__device__ __forceinline__ unsigned quotient(unsigned u, unsigned d, unsigned inv)
+{
+    return inv ? __umulhi(u, inv) : u / d;
+}
 
 __device__ __forceinline__ uint32_t bshl(uint32_t below, uint32_t cur, int s) { return __funnelshift_l(below, cur, s); }
 __device__ __forceinline__ uint32_t bshr(uint32_t cur, uint32_t above, int s) { return __funnelshift_r(cur, above, s); }
@@ -1094,13 +1102,14 @@ __device__ __forceinline__ void load32(const uint8_t* p, uint32_t (&v)[8])
 }
 
 // mask0 of the byte plane with the banding (see ph_band_copy) into aux; the other planes cleared.
-__device__ void bits_pack(const Grid2& g, const Bits2& B, const uint8_t* __restrict__ m, Span sp)
+__device__ void bits_pack(const Grid2& g, const Bits2& B, const uint8_t* __restrict__ m, Span sp, int done)
 {
     const unsigned n = (unsigned)g.rows * (unsigned)B.nwx;
     for (unsigned w = sp.t0; w < n; w += sp.stride) {
-        const int r = (int)(w / (unsigned)B.nwx), x = (int)w - r * B.nwx, j = r - kGhost;
+        const int r = (int)quotient(w, (unsigned)B.nwx, B.nwx_inv), x = (int)w - r * B.nwx, j = r - kGhost;
         uint32_t v[8];
         load32(m + 32 * (size_t)w, v);
+        if (done) return;
         uint32_t b = gather_bits(v, 0);
         if (j >= 0 && j < g.ny) {
             uint32_t inner = j >= 2 && j <= g.ny - 3 ? cols_in(x, 2, g.nx - 3) : 0u;
@@ -1138,14 +1147,15 @@ __device__ __forceinline__ void push_cols(uint32_t* P, int nwx, int x, uint32_t 
 }
 
 // AddAdjacentZone (see ph_aaz) of aux into mask0 (clear before).
-__device__ void bits_zone(const Grid2& g, const Bits2& B, Span sp)
+__device__ void bits_zone(const Grid2& g, const Bits2& B, Span sp, int done)
 {
     const int NX = g.nx - 1, NY = g.ny - 1, nwx = B.nwx;
     const unsigned n = (unsigned)g.rows * (unsigned)nwx;
     for (unsigned w = sp.t0; w < n; w += sp.stride) {
         const uint32_t a = B.aux[w];
+        if (done) return;
         if (!a) continue;
-        const int r = (int)(w / (unsigned)nwx), x = (int)w - r * nwx, j = r - kGhost;
+        const int r = (int)quotient(w, (unsigned)nwx, B.nwx_inv), x = (int)w - r * nwx, j = r - kGhost;
         uint32_t own = a;
         const uint32_t d = j >= 0 && j <= NY ? a & cols_in(x, 0, NX) : 0u;
         if (d) {
@@ -1176,8 +1186,8 @@ __device__ void bits_zone(const Grid2& g, const Bits2& B, Span sp)
     }
 }
 
-// CheckReconstruction (AWCM_MANAGER_2D.h:63-158, see ph_cr) of the level of spacing h = 2^t.  Rows j =
-// 0, h, 2h .. are base + (j >> sh) nwx (base: row 0).  Up to h = 16 it is a gather:
+// CheckReconstruction (AWCM_MANAGER_2D.h:63-158, see ph_cr) of the level of spacing h = 2^t of the plane
+// whose row 0 is `base`.  done: nothing is written.  Up to h = 16 it is a gather:
 //   an odd row takes, on its even columns, the columns -+h, -+3h of its own d3 points;
 //   an even row takes from the odd rows -+h, -+3h their d3 points (marking d1 points there) and d2 points
 //   (marking c points), and on its even columns the columns -+h, -+3h of those d3 points and of its own
@@ -1195,8 +1205,9 @@ __host__ __device__ __forceinline__ long close_warps(long nr, int nwx)
     if (nwx > 32) return nr * ((nwx + kCloseKeep - 1) / kCloseKeep);
     return (nr + close_rows_per_warp(nwx) - 1) / close_rows_per_warp(nwx);
 }
-__device__ void bits_close_level(const Grid2& g, uint32_t* base, int sh, int nwx, int t, Span sp)
+__device__ void bits_close_level(const Grid2& g, const Bits2& B, uint32_t* base, int t, Span sp, int done)
 {
+    const int nwx = B.nwx;
     const int h = 1 << t, NX = g.nx - 1, NY = g.ny - 1;
     if (t >= 5) {
         const unsigned nc = (unsigned)(NX >> t) + 1u, n = ((unsigned)(NY >> t) + 1u) * nc;
@@ -1206,8 +1217,8 @@ __device__ void bits_close_level(const Grid2& g, uint32_t* base, int sh, int nwx
             const int i = (int)a << t, j = (int)b << t, D = 2 * h;
             if (!io && (!jo || i == 0 || i == NX)) continue;
             if (!jo && (j == 0 || j == NY)) continue;
-            if (!((base[(size_t)(j >> sh) * nwx + (i >> 5)] >> kGhost) & 1u)) continue;
-            auto put = [&](int ii, int jj) { atomicOr(&base[(size_t)(jj >> sh) * nwx + (ii >> 5)], 1u << kGhost); };
+            if (!((base[(size_t)j * nwx + (i >> 5)] >> kGhost) & 1u) || done) continue;
+            auto put = [&](int ii, int jj) { atomicOr(&base[(size_t)jj * nwx + (ii >> 5)], 1u << kGhost); };
             int is = 0, js = 0, k;
             if (io) predict_stencil(i, D, NX, is, k);
             if (jo) predict_stencil(j, D, NY, js, k);
@@ -1221,31 +1232,30 @@ __device__ void bits_close_level(const Grid2& g, uint32_t* base, int sh, int nwx
         return;
     }
     const int nr = (NY >> t) + 1, lane = threadIdx.x & 31;
-    const int rpw = close_rows_per_warp(nwx), chunks = nwx > 32 ? (nwx + kCloseKeep - 1) / kCloseKeep : 1;
+    const int lane_row = nwx <= 32 ? (lane * (65536 / nwx + 1)) >> 16 : 0;  // lane / nwx
     const int fa = h + kGhost, fb = 3 * h + kGhost, la = NX - h + kGhost;
-    const unsigned n = (unsigned)close_warps(nr, nwx);
+    const unsigned n = nwx > 32 ? (unsigned)nr * (unsigned)B.chunks : (unsigned)((nr + B.rpw - 1) / B.rpw);
     for (unsigned it = sp.t0 >> 5; it < n; it += sp.stride >> 5) {
         int rr, x;
         bool keep;
         if (nwx <= 32) {
-            const int sub = lane / nwx;
-            x = lane - sub * nwx;
-            rr = (int)it * rpw + sub;
-            keep = sub < rpw && rr < nr;
+            x = lane - lane_row * nwx;
+            rr = (int)it * B.rpw + lane_row;
+            keep = lane_row < B.rpw && rr < nr;
         } else {
-            rr = (int)(it / (unsigned)chunks);
-            x = ((int)it - rr * chunks) * kCloseKeep - kCloseLeft + lane;
+            rr = (int)quotient(it, (unsigned)B.chunks, B.chunks_inv);
+            x = ((int)it - rr * B.chunks) * kCloseKeep - kCloseLeft + lane;
             keep = lane >= kCloseLeft && lane < kCloseLeft + kCloseKeep;
         }
         const bool on = x >= 0 && x < nwx && rr < nr && (nwx > 32 || keep);
         const int j = rr << t;
         const bool odd_row = rr & 1;
-        uint32_t* R = base + (size_t)(j >> sh) * nwx + x;
+        uint32_t* R = base + (size_t)j * nwx + x;
         uint32_t own = 0, v = 0;  // this word; the rows around it (even rows)
         if (on) {
             own = *R;
             if (!odd_row) {
-                const long st = (long)(h >> sh) * nwx;
+                const long st = (long)h * nwx;
 #pragma unroll
                 for (int k = -3; k <= 3; k += 2)
                     if (j + k * h > 0 && j + k * h < NY) v |= R[k * st];
@@ -1284,7 +1294,7 @@ __device__ void bits_close_level(const Grid2& g, uint32_t* base, int sh, int nwx
         // the d3 and d2 points around (d2 points do not include the two end columns)
         mark |= v & cols_mult(x, t) & cols_in(x, 1, NX - 1);
         mark &= in;
-        if (keep && on && (mark & ~own)) *R = own | mark;
+        if (keep && on && (mark & ~own) && !done) *R = own | mark;
     }
 }
 
@@ -1297,7 +1307,8 @@ __device__ __forceinline__ uint32_t padded2(const Grid2& g, const uint32_t* M, i
 // ComputeLevel(level_{k-1}, mask_{k-1}), mask_k = mask_{k-1} and AddPointForDifferentiation(mask_k,
 // level_{k-1}) (see ph_cl, ph_apd) into mask_k (clear before).  A distance of the level search is one shift of
 // the word's row and a word of two other rows.
-__device__ void bits_next(const Grid2& g, const Bits2& B, int8_t* lvl, int k, Span sp)
+// (Fetching the words of four distances ahead of their use was slower: most words end at distance 1.)
+__device__ void bits_next(const Grid2& g, const Bits2& B, int8_t* lvl, int k, Span sp, int done)
 {
     const int NX = g.nx - 1, NY = g.ny - 1, nwx = B.nwx;
     const uint32_t* A = B.m[k - 1];
@@ -1305,20 +1316,22 @@ __device__ void bits_next(const Grid2& g, const Bits2& B, int8_t* lvl, int k, Sp
     const unsigned n = (unsigned)g.rows * (unsigned)nwx;
     for (unsigned w = sp.t0; w < n; w += sp.stride) {
         const uint32_t a = A[w], was = B.live[k - 1][w];
+        if (done) return;
         if (!(a | was)) continue;
-        const int r = (int)(w / (unsigned)nwx), x = (int)w - r * nwx, j = r - kGhost;
+        const int r = (int)quotient(w, (unsigned)nwx, B.nwx_inv), x = (int)w - r * nwx, j = r - kGhost;
         const uint32_t in = j >= 0 && j <= NY ? cols_in(x, 0, NX) : 0u;
         const uint32_t on = a & in;
         uint32_t own = a;
         if (on | (was & in)) {
-            uint32_t lev4[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            uint32_t S[5] = {0, 0, 0, 0, 0};  // the level, bit-sliced
             const uint32_t mid = j >= 1 && j <= NY - 1 ? cols_in(x, 1, NX - 1) : 0u;
             uint32_t* row = M + (size_t)r * nwx;
-            // the points `s` of level maxl - e: their level bytes, and their stencils into mask_k
+            // the points `s` of level maxl - e: their levels, and their stencils into mask_k
             auto take = [&](uint32_t s, int e) {
-                const uint32_t lev = (uint32_t)(g.maxl - e);
+                const int lev = g.maxl - e;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) lev4[q] |= spread4(s >> (4 * q)) * lev;
+                for (int b = 0; b < 5; ++b)
+                    if ((lev >> b) & 1) S[b] |= s;
                 s &= mid;
                 if (!s) return;
                 if (e == 0) {
@@ -1347,30 +1360,43 @@ __device__ void bits_next(const Grid2& g, const Bits2& B, int8_t* lvl, int k, Sp
             uint32_t todo = on;
             if (todo) {
                 const uint32_t l = padded2(g, A, nwx, r, x - 1), rt = padded2(g, A, nwx, r, x + 1);
-                for (int e = 0; e <= g.maxl && todo; ++e) {
+                // most points have a neighbour at distance 1
+                const uint32_t got = todo & (padded2(g, A, nwx, r - 1, x) | padded2(g, A, nwx, r + 1, x) | bshl(l, a, 1) | bshr(a, rt, 1));
+                todo &= ~got;
+                if (got) take(got, 0);
+                for (int e = 1; e <= g.maxl && todo; ++e) {
                     const int d = 1 << e;
                     uint32_t near = padded2(g, A, nwx, r - d, x) | padded2(g, A, nwx, r + d, x);
                     if (e < 5) near |= bshl(l, a, d) | bshr(a, rt, d);
                     else near |= padded2(g, A, nwx, r, x - (d >> 5)) | padded2(g, A, nwx, r, x + (d >> 5));
-                    const uint32_t got = todo & near;
-                    todo &= ~got;
-                    if (got) take(got, e);
+                    const uint32_t hit = todo & near;
+                    todo &= ~hit;
+                    if (hit) take(hit, e);
                 }
             }
             int8_t* lp = lvl + 32 * (size_t)w;
-            for (uint32_t u = todo; u; u &= u - 1) {  // no neighbour found: the level stays as it was
+            uint32_t odd = 0;  // the levels of the points without any neighbour stay as they were
+            for (uint32_t u = todo; u; u &= u - 1) {
                 const int b = __ffs(u) - 1, lev = lp[b];
                 if (lev >= 0 && lev <= g.maxl) take(1u << b, g.maxl - lev);
-                else lev4[b >> 2] |= (uint32_t)(uint8_t)lev << (8 * (b & 3));
+                else odd |= 1u << b;
             }
             uint32_t* lw = reinterpret_cast<uint32_t*>(lp);
-            if (in == ~0u) {
+            uint32_t lev4[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                lev4[q] = 0;
+#pragma unroll
+                for (int b = 0; b < 5; ++b)
+                    if (S[b]) lev4[q] |= spread4(S[b] >> (4 * q)) << b;
+            }
+            if (in == ~0u && !odd) {
                 reinterpret_cast<uint4*>(lw)[0] = make_uint4(lev4[0], lev4[1], lev4[2], lev4[3]);
                 reinterpret_cast<uint4*>(lw)[1] = make_uint4(lev4[4], lev4[5], lev4[6], lev4[7]);
             } else {
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    const uint32_t keep = ~(spread4(in >> (4 * q)) * 255u);  // ghosts keep theirs
+                    const uint32_t keep = ~(spread4((in & ~odd) >> (4 * q)) * 255u);  // ghosts keep theirs too
                     if (keep != ~0u) lw[q] = (lw[q] & keep) | lev4[q];
                 }
             }
@@ -1383,13 +1409,14 @@ __device__ void bits_next(const Grid2& g, const Bits2& B, int8_t* lvl, int k, Sp
 }
 
 // The planes mask0..mask3 back into the byte plane (its other bits stay).
-__device__ void bits_unpack(const Grid2& g, const Bits2& B, uint8_t* m, Span sp)
+__device__ void bits_unpack(const Grid2& g, const Bits2& B, uint8_t* m, Span sp, int done)
 {
     const unsigned n = (unsigned)g.rows * (unsigned)B.nwx;
     for (unsigned w = sp.t0; w < n; w += sp.stride) {
         uint32_t v[8], o[8];
         load32(m + 32 * (size_t)w, v);
         const uint32_t b[4] = {B.m[0][w], B.m[1][w], B.m[2][w], B.m[3][w]};
+        if (done) return;
         uint32_t diff = 0;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
@@ -1408,32 +1435,27 @@ __device__ void bits_unpack(const Grid2& g, const Bits2& B, uint8_t* m, Span sp)
 __global__ void k_bits_pack(Grid2 g, Bits2 B, const uint8_t* m, const StepState* st)
 {
     pdl_begin();
-    if (st && st->done) return;
-    bits_pack(g, B, m, grid_span());
+    bits_pack(g, B, m, grid_span(), st ? st->done : 0);
 }
 __global__ void k_bits_zone(Grid2 g, Bits2 B, const StepState* st)
 {
     pdl_begin();
-    if (st && st->done) return;
-    bits_zone(g, B, grid_span());
+    bits_zone(g, B, grid_span(), st ? st->done : 0);
 }
-__global__ void k_bits_close(Grid2 g, uint32_t* M, int nwx, int t, const StepState* st)
+__global__ void k_bits_close(Grid2 g, Bits2 B, int k, int t, const StepState* st)
 {
     pdl_begin();
-    if (st && st->done) return;
-    bits_close_level(g, M + (size_t)kGhost * nwx, 0, nwx, t, grid_span());
+    bits_close_level(g, B, B.m[k] + (size_t)kGhost * B.nwx, t, grid_span(), st ? st->done : 0);
 }
 __global__ void k_bits_next(Grid2 g, Bits2 B, int8_t* lvl, int k, const StepState* st)
 {
     pdl_begin();
-    if (st && st->done) return;
-    bits_next(g, B, lvl, k, grid_span());
+    bits_next(g, B, lvl, k, grid_span(), st ? st->done : 0);
 }
 __global__ void k_bits_unpack(Grid2 g, Bits2 B, uint8_t* m, const StepState* st)
 {
     pdl_begin();
-    if (st && st->done) return;
-    bits_unpack(g, B, m, grid_span());
+    bits_unpack(g, B, m, grid_span(), st ? st->done : 0);
 }
 constexpr int kBitsThreads = 1024;
 // The whole chain of a small grid in one CTA, its planes in shared memory: no launch per pass.
@@ -1447,21 +1469,21 @@ __global__ void __launch_bounds__(kBitsThreads) k_bits_all(Grid2 g, Bits2 B, uin
     B.aux = rows_sm;
     for (int k = 0; k < 4; ++k) B.m[k] = rows_sm + (k + 1) * n;
     const Span sp{threadIdx.x, blockDim.x};
-    bits_pack(g, B, m, sp);
+    bits_pack(g, B, m, sp, 0);
     __syncthreads();
-    bits_zone(g, B, sp);
+    bits_zone(g, B, sp, 0);
     __syncthreads();
     for (int k = 0; k <= 3; ++k) {
         if (k) {
-            bits_next(g, B, k == 1 ? l0 : k == 2 ? l1 : l2, k, sp);
+            bits_next(g, B, k == 1 ? l0 : k == 2 ? l1 : l2, k, sp, 0);
             __syncthreads();
         }
         for (int t = 0; t < g.maxl; ++t) {
-            bits_close_level(g, B.m[k] + (size_t)kGhost * B.nwx, 0, B.nwx, t, sp);
+            bits_close_level(g, B, B.m[k] + (size_t)kGhost * B.nwx, t, sp, 0);
             __syncthreads();
         }
     }
-    bits_unpack(g, B, m, sp);
+    bits_unpack(g, B, m, sp, 0);
 }
 
 // ------------------------------------------------------------------- persistent PrepareEuler
@@ -2219,11 +2241,12 @@ __global__ void __launch_bounds__(128, AWCM_FACE_MIN_CTAS)
            const double* __restrict__ alpha, const StepState* st, StepState* dt_st)
 {
     pdl_begin();
-    if (st->done) return;
+    const int done = st->done;
+    const unsigned n = *count;
+    if (done) return;
     // dt_st: this launch also computes the step's dt (from the CFL speed of the scan before it);
     // the faces do not read it, the point updates after them do
     if (dt_st && blockIdx.x == 0 && threadIdx.x == 0) compute_dt(g, dt_st);
-    const unsigned n = *count;
     const long stride = (long)gridDim.x * blockDim.x;
     for (long e = gtid(); e < n; e += stride) {
         const uint32_t idx = list[e];
@@ -2358,9 +2381,10 @@ __global__ void __launch_bounds__(256) k_update(Grid2 g, Field4 in, Field4 inx, 
                                                 const StepState* st)
 {
     pdl_begin();
-    if (st->done) return;
+    const int done = st->done;
     const unsigned n0 = *nf, n = n0 + *nc;
     const double sc = st->sc[g.maxl];
+    if (done) return;
     const long stride = (long)gridDim.x * blockDim.x;
     for (long e = gtid(); e < n; e += stride) {
         if (e < n0) update_fin_point<KIND>(g, in, out, qn, fx, fy, lf[e], sc);
@@ -2773,6 +2797,14 @@ struct Solver2D {
         }
         AWCM_CUDA_TRY(cudaMalloc(&m, plane));
         bits.nwx = g.pitch / 32;
+        auto inverse = [](unsigned long long d, unsigned long long most) -> unsigned {
+            const unsigned long long inv = ((1ull << 32) + d - 1) / d;  // exact while u (inv d - 2^32) < 2^32
+            return d > 1 && most * (inv * d - (1ull << 32)) < (1ull << 32) ? (unsigned)inv : 0u;
+        };
+        bits.nwx_inv = inverse(bits.nwx, plane / 32);
+        bits.rpw = close_rows_per_warp(bits.nwx);
+        bits.chunks = (bits.nwx + kCloseKeep - 1) / kCloseKeep;
+        bits.chunks_inv = inverse(bits.chunks, (unsigned long long)g.rows * bits.chunks);
         AWCM_CUDA_TRY(cudaMalloc(&bits_mem, 8 * bit_words() * sizeof(uint32_t)));
         for (int k = 0; k < 4; ++k) bits.m[k] = bits_mem + k * bit_words();
         bits.aux = bits_mem + 4 * bit_words();
@@ -3068,7 +3100,7 @@ struct Solver2D {
             for (int t = 0; t < g.maxl; ++t) {
                 const long rows = (((long)g.ny - 1) >> t) + 1;
                 const long threads = t < 5 ? 32 * close_warps(rows, bits.nwx) : rows * (((g.nx - 1) >> t) + 1);
-                launch(k_bits_close, pb(threads), 256, g, bits.m[k], bits.nwx, t, s);
+                launch(k_bits_close, pb(threads), 256, g, bits, k, t, s);
                 after("k_bits_close");
             }
             launches += (k ? 1 : 0) + g.maxl;
