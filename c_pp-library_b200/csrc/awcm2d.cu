@@ -45,6 +45,18 @@ struct StepState {
     unsigned spin_limit;           // polls before a grid-barrier wait gives up (0 = kSpinLimit)
 };
 
+// u / d by the reciprocal inv = ceil(2^32 / d) (0: by division).  Exact while u (inv d - 2^32) < 2^32.
+__device__ __forceinline__ unsigned quotient(unsigned u, unsigned d, unsigned inv)
+{
+    return inv ? __umulhi(u, inv) : u / d;
+}
+// Row (from the bottom ghost row) of point a of a plane, and of 32-bit word w of a byte plane.
+__device__ __forceinline__ unsigned row_of(const Grid2& g, unsigned a) { return quotient(a, (unsigned)g.pitch, g.pitch_inv); }
+__device__ __forceinline__ unsigned row_of_word(const Grid2& g, unsigned w)
+{
+    return quotient(w, (unsigned)g.pitch / 4u, g.wpr_inv);
+}
+
 __device__ __forceinline__ int ctz_or(int v, int big) { return v == 0 ? big : __ffs(v) - 1; }
 
 // Sub-band geometry of level lev: which 0 = d1 (half x, coarse y), 1 = d2 (coarse x, half y),
@@ -56,7 +68,8 @@ struct Band {
 __host__ __device__ __forceinline__ Band band_of(const Grid2& g, int lev, int which)
 {
     const int D = g.D(lev), h = D >> 1;
-    const int MX = (g.nx - 1) / D, MY = (g.ny - 1) / D;
+    // by shifts: a dozen divisions by the spacing were a quarter of a small launch
+    const int MX = (g.nx - 1) >> (g.maxl - lev), MY = (g.ny - 1) >> (g.maxl - lev);
     Band b;
     b.D = D;
     switch (which) {
@@ -154,8 +167,8 @@ struct MaskWord {
 };
 __device__ __forceinline__ MaskWord mask_word(const Grid2& g, unsigned w)
 {
-    const unsigned a = 4u * w, row = a / (unsigned)g.pitch;
-    return MaskWord{w, (int)(a - row * (unsigned)g.pitch) - kGhost, (int)row - kGhost};
+    const unsigned row = row_of_word(g, w);
+    return MaskWord{w, (int)(4u * w - row * (unsigned)g.pitch) - kGhost, (int)row - kGhost};
 }
 __device__ __forceinline__ unsigned plane_words(const Grid2& g) { return (unsigned)g.pitch * (unsigned)g.rows / 4u; }
 // Lanes (bit L = byte L) whose column i0 + L lies in [lo, hi].
@@ -392,7 +405,7 @@ __device__ __forceinline__ void fine_rows(const Grid2& g, const uint8_t* m, int 
         const unsigned v = mp[row0 + t];
         unsigned hit = ((v >> b1) | (v >> b2)) & kLaneBits;
         if (!hit) continue;
-        const unsigned r = t / wpr, wi = t - r * wpr;
+        const unsigned r = row_of_word(g, t), wi = t - r * wpr;
         const int j = (int)r, i0 = 4 * (int)wi - kGhost;
         hit &= lane_bits(lanes_in(i0, 0, g.nx - 1));
         while (hit) {
@@ -487,8 +500,7 @@ __device__ void ph_cr(const Grid2& g, uint8_t* __restrict__ m, int lev, int bit,
 constexpr int kRowScanMaxH = 2;
 __device__ __forceinline__ unsigned rowscan_n(const Grid2& g, int lev, int rows)
 {
-    const int h = g.D(lev) >> 1;
-    const unsigned nr = (unsigned)((g.ny - 1) / h) + 1u;  // rows 0, h, .., NY
+    const unsigned nr = (unsigned)((g.ny - 1) >> (g.maxl - lev - 1)) + 1u;  // rows 0, h, .., NY
     const unsigned wpr = (unsigned)g.pitch / 4u;
     return (rows == 2 ? nr : (rows == 0 ? (nr + 1u) / 2u : nr / 2u)) * wpr;
 }
@@ -500,7 +512,7 @@ __device__ __forceinline__ unsigned rowscan_word(const Grid2& g, int lev, int ro
 {
     const int h = g.D(lev) >> 1;
     const unsigned wpr = (unsigned)g.pitch / 4u;
-    const unsigned r = t / wpr, wi = t - r * wpr;
+    const unsigned r = row_of_word(g, t), wi = t - r * wpr;
     const unsigned rr = rows == 2 ? r : 2u * r + (unsigned)rows;
     j = (int)rr * h;
     i0 = 4 * (int)wi - kGhost;
@@ -512,7 +524,7 @@ __device__ __forceinline__ unsigned rowscan_word(const Grid2& g, int lev, int ro
 // Sub-band of the level point (i, j) (h = spacing): 2 = d3, 0 = d1, 1 = d2, -1 = none.
 __device__ __forceinline__ int rowscan_band(const Grid2& g, int i, int j, int h)
 {
-    const bool io = (i / h) & 1, jo = (j / h) & 1;
+    const bool io = i & h, jo = j & h;  // i and j are multiples of h
     if (io && jo) return 2;
     if (io) return (j == 0 || j == g.ny - 1) ? -1 : 0;
     if (jo) return (i == 0 || i == g.nx - 1) ? -1 : 1;
@@ -1061,11 +1073,6 @@ struct Bits2 {
     int rpw, chunks;    // close_rows_per_warp, warps per row of a longer one
     unsigned chunks_inv;
 };
-// u / d by the reciprocal inv = ceil(2^32 / d) (0: by division).  Exact while u (inv d - 2^32) < 2^32.
-__device__ __forceinline__ unsigned quotient(unsigned u, unsigned d, unsigned inv)
-{
-    return inv ? __umulhi(u, inv) : u / d;
-}
 
 __device__ __forceinline__ uint32_t bshl(uint32_t below, uint32_t cur, int s) { return __funnelshift_l(below, cur, s); }
 __device__ __forceinline__ uint32_t bshr(uint32_t cur, uint32_t above, int s) { return __funnelshift_r(cur, above, s); }
@@ -1952,8 +1959,9 @@ __device__ void alpha_list_run(const Grid2& g, Field4 f, const uint32_t* __restr
         double sx = 0;
         if (on) {
             const uint32_t idx = e < n0 ? la[e] : lb[e - n0];
-            const int i = (int)(idx % (uint32_t)g.pitch) - kGhost;
-            j = (int)(idx / (uint32_t)g.pitch) - kGhost;
+            const unsigned row = row_of(g, idx);
+            const int i = (int)(idx - row * (unsigned)g.pitch) - kGhost;
+            j = (int)row - kGhost;
             const double q[4] = {f.p[0][idx], f.p[1][idx], f.p[2][idx], f.p[3][idx]};
             double sy;
             speeds(q, g.gamma, sx, sy);
@@ -2250,8 +2258,8 @@ __global__ void __launch_bounds__(128, AWCM_FACE_MIN_CTAS)
     const long stride = (long)gridDim.x * blockDim.x;
     for (long e = gtid(); e < n; e += stride) {
         const uint32_t idx = list[e];
-        const int ii = (int)(idx % (uint32_t)g.pitch) - kGhost;
-        const int jj = (int)(idx / (uint32_t)g.pitch) - kGhost;
+        const unsigned row = row_of(g, idx);
+        const int ii = (int)(idx - row * (unsigned)g.pitch) - kGhost, jj = (int)row - kGhost;
         const long step = DIR == 0 ? 1 : g.pitch;
         const double al = DIR == 0 ? alpha[jj] : alpha[ii];
         SharedDiv dv;
@@ -2314,8 +2322,8 @@ __device__ __forceinline__ void update_crs_point(const Grid2& g, Field4 in, Fiel
                                                  const int8_t* __restrict__ lvl, size_t a, const StepState* st)
 {
     const int NX = g.nx - 1, NY = g.ny - 1;
-    const int i = (int)((unsigned)a % (unsigned)g.pitch) - kGhost;
-    const int j = (int)((unsigned)a / (unsigned)g.pitch) - kGhost;
+    const unsigned row = row_of(g, (unsigned)a);
+    const int i = (int)((unsigned)a - row * (unsigned)g.pitch) - kGhost, j = (int)row - kGhost;
     const int lev = lvl[a];
     if (lev < 0 || lev > g.maxl) return;
     const int d = g.D(lev);
@@ -2456,8 +2464,8 @@ __global__ void __launch_bounds__(256) k_update_crs_scalar(Grid2 g, const double
     const int NX = g.nx - 1, NY = g.ny - 1;
     for (unsigned e = gtid(); e < n; e += gridDim.x * blockDim.x) {
         const size_t a = list[e];
-        const int i = (int)((unsigned)a % (unsigned)g.pitch) - kGhost;
-        const int j = (int)((unsigned)a / (unsigned)g.pitch) - kGhost;
+        const unsigned row = row_of(g, (unsigned)a);
+        const int i = (int)((unsigned)a - row * (unsigned)g.pitch) - kGhost, j = (int)row - kGhost;
         const int lev = lvl[a];
         if (lev < 0 || lev > g.maxl) continue;
         const int d = g.D(lev);
@@ -2772,6 +2780,13 @@ struct Solver2D {
         }
         g.W = make_weights();
         plane = (size_t)g.pitch * g.rows;
+        // reciprocals for quotient(): of d for dividends below `most`
+        auto inverse = [](unsigned long long d, unsigned long long most) -> unsigned {
+            const unsigned long long inv = ((1ull << 32) + d - 1) / d;
+            return d > 1 && most * (inv * d - (1ull << 32)) < (1ull << 32) ? (unsigned)inv : 0u;
+        };
+        g.pitch_inv = inverse(g.pitch, plane);
+        g.wpr_inv = inverse(g.pitch / 4, plane / 4);
         AWCM_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         AWCM_CUDA_TRY(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
         AWCM_CUDA_TRY(cudaStreamCreateWithFlags(&side2, cudaStreamNonBlocking));
@@ -2797,10 +2812,6 @@ struct Solver2D {
         }
         AWCM_CUDA_TRY(cudaMalloc(&m, plane));
         bits.nwx = g.pitch / 32;
-        auto inverse = [](unsigned long long d, unsigned long long most) -> unsigned {
-            const unsigned long long inv = ((1ull << 32) + d - 1) / d;  // exact while u (inv d - 2^32) < 2^32
-            return d > 1 && most * (inv * d - (1ull << 32)) < (1ull << 32) ? (unsigned)inv : 0u;
-        };
         bits.nwx_inv = inverse(bits.nwx, plane / 32);
         bits.rpw = close_rows_per_warp(bits.nwx);
         bits.chunks = (bits.nwx + kCloseKeep - 1) / kCloseKeep;
