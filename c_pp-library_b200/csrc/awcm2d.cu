@@ -64,6 +64,7 @@ __device__ __forceinline__ int ctz_or(int v, int big) { return v == 0 ? big : __
 // (Wavelet/MRA_GRID_UNIFORM_2D.h:101-131).
 struct Band {
     int i0, j0, cx, cy, D;
+    unsigned inv;  // reciprocal of cx (see quotient)
 };
 __host__ __device__ __forceinline__ Band band_of(const Grid2& g, int lev, int which)
 {
@@ -78,6 +79,7 @@ __host__ __device__ __forceinline__ Band band_of(const Grid2& g, int lev, int wh
         case 2: b.i0 = h, b.cx = MX, b.j0 = h, b.cy = MY; break;
         default: b.i0 = D, b.cx = MX - 1, b.j0 = D, b.cy = MY - 1; break;
     }
+    b.inv = which == 0 || which == 2 ? g.cx_inv[lev] : g.cx1_inv[lev];
     if (b.cx < 0) b.cx = 0;
     if (b.cy < 0) b.cy = 0;
     return b;
@@ -121,8 +123,9 @@ __device__ __forceinline__ bool union_point(const Grid2& g, int lev, const int (
         const Band b = band_of(g, lev, which[k]);
         const unsigned n = (unsigned)b.cx * (unsigned)b.cy;
         if (t < n) {
-            i = b.i0 + (int)(t % (unsigned)b.cx) * b.D;
-            j = b.j0 + (int)(t / (unsigned)b.cx) * b.D;
+            const unsigned q = quotient(t, (unsigned)b.cx, b.inv);
+            i = b.i0 + (int)(t - q * (unsigned)b.cx) * b.D;
+            j = b.j0 + (int)q * b.D;
             w = which[k];
             return true;
         }
@@ -198,6 +201,11 @@ struct Span {
     unsigned t0, stride;
 };
 __device__ __forceinline__ Span grid_span() { return Span{gtid(), gridDim.x * blockDim.x}; }
+
+// Every transform pass gives a thread to each point of its sub-bands, active or not.  Scanning mask rows instead,
+// word by word past the empty ones, was slower at every size but the largest (129^2 168 us a step against 145,
+// 641x385 282 against 270, 2049x513 412 against 392, 2049^2 760 against 764): a point's mask byte is one load
+// that its warp shares, a scanned word's points follow one another on one lane.
 
 __device__ __forceinline__ unsigned band_n(const Grid2& g, int lev, int which)
 {
@@ -381,72 +389,6 @@ __device__ void ph_iwt(const Grid2& g, double* __restrict__ q, const uint8_t* __
     }
 }
 
-// The finest level (point spacing 1) of the step's transforms as a row scan: word t of the grid rows
-// is tested for the two mask bits that can make one of its points need work before its row and
-// column are decoded (most words have neither), and the set lanes are classified by parity:
-// 2 = d3 (odd, odd), 0 = d1 (odd, even; not the top or bottom row), 1 = d2 (even, odd; not the left
-// or right column), 3 = c (even, even; not on the boundary), -1 = none -- the extents of band_of.
-__device__ __forceinline__ int fine_band(const Grid2& g, int i, int j)
-{
-    const bool io = i & 1, jo = j & 1;
-    if (io && jo) return 2;
-    if (io) return (j == 0 || j == g.ny - 1) ? -1 : 0;
-    if (jo) return (i == 0 || i == g.nx - 1) ? -1 : 1;
-    return (i == 0 || i == g.nx - 1 || j == 0 || j == g.ny - 1) ? -1 : 3;
-}
-// f(i, j, a, byte) for the grid points of the scanned words whose byte has bit b1 or b2.
-template <class F>
-__device__ __forceinline__ void fine_rows(const Grid2& g, const uint8_t* m, int b1, int b2, Span sp, F&& f)
-{
-    const unsigned wpr = (unsigned)g.pitch / 4u, row0 = (unsigned)kGhost * wpr;
-    const unsigned n = (unsigned)g.ny * wpr;
-    const unsigned* mp = reinterpret_cast<const unsigned*>(m);
-    for (unsigned t = sp.t0; t < n; t += sp.stride) {
-        const unsigned v = mp[row0 + t];
-        unsigned hit = ((v >> b1) | (v >> b2)) & kLaneBits;
-        if (!hit) continue;
-        const unsigned r = row_of_word(g, t), wi = t - r * wpr;
-        const int j = (int)r, i0 = 4 * (int)wi - kGhost;
-        hit &= lane_bits(lanes_in(i0, 0, g.nx - 1));
-        while (hit) {
-            const int L = (__ffs(hit) - 1) >> 3;
-            hit &= hit - 1;
-            f(i0 + L, j, 4u * (row0 + t) + (unsigned)L, (v >> (8 * L)) & 0xffu);
-        }
-    }
-}
-// Row-scan forms of the finest level (idle mode / sparse zeroing, see ph_fwt_a and ph_iwt).
-__device__ void ph_fwt_a_fine(const Grid2& g, double* __restrict__ q, double* __restrict__ tb,
-                              uint8_t* __restrict__ m, double tol, Span sp)
-{
-    fine_rows(g, m, 0, 0, sp, [&](int i, int j, size_t a, unsigned) {
-        const int w = fine_band(g, i, j);
-        if (w >= 0 && w != 3) fwt_a_point(g, q, tb, m, i, j, a, 2, w, tol, true);
-    });
-}
-__device__ void ph_fwt_b_fine(const Grid2& g, double* __restrict__ q, const double* __restrict__ tb,
-                              const uint8_t* __restrict__ m, Span sp)
-{
-    fine_rows(g, m, 0, kBitTemp, sp, [&](int i, int j, size_t a, unsigned byte) {
-        const int w = fine_band(g, i, j);
-        if (w == 3) {
-            if (byte & 1u) fwt_b_point(g, q, tb, m, i, j, a, 2, true);
-        } else if (w == 0 || w == 1) {
-            if ((byte >> kBitTemp) & 1u) q[a] = tb[a];
-        }
-    });
-}
-template <int PH>
-__device__ void ph_iwt_fine(const Grid2& g, double* __restrict__ q, const uint8_t* __restrict__ m, int bit, Span sp)
-{
-    fine_rows(g, m, bit, kBitTemp, sp, [&](int i, int j, size_t a, unsigned byte) {
-        const int w = fine_band(g, i, j);
-        if (PH == 0 ? w != 3 : PH == 1 ? (w != 0 && w != 1) : w != 2) return;
-        if ((byte >> bit) & 1u) iwt_point(g, q, i, j, a, 2, w);
-        else q[a] = 0;  // in mask_temp, not in the mask
-    });
-}
-
 // CheckReconstruction of one level (AWCM_MANAGER_2D.h:63-158) in one phase.  The reference runs
 // d3 -> d1 -> d2 so that d1/d2 points switched on by a d3 point also mark their stencils; those
 // stencils ((is..is+3D, n) for a d1 point (i, n), (m, js..js+3D) for a d2 point (m, j)) lie inside
@@ -626,36 +568,6 @@ __device__ void ph_interp(const Grid2& g, Field4 q, const uint8_t* __restrict__ 
         const unsigned mb = m[a];
         if (!((mb >> work) & 1u) || ((mb >> from_bit) & 1u)) continue;
         interp_point(g, q, i, j, a, D, w, p0);
-    }
-}
-
-// Row-scan form of ph_interp for the fine levels: PH 0 scans every row of the level (d1 on the
-// even ones, d2 on the odd ones), PH 1 only the odd rows (d3).
-template <int PH>
-__device__ void ph_interp_rows(const Grid2& g, Field4 q, const uint8_t* __restrict__ m, int lev, int work, int from_bit,
-                               int p0, Span sp)
-{
-    const int D = g.D(lev), h = D >> 1;
-    const int rows = PH == 0 ? 2 : 1;
-    const unsigned n = rowscan_n(g, lev, rows);
-    const unsigned* mp = reinterpret_cast<const unsigned*>(m);
-    const unsigned row0 = (unsigned)kGhost * ((unsigned)g.pitch / 4u);
-    for (unsigned t = sp.t0; t < n; t += sp.stride) {
-        // every row of the finest detail level (h = 1, PH 0): word t of the grid rows
-        if (PH == 0 && h == 1 && !((mp[row0 + t] >> work) & ~(mp[row0 + t] >> from_bit) & kLaneBits)) continue;
-        int j, i0;
-        unsigned wdx;
-        const unsigned lanes = rowscan_word(g, lev, rows, t, j, i0, wdx);
-        const unsigned v = mp[wdx];
-        unsigned hit = (v >> work) & ~(v >> from_bit) & lane_bits(lanes);
-        while (hit) {
-            const int L = (__ffs(hit) - 1) >> 3;
-            hit &= hit - 1;
-            const int i = i0 + L;
-            const int w = rowscan_band(g, i, j, h);
-            if (w < 0 || (PH == 0) == (w == 2)) continue;
-            interp_point(g, q, i, j, 4u * wdx + L, D, w, p0);
-        }
     }
 }
 
@@ -912,15 +824,13 @@ __global__ void k_fwt_a(Grid2 g, double* q, double* tb, uint8_t* m, int lev, int
 {
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
-    if (idle && lev == g.maxl - 1) ph_fwt_a_fine(g, q, tb, m, st->tol, grid_span());
-    else ph_fwt_a(g, q, tb, m, lev, st->tol, idle != 0, grid_span());
+    ph_fwt_a(g, q, tb, m, lev, st->tol, idle != 0, grid_span());
 }
 __global__ void k_fwt_b(Grid2 g, double* q, const double* tb, const uint8_t* m, int lev, int idle, const StepState* st)
 {
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
-    if (idle && lev == g.maxl - 1) ph_fwt_b_fine(g, q, tb, m, grid_span());
-    else ph_fwt_b(g, q, tb, m, lev, idle != 0, grid_span());
+    ph_fwt_b(g, q, tb, m, lev, idle != 0, grid_span());
 }
 template <int PH>
 __global__ void k_iwt(Grid2 g, double* q, const uint8_t* m, int lev, int bit, int sparse, const StepState* st)
@@ -928,8 +838,7 @@ __global__ void k_iwt(Grid2 g, double* q, const uint8_t* m, int lev, int bit, in
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
     const bool zero_all = !sparse || !st || st->full_zero;
-    if (!zero_all && lev == g.maxl - 1) ph_iwt_fine<PH>(g, q, m, bit, grid_span());
-    else ph_iwt<PH>(g, q, m, lev, bit, zero_all, grid_span());
+    ph_iwt<PH>(g, q, m, lev, bit, zero_all, grid_span());
 }
 __global__ void k_cr(Grid2 g, uint8_t* m, int lev, int bit, const StepState* st)
 {
@@ -993,14 +902,6 @@ __global__ void k_interp(Grid2 g, Field4 q, const uint8_t* m, int lev, int work,
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
     ph_interp<PH>(g, q, m, lev, work, from_bit, p0, grid_span());
-}
-template <int PH>
-__global__ void k_interp_rows(Grid2 g, Field4 q, const uint8_t* m, int lev, int work, int from_bit, int p0,
-                              const StepState* st)
-{
-    pdl_begin();
-    AWCM_SKIP_IF_DONE(st);
-    ph_interp_rows<PH>(g, q, m, lev, work, from_bit, p0, grid_span());
 }
 // The first launch of an Euler step: k_begin's bookkeeping by its first thread, and mask_temp = mask0.
 // Nothing in it reads what the bookkeeping writes.
@@ -2787,6 +2688,11 @@ struct Solver2D {
         };
         g.pitch_inv = inverse(g.pitch, plane);
         g.wpr_inv = inverse(g.pitch / 4, plane / 4);
+        for (int lev = 0; lev < g.maxl; ++lev) {
+            const int MX = (g.nx - 1) >> (g.maxl - lev);
+            g.cx_inv[lev] = inverse(MX, plane);
+            g.cx1_inv[lev] = MX > 1 ? inverse(MX - 1, plane) : 0u;
+        }
         AWCM_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         AWCM_CUDA_TRY(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
         AWCM_CUDA_TRY(cudaStreamCreateWithFlags(&side2, cudaStreamNonBlocking));
@@ -3070,17 +2976,10 @@ struct Solver2D {
             launches += 1;
         }
         for (int lev = top + 1; lev < g.maxl; ++lev) {
-            if (row_scan(lev)) {
-                launch(k_interp_rows<0>, pb(rowscan_threads(lev, 2)), 256, g, q, m, lev, work, from, p0, s);
-                after("k_interp_rows<0>");
-                launch(k_interp_rows<1>, pb(rowscan_threads(lev, 1)), 256, g, q, m, lev, work, from, p0, s);
-                after("k_interp_rows<1>");
-            } else {
-                launch(k_interp<0>, pb(band_count(lev, 0) + band_count(lev, 1)), 256, g, q, m, lev, work, from, p0, s);
-                after("k_interp<0>");
-                launch(k_interp<1>, pb(band_count(lev, 2)), 256, g, q, m, lev, work, from, p0, s);
-                after("k_interp<1>");
-            }
+            launch(k_interp<0>, pb(band_count(lev, 0) + band_count(lev, 1)), 256, g, q, m, lev, work, from, p0, s);
+            after("k_interp<0>");
+            launch(k_interp<1>, pb(band_count(lev, 2)), 256, g, q, m, lev, work, from, p0, s);
+            after("k_interp<1>");
             launches += 2;
         }
     }

@@ -16,6 +16,7 @@ struct Grid2 {
     double wz_delta;  // > 0: tau = sqrt((b0-b2)^2 + wz_delta^2) instead of |b0 - b2| (0 as in the reference)
     const int8_t* bcf;  // kind AWCM_BC_GENERIC: BOUNDARY_CONDITION of every ghosted point (plane layout)
     unsigned pitch_inv, wpr_inv;  // reciprocals of pitch and pitch / 4, 0 where a division is needed
+    unsigned cx_inv[kMaxLevels], cx1_inv[kMaxLevels];  // of the details per row of a level, and of one less
     int wt_i, wt_j;     // kind AWCM_BC_WIND_TUNNEL: the step corner int(0.6/dx), int(0.2/dy)
     Weights W;
     __host__ __device__ __forceinline__ size_t at(int i, int j) const
