@@ -812,11 +812,7 @@ __device__ __forceinline__ void begin_step(StepState* st, bool done, int keep_li
 }
 
 // ------------------------------------------------------------------------ standalone kernels
-#ifndef AWCM_COARSE_POINTS
-#define AWCM_COARSE_POINTS 1024
-#endif
 constexpr int kCoarseThreads = 1024;
-constexpr long kCoarsePoints = AWCM_COARSE_POINTS;
 #define AWCM_SKIP_IF_DONE(st) \
     if ((st) && (st)->done) return
 
@@ -852,49 +848,97 @@ __global__ void k_cr_rows(Grid2 g, uint8_t* m, int lev, int bit, const StepState
     AWCM_SKIP_IF_DONE(st);
     ph_cr_rows(g, m, lev, bit, grid_span());
 }
-// The coarse levels top, top-1 .. 0 (0 .. top) of a transform in one CTA: a level of a few thousand points
-// takes about as long there as its launch does.
-__global__ void __launch_bounds__(kCoarseThreads) k_fwt_coarse(Grid2 g, double* q, double* tb, uint8_t* m, int top, int idle,
+// The coarse levels top, top-1 .. 0 (0 .. top) of a transform in one CTA, on a copy of their grid in shared
+// memory: c is that grid (the points whose indices are multiples of 2^s, s = maxl-1-top; the same levels), and a
+// pass on it is the pass on the plane.  A phase takes about a microsecond there, as a launch of its own 4 to 6.
+extern __shared__ double coarse_sm[];
+struct CoarsePlanes {
+    const Grid2 &g, &c;
+    int s, n;  // shift; doubles of a plane of c
+    __device__ CoarsePlanes(const Grid2& g_, const Grid2& c_) : g(g_), c(c_), s(g_.maxl - c_.maxl), n(c_.pitch * c_.ny) {}
+    // Plane k, so that point (i, j) of c is at plane(k)[c.at(i, j)]; the mask bytes follow `planes` planes.
+    __device__ double* plane(int k) const { return coarse_sm + (size_t)k * n - origin(); }
+    __device__ uint8_t* mask(int planes) const { return reinterpret_cast<uint8_t*>(coarse_sm + (size_t)planes * n) - origin(); }
+    __device__ size_t origin() const { return c.at(0, 0); }
+    // f(a, b) for the points: place a in the plane, b in the copy.
+    template <class F>
+    __device__ void each(F&& f) const
+    {
+        const unsigned np = (unsigned)c.nx * (unsigned)c.ny;
+        for (unsigned u = threadIdx.x; u < np; u += blockDim.x) {
+            const int j = (int)(u / (unsigned)c.nx), i = (int)(u - (unsigned)j * (unsigned)c.nx);
+            f(g.at(i << s, j << s), c.at(i, j));
+        }
+    }
+};
+__global__ void __launch_bounds__(kCoarseThreads) k_fwt_coarse(Grid2 g, Grid2 c, double* q, uint8_t* m, int idle,
                                                               const StepState* st)
 {
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
+    const CoarsePlanes P(g, c);
+    double *Q = P.plane(0), *T = P.plane(1);
+    uint8_t* M = P.mask(2);
+    P.each([&](size_t a, size_t b) { Q[b] = q[a], M[b] = m[a]; });
+    __syncthreads();
     const Span sp{threadIdx.x, blockDim.x};
-    for (int lev = top; lev >= 0; --lev) {
-        ph_fwt_a(g, q, tb, m, lev, st->tol, idle != 0, sp);
+    for (int lev = c.maxl - 1; lev >= 0; --lev) {
+        ph_fwt_a(c, Q, T, M, lev, st->tol, idle != 0, sp);
         __syncthreads();
-        ph_fwt_b(g, q, tb, m, lev, idle != 0, sp);
+        ph_fwt_b(c, Q, T, M, lev, idle != 0, sp);
         __syncthreads();
     }
+    P.each([&](size_t a, size_t b) { q[a] = Q[b], m[a] = M[b]; });
 }
-__global__ void __launch_bounds__(kCoarseThreads) k_iwt_coarse(Grid2 g, double* q, const uint8_t* m, int top, int bit, int sparse,
+__global__ void __launch_bounds__(kCoarseThreads) k_iwt_coarse(Grid2 g, Grid2 c, double* q, const uint8_t* m, int bit, int sparse,
                                                               const StepState* st)
 {
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
     const bool zero_all = !sparse || !st || st->full_zero;
+    const CoarsePlanes P(g, c);
+    double* Q = P.plane(0);
+    uint8_t* M = P.mask(1);
+    P.each([&](size_t a, size_t b) { Q[b] = q[a], M[b] = m[a]; });
+    __syncthreads();
     const Span sp{threadIdx.x, blockDim.x};
-    for (int lev = 0; lev <= top; ++lev) {
-        ph_iwt<0>(g, q, m, lev, bit, zero_all, sp);
+    for (int lev = 0; lev < c.maxl; ++lev) {
+        ph_iwt<0>(c, Q, M, lev, bit, zero_all, sp);
         __syncthreads();
-        ph_iwt<1>(g, q, m, lev, bit, zero_all, sp);
+        ph_iwt<1>(c, Q, M, lev, bit, zero_all, sp);
         __syncthreads();
-        ph_iwt<2>(g, q, m, lev, bit, zero_all, sp);
+        ph_iwt<2>(c, Q, M, lev, bit, zero_all, sp);
         __syncthreads();
     }
+    P.each([&](size_t a, size_t b) { q[a] = Q[b]; });
 }
-__global__ void __launch_bounds__(kCoarseThreads) k_interp_coarse(Grid2 g, Field4 q, const uint8_t* m, int top, int work,
+__global__ void __launch_bounds__(kCoarseThreads) k_interp_coarse(Grid2 g, Grid2 c, Field4 q, const uint8_t* m, int work,
                                                                  int from_bit, int p0, const StepState* st)
 {
     pdl_begin();
     AWCM_SKIP_IF_DONE(st);
+    const CoarsePlanes P(g, c);
+    const Field4 Q{{P.plane(0), P.plane(1), P.plane(2), P.plane(3)}};
+    uint8_t* M = P.mask(4);
+    P.each([&](size_t a, size_t b) {
+        M[b] = m[a];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k >= p0) Q.p[k][b] = q.p[k][a];
+    });
+    __syncthreads();
     const Span sp{threadIdx.x, blockDim.x};
-    for (int lev = 0; lev <= top; ++lev) {
-        ph_interp<0>(g, q, m, lev, work, from_bit, p0, sp);
+    for (int lev = 0; lev < c.maxl; ++lev) {
+        ph_interp<0>(c, Q, M, lev, work, from_bit, p0, sp);
         __syncthreads();
-        ph_interp<1>(g, q, m, lev, work, from_bit, p0, sp);
+        ph_interp<1>(c, Q, M, lev, work, from_bit, p0, sp);
         __syncthreads();
     }
+    P.each([&](size_t a, size_t b) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k >= p0) q.p[k][a] = Q.p[k][b];
+    });
 }
 template <int PH>
 __global__ void k_interp(Grid2 g, Field4 q, const uint8_t* m, int lev, int work, int from_bit, int p0, const StepState* st)
@@ -2727,6 +2771,9 @@ struct Solver2D {
         bits.aux = bits_mem + 4 * bit_words();
         for (int k = 0; k < 3; ++k) bits.live[k] = bits_mem + (5 + k) * bit_words();
         mark_levels();
+        AWCM_CUDA_TRY(cudaFuncSetAttribute(k_fwt_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem));
+        AWCM_CUDA_TRY(cudaFuncSetAttribute(k_iwt_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem));
+        AWCM_CUDA_TRY(cudaFuncSetAttribute(k_interp_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem));
         AWCM_CUDA_TRY(cudaFuncSetAttribute(k_bits_all, cudaFuncAttributeMaxDynamicSharedMemorySize, kBitsSmem));
         for (int s = 0; s < kStages; ++s) {
             AWCM_CUDA_TRY(cudaMalloc(&ax[s], sizeof(double) * g.ny));
@@ -2877,14 +2924,32 @@ struct Solver2D {
         const Band b = band_of(g, lev, which);
         return (long)b.cx * b.cy;
     }
-    // The finest of the coarse levels that share one launch (-1: none; one level alone gains nothing; the
-    // finest level has its own form).
+    // The finest of the coarse levels that share one launch (-1: none): those of up to 1024 details, one a thread,
+    // and on grids of many levels one of up to 4096 behind them.  Steps without / with up to 1024 / with up to 4096:
+    // 129^2 (3 levels) 142 / 138.5 / 141 us, 641x385 264 / 250 / 248, 2049^2 758 / 752 / 740; 2049x513, whose first
+    // level has 3072 details, 390 / 390 / 403.
     int coarse_top() const
     {
         int top = -1;
-        while (top + 2 < g.maxl && details(top + 1) <= kCoarsePoints) ++top;
+        while (top + 1 < g.maxl && details(top + 1) <= kCoarseThreads) ++top;
+        if (top >= 0 && g.maxl >= 5 && top + 1 < g.maxl && details(top + 1) <= 4 * kCoarseThreads) ++top;
+        while (top >= 0 && coarse_bytes(coarse_grid(top), 4) > kCoarseSmem) --top;
         return top;
     }
+    // The grid of the levels 0 .. top, its rows odd in length (the banks of a column).
+    Grid2 coarse_grid(int top) const
+    {
+        Grid2 c = g;
+        const int s = g.maxl - 1 - top;
+        c.nx = ((g.nx - 1) >> s) + 1;
+        c.ny = ((g.ny - 1) >> s) + 1;
+        c.maxl = top + 1;
+        c.pitch = c.nx | 1;
+        c.rows = c.ny;
+        return c;
+    }
+    static constexpr size_t kCoarseSmem = 200 * 1024;
+    static size_t coarse_bytes(const Grid2& c, int planes) { return (size_t)c.pitch * c.ny * (planes * sizeof(double) + 1); }
     long details(int lev) const { return band_count(lev, 0) + band_count(lev, 1) + band_count(lev, 2); }
 
     // Fine levels (point spacing <= kRowScanMaxH) scan mask words row by row and skip empty words;
@@ -2928,7 +2993,8 @@ struct Solver2D {
             launches += 2;
         }
         if (top >= 0) {
-            launch(k_fwt_coarse, 1, kCoarseThreads, g, q.p[0], fx.p[0], m, top, id, s);
+            const Grid2 c = coarse_grid(top);
+            launch_smem(k_fwt_coarse, 1, kCoarseThreads, coarse_bytes(c, 2), g, c, q.p[0], m, id, s);
             after("k_fwt_coarse");
             launches += 1;
         }
@@ -2939,7 +3005,8 @@ struct Solver2D {
     {
         const int sp = sparse ? 1 : 0, top = coarse_top();
         if (top >= 0) {
-            launch(k_iwt_coarse, 1, kCoarseThreads, g, q.p[0], m, top, bit, sp, s);
+            const Grid2 c = coarse_grid(top);
+            launch_smem(k_iwt_coarse, 1, kCoarseThreads, coarse_bytes(c, 1), g, c, q.p[0], m, bit, sp, s);
             after("k_iwt_coarse");
             launches += 1;
         }
@@ -2971,7 +3038,8 @@ struct Solver2D {
     {
         const int top = coarse_top();
         if (top >= 0) {
-            launch(k_interp_coarse, 1, kCoarseThreads, g, q, m, top, work, from, p0, s);
+            const Grid2 c = coarse_grid(top);
+            launch_smem(k_interp_coarse, 1, kCoarseThreads, coarse_bytes(c, 4), g, c, q, m, work, from, p0, s);
             after("k_interp_coarse");
             launches += 1;
         }
