@@ -60,11 +60,15 @@ __device__ __forceinline__ void atomic_add(double* p, double v)
     if (v != 0.0) atomicAdd(p, v);
 }
 
+// Divisors of the WENO-Z reverse: smoothness + eps, tau and the weights' sum.
+constexpr int kSafeWenoLo = -640, kSafeWenoHi = 900;
+
 // ---------------------------------------------------------------------------- WENO-Z reverse
 // Reverse of recon_left<kWenoZ> (WENOZ5::ReconstructLeft, WENOZ.h:75-104): adds d(out)/d(input)
 // times ob to g[0..4] for the inputs (ll, l, c, r, rr) and returns out itself.  tau = |b0 - b2| is differentiated as
 // sign(b0 - b2); with delta > 0, tau = sqrt((b0 - b2)^2 + delta^2) and dtau = (b0 - b2) / tau.
-__device__ __forceinline__ double recon_left_vjp(double ll, double l, double c, double r, double rr, double ob,
+template <class DV>
+__device__ __forceinline__ double recon_left_vjp(DV& dv, double ll, double l, double c, double r, double rr, double ob,
                                                  double eps, double delta, double* g)
 {
     const double A0 = c - 2 * r + rr, B0 = 3 * c - 4 * r + rr;
@@ -77,14 +81,20 @@ __device__ __forceinline__ double recon_left_vjp(double ll, double l, double c, 
     double tau, sg;
     if (delta > 0) {
         tau = sqrt(dl * dl + delta * delta);
-        sg = dl / tau;
+        dv.range(tau, kSafeWenoLo, kSafeWenoHi);
+        sg = dv.quot_pos(dl, dv.by(tau));
     } else {
         tau = fabs(dl);
         sg = dl > 0 ? 1.0 : (dl < 0 ? -1.0 : 0.0);
     }
-    const double ie0 = 1.0 / (b0 + eps), ie1 = 1.0 / (b1 + eps), ie2 = 1.0 / (b2 + eps);
+    const double d0 = b0 + eps, d1 = b1 + eps, d2 = b2 + eps;
+    dv.range(d0, kSafeWenoLo, kSafeWenoHi), dv.range(d1, kSafeWenoLo, kSafeWenoHi);
+    dv.range(d2, kSafeWenoLo, kSafeWenoHi);
+    const double ie0 = dv.recip(d0), ie1 = dv.recip(d1), ie2 = dv.recip(d2);
     const double a0 = 0.1 * (1 + tau * ie0), a1 = 0.6 * (1 + tau * ie1), a2 = 0.3 * (1 + tau * ie2);
-    const double iS = 1.0 / (a0 + a1 + a2);
+    const double as = a0 + a1 + a2;
+    dv.range(as, kSafeWenoLo, kSafeWenoHi);
+    const double iS = dv.recip(as);
     const double w0 = a0 * iS, w1 = a1 * iS, w2 = a2 * iS;
     const double P0 = kC11_6 * c + kCm7_6 * r + kC1_3 * rr;
     const double P1 = kC1_3 * l + kC5_6 * c + kCm1_6 * r;
@@ -115,10 +125,9 @@ __device__ __forceinline__ double recon_left_vjp(double ll, double l, double c, 
 // Reverse of flux2<DIR> (EULER_EQUATION_2D::ComputeFu/ComputeGu, EULER_EQUATION.h:74-99):
 // adds (dF/dq)^T fb to qb.
 template <int DIR>
-__device__ __forceinline__ void flux2_vjp(const double* q, double g, const double* fb, double* qb)
+__device__ __forceinline__ void flux2_vjp(const double* q, double iq0, double g, const double* fb, double* qb)
 {
     const double gm1 = g - 1;
-    const double iq0 = 1.0 / q[0];
     const double u = q[1] * iq0, v = q[2] * iq0;
     const double p = gm1 * (q[3] - 0.5 * (q[1] * q[1] + q[2] * q[2]) * iq0);
     double pb = 0;
@@ -158,19 +167,20 @@ __device__ __forceinline__ void flux2_vjp(const double* q, double g, const doubl
 }
 
 struct RoeAdj {
-    double u, v, H, c, kc;
+    double u, v, H, c, kc, i2c;  // i2c = 1 / (2 c)
 };
 
 // Reverse of inv2<DIR> (ROE_SOLVER_2D::Inversion_X/_Y, ROESOLVER.h:73-96): adds (dx/db)^T xb to
 // bb and the parameter adjoints to P.
-template <int DIR>
-__device__ __forceinline__ void inv2_vjp(const RoeAdj& R, const double* b, const double* xb, double* bb, RoeAdj& P)
+template <int DIR, class DV>
+__device__ __forceinline__ void inv2_vjp(DV& dv, const RoeAdj& R, const typename DV::Divisor& c1, const double* b,
+                                         const double* xb, double* bb, RoeAdj& P)
 {
     const double u = R.u, v = R.v, H = R.H, c = R.c, kc = R.kc;
     const double A = H - u * u - v * v;
     const double y3 = DIR == 0 ? A * b[0] + u * b[1] + v * b[2] - b[3] : A * b[0] + v * b[2] + u * b[1] - b[3];
     const double x3 = y3 * kc;
-    const double i2c = 0.5 / c;
+    const double i2c = R.i2c;
     const double y4 = DIR == 0 ? b[1] + (c - u) * b[0] - c * x3 : b[2] + (c - v) * b[0] - c * x3;
     const double x4 = y4 * i2c;
     // x1 = b0 - x3 - x4
@@ -179,7 +189,7 @@ __device__ __forceinline__ void inv2_vjp(const RoeAdj& R, const double* b, const
     const double x4b = xb[3] - xb[0];
     // x4 = y4 / (2c)
     const double y4b = x4b * i2c;
-    P.c -= x4b * x4 / c;
+    P.c -= dv.quot(x4b * x4, c1);
     if (DIR == 0) {
         bb[1] += y4b;
         bb[0] += y4b * (c - u);
@@ -217,39 +227,52 @@ __device__ __forceinline__ void inv2_vjp(const RoeAdj& R, const double* b, const
 // d(face flux)/d(six cells)^T ob (WENOZ_EULER_SOLVER_2D::ComputeFluxX/Y, WENOZ.h:236-320).
 // Forward values are recomputed here; alpha (the frozen LF speed) has no adjoint.  The 6 x 4
 // characteristic states and fluxes (and, in place, their adjoints) live in shared memory:
-// `sh` points at this thread's slot, element e at sh[e * kAdjThreads].
+// `sh` points at this thread's slot, element e at sh[e * kAdjThreads].  cell(p, q) reads cell p,
+// add(p, qb) adds to its adjoint; false, with nothing added, where the divisions of DV do not apply.
+// A face's hundred divisions are what its time went to: by shared reciprocals, with the cells read twice instead
+// of kept (no spills; 260 bytes before), the reverse sweep over 513 x 513 takes 22.8 instead of 25.0 ms for
+// 100 steps.  168 registers and 3 CTAs an SM spill and take 25.1.
 constexpr int kAdjThreads = 128;
-template <int DIR>
-__device__ void face_flux_2d_vjp(const double (&s)[6][4], double alpha, double g, const double* ob, double eps,
-                                 double delta, double (&gs)[6][4], double* sh)
+template <int DIR, class DV, class Cell, class Add>
+__device__ __forceinline__ bool face_flux_2d_vjp(DV& dv, const Cell& cell, const Add& add, double alpha, double g,
+                                                 const double* ob, double eps, double delta, double* sh)
 {
     auto RQs = [&](int p, int k) -> double& { return sh[(p * 4 + k) * kAdjThreads]; };
     auto RFs = [&](int p, int k) -> double& { return sh[(24 + p * 4 + k) * kAdjThreads]; };
     // ---- forward: Roe average of the face states s[2], s[3] (ROESOLVER.h:49-70)
-    const double* L = s[2];
-    const double* Rr = s[3];
+    double L[4], Rr[4];
+    cell(2, L), cell(3, Rr);
     const double gm1 = g - 1;
-    const double iL0 = 1.0 / L[0], iR0 = 1.0 / Rr[0];
+    dv.range(alpha, kSafeLo, kSafeAlpha);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) dv.range_or_0(ob[k], -1022, 200);
+    dv.range(L[0], -kSafeRho, kSafeRho), dv.range(Rr[0], -kSafeRho, kSafeRho);
+    const double iL0 = dv.recip(L[0]), iR0 = dv.recip(Rr[0]);
     const double KL = L[1] * L[1] + L[2] * L[2], KR = Rr[1] * Rr[1] + Rr[2] * Rr[2];
     const double pL = gm1 * (L[3] - 0.5 * KL * iL0), pR = gm1 * (Rr[3] - 0.5 * KR * iR0);
     const double HL = (L[3] + pL) * iL0, HR = (Rr[3] + pR) * iR0;
     const double uL = L[1] * iL0, uR = Rr[1] * iR0, vL = L[2] * iL0, vR = Rr[2] * iR0;
     const double sL = sqrt(L[0]), sR = sqrt(Rr[0]);
-    const double iden = 1.0 / (sL + sR);
+    const double iden = dv.recip(sL + sR);
     RoeAdj R;
     R.u = (sL * uL + sR * uR) * iden;
     R.v = (sL * vL + sR * vR) * iden;
     R.H = (sL * HL + sR * HR) * iden;
     const double q2 = R.u * R.u + R.v * R.v;
     R.c = sqrt(0.4 * (R.H - 0.5 * q2));
-    R.kc = 0.4 / (R.c * R.c);
+    dv.range(R.c, kSafeC, kSafeHi);
+    const auto c1 = dv.by(R.c);
+    const auto c2 = dv.twice(c1);
+    R.kc = dv.quot_pos(0.4, dv.by(R.c * R.c));
+    R.i2c = dv.quot_pos(0.5, c1);
     // ---- forward: characteristic variables and LF split of the six cells
 #pragma unroll
     for (int p = 0; p < 6; ++p) {
-        double f[4], rq[4], rf[4];
-        flux2<DIR>(s[p], g, f);
-        inv2<DIR>(R.u, R.v, R.H, R.c, R.kc, s[p], rq);
-        inv2<DIR>(R.u, R.v, R.H, R.c, R.kc, f, rf);
+        double s[4], f[4], rq[4], rf[4];
+        cell(p, s);
+        cell_flux2<DIR>(dv, s, g, f, nullptr);
+        inv2<DIR>(dv, R.u, R.v, R.H, R.c, R.kc, c2, s, rq);
+        inv2<DIR>(dv, R.u, R.v, R.H, R.c, R.kc, c2, f, rf);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             RQs(p, k) = rq[k];
@@ -284,8 +307,8 @@ __device__ void face_flux_2d_vjp(const double (&s)[6][4], double alpha, double g
         }
         // left_r = ReconstructLeft(fp4, fp3, fp2, fp1, fp0); right_l = ReconstructLeft(fm1..fm5)
         double gl[5] = {0, 0, 0, 0, 0}, gr[5] = {0, 0, 0, 0, 0};
-        S[k] = recon_left_vjp(fp[4], fp[3], fp[2], fp[1], fp[0], Sb[k], eps, delta, gl) +
-               recon_left_vjp(fm[1], fm[2], fm[3], fm[4], fm[5], Sb[k], eps, delta, gr);
+        S[k] = recon_left_vjp(dv, fp[4], fp[3], fp[2], fp[1], fp[0], Sb[k], eps, delta, gl) +
+               recon_left_vjp(dv, fm[1], fm[2], fm[3], fm[4], fm[5], Sb[k], eps, delta, gr);
         fpb[4] += gl[0], fpb[3] += gl[1], fpb[2] += gl[2], fpb[1] += gl[3], fpb[0] += gl[4];
         fmb[1] += gr[0], fmb[2] += gr[1], fmb[3] += gr[2], fmb[4] += gr[3], fmb[5] += gr[4];
 #pragma unroll
@@ -294,7 +317,7 @@ __device__ void face_flux_2d_vjp(const double (&s)[6][4], double alpha, double g
             RQs(p, k) = 0.5 * alpha * (fpb[p] - fmb[p]);
         }
     }
-    RoeAdj P{0, 0, 0, 0, 0};
+    RoeAdj P{0, 0, 0, 0, 0, 0};
     if (DIR == 0) {
         P.u += ob[1] * (S[0] + S[2] + S[3]) + ob[3] * (-S[0] * c + S[2] * u + S[3] * c);
         P.v += ob[2] * (S[0] + S[2] + S[3]) + ob[3] * (S[1] + S[2] * v);
@@ -305,23 +328,32 @@ __device__ void face_flux_2d_vjp(const double (&s)[6][4], double alpha, double g
         P.c += ob[2] * (S[3] - S[0]) + ob[3] * v * (S[3] - S[0]);
     }
     P.H += ob[3] * (S[0] + S[3]);
-    // ---- reverse: characteristic projections and physical fluxes
+    // every range is checked by here
+    if constexpr (DV::checked)
+        if (dv.bad) return false;
+    // ---- reverse: characteristic projections and physical fluxes.  The cells are read and their fluxes
+    // computed again rather than kept live across the WENO-Z reverse.
+    asm volatile("" ::: "memory");
+    double gl[4] = {0, 0, 0, 0}, gr[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int p = 0; p < 6; ++p) {
-        double f[4], fb[4] = {0, 0, 0, 0}, rqb[4], rfb[4];
-        flux2<DIR>(s[p], g, f);  // recomputed rather than kept live across the WENO-Z reverse
+        double s[4], go[4] = {0, 0, 0, 0}, f[4], fb[4] = {0, 0, 0, 0}, rqb[4], rfb[4];
+        double* gs = p == 2 ? gl : p == 3 ? gr : go;
+        cell(p, s);
+        cell_flux2<DIR>(dv, s, g, f, nullptr);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             rqb[k] = RQs(p, k);
             rfb[k] = RFs(p, k);
         }
-        inv2_vjp<DIR>(R, s[p], rqb, gs[p], P);
-        inv2_vjp<DIR>(R, f, rfb, fb, P);
-        flux2_vjp<DIR>(s[p], g, fb, gs[p]);
+        inv2_vjp<DIR>(dv, R, c1, s, rqb, gs, P);
+        inv2_vjp<DIR>(dv, R, c1, f, rfb, fb, P);
+        flux2_vjp<DIR>(s, dv.recip(s[0]), g, fb, gs);
+        if (p != 2 && p != 3) add(p, gs);
     }
     // ---- reverse: Roe average (kc = 0.4 / c^2, c = sqrt(0.4 (H - q2/2)))
-    P.c += P.kc * (-2.0 * R.kc / R.c);
-    const double ccb = P.c * 0.5 / R.c;
+    P.c += P.kc * dv.quot(-2.0 * R.kc, c1);
+    const double ccb = dv.quot(P.c * 0.5, c1);
     P.H += 0.4 * ccb;
     const double q2b = -0.2 * ccb;
     P.u += 2 * R.u * q2b;
@@ -334,7 +366,7 @@ __device__ void face_flux_2d_vjp(const double (&s)[6][4], double alpha, double g
     // H = (q3 + p)/q0, u = q1/q0, v = q2/q0, p = gm1 (q3 - K/(2 q0)), s = sqrt(q0)
     auto side = [&](const double* q, double iq0, double K, double Hs, double us, double vs, double sq, double sb,
                     double ub, double vb, double hb, double* qb) {
-        qb[0] += sb * 0.5 / sq;
+        qb[0] += dv.quot(sb * 0.5, dv.by(sq));
         qb[1] += ub * iq0;
         qb[0] -= ub * us * iq0;
         qb[2] += vb * iq0;
@@ -348,8 +380,10 @@ __device__ void face_flux_2d_vjp(const double (&s)[6][4], double alpha, double g
         qb[1] += 2 * q[1] * Kb;
         qb[2] += 2 * q[2] * Kb;
     };
-    side(L, iL0, KL, HL, uL, vL, sL, sLb, uLb, vLb, HLb, gs[2]);
-    side(Rr, iR0, KR, HR, uR, vR, sR, sRb, uRb, vRb, HRb, gs[3]);
+    side(L, iL0, KL, HL, uL, vL, sL, sLb, uLb, vLb, HLb, gl);
+    side(Rr, iR0, KR, HR, uR, vR, sR, sRb, uRb, vRb, HRb, gr);
+    add(2, gl), add(3, gr);
+    return true;
 }
 
 __device__ __forceinline__ bool fin_point(const Grid2& g, const uint8_t* m, const int8_t* lvl, int i, int j, int bit)
@@ -362,68 +396,69 @@ __device__ __forceinline__ bool fin_point(const Grid2& g, const uint8_t* m, cons
 // Face VJP over the stage's face list: the weight of face f (between f and f+1 along DIR) is
 // nu(f) for a finest-level point f (R_f += F_f) minus nu(f+1) for a finest point f+1
 // (R_{f+1} -= F_f); lam -= weight . dF_f/dcells.
-#ifndef AWCM_ADJ_MIN_CTAS
-#define AWCM_ADJ_MIN_CTAS 1  // 255 registers and 2 CTAs per SM; forcing more CTAs spills and runs slower
-#endif
-template <int DIR>
-__global__ void __launch_bounds__(kAdjThreads, AWCM_ADJ_MIN_CTAS) k_adj_face(AdjStage A, const uint32_t* __restrict__ list,
-                                                  const unsigned* __restrict__ count,
-                                                  const double* __restrict__ alpha)
+// One face with the divisions of DV; false, with nothing written, where they do not apply.
+template <int DIR, class DV>
+__device__ __forceinline__ bool face_vjp(const AdjStage& A, uint32_t idx, const double* __restrict__ alpha, double* sh)
 {
-    pdl_begin();
-    __shared__ double sh[48 * kAdjThreads];
     const Grid2& g = A.g;
-    const unsigned n = *count;
-    const unsigned stride = gridDim.x * blockDim.x;
     const long step = DIR == 0 ? 1 : g.pitch;
-    for (unsigned e = gtid(); e < n; e += stride) {
+    const int ii = (int)(idx % (uint32_t)g.pitch) - kGhost;
+    const int jj = (int)(idx / (uint32_t)g.pitch) - kGhost;
+    const int i1 = DIR == 0 ? ii + 1 : ii, j1 = DIR == 0 ? jj : jj + 1;
+    double w[4] = {0, 0, 0, 0};
+    bool any = false;
+    if (fin_point(g, A.m, A.lvl, ii, jj, A.bit)) {
+        for (int k = 0; k < 4; ++k) w[k] += A.nu.p[k][idx];
+        any = true;
+    }
+    if (fin_point(g, A.m, A.lvl, i1, j1, A.bit)) {
+        const size_t b = (size_t)idx + step;
+        for (int k = 0; k < 4; ++k) w[k] -= A.nu.p[k][b];
+        any = true;
+    }
+    if (!any || (w[0] == 0 && w[1] == 0 && w[2] == 0 && w[3] == 0)) return true;
+    const double al = DIR == 0 ? alpha[jj] : alpha[ii];
+    DV dv;
+    return face_flux_2d_vjp<DIR>(
+        dv,
+        [&](int p, double* s) {
+            const long a = (long)idx + (p - 2) * step;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s[k] = A.qin.p[k][a];
+        },
+        [&](int p, const double* gs) {
+            const long a = (long)idx + (p - 2) * step;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) atomic_sub(&A.lam.p[k][a], gs[k]);
+        },
+        al, g.gamma, w, g.wz_eps, g.wz_delta, sh);
+}
+template <int DIR>
+__device__ __noinline__ void face_vjp_any(const AdjStage& A, uint32_t idx, const double* alpha, double* sh)
+{
+    face_vjp<DIR, IeeeDiv>(A, idx, alpha, sh);
+}
+
+template <int DIR>
+__device__ __forceinline__ void face_list_vjp(const AdjStage& A, const uint32_t* __restrict__ list,
+                                              const unsigned* __restrict__ count, const double* __restrict__ alpha,
+                                              unsigned first, unsigned stride, double* sh)
+{
+    const unsigned n = *count;
+    for (unsigned e = first; e < n; e += stride) {
         const uint32_t idx = list[e];
-        const int ii = (int)(idx % (uint32_t)g.pitch) - kGhost;
-        const int jj = (int)(idx / (uint32_t)g.pitch) - kGhost;
-        const int i1 = DIR == 0 ? ii + 1 : ii, j1 = DIR == 0 ? jj : jj + 1;
-        double w[4] = {0, 0, 0, 0};
-        bool any = false;
-        if (fin_point(g, A.m, A.lvl, ii, jj, A.bit)) {
-            for (int k = 0; k < 4; ++k) w[k] += A.nu.p[k][idx];
-            any = true;
-        }
-        if (fin_point(g, A.m, A.lvl, i1, j1, A.bit)) {
-            const size_t b = (size_t)idx + step;
-            for (int k = 0; k < 4; ++k) w[k] -= A.nu.p[k][b];
-            any = true;
-        }
-        if (!any || (w[0] == 0 && w[1] == 0 && w[2] == 0 && w[3] == 0)) continue;
-        double s[6][4], gs[6][4];
-#pragma unroll
-        for (int p = 0; p < 6; ++p) {
-            const long a = (long)idx + (p - 2) * step;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                s[p][k] = A.qin.p[k][a];
-                gs[p][k] = 0;
-            }
-        }
-        const double al = DIR == 0 ? alpha[jj] : alpha[ii];
-        face_flux_2d_vjp<DIR>(s, al, g.gamma, w, g.wz_eps, g.wz_delta, gs, sh + threadIdx.x);
-#pragma unroll
-        for (int p = 0; p < 6; ++p) {
-            const long a = (long)idx + (p - 2) * step;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) atomic_sub(&A.lam.p[k][a], gs[p][k]);
-        }
+        if (!face_vjp<DIR, SharedDiv>(A, idx, alpha, sh)) face_vjp_any<DIR>(A, idx, alpha, sh);
     }
 }
 
 // Coarse points: R = dF + dG from physical fluxes at spacing d (central, or the reference's
 // one-sided forms at the edges; same branch selection as the forward).
-__global__ void __launch_bounds__(256) k_adj_coarse(AdjStage A)
+__device__ __forceinline__ void coarse_list_vjp(const AdjStage& A, unsigned first, unsigned stride)
 {
-    pdl_begin();
     const Grid2& g = A.g;
     const unsigned n = *A.ncrs;
-    const unsigned stride = gridDim.x * blockDim.x;
     const int NX = g.nx - 1, NY = g.ny - 1;
-    for (unsigned e = gtid(); e < n; e += stride) {
+    for (unsigned e = first; e < n; e += stride) {
         const size_t a = A.crs[e];
         const int i = (int)((unsigned)a % (unsigned)g.pitch) - kGhost;
         const int j = (int)((unsigned)a / (unsigned)g.pitch) - kGhost;
@@ -462,12 +497,33 @@ __global__ void __launch_bounds__(256) k_adj_coarse(AdjStage A)
                     q[k] = A.qin.p[k][b];
                     fb[k] = ws[o] * nu[k];
                 }
-                if (dir == 0) flux2_vjp<0>(q, g.gamma, fb, qb);
-                else flux2_vjp<1>(q, g.gamma, fb, qb);
+                if (dir == 0) flux2_vjp<0>(q, 1.0 / q[0], g.gamma, fb, qb);
+                else flux2_vjp<1>(q, 1.0 / q[0], g.gamma, fb, qb);
                 for (int k = 0; k < 4; ++k) atomic_sub(&A.lam.p[k][b], qb[k]);
             }
         }
     }
+}
+
+// A stage's x faces and its coarse points in one launch (DIR 0), then its y faces (DIR 1).  The faces are
+// bound by the latency of their arithmetic: 250 registers leave 8 warps on an SM, and a list of 15,000 to
+// 40,000 faces fills half to all of the 37,888 threads that fit.  The coarse points, bound by their loads and
+// atomics, run in the first `coarse` CTAs beside the faces instead of in a launch of their own.
+// 513 x 513, 100 steps, whole reverse sweep: three launches 22.8 ms, coarse points beside the x faces 20.8
+// (as the last CTAs 21.4, beside the y faces 20.9), x and y faces beside each other as well 22.0: the two
+// face codes together no longer fit the instruction cache.
+template <int DIR>
+__global__ void __launch_bounds__(kAdjThreads) k_adj_face(const __grid_constant__ AdjStage A, unsigned coarse)
+{
+    pdl_begin();
+    __shared__ double sh[48 * kAdjThreads];
+    if (blockIdx.x < coarse) {
+        coarse_list_vjp(A, gtid(), coarse * kAdjThreads);
+        return;
+    }
+    const unsigned first = gtid() - coarse * kAdjThreads, stride = (gridDim.x - coarse) * kAdjThreads;
+    if (DIR == 0) face_list_vjp<0>(A, A.xf, A.nxf, A.ax, first, stride, sh + threadIdx.x);
+    else face_list_vjp<1>(A, A.yf, A.nyf, A.ay, first, stride, sh + threadIdx.x);
 }
 
 // RK combination adjoints, one dense pass per stage over the plane (points off the grid are
@@ -619,10 +675,10 @@ __global__ void __launch_bounds__(kSeedThreads) k_sum_rows(const double* rowsum,
 
 void adj_launch_stage(const AdjStage& a, int face_blocks, cudaStream_t s)
 {
-    // 16 CTAs per SM over the face list (2 resident): 0.9 % faster reverse sweep than 8
-    launch_pdl(k_adj_face<0>, 2 * face_blocks, kAdjThreads, s, a, a.xf, a.nxf, a.ax);
-    launch_pdl(k_adj_face<1>, 2 * face_blocks, kAdjThreads, s, a, a.yf, a.nyf, a.ay);
-    launch_pdl(k_adj_coarse, face_blocks / 2, 256, s, a);
+    // face_blocks is 8 CTAs an SM: 16 for the faces (8: 0.5 % slower), 4 for the coarse points (8: 1 % slower)
+    const unsigned faces = 2 * face_blocks, coarse = face_blocks / 2;
+    launch_pdl(k_adj_face<0>, faces + coarse, kAdjThreads, s, a, coarse);
+    launch_pdl(k_adj_face<1>, faces, kAdjThreads, s, a, 0u);
 }
 
 void adj_launch_rk(int stage, const Grid2& g, size_t plane, const uint8_t* m, const int8_t* lvl, const double* sc,

@@ -60,6 +60,7 @@ struct IeeeDiv {
     __device__ __forceinline__ double twice(double b) { return 2 * b; }
     __device__ __forceinline__ double quot(double a, double b) { return a / b; }
     __device__ __forceinline__ double quot_pos(double a, double b) { return a / b; }
+    __device__ __forceinline__ double recip(double b) { return 1.0 / b; }
     __device__ __forceinline__ void range(double, int, int) {}
     __device__ __forceinline__ void range_or_0(double, int, int) {}
 };
@@ -94,6 +95,7 @@ struct SharedDiv {
         const bool ones = (((unsigned)__double2hiint(b) | 0xfff00000u) & lo) == 0xffffffffu;
         return Divisor{b, __hiloint2double(__double2hiint(y), __double2loint(y) | (ones ? 1 : 0))};
     }
+    __device__ __forceinline__ double recip(double b) { return by(b).y; }
     // The divisor 2 b from that of b.
     __device__ __forceinline__ Divisor twice(const Divisor& d) { return Divisor{2 * d.b, 0.5 * d.y}; }
     // a > 0, or any a where the sign of a zero quotient does not matter
