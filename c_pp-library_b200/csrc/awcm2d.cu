@@ -1960,15 +1960,18 @@ __global__ void __launch_bounds__(256) k_bc_alpha(Grid2 g, Field4 f, const uint3
 
 // dt = cfl dx / max speed, clipped to the output time (main_2d_euler(quad).cpp:76-83), and the
 // per-level stage factor dt / (dx 2^(maxl-lev)) of the RK updates.
-__device__ void compute_dt(const Grid2& g, StepState* st)
+__device__ __forceinline__ double step_dt(const Grid2& g, const StepState* st, bool& clipped)
 {
     double dt = st->cfl * g.dx / st->mv;
     if (st->dt_fixed > 0) dt = st->dt_fixed;
-    st->do_print = 0;
-    if (st->t + dt > st->t_end) {
-        dt = st->t_end - st->t;
-        st->do_print = 1;
-    }
+    clipped = st->t + dt > st->t_end;
+    return clipped ? st->t_end - st->t : dt;
+}
+__device__ void compute_dt(const Grid2& g, StepState* st)
+{
+    bool clipped;
+    const double dt = step_dt(g, st, clipped);
+    st->do_print = clipped ? 1 : 0;
     st->dt = dt;
     for (int lev = 0; lev <= g.maxl; ++lev) {
         const double dxl = g.dx * g.D(lev);
@@ -2154,64 +2157,41 @@ __global__ void __launch_bounds__(256) k_lists(Grid2 g, const uint8_t* __restric
 }
 
 // --------------------------------------------------------------------------------- stage kernels
-// Face flux from the compacted face list: x faces (DIR 0) read cells i-2..i+3 of row j, y faces
-// (DIR 1) cells j-2..j+3 of column i (WENOZ_EULER_SOLVER_2D::ComputeFluxX/Y, WENOZ.h:236-320).
-// What bounds it: the FP64 pipe (2 cycles a warp instruction).  With divisions by shared reciprocals
-// (SharedDiv) a million faces take 120-126 us against 165 us with IEEE divisions.
+// Face flux: x faces read cells i-2..i+3 of row j, y faces cells j-2..j+3 of column i with the momenta
+// exchanged (WENOZ_EULER_SOLVER_2D::ComputeFluxX/Y, WENOZ.h:236-320).  What bounds it: the FP64 pipe (2 cycles
+// a warp instruction).  With divisions by shared reciprocals (SharedDiv) a million faces take 120-126 us
+// against 165 us with IEEE divisions.
 // CUSTOM false: the reference's WENO-Z parameters as compile-time constants (eps 1e-40, exact
 // |b0 - b2|); true: the instance's runtime parameters (the differentiable mode).
 #ifndef AWCM_FACE_MIN_CTAS
 #define AWCM_FACE_MIN_CTAS 4
 #endif
-template <int DIR, bool CUSTOM, class DV>
-__device__ __forceinline__ void face2(DV& dv, const Field4& f, long idx, long step, double al, double gamma, double eps,
-                                      double delta, const Field4& out)
+template <bool CUSTOM, class DV>
+__device__ __forceinline__ void face2(DV& dv, const Field4& f, uint32_t idx, bool y, int step, double al, double gamma,
+                                      double eps, double delta, const Field4& out)
 {
+    const double* const f1 = y ? f.p[2] : f.p[1];
+    const double* const f2 = y ? f.p[1] : f.p[2];
     double s[6][4], o[4];
 #pragma unroll
     for (int p = 0; p < 6; ++p) {
-        const long a = idx + (p - 2) * step;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) s[p][k] = f.p[k][a];
+        const long a = (long)idx + (p - 2) * step;
+        s[p][0] = f.p[0][a], s[p][1] = f1[a], s[p][2] = f2[a], s[p][3] = f.p[3][a];
     }
-    if (CUSTOM) face_flux_2d<DIR>(dv, s, al, gamma, o, eps, delta);
-    else face_flux_2d<DIR>(dv, s, al, gamma, o);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) out.p[k][idx] = o[k];
+    if (CUSTOM) face_flux_2d(dv, s, y, al, gamma, o, eps, delta);
+    else face_flux_2d(dv, s, y, al, gamma, o);
+    out.p[0][idx] = o[0];
+    (y ? out.p[2] : out.p[1])[idx] = o[1];
+    (y ? out.p[1] : out.p[2])[idx] = o[2];
+    out.p[3][idx] = o[3];
 }
 // A face whose operands are outside the range of SharedDiv, with IEEE divisions.
-template <int DIR, bool CUSTOM>
-__device__ __noinline__ void face_any2(Field4 f, long idx, long step, double al, double gamma, double eps, double delta,
-                                       Field4 out)
+template <bool CUSTOM>
+__device__ __noinline__ void face_any2(Field4 f, uint32_t idx, bool y, int step, double al, double gamma, double eps,
+                                       double delta, Field4 out)
 {
     IeeeDiv dv;
-    face2<DIR, CUSTOM>(dv, f, idx, step, al, gamma, eps, delta, out);
-}
-
-template <int DIR, bool CUSTOM>
-__global__ void __launch_bounds__(128, AWCM_FACE_MIN_CTAS)
-    k_face(Grid2 g, Field4 f, Field4 out, const uint32_t* __restrict__ list, const unsigned* __restrict__ count,
-           const double* __restrict__ alpha, const StepState* st, StepState* dt_st)
-{
-    pdl_begin();
-    const int done = st->done;
-    const unsigned n = *count;
-    if (done) return;
-    // dt_st: this launch also computes the step's dt (from the CFL speed of the scan before it);
-    // the faces do not read it, the point updates after them do
-    if (dt_st && blockIdx.x == 0 && threadIdx.x == 0) compute_dt(g, dt_st);
-    const long stride = (long)gridDim.x * blockDim.x;
-    for (long e = gtid(); e < n; e += stride) {
-        const uint32_t idx = list[e];
-        const unsigned row = row_of(g, idx);
-        const int ii = (int)(idx - row * (unsigned)g.pitch) - kGhost, jj = (int)row - kGhost;
-        const long step = DIR == 0 ? 1 : g.pitch;
-        const double al = DIR == 0 ? alpha[jj] : alpha[ii];
-        SharedDiv dv;
-        if (CUSTOM) dv.bad = !(g.wz_eps >= 1e-40 && g.wz_eps < 1e40 && g.wz_delta < 1e40);
-        face2<DIR, CUSTOM>(dv, f, idx, step, al, g.gamma, g.wz_eps, g.wz_delta, out);
-        if (dv.bad) face_any2<DIR, CUSTOM>(f, idx, step, al, g.gamma, g.wz_eps, g.wz_delta, out);
-    }
+    face2<CUSTOM>(dv, f, idx, y, step, al, gamma, eps, delta, out);
 }
 
 // RK combinations of the three stages (main_2d_euler(quad).cpp:162, 242, 321 and 325-332):
@@ -2262,9 +2242,11 @@ __device__ __forceinline__ void update_fin_point(const Grid2& g, Field4 in, Fiel
 // the reference's one-sided forms next to the boundary (AWCM_2D::Differentiate*, Wavelet/AWCM_2D.h:154-187,
 // branch selection main_2d_euler(quad).cpp:132-160).
 // inx: the field of the x-direction fluxes (the wind tunnel's x-sweep copy of the stage input, else in).
+// dt: the step's dt where the level factors st->sc may not be written yet, else null.
 template <int KIND>
 __device__ __forceinline__ void update_crs_point(const Grid2& g, Field4 in, Field4 inx, Field4 out, Field4 qn,
-                                                 const int8_t* __restrict__ lvl, size_t a, const StepState* st)
+                                                 const int8_t* __restrict__ lvl, size_t a, const StepState* st,
+                                                 const double* dt = nullptr)
 {
     const int NX = g.nx - 1, NY = g.ny - 1;
     const unsigned row = row_of(g, (unsigned)a);
@@ -2321,28 +2303,71 @@ __device__ __forceinline__ void update_crs_point(const Grid2& g, Field4 in, Fiel
             for (int k = 0; k < 4; ++k) dG[k] = kD1 * (gt[k] - gb[k]) + kD2 * (go[k] - gbb[k]);
         }
     }
-    rk_store<KIND>(in, out, qn, a, dF, dG, st->sc[lev]);
+    rk_store<KIND>(in, out, qn, a, dF, dG, dt ? *dt / (g.dx * g.D(lev)) : st->sc[lev]);
 }
 
-// The finest-level and the coarse points of a stage in one launch: the two sets are disjoint and
-// neither reads what the other writes (the stage output, or qn at the point itself).
-template <int KIND>
-__global__ void __launch_bounds__(256) k_update(Grid2 g, Field4 in, Field4 inx, Field4 out, Field4 qn, Field4 fx,
-                                                Field4 fy, const int8_t* __restrict__ lvl,
-                                                const uint32_t* __restrict__ lf, const unsigned* __restrict__ nf,
-                                                const uint32_t* __restrict__ lc, const unsigned* __restrict__ nc,
-                                                const StepState* st)
+// The x faces, the y faces and the coarse points of a stage in one launch: all three read the stage input,
+// and none reads what another writes.  The faces are bound by the FP64 pipe where their lists fill the chip,
+// by the latency of their arithmetic where they do not: one list of both directions with one code (two
+// codes side by side do not fit the instruction cache: 2049 x 2049 757 us) has no launch and no ragged wave between
+// them, and the coarse points, bound by their loads, run in the first CTAs beside them.  Steps against a
+// launch a direction in parallel branches and the coarse points with the finest ones: 129 x 129 137 -> 129 us,
+// 641 x 385 247 -> 237, 2049 x 513 388 -> 357, 2049 x 2049 737 -> 726; 100 frozen steps of 513 x 513
+// 9.3 -> 7.7 ms.  With the coarse points in k_update: 140, 246, 384, 740 us and 8.7 ms.
+struct StageArgs {
+    Field4 in, inx, out, qn, fx, fy;          // inx: the field of the x-direction fluxes (see update_crs_point)
+    const int8_t* lvl;
+    const uint32_t *fin, *crs, *xf, *yf;      // finest points, coarse points, x faces, y faces
+    const unsigned* n;                        // their four counts
+    const double *ax, *ay;                    // LF speeds
+    const StepState* st;
+    StepState* dt_st;                         // set: this launch also computes the step's dt
+    unsigned coarse;                          // CTAs of the coarse points, the first ones
+};
+template <bool CUSTOM, int KIND>
+__global__ void __launch_bounds__(128, AWCM_FACE_MIN_CTAS) k_faces(Grid2 g, const __grid_constant__ StageArgs A)
 {
     pdl_begin();
-    const int done = st->done;
-    const unsigned n0 = *nf, n = n0 + *nc;
-    const double sc = st->sc[g.maxl];
-    if (done) return;
-    const long stride = (long)gridDim.x * blockDim.x;
-    for (long e = gtid(); e < n; e += stride) {
-        if (e < n0) update_fin_point<KIND>(g, in, out, qn, fx, fy, lf[e], sc);
-        else update_crs_point<KIND>(g, in, inx, out, qn, lvl, lc[e - n0], st);
+    if (A.st->done) return;
+    // dt from the CFL speed of the scan before: the faces do not need it, the coarse points take it
+    // themselves, the finest points follow in k_update
+    if (A.dt_st && blockIdx.x == 0 && threadIdx.x == 0) compute_dt(g, A.dt_st);
+    if (blockIdx.x < A.coarse) {
+        const unsigned n = A.n[1];
+        bool clipped;
+        const double dt = A.dt_st ? step_dt(g, A.st, clipped) : 0.0;
+        for (unsigned e = gtid(); e < n; e += A.coarse * 128)
+            update_crs_point<KIND>(g, A.in, A.inx, A.out, A.qn, A.lvl, A.crs[e], A.st, A.dt_st ? &dt : nullptr);
+        return;
     }
+    const unsigned nx = A.n[2], n = nx + A.n[3];
+    for (unsigned e = (blockIdx.x - A.coarse) * 128 + threadIdx.x; e < n; e += (gridDim.x - A.coarse) * 128) {
+        const bool y = e >= nx;
+        const uint32_t idx = y ? A.yf[e - nx] : A.xf[e];
+        const unsigned row = row_of(g, idx);
+        const int ii = (int)(idx - row * (unsigned)g.pitch) - kGhost, jj = (int)row - kGhost;
+        const double al = y ? A.ay[ii] : A.ax[jj];
+        const int step = y ? g.pitch : 1;
+        const Field4& in = y ? A.in : A.inx;
+        const Field4& out = y ? A.fy : A.fx;
+        SharedDiv dv;
+        if (CUSTOM) dv.bad = !(g.wz_eps >= 1e-40 && g.wz_eps < 1e40 && g.wz_delta < 1e40);
+        face2<CUSTOM>(dv, in, idx, y, step, al, g.gamma, g.wz_eps, g.wz_delta, out);
+        if (dv.bad) face_any2<CUSTOM>(in, idx, y, step, al, g.gamma, g.wz_eps, g.wz_delta, out);
+    }
+}
+
+// The finest-level points of a stage, from its face fluxes.
+template <int KIND>
+__global__ void __launch_bounds__(256) k_update(Grid2 g, const __grid_constant__ StageArgs A)
+{
+    pdl_begin();
+    const int done = A.st->done;
+    const unsigned n = A.n[0];
+    const double sc = A.st->sc[g.maxl];
+    if (done) return;
+    for (unsigned e = gtid(); e < n; e += gridDim.x * blockDim.x)
+        update_fin_point<KIND>(g, A.in, A.out, A.qn, A.fx, A.fy, A.fin[e], sc);
 }
 
 // ------------------------------------------------------------------------- layout conversions
@@ -2568,19 +2593,13 @@ struct Solver2D {
     int8_t* bcf_dev = nullptr;  // BOUNDARY_CONDITION plane of the generic manager
     cudaStream_t stream = nullptr;
     // Second branch of the step graph: PrepareEuler's interpolation of the momenta and energy runs
-    // beside the density's inverse transform, and the x faces beside the y faces.  `cur` is the
-    // stream the launch helper enqueues on (null = `stream`).
+    // beside the density's inverse transform.  `cur` is the stream the launch helper enqueues on
+    // (null = `stream`).
     cudaStream_t side = nullptr, side2 = nullptr;
     cudaStream_t cur = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr;
     // a finely profiled step keeps one stream: its per-kernel events time the launches in order
     bool fork_ok() const { return side && !fine; }
-    void fork(cudaStream_t to)
-    {
-        cudaEventRecord(ev_fork, stream);
-        cudaStreamWaitEvent(to, ev_fork, 0);
-        cur = to;
-    }
     void join(cudaStream_t from, cudaEvent_t ev)
     {
         cur = nullptr;
@@ -3267,43 +3286,28 @@ struct Solver2D {
     void enq_faces_update(int stage, Field4 in, Field4 out, const double* axp = nullptr, const double* ayp = nullptr,
                           bool with_dt = false)
     {
-        StepState* dts = with_dt ? st : nullptr;
         uint32_t* const* L = lists + 4 * stage;
         const unsigned* C = st->cnt + 4 * stage;
-        const double* sx = axp ? axp : ax[stage];
-        // face kernels: 16 CTAs of 128 per SM over the face list (4 resident, so four waves); 8 or 4
-        // per SM measured 1.3 % and 7 % slower faces
-        const double* sy = ayp ? ayp : ay[stage];
+        StageArgs A;
+        A.in = in, A.inx = xin(in), A.out = out, A.qn = q, A.fx = fx, A.fy = fy, A.lvl = lvl[2 - stage];
+        A.fin = L[0], A.crs = L[1], A.xf = L[2], A.yf = L[3], A.n = C;
+        A.ax = axp ? axp : ax[stage], A.ay = ayp ? ayp : ay[stage];
+        A.st = st, A.dt_st = with_dt ? st : nullptr;
+        // face_blocks is 8 CTAs an SM: 12 for the faces (8 and 16: up to 1.3 % slower 2049 x 2049 steps), 2 for
+        // the coarse points (3 and 4: a 129 x 129 step 135 us instead of 129)
+        A.coarse = face_blocks / 4;
+        const unsigned nb = A.coarse + face_blocks / 2 * 3;
+        const bool custom = !(g.wz_eps == 1e-40 && g.wz_delta == 0.0);
         mark();
-        // the x faces (fx) and the y faces (fy) read the same stage input: parallel branches
-        const bool par = fork_ok();
-        if (par) fork(side);
-        if (g.wz_eps == 1e-40 && g.wz_delta == 0.0)
-            launch(k_face<0, false>, 2 * face_blocks, 128, g, xin(in), fx, L[2], C + 2, sx, st, (StepState*)nullptr);
-        else
-            launch(k_face<0, true>, 2 * face_blocks, 128, g, xin(in), fx, L[2], C + 2, sx, st, (StepState*)nullptr);
-        after("k_face<0>");
-        cur = nullptr;
-        if (g.wz_eps == 1e-40 && g.wz_delta == 0.0)
-            launch(k_face<1, false>, 2 * face_blocks, 128, g, in, fy, L[3], C + 3, sy, st, dts);
-        else
-            launch(k_face<1, true>, 2 * face_blocks, 128, g, in, fy, L[3], C + 3, sy, st, dts);
-        after("k_face<1>");
-        if (par) join(side, ev_join);
+        launch(stage == 0   ? (custom ? k_faces<true, 1> : k_faces<false, 1>)
+               : stage == 1 ? (custom ? k_faces<true, 2> : k_faces<false, 2>)
+                            : (custom ? k_faces<true, 3> : k_faces<false, 3>),
+               nb, 128, g, A);
+        after("k_faces");
+        mark();
+        launch(stage == 0 ? k_update<1> : stage == 1 ? k_update<2> : k_update<3>, face_blocks / 2, 256, g, A);
+        after("k_update");
         launches += 2;
-        mark();
-        const int ub = face_blocks / 2;
-        if (stage == 0) {
-            launch(k_update<1>, ub, 256, g, in, xin(in), out, q, fx, fy, lvl[2], L[0], C + 0, L[1], C + 1, st);
-            after("k_update<1>");
-        } else if (stage == 1) {
-            launch(k_update<2>, ub, 256, g, in, xin(in), out, q, fx, fy, lvl[1], L[0], C + 0, L[1], C + 1, st);
-            after("k_update<2>");
-        } else {
-            launch(k_update<3>, ub, 256, g, in, xin(in), out, q, fx, fy, lvl[0], L[0], C + 0, L[1], C + 1, st);
-            after("k_update<3>");
-        }
-        launches += 1;
         mark();
     }
 

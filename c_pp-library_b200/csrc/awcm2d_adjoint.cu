@@ -265,14 +265,15 @@ __device__ __forceinline__ bool face_flux_2d_vjp(DV& dv, const Cell& cell, const
     const auto c2 = dv.twice(c1);
     R.kc = dv.quot_pos(0.4, dv.by(R.c * R.c));
     R.i2c = dv.quot_pos(0.5, c1);
+    const double A = R.H - R.u * R.u - R.v * R.v;
     // ---- forward: characteristic variables and LF split of the six cells
 #pragma unroll
     for (int p = 0; p < 6; ++p) {
         double s[4], f[4], rq[4], rf[4];
         cell(p, s);
         cell_flux2<DIR>(dv, s, g, f, nullptr);
-        inv2<DIR>(dv, R.u, R.v, R.H, R.c, R.kc, c2, s, rq);
-        inv2<DIR>(dv, R.u, R.v, R.H, R.c, R.kc, c2, f, rf);
+        inv2<DIR>(dv, A, R.u, R.v, R.c, R.kc, c2, s, rq);
+        inv2<DIR>(dv, A, R.u, R.v, R.c, R.kc, c2, f, rf);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             RQs(p, k) = rq[k];

@@ -333,14 +333,14 @@ __device__ __forceinline__ void speeds2(DV& dv, const double* q, double g, doubl
 }
 
 // ROE_SOLVER_2D::Inversion_X / Inversion_Y (ROESOLVER.h:73-96); kc = 0.4 / c / c, same value, c2 the
-// divisor 2 c.
+// divisor 2 c, A = H - u * u - v * v.
 template <int DIR, class DV>
-__device__ __forceinline__ void inv2(DV& dv, double u, double v, double H, double c, double kc,
+__device__ __forceinline__ void inv2(DV& dv, double A, double u, double v, double c, double kc,
                                      const typename DV::Divisor& c2, const double* b, double* x)
 {
     double x3;
-    if (DIR == 0) x3 = (H - u * u - v * v) * b[0] + u * b[1] + v * b[2] - b[3];
-    else x3 = (H - u * u - v * v) * b[0] + v * b[2] + u * b[1] - b[3];
+    if (DIR == 0) x3 = A * b[0] + u * b[1] + v * b[2] - b[3];
+    else x3 = A * b[0] + v * b[2] + u * b[1] - b[3];
     x3 *= kc;
     const double x2 = DIR == 0 ? b[2] - v * b[0] : b[1] - u * b[0];
     double x4 = DIR == 0 ? b[1] + (c - u) * b[0] - c * x3 : b[2] + (c - v) * b[0] - c * x3;
@@ -349,12 +349,6 @@ __device__ __forceinline__ void inv2(DV& dv, double u, double v, double H, doubl
     x[1] = x2;
     x[2] = x3;
     x[3] = x4;
-}
-template <int DIR>
-__device__ __forceinline__ void inv2(double u, double v, double H, double c, double kc, const double* b, double* x)
-{
-    IeeeDiv dv;
-    inv2<DIR>(dv, u, v, H, c, kc, 2 * c, b, x);
 }
 
 // The flux of one cell (flux2) with its total enthalpy, velocities and pressure from one reciprocal.
@@ -386,17 +380,19 @@ __device__ __forceinline__ void cell_flux2(DV& dv, const double* q, double g, do
     }
 }
 
-// WENOZ_EULER_SOLVER_2D::ComputeFluxX (DIR 0) / ComputeFluxY (DIR 1), WENOZ.h:236-320, with the Roe
-// average of the two cells at the face (ROE_SOLVER_2D::RoeAverage, ROESOLVER.h:49-70).
-// s[p] = cells -3..+2 across the face along DIR.
-template <int DIR, class DV>
-__device__ __forceinline__ void face_flux_2d(DV& dv, const double (&s)[6][4], double alpha, double g, double* out,
+// WENOZ_EULER_SOLVER_2D::ComputeFluxX / ComputeFluxY, WENOZ.h:236-320, with the Roe average of the two
+// cells at the face (ROE_SOLVER_2D::RoeAverage, ROESOLVER.h:49-70).  s[p] = cells -3..+2 across the face.
+// One code for both directions: a y face passes its cells, and gets its flux, with the momenta exchanged.
+// ComputeFluxY then takes the same operations on the same operands, but for the order in which the Roe
+// velocities' squares are subtracted from H.
+template <class DV>
+__device__ __forceinline__ void face_flux_2d(DV& dv, const double (&s)[6][4], bool y, double alpha, double g, double* out,
                                              double wz_eps = 1e-40, double wz_delta = 0.0)
 {
     double f[6][4], L[3], R[3];
     dv.range(alpha, kSafeLo, kSafeAlpha);
 #pragma unroll
-    for (int p = 0; p < 6; ++p) cell_flux2<DIR>(dv, s[p], g, f[p], p == 2 ? L : p == 3 ? R : nullptr);
+    for (int p = 0; p < 6; ++p) cell_flux2<0>(dv, s[p], g, f[p], p == 2 ? L : p == 3 ? R : nullptr);
     const double sl = sqrt(s[2][0]), sr = sqrt(s[3][0]);
     const auto den = dv.by(sl + sr);
     const double u = dv.quot(sl * L[0] + sr * R[0], den);
@@ -407,12 +403,14 @@ __device__ __forceinline__ void face_flux_2d(DV& dv, const double (&s)[6][4], do
     const auto c1 = dv.by(c);
     const double kc = dv.quot_pos(dv.quot_pos(0.4, c1), c1);
     const auto c2 = dv.twice(c1);
+    const double uu = u * u, vv = v * v;
+    const double A = y ? (H - vv) - uu : (H - uu) - vv;
     double fp[6][4], fm[6][4];
 #pragma unroll
     for (int p = 0; p < 6; ++p) {
         double RQ[4], RF[4];
-        inv2<DIR>(dv, u, v, H, c, kc, c2, s[p], RQ);
-        inv2<DIR>(dv, u, v, H, c, kc, c2, f[p], RF);
+        inv2<0>(dv, A, u, v, c, kc, c2, s[p], RQ);
+        inv2<0>(dv, A, u, v, c, kc, c2, f[p], RF);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             fp[p][k] = 0.5 * (RF[k] + alpha * RQ[k]);
@@ -427,17 +425,10 @@ __device__ __forceinline__ void face_flux_2d(DV& dv, const double (&s)[6][4], do
         S[k] = lr + rl;
     }
     double r1[4], r2[4], r3[4], r4[4];
-    if (DIR == 0) {
-        r1[0] = 1, r2[0] = 0, r3[0] = 1, r4[0] = 1;
-        r1[1] = u - c, r2[1] = 0, r3[1] = u, r4[1] = u + c;
-        r1[2] = v, r2[2] = 1, r3[2] = v, r4[2] = v;
-        r1[3] = H - u * c, r2[3] = v, r3[3] = 0.5 * (u * u + v * v), r4[3] = H + u * c;
-    } else {
-        r1[0] = 1, r2[0] = 0, r3[0] = 1, r4[0] = 1;
-        r1[1] = u, r2[1] = 1, r3[1] = u, r4[1] = u;
-        r1[2] = v - c, r2[2] = 0, r3[2] = v, r4[2] = v + c;
-        r1[3] = H - v * c, r2[3] = u, r3[3] = 0.5 * (u * u + v * v), r4[3] = H + v * c;
-    }
+    r1[0] = 1, r2[0] = 0, r3[0] = 1, r4[0] = 1;
+    r1[1] = u - c, r2[1] = 0, r3[1] = u, r4[1] = u + c;
+    r1[2] = v, r2[2] = 1, r3[2] = v, r4[2] = v;
+    r1[3] = H - u * c, r2[3] = v, r3[3] = 0.5 * (u * u + v * v), r4[3] = H + u * c;
 #pragma unroll
     for (int k = 0; k < 4; ++k) out[k] = S[0] * r1[k] + S[1] * r2[k] + S[2] * r3[k] + S[3] * r4[k];
 }
