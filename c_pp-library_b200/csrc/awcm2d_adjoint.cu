@@ -170,18 +170,18 @@ struct RoeAdj {
     double u, v, H, c, kc, i2c;  // i2c = 1 / (2 c)
 };
 
-// Reverse of inv2<DIR> (ROE_SOLVER_2D::Inversion_X/_Y, ROESOLVER.h:73-96): adds (dx/db)^T xb to
+// Reverse of inv2<0> (ROE_SOLVER_2D::Inversion_X, ROESOLVER.h:73-96): adds (dx/db)^T xb to
 // bb and the parameter adjoints to P.
-template <int DIR, class DV>
+template <class DV>
 __device__ __forceinline__ void inv2_vjp(DV& dv, const RoeAdj& R, const typename DV::Divisor& c1, const double* b,
                                          const double* xb, double* bb, RoeAdj& P)
 {
     const double u = R.u, v = R.v, H = R.H, c = R.c, kc = R.kc;
     const double A = H - u * u - v * v;
-    const double y3 = DIR == 0 ? A * b[0] + u * b[1] + v * b[2] - b[3] : A * b[0] + v * b[2] + u * b[1] - b[3];
+    const double y3 = A * b[0] + u * b[1] + v * b[2] - b[3];
     const double x3 = y3 * kc;
     const double i2c = R.i2c;
-    const double y4 = DIR == 0 ? b[1] + (c - u) * b[0] - c * x3 : b[2] + (c - v) * b[0] - c * x3;
+    const double y4 = b[1] + (c - u) * b[0] - c * x3;
     const double x4 = y4 * i2c;
     // x1 = b0 - x3 - x4
     bb[0] += xb[0];
@@ -190,23 +190,13 @@ __device__ __forceinline__ void inv2_vjp(DV& dv, const RoeAdj& R, const typename
     // x4 = y4 / (2c)
     const double y4b = x4b * i2c;
     P.c -= dv.quot(x4b * x4, c1);
-    if (DIR == 0) {
-        bb[1] += y4b;
-        bb[0] += y4b * (c - u);
-        P.u -= y4b * b[0];
-        // x2 = b2 - v b0
-        bb[2] += xb[1];
-        bb[0] -= xb[1] * v;
-        P.v -= xb[1] * b[0];
-    } else {
-        bb[2] += y4b;
-        bb[0] += y4b * (c - v);
-        P.v -= y4b * b[0];
-        // x2 = b1 - u b0
-        bb[1] += xb[1];
-        bb[0] -= xb[1] * u;
-        P.u -= xb[1] * b[0];
-    }
+    bb[1] += y4b;
+    bb[0] += y4b * (c - u);
+    P.u -= y4b * b[0];
+    // x2 = b2 - v b0
+    bb[2] += xb[1];
+    bb[0] -= xb[1] * v;
+    P.v -= xb[1] * b[0];
     P.c += y4b * (b[0] - x3);
     x3b -= y4b * c;
     // x3 = y3 kc
@@ -228,12 +218,12 @@ __device__ __forceinline__ void inv2_vjp(DV& dv, const RoeAdj& R, const typename
 // Forward values are recomputed here; alpha (the frozen LF speed) has no adjoint.  The 6 x 4
 // characteristic states and fluxes (and, in place, their adjoints) live in shared memory:
 // `sh` points at this thread's slot, element e at sh[e * kAdjThreads].  cell(p, q) reads cell p,
-// add(p, qb) adds to its adjoint; false, with nothing added, where the divisions of DV do not apply.
+// add(p, qb) adds to its adjoint, both with the momenta exchanged for a y face, as ob is; false, with nothing added, where the divisions of DV do not apply.
 // A face's hundred divisions are what its time went to: by shared reciprocals, with the cells read twice instead
 // of kept (no spills; 260 bytes before), the reverse sweep over 513 x 513 takes 22.8 instead of 25.0 ms for
 // 100 steps.  168 registers and 3 CTAs an SM spill and take 25.1.
 constexpr int kAdjThreads = 128;
-template <int DIR, class DV, class Cell, class Add>
+template <class DV, class Cell, class Add>
 __device__ __forceinline__ bool face_flux_2d_vjp(DV& dv, const Cell& cell, const Add& add, double alpha, double g,
                                                  const double* ob, double eps, double delta, double* sh)
 {
@@ -271,9 +261,9 @@ __device__ __forceinline__ bool face_flux_2d_vjp(DV& dv, const Cell& cell, const
     for (int p = 0; p < 6; ++p) {
         double s[4], f[4], rq[4], rf[4];
         cell(p, s);
-        cell_flux2<DIR>(dv, s, g, f, nullptr);
-        inv2<DIR>(dv, A, R.u, R.v, R.c, R.kc, c2, s, rq);
-        inv2<DIR>(dv, A, R.u, R.v, R.c, R.kc, c2, f, rf);
+        cell_flux2<0>(dv, s, g, f, nullptr);
+        inv2<0>(dv, A, R.u, R.v, R.c, R.kc, c2, s, rq);
+        inv2<0>(dv, A, R.u, R.v, R.c, R.kc, c2, f, rf);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             RQs(p, k) = rq[k];
@@ -285,17 +275,10 @@ __device__ __forceinline__ bool face_flux_2d_vjp(DV& dv, const Cell& cell, const
     // reverse below, which recomputes the reconstructions anyway.
     const double u = R.u, v = R.v, H = R.H, c = R.c;
     double Sb[4];
-    if (DIR == 0) {
-        Sb[0] = ob[0] + ob[1] * (u - c) + ob[2] * v + ob[3] * (H - u * c);
-        Sb[1] = ob[2] + ob[3] * v;
-        Sb[2] = ob[0] + ob[1] * u + ob[2] * v + ob[3] * 0.5 * q2;
-        Sb[3] = ob[0] + ob[1] * (u + c) + ob[2] * v + ob[3] * (H + u * c);
-    } else {
-        Sb[0] = ob[0] + ob[1] * u + ob[2] * (v - c) + ob[3] * (H - v * c);
-        Sb[1] = ob[1] + ob[3] * u;
-        Sb[2] = ob[0] + ob[1] * u + ob[2] * v + ob[3] * 0.5 * q2;
-        Sb[3] = ob[0] + ob[1] * u + ob[2] * (v + c) + ob[3] * (H + v * c);
-    }
+    Sb[0] = ob[0] + ob[1] * (u - c) + ob[2] * v + ob[3] * (H - u * c);
+    Sb[1] = ob[2] + ob[3] * v;
+    Sb[2] = ob[0] + ob[1] * u + ob[2] * v + ob[3] * 0.5 * q2;
+    Sb[3] = ob[0] + ob[1] * (u + c) + ob[2] * v + ob[3] * (H + u * c);
     // ---- reverse: WENO-Z reconstructions and the LF split, per characteristic field
     double S[4];
 #pragma unroll
@@ -319,15 +302,9 @@ __device__ __forceinline__ bool face_flux_2d_vjp(DV& dv, const Cell& cell, const
         }
     }
     RoeAdj P{0, 0, 0, 0, 0, 0};
-    if (DIR == 0) {
-        P.u += ob[1] * (S[0] + S[2] + S[3]) + ob[3] * (-S[0] * c + S[2] * u + S[3] * c);
-        P.v += ob[2] * (S[0] + S[2] + S[3]) + ob[3] * (S[1] + S[2] * v);
-        P.c += ob[1] * (S[3] - S[0]) + ob[3] * u * (S[3] - S[0]);
-    } else {
-        P.u += ob[1] * (S[0] + S[2] + S[3]) + ob[3] * (S[1] + S[2] * u);
-        P.v += ob[2] * (S[0] + S[2] + S[3]) + ob[3] * (-S[0] * c + S[2] * v + S[3] * c);
-        P.c += ob[2] * (S[3] - S[0]) + ob[3] * v * (S[3] - S[0]);
-    }
+    P.u += ob[1] * (S[0] + S[2] + S[3]) + ob[3] * (-S[0] * c + S[2] * u + S[3] * c);
+    P.v += ob[2] * (S[0] + S[2] + S[3]) + ob[3] * (S[1] + S[2] * v);
+    P.c += ob[1] * (S[3] - S[0]) + ob[3] * u * (S[3] - S[0]);
     P.H += ob[3] * (S[0] + S[3]);
     // every range is checked by here
     if constexpr (DV::checked)
@@ -341,15 +318,15 @@ __device__ __forceinline__ bool face_flux_2d_vjp(DV& dv, const Cell& cell, const
         double s[4], go[4] = {0, 0, 0, 0}, f[4], fb[4] = {0, 0, 0, 0}, rqb[4], rfb[4];
         double* gs = p == 2 ? gl : p == 3 ? gr : go;
         cell(p, s);
-        cell_flux2<DIR>(dv, s, g, f, nullptr);
+        cell_flux2<0>(dv, s, g, f, nullptr);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             rqb[k] = RQs(p, k);
             rfb[k] = RFs(p, k);
         }
-        inv2_vjp<DIR>(dv, R, c1, s, rqb, gs, P);
-        inv2_vjp<DIR>(dv, R, c1, f, rfb, fb, P);
-        flux2_vjp<DIR>(s, dv.recip(s[0]), g, fb, gs);
+        inv2_vjp(dv, R, c1, s, rqb, gs, P);
+        inv2_vjp(dv, R, c1, f, rfb, fb, P);
+        flux2_vjp<0>(s, dv.recip(s[0]), g, fb, gs);
         if (p != 2 && p != 3) add(p, gs);
     }
     // ---- reverse: Roe average (kc = 0.4 / c^2, c = sqrt(0.4 (H - q2/2)))
@@ -398,58 +375,48 @@ __device__ __forceinline__ bool fin_point(const Grid2& g, const uint8_t* m, cons
 // nu(f) for a finest-level point f (R_f += F_f) minus nu(f+1) for a finest point f+1
 // (R_{f+1} -= F_f); lam -= weight . dF_f/dcells.
 // One face with the divisions of DV; false, with nothing written, where they do not apply.
-template <int DIR, class DV>
-__device__ __forceinline__ bool face_vjp(const AdjStage& A, uint32_t idx, const double* __restrict__ alpha, double* sh)
+template <class DV>
+__device__ __forceinline__ bool face_vjp(const AdjStage& A, uint32_t idx, bool y, double* sh)
 {
     const Grid2& g = A.g;
-    const long step = DIR == 0 ? 1 : g.pitch;
+    const int step = y ? g.pitch : 1;
     const int ii = (int)(idx % (uint32_t)g.pitch) - kGhost;
     const int jj = (int)(idx / (uint32_t)g.pitch) - kGhost;
-    const int i1 = DIR == 0 ? ii + 1 : ii, j1 = DIR == 0 ? jj : jj + 1;
+    const int k1 = y ? 2 : 1, k2 = 3 - k1;
     double w[4] = {0, 0, 0, 0};
     bool any = false;
     if (fin_point(g, A.m, A.lvl, ii, jj, A.bit)) {
-        for (int k = 0; k < 4; ++k) w[k] += A.nu.p[k][idx];
+        w[0] += A.nu.p[0][idx], w[1] += A.nu.p[k1][idx], w[2] += A.nu.p[k2][idx], w[3] += A.nu.p[3][idx];
         any = true;
     }
-    if (fin_point(g, A.m, A.lvl, i1, j1, A.bit)) {
+    if (fin_point(g, A.m, A.lvl, y ? ii : ii + 1, y ? jj + 1 : jj, A.bit)) {
         const size_t b = (size_t)idx + step;
-        for (int k = 0; k < 4; ++k) w[k] -= A.nu.p[k][b];
+        w[0] -= A.nu.p[0][b], w[1] -= A.nu.p[k1][b], w[2] -= A.nu.p[k2][b], w[3] -= A.nu.p[3][b];
         any = true;
     }
     if (!any || (w[0] == 0 && w[1] == 0 && w[2] == 0 && w[3] == 0)) return true;
-    const double al = DIR == 0 ? alpha[jj] : alpha[ii];
+    const double al = y ? A.ay[ii] : A.ax[jj];
+    const double* const f1 = A.qin.p[k1];
+    const double* const f2 = A.qin.p[k2];
+    double* const l1 = A.lam.p[k1];
+    double* const l2 = A.lam.p[k2];
     DV dv;
-    return face_flux_2d_vjp<DIR>(
+    return face_flux_2d_vjp(
         dv,
         [&](int p, double* s) {
             const long a = (long)idx + (p - 2) * step;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) s[k] = A.qin.p[k][a];
+            s[0] = A.qin.p[0][a], s[1] = f1[a], s[2] = f2[a], s[3] = A.qin.p[3][a];
         },
         [&](int p, const double* gs) {
             const long a = (long)idx + (p - 2) * step;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) atomic_sub(&A.lam.p[k][a], gs[k]);
+            atomic_sub(&A.lam.p[0][a], gs[0]), atomic_sub(&l1[a], gs[1]);
+            atomic_sub(&l2[a], gs[2]), atomic_sub(&A.lam.p[3][a], gs[3]);
         },
         al, g.gamma, w, g.wz_eps, g.wz_delta, sh);
 }
-template <int DIR>
-__device__ __noinline__ void face_vjp_any(const AdjStage& A, uint32_t idx, const double* alpha, double* sh)
+__device__ __noinline__ void face_vjp_any(const AdjStage& A, uint32_t idx, bool y, double* sh)
 {
-    face_vjp<DIR, IeeeDiv>(A, idx, alpha, sh);
-}
-
-template <int DIR>
-__device__ __forceinline__ void face_list_vjp(const AdjStage& A, const uint32_t* __restrict__ list,
-                                              const unsigned* __restrict__ count, const double* __restrict__ alpha,
-                                              unsigned first, unsigned stride, double* sh)
-{
-    const unsigned n = *count;
-    for (unsigned e = first; e < n; e += stride) {
-        const uint32_t idx = list[e];
-        if (!face_vjp<DIR, SharedDiv>(A, idx, alpha, sh)) face_vjp_any<DIR>(A, idx, alpha, sh);
-    }
+    face_vjp<IeeeDiv>(A, idx, y, sh);
 }
 
 // Coarse points: R = dF + dG from physical fluxes at spacing d (central, or the reference's
@@ -506,15 +473,14 @@ __device__ __forceinline__ void coarse_list_vjp(const AdjStage& A, unsigned firs
     }
 }
 
-// A stage's x faces and its coarse points in one launch (DIR 0), then its y faces (DIR 1).  The faces are
-// bound by the latency of their arithmetic: 250 registers leave 8 warps on an SM, and a list of 15,000 to
-// 40,000 faces fills half to all of the 37,888 threads that fit.  The coarse points, bound by their loads and
-// atomics, run in the first `coarse` CTAs beside the faces instead of in a launch of their own.
-// 513 x 513, 100 steps, whole reverse sweep: three launches 22.8 ms, coarse points beside the x faces 20.8
-// (as the last CTAs 21.4, beside the y faces 20.9), x and y faces beside each other as well 22.0: the two
-// face codes together no longer fit the instruction cache.
-template <int DIR>
-__global__ void __launch_bounds__(kAdjThreads) k_adj_face(const __grid_constant__ AdjStage A, unsigned coarse)
+// A stage's faces, in both directions with one code, and its coarse points in one launch.  The faces are
+// bound by the latency of their arithmetic: 220 registers leave 8 warps on an SM, and 15,000 to 40,000 x faces
+// and as many y faces make one or two waves of the 37,888 threads that fit.  The coarse points, bound by their
+// loads and atomics, run in the first `coarse` CTAs beside them.
+// 513 x 513, 100 steps, whole reverse sweep: three launches 22.8 ms, coarse points beside the x faces 20.2
+// (as the last CTAs 0.6 more), all in one launch 18.0
+// (x and y faces in one launch with a code each 22.0: the two codes do not fit the instruction cache).
+__global__ void __launch_bounds__(kAdjThreads) k_adj_stage(const __grid_constant__ AdjStage A, unsigned coarse)
 {
     pdl_begin();
     __shared__ double sh[48 * kAdjThreads];
@@ -522,9 +488,12 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_face(const __grid_constant_
         coarse_list_vjp(A, gtid(), coarse * kAdjThreads);
         return;
     }
-    const unsigned first = gtid() - coarse * kAdjThreads, stride = (gridDim.x - coarse) * kAdjThreads;
-    if (DIR == 0) face_list_vjp<0>(A, A.xf, A.nxf, A.ax, first, stride, sh + threadIdx.x);
-    else face_list_vjp<1>(A, A.yf, A.nyf, A.ay, first, stride, sh + threadIdx.x);
+    const unsigned nx = *A.nxf, n = nx + *A.nyf;
+    for (unsigned e = gtid() - coarse * kAdjThreads; e < n; e += (gridDim.x - coarse) * kAdjThreads) {
+        const bool y = e >= nx;
+        const uint32_t idx = y ? A.yf[e - nx] : A.xf[e];
+        if (!face_vjp<SharedDiv>(A, idx, y, sh + threadIdx.x)) face_vjp_any(A, idx, y, sh + threadIdx.x);
+    }
 }
 
 // RK combination adjoints, one dense pass per stage over the plane (points off the grid are
@@ -676,10 +645,9 @@ __global__ void __launch_bounds__(kSeedThreads) k_sum_rows(const double* rowsum,
 
 void adj_launch_stage(const AdjStage& a, int face_blocks, cudaStream_t s)
 {
-    // face_blocks is 8 CTAs an SM: 16 for the faces (8: 0.5 % slower), 4 for the coarse points (8: 1 % slower)
-    const unsigned faces = 2 * face_blocks, coarse = face_blocks / 2;
-    launch_pdl(k_adj_face<0>, faces + coarse, kAdjThreads, s, a, coarse);
-    launch_pdl(k_adj_face<1>, faces, kAdjThreads, s, a, 0u);
+    // face_blocks is 8 CTAs an SM, for the faces (16 and 32: 2 to 3 % slower sweeps); 2 for the coarse points
+    const unsigned coarse = face_blocks / 4;
+    launch_pdl(k_adj_stage, coarse + face_blocks, kAdjThreads, s, a, coarse);
 }
 
 void adj_launch_rk(int stage, const Grid2& g, size_t plane, const uint8_t* m, const int8_t* lvl, const double* sc,
