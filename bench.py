@@ -726,7 +726,7 @@ def run_b200(args):
         "config": dict(WORKLOAD, parallelism=f"replicas{world}" if world > 1 else "single GPU",
                        l2="no flush: device state %.0f MB > 126 MB L2" % (state_bytes / 1e6),
                        steps_from=f"after {warmup} warm-up steps from t=0 (t={t_after_warmup:.3e})"),
-        "roofline": {"bound": "fp64", "kernel": "k_face (WENO-Z/Roe face flux)", "achieved": achieved,
+        "roofline": {"bound": "fp64", "kernel": "k_faces (WENO-Z/Roe face flux, with the coarse points)", "achieved": achieved,
                      "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "traffic": traffic,
                      "peak_note": "of measured: dense DFMA probe on this GPU (2 flops per FMA)",
                      "flops_per_face": FLOPS_PER_FACE, "faces_per_step": faces / len(prof),
@@ -755,7 +755,7 @@ def run_b200(args):
 
 def run_capture(k: int):
     """Small, self-ending run for ncu: the benchmark instance, k graph-replayed steps and one
-    profiled step (its face kernels are launches 6k+1 .. 6k+6 of k_face)."""
+    profiled step (its face kernels are launches 3k+1 .. 3k+3 of k_faces)."""
     import awcm
 
     w = WORKLOAD
