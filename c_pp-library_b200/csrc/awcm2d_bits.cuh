@@ -164,12 +164,14 @@ __device__ void bits_zone(const Grid2& g, const Bits2& B, Span sp, int done)
 //   (marking c points), and on its even columns the columns -+h, -+3h of those d3 points and of its own
 //   d1 points.
 // At the ends the stencil of the first detail h is that of the detail 3h, and likewise at the other end,
-// so the first one counts as both.  A warp takes consecutive words of a row (two words of margin on the
-// left, one on the right; short rows several to a warp), so a word's neighbours come by shuffles.
+// so the first one counts as both.  A warp takes consecutive words of a row (two words of margin on
+// either side; short rows several to a warp), so a word's neighbours come by shuffles.  Two words are what
+// h = 16 needs: a detail marks the words at -1, 0, +1 and +2 of its own, and the last detail NX - 16, as
+// NX - 48, marks NX - 96, two words below its own.
 // A row's thread writes points of the row that no other thread of the pass reads, or (d1, d2 points
 // set by a d3 point) whose marks lie among those of the d3 point.
 // The coarser levels, whose columns are one bit of every (h / 32)-th word, push point by point.
-constexpr int kCloseKeep = 29, kCloseLeft = 2;
+constexpr int kCloseKeep = 28, kCloseLeft = 2;
 __host__ __device__ __forceinline__ int close_rows_per_warp(int nwx) { return nwx <= 32 ? 32 / nwx : 1; }
 __host__ __device__ __forceinline__ long close_warps(long nr, int nwx)
 {
