@@ -1869,7 +1869,6 @@ struct Batch1D {
 // of 8199 doubles and two list regions of 16-bit entries, about 641 KiB,
 // which every GPU that loads this library holds until the process exits.
 constexpr int kNoAllocThreads = 512;
-constexpr size_t kNoAllocSmem = (227 * 1024 - sizeof(Work1)) & ~(size_t)15;
 constexpr int kNoAllocMaxNx = 8193;
 constexpr int kNoAllocMaxW = kNoAllocMaxNx + 2 * kGhost;
 constexpr size_t kNoAllocLists = (size_t)kNoAllocMaxW + 32;  // 4 (w + 32) entries of 2 bytes
@@ -1915,26 +1914,37 @@ __global__ void __launch_bounds__(kNoAllocThreads, 1)
     }
 }
 
-// Device address of the scratch array, resolved once per device (host code must not use the
-// symbol itself: on the host it is only a stand-in for the device copy).
+// Device address of the scratch array (host code must not use the symbol itself: on the host it is only
+// a stand-in for the device copy) and the dynamic shared memory that a launch can take beside the
+// kernel's static one (sizeof(Work1) and what the compiler pads it with), resolved once per device.
 constexpr int kMaxDevices = 64;
+struct NoAlloc {
+    double* scratch;
+    size_t smem;
+};
 std::mutex g_noalloc_mu;
-void* g_noalloc_addr[kMaxDevices] = {};
+NoAlloc g_noalloc[kMaxDevices] = {};
 
-int noalloc_scratch(int dev, double** ptr)
+int noalloc_resources(int dev, NoAlloc* out)
 {
     if (dev < 0 || dev >= kMaxDevices) return kErrArg;
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
-    if (!g_noalloc_addr[dev]) {
+    NoAlloc& N = g_noalloc[dev];
+    if (!N.scratch) {
+        cudaFuncAttributes fa{};
+        int optin = 0;
+        AWCM_CUDA_TRY(cudaFuncGetAttributes(&fa, k_step1d_noalloc));
+        AWCM_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         void* p = nullptr;
         const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess || !p) {
             set_last_error(cudaGetErrorString(e), __FILE__, __LINE__);
             return kErrCuda;
         }
-        g_noalloc_addr[dev] = p;
+        N.smem = ((size_t)optin - fa.sharedSizeBytes) & ~(size_t)15;
+        N.scratch = static_cast<double*>(p);
     }
-    *ptr = static_cast<double*>(g_noalloc_addr[dev]);
+    *out = N;
     return kOk;
 }
 
@@ -2207,8 +2217,8 @@ int awcm1d_step_noalloc(int num_levels, int nx_coarse, double x_min, double x_ma
     }
     int dev = 0;
     AWCM_CUDA_TRY(cudaGetDevice(&dev));
-    double* scratch = nullptr;
-    const int rc = noalloc_scratch(dev, &scratch);
+    NoAlloc N{};
+    const int rc = noalloc_resources(dev, &N);
     if (rc) return rc;
     Inst1 I{};
     I.nx = (int)nx;
@@ -2221,10 +2231,9 @@ int awcm1d_step_noalloc(int num_levels, int nx_coarse, double x_min, double x_ma
     I.cfl = cfl;
     I.t = t;
     I.t_end = t_end;
-    // what fits beside the kernel's static shared memory
-    const unsigned smem = (unsigned)pick_layout((int)nx, num_levels - 1, kNoAllocSmem, false).bytes;
+    const unsigned smem = (unsigned)pick_layout((int)nx, num_levels - 1, N.smem, false).bytes;
     AWCM_CUDA_TRY(cudaFuncSetAttribute(k_step1d_noalloc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_step1d_noalloc<<<1, kNoAllocThreads, smem, (cudaStream_t)stream>>>(I, q_dev, state_dev, scratch, out_dev, make_weights(),
+    k_step1d_noalloc<<<1, kNoAllocThreads, smem, (cudaStream_t)stream>>>(I, q_dev, state_dev, N.scratch, out_dev, make_weights(),
                                                                          smem);
     AWCM_CUDA_TRY(cudaGetLastError());
     return kOk;
