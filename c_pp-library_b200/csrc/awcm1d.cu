@@ -1660,7 +1660,7 @@ struct Batch1D {
         const int stat = (int)fa.sharedSizeBytes;
         smem_cap = (size_t)std::min(optin - stat, per_sm / occ - 1024 - stat) & ~(size_t)15;
         smem = smem_bytes();
-        cudaFuncSetAttribute(k_step1d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        AWCM_CUDA_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(k_step1d), optin - stat));
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_step1d, block, smem);
         if (occ < 1) occ = 1;
         if (ctas_per_sm > 0) occ = std::min(occ, ctas_per_sm);
@@ -1673,7 +1673,6 @@ struct Batch1D {
     void enq_step(int nsteps = 1)
     {
         cudaMemsetAsync(d_queue, 0, sizeof(unsigned), stream);
-        cudaFuncSetAttribute(k_step1d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_step1d<<<grid, block, smem, stream>>>(d_inst, n, d_order, d_queue, P, (unsigned)smem, nsteps);
     }
 
@@ -1916,7 +1915,8 @@ __global__ void __launch_bounds__(kNoAllocThreads, 1)
 
 // Device address of the scratch array (host code must not use the symbol itself: on the host it is only
 // a stand-in for the device copy) and the dynamic shared memory that a launch can take beside the
-// kernel's static one (sizeof(Work1) and what the compiler pads it with), resolved once per device.
+// kernel's static one (sizeof(Work1) and what the compiler pads it with), allowed and resolved once per
+// device.
 constexpr int kMaxDevices = 64;
 struct NoAlloc {
     double* scratch;
@@ -1942,6 +1942,7 @@ int noalloc_resources(int dev, NoAlloc* out)
             return kErrCuda;
         }
         N.smem = ((size_t)optin - fa.sharedSizeBytes) & ~(size_t)15;
+        AWCM_CUDA_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(k_step1d_noalloc), (int)N.smem));
         N.scratch = static_cast<double*>(p);
     }
     *out = N;
@@ -2232,7 +2233,6 @@ int awcm1d_step_noalloc(int num_levels, int nx_coarse, double x_min, double x_ma
     I.t = t;
     I.t_end = t_end;
     const unsigned smem = (unsigned)pick_layout((int)nx, num_levels - 1, N.smem, false).bytes;
-    AWCM_CUDA_TRY(cudaFuncSetAttribute(k_step1d_noalloc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_step1d_noalloc<<<1, kNoAllocThreads, smem, (cudaStream_t)stream>>>(I, q_dev, state_dev, N.scratch, out_dev, make_weights(),
                                                                          smem);
     AWCM_CUDA_TRY(cudaGetLastError());

@@ -2396,10 +2396,10 @@ struct Solver2D {
         bits.aux = bits_mem + 4 * bit_words();
         for (int k = 0; k < 3; ++k) bits.live[k] = bits_mem + (5 + k) * bit_words();
         mark_levels();
-        AWCM_CUDA_TRY(cudaFuncSetAttribute(k_fwt_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem));
-        AWCM_CUDA_TRY(cudaFuncSetAttribute(k_iwt_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem));
-        AWCM_CUDA_TRY(cudaFuncSetAttribute(k_interp_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem));
-        AWCM_CUDA_TRY(cudaFuncSetAttribute(k_bits_all, cudaFuncAttributeMaxDynamicSharedMemorySize, kBitsSmem));
+        AWCM_CUDA_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(k_fwt_coarse), (int)kCoarseSmem));
+        AWCM_CUDA_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(k_iwt_coarse), (int)kCoarseSmem));
+        AWCM_CUDA_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(k_interp_coarse), (int)kCoarseSmem));
+        AWCM_CUDA_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(k_bits_all), kBitsSmem));
         for (int s = 0; s < kStages; ++s) {
             AWCM_CUDA_TRY(cudaMalloc(&ax[s], sizeof(double) * g.ny));
             AWCM_CUDA_TRY(cudaMalloc(&ay[s], sizeof(double) * g.nx));

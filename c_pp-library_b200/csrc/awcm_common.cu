@@ -1,6 +1,7 @@
 // Library-wide C-ABI helpers: per-thread last-error text and the version string.
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "awcm_b200.h"
 #include "awcm_common.cuh"
@@ -13,6 +14,16 @@ void set_last_error(const char* msg, const char* file, int line)
 {
     const char* base = std::strrchr(file, '/');
     std::snprintf(g_last_error, sizeof(g_last_error), "%s (%s:%d)", msg, base ? base + 1 : file, line);
+}
+
+cudaError_t allow_dynamic_smem(const void* kernel, int bytes)
+{
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    cudaFuncAttributes fa{};
+    const cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+    if (e != cudaSuccess || fa.maxDynamicSharedSizeBytes >= bytes) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 // FP64 peak probe: independent DFMA chains on every SM (2 flops per DFMA).

@@ -96,4 +96,9 @@ __device__ __forceinline__ double warp_max(double v)
 
 void set_last_error(const char* msg, const char* file, int line);
 
+// Lets launches of `kernel` on the current device take up to `bytes` of dynamic shared memory.  The limit
+// is the process's, not a handle's: it is only ever raised, by one thread at a time, and a launch passes
+// what it needs itself.
+cudaError_t allow_dynamic_smem(const void* kernel, int bytes);
+
 }  // namespace awcm
