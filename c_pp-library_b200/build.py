@@ -20,7 +20,7 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 LIB = os.path.join(HERE, "libawcm_b200.so")
 SOURCES = ["awcm_common.cu", "awcm2d.cu", "awcm1d.cu", "awcm2d_adjoint.cu", "awcm_state.cpp"]
-HEADERS = ["awcm_common.cuh", "awcm_numerics.cuh", "awcm2d_types.cuh", "awcm2d_bits.cuh"]
+HEADERS = ["awcm_common.cuh", "awcm_numerics.cuh", "awcm2d_types.cuh", "awcm2d_bits.cuh", "awcm1d_layout.cuh"]
 # per-file overrides of the contraction flags
 FMA_SOURCES = {"awcm2d_adjoint.cu"}
 
