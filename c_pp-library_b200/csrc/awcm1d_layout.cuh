@@ -64,7 +64,8 @@ __host__ __device__ __forceinline__ Layout1 pick_layout(int nx, int maxl, size_t
 {
     const int w = nx + 2 * kGhost;
     const size_t full = list_entries1(w), eb = 2 * entry_bytes(w), np = plane_bytes1(nx, maxl);
-    const size_t least = full < 512 ? full : 512;
+    // in whole eights like cap, so that the bytes of a layout give that layout again
+    const size_t least = full < 512 ? full & ~(size_t)7 : 512;
     for (int tier = kInAll; tier >= kInNone; --tier) {
         const size_t fixed = tier == kInNone ? 0 : np + align16(sizeof(double) * tier_doubles(tier, scalar, w));
         if (tier != kInNone && fixed + eb * least > avail) continue;
