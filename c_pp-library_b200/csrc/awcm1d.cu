@@ -85,6 +85,7 @@ struct Work1 {
 
 // A list of points (stored as i + kGhost) with 16- or 32-bit entries.
 struct List {
+    static constexpr bool kSome = false;
     void* p;
     bool half;
     __device__ __forceinline__ int get(unsigned e) const
@@ -204,47 +205,96 @@ __device__ __forceinline__ double reduce_get(const Work1* wk, int slot, int whic
 }
 
 // ------------------------------------------------------------------ masks and levels, bytes <-> planes
-// One warp per word, one point per lane.
-__device__ void load_planes(const Ctx& c, const uint8_t* mb, const int8_t* lb)
+// Sets of planes: bits 0..4 mask0..mask3 and the previous mask0 (as in a mask byte), bits 8..11 the levels.
+constexpr unsigned kAllPlanes = 0xf1fu;
+__host__ __device__ constexpr unsigned level_plane(int k) { return 0x100u << k; }
+// One warp per word, one point per lane: warp `warp` of `nwarp`, four words at a time, so that the latencies
+// of their loads overlap.
+constexpr int kConvWords = 4;
+__device__ __forceinline__ void load_planes(const Ctx& c, const uint8_t* mb, const int8_t* lb, unsigned which, int warp, int nwarp)
 {
-    const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-    for (int x = threadIdx.x >> 5; x < c.nw; x += nwarp) {
-        const int i = 32 * (x - 1) + lane;
-        const bool on = i >= -kGhost && i <= c.N1 + kGhost;
-        const unsigned v = on ? mb[i + kGhost] : 0x1fu;
-        for (int k = 0; k < 5; ++k) {
-            const uint32_t b = __ballot_sync(0xffffffffu, (v >> k) & 1u);
-            if (lane == 0) (k == kPlTemp ? c.plane(kPlTemp) : c.mask(k))[x] = b;
+    const int lane = threadIdx.x & 31;
+    for (int x0 = warp; x0 < c.nw; x0 += kConvWords * nwarp) {
+        auto word = [&](int u) { return x0 + u * nwarp; };
+        auto point = [&](int u) { return 32 * (word(u) - 1) + lane; };
+        if (which & 0x1fu) {
+            unsigned v[kConvWords];
+#pragma unroll
+            for (int u = 0; u < kConvWords; ++u)
+                v[u] = point(u) >= -kGhost && point(u) <= c.N1 + kGhost ? mb[point(u) + kGhost] : 0x1fu;
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                if (!((which >> k) & 1u)) continue;
+                uint32_t* P = k == kPlTemp ? c.plane(kPlTemp) : c.mask(k);
+#pragma unroll
+                for (int u = 0; u < kConvWords; ++u) {
+                    const uint32_t b = __ballot_sync(0xffffffffu, (v[u] >> k) & 1u);
+                    if (lane == 0 && word(u) < c.nw) P[word(u)] = b;
+                }
+            }
         }
+#pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int l = on && i >= 0 && i <= c.N1 ? lb[k * c.w + i + kGhost] : 0;
-            const int s = l < 0 || l > c.maxl ? c.no_level() : l;
-            const uint32_t f = __ballot_sync(0xffffffffu, s == c.maxl);
-            if (lane == 0) c.fine(k)[x] = f;
-            for (int b = 0; b < c.nb; ++b) {
-                const uint32_t y = __ballot_sync(0xffffffffu, (s >> b) & 1);
-                if (lane == 0) c.slice(k, b)[x] = y;
+            if (!(which & level_plane(k))) continue;
+            int l[kConvWords];
+#pragma unroll
+            for (int u = 0; u < kConvWords; ++u)
+                l[u] = point(u) >= 0 && point(u) <= c.N1 ? lb[k * c.w + point(u) + kGhost] : 0;
+#pragma unroll
+            for (int u = 0; u < kConvWords; ++u) {
+                const int s = l[u] < 0 || l[u] > c.maxl ? c.no_level() : l[u];
+                const bool put = lane == 0 && word(u) < c.nw;
+                const uint32_t f = __ballot_sync(0xffffffffu, s == c.maxl);
+                if (put) c.fine(k)[word(u)] = f;
+                for (int b = 0; b < c.nb; ++b) {
+                    const uint32_t y = __ballot_sync(0xffffffffu, (s >> b) & 1);
+                    if (put) c.slice(k, b)[word(u)] = y;
+                }
             }
         }
     }
 }
-// A level outside 0..maxl keeps its byte.
-__device__ void store_planes(const Ctx& c, uint8_t* mb, int8_t* lb)
+// A level outside 0..maxl keeps its byte, and so do the bits of the planes left out.
+__device__ __forceinline__ void store_planes(const Ctx& c, uint8_t* mb, int8_t* lb, unsigned which, int warp, int nwarp)
 {
-    const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-    for (int x = threadIdx.x >> 5; x < c.nw; x += nwarp) {
-        const int i = 32 * (x - 1) + lane;
-        if (i < -kGhost || i > c.N1 + kGhost) continue;
-        const bool ghost = i < 0 || i > c.N1;
-        unsigned v = ghost ? 0xe0u : 0u;
-        for (int k = 0; k < 4; ++k) v |= ((c.mask(k)[x] >> lane) & 1u) << k;
-        v |= ((c.plane(kPlTemp)[x] >> lane) & 1u) << kBitTemp;
-        mb[i + kGhost] = (uint8_t)v;
-        if (ghost) continue;
+    const int lane = threadIdx.x & 31;
+    const unsigned masks = which & 0x1fu;
+    for (int x0 = warp; x0 < c.nw; x0 += kConvWords * nwarp) {
+        auto word = [&](int u) { return x0 + u * nwarp; };
+        auto point = [&](int u) { return 32 * (word(u) - 1) + lane; };
+        auto on = [&](int u, int g) { return point(u) >= -g && point(u) <= c.N1 + g; };
+        if (masks) {
+            unsigned v[kConvWords];
+#pragma unroll
+            for (int u = 0; u < kConvWords; ++u) {
+                v[u] = on(u, 0) ? 0u : 0xe0u;
+                if (masks != 0x1fu && on(u, kGhost)) v[u] = mb[point(u) + kGhost] & ~masks;
+            }
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                if (!((which >> k) & 1u)) continue;
+                const uint32_t* P = k == kPlTemp ? c.plane(kPlTemp) : c.mask(k);
+#pragma unroll
+                for (int u = 0; u < kConvWords; ++u)
+                    if (on(u, kGhost)) v[u] |= ((P[word(u)] >> lane) & 1u) << k;
+            }
+#pragma unroll
+            for (int u = 0; u < kConvWords; ++u)
+                if (on(u, kGhost)) mb[point(u) + kGhost] = (uint8_t)v[u];
+        }
+#pragma unroll
         for (int k = 0; k < 4; ++k) {
-            int l = 0;
-            for (int b = 0; b < c.nb; ++b) l |= (int)((c.slice(k, b)[x] >> lane) & 1u) << b;
-            if (l != c.no_level()) lb[k * c.w + i + kGhost] = (int8_t)l;
+            if (!(which & level_plane(k))) continue;
+            int l[kConvWords] = {};
+            for (int b = 0; b < c.nb; ++b) {
+                const uint32_t* P = c.slice(k, b);
+#pragma unroll
+                for (int u = 0; u < kConvWords; ++u)
+                    if (on(u, 0)) l[u] |= (int)((P[word(u)] >> lane) & 1u) << b;
+            }
+#pragma unroll
+            for (int u = 0; u < kConvWords; ++u)
+                if (on(u, 0) && l[u] != c.no_level()) lb[k * c.w + point(u) + kGhost] = (int8_t)l[u];
         }
     }
 }
@@ -382,14 +432,15 @@ __device__ void build_stage_lists(const Ctx& c, int k, int region)
 // The weights away from the ends, -1/16 and 9/16 (make_weights gives them exactly).
 constexpr double kInnerW0 = -0.0625, kInnerW1 = 0.5625;
 enum Lift1 { kPredictF, kUpdateF, kUpdateI, kPredictI };
-template <int OP>
-__device__ __forceinline__ void lift1(const Ctx& c, const List& L, unsigned lo, unsigned hi, int D,
+template <int OP, class Points>
+__device__ __forceinline__ void lift1(const Ctx& c, const Points& L, unsigned lo, unsigned hi, int D,
                                       const uint32_t* temp = nullptr)
 {
     constexpr bool predict = OP == kPredictF || OP == kPredictI;
     const double tol = c.I.tol;
     for (unsigned e = lo + threadIdx.x; e < hi; e += blockDim.x) {
         const int i = L.get(e);
+        if (Points::kSome && i < 0) continue;
         if (!predict && (i == 0 || i == c.N1)) continue;
         int s, k;
         if (predict) predict_stencil(i, D, c.N1, s, k);
@@ -429,6 +480,28 @@ __device__ void fwt1(const Ctx& c, const List& L)
         lift1<kPredictF>(c, L, off[lev + 1], off[lev + 2], c.D(lev));
         __syncthreads();
         lift1<kUpdateF>(c, L, 0, off[lev + 1], c.D(lev));
+        __syncthreads();
+    }
+}
+
+// The same without a list, for a pass on a short line: a thread per point of a level.
+struct SomePoints {  // first, first + D, .. : those of plane P, else -1
+    static constexpr bool kSome = true;
+    const uint32_t* P;
+    int first, D;
+    __device__ __forceinline__ int get(unsigned e) const
+    {
+        const int i = first + (int)e * D;
+        return Ctx::bit(P, i) ? i : -1;
+    }
+};
+__device__ void fwt_short1(const Ctx& c)
+{
+    for (int lev = c.maxl - 1; lev >= 0; --lev) {
+        const int D = c.D(lev), nd = c.N1 / D;
+        lift1<kPredictF>(c, SomePoints{c.m0, D >> 1, D}, 0, nd, D);
+        __syncthreads();
+        lift1<kUpdateF>(c, SomePoints{c.m0, D, D}, 0, nd - 1, D);
         __syncthreads();
     }
 }
@@ -1235,7 +1308,7 @@ __device__ void step_inst(const Buffers1& g, const Weights& W, uint8_t* smem, si
     c.ls = p;
     c.cap = lay.cap;
     if (threadIdx.x < 32) wk->cls[threadIdx.x] = 0;
-    load_planes(c, g.mask, g.level);
+    load_planes(c, g.mask, g.level, kAllPlanes, threadIdx.x >> 5, blockDim.x >> 5);
     __syncthreads();
     // Between steps the field is zero off mask0 (RemoveResidue); a field or masks set from outside
     // need not be, and then the first step removes the residue everywhere.
@@ -1252,7 +1325,7 @@ __device__ void step_inst(const Buffers1& g, const Weights& W, uint8_t* smem, si
         else stages1(I, c, L3, dense);
         dense = false;
     }
-    store_planes(c, g.mask, g.level);
+    store_planes(c, g.mask, g.level, kAllPlanes, threadIdx.x >> 5, blockDim.x >> 5);
     for (int t = threadIdx.x; t < w; t += blockDim.x) {
         if (c.f.m0) g.q[t] = c.f.q0[place(t, kPlaceMask)];
         if (c.f.m12) {
@@ -1320,9 +1393,16 @@ __global__ void __launch_bounds__(kMaxThreads1, 1) k_step1d(Inst1* insts, int n,
 }
 
 // Single passes for the C-ABI manager surface (one CTA per instance), on planes in global memory.
+constexpr int kPassThreads = 512;
+// Points up to which a transform goes without lists (whole calls of the forward transform without / with, the
+// host's share of 12 us a call and 20 us of parameters included: 257 points 35 / 37 us, 2049 41 / 43, 4097 46.5 / 46,
+// 8193 55 / 52).
+constexpr int kShortLine1 = 2100;
 // The inverse transform of any mask: unlike in the step the mask need not be closed, so points
 // outside it are zeroed in their level's own phase, as in the reference.
-__device__ void iwt_any1(const Ctx& c, const uint32_t* M)
+// on(i): whether point i is in the mask.
+template <class On>
+__device__ void iwt_any1(const Ctx& c, On&& on)
 {
     for (int lev = 0; lev < c.maxl; ++lev) {
         const int D = c.D(lev), h = D >> 1, nd = c.N1 / D;
@@ -1330,7 +1410,7 @@ __device__ void iwt_any1(const Ctx& c, const uint32_t* M)
             for (int a = threadIdx.x; a < (ph ? nd : nd - 1); a += blockDim.x) {
                 const int i = ph ? h + a * D : D + a * D;
                 double v = 0;
-                if (Ctx::bit(M, i)) {
+                if (on(i)) {
                     int s, k;
                     if (ph) predict_stencil(i, D, c.N1, s, k);
                     else update_stencil(i, D, c.N1, s, k);
@@ -1348,27 +1428,35 @@ __device__ void iwt_any1(const Ctx& c, const uint32_t* M)
     }
 }
 // InterpolateEuler(q, mra, from, to) (Wavelet/WAVELET_1D.h:393-431) for any two masks.
+template <class Points>
+__device__ __forceinline__ void interp_level1(const Ctx& c, const Points& L, unsigned lo, unsigned hi, int D, const uint32_t* from)
+{
+    for (unsigned e = lo + threadIdx.x; e < hi; e += blockDim.x) {
+        const int i = L.get(e);
+        if (Points::kSome && (i < 0 || Ctx::bit(from, i))) continue;
+        int s, k;
+        predict_stencil(i, D, c.N1, s, k);
+        for (int p = 1; p < 3; ++p) {
+            double v = 0;
+            for (int cnt = 0; cnt < 4; ++cnt) v += c.w_(cnt, k) * c.Q(p, s + cnt * D);
+            c.Q(p, i) = v;
+        }
+    }
+    __syncthreads();
+}
 __device__ void interp_any1(const Ctx& c, const uint32_t* from, const uint32_t* to)
 {
     for (int x = threadIdx.x; x < c.nw; x += blockDim.x) c.aux[x] = c.points(to, x) & ~from[x];
     __syncthreads();
     close1(c, c.aux);
+    if (c.nx <= kShortLine1) {
+        for (int lev = 0; lev < c.maxl; ++lev)
+            interp_level1(c, SomePoints{c.aux, c.D(lev) >> 1, c.D(lev)}, 0, c.N1 / c.D(lev), c.D(lev), from);
+        return;
+    }
     const List L = order_points(c, 0, c.aux, from);
     const unsigned* off = c.wk->off;
-    for (int lev = 0; lev < c.maxl; ++lev) {
-        const int D = c.D(lev);
-        for (unsigned e = off[lev + 1] + threadIdx.x; e < off[lev + 2]; e += blockDim.x) {
-            const int i = L.get(e);
-            int s, k;
-            predict_stencil(i, D, c.N1, s, k);
-            for (int p = 1; p < 3; ++p) {
-                double v = 0;
-                for (int cnt = 0; cnt < 4; ++cnt) v += c.w_(cnt, k) * c.Q(p, s + cnt * D);
-                c.Q(p, i) = v;
-            }
-        }
-        __syncthreads();
-    }
+    for (int lev = 0; lev < c.maxl; ++lev) interp_level1(c, L, off[lev + 1], off[lev + 2], c.D(lev), from);
 }
 // Density (or scalar field) to 0 at the interior points outside M (the inverse transform's zeros).
 __device__ void zero_off1(const Ctx& c, const uint32_t* M)
@@ -1377,16 +1465,47 @@ __device__ void zero_off1(const Ctx& c, const uint32_t* M)
         if (!Ctx::bit(M, i)) c.Q(0, i) = 0;
 }
 
-__global__ void k_pass1d(Inst1* insts, int inst, Pool P, int op, int bit, int level_id)
+// A single pass converts the planes that it reads and the ones that it writes, no others: a step converts
+// all of them once for some twenty passes, a pass alone would spend its time on them.  (With all of them, on
+// one CTA, every pass over 32769 points took 420 to 600 us; now 11 to 117.)
+struct PassPlanes {
+    unsigned in, out;
+};
+PassPlanes pass_planes(int op, int bit, int level_id)
+{
+    const unsigned M = 1u << bit;
+    switch (op) {
+        case 0: case 1: return {M, M};
+        case 2: return {M | level_plane(level_id), M};
+        case 3: return {M, level_plane(level_id)};
+        case 10: return {kAllPlanes, kAllPlanes};
+        case 11: return {1u, 1u};
+        case 13: return {M | 1u << level_id, 0u};
+        default: return {0u, 0u};  // the passes that read or write single bits of the bytes
+    }
+}
+// The conversions of a pass on all SMs.
+__global__ void k_planes1d(Inst1* insts, int inst, Pool P, unsigned which, int store)
+{
+    const Inst1& I = insts[inst];
+    const Buffers1 g = pool_buffers(I, P);
+    const Ctx c = make_ctx(I, g, nullptr, P.W);
+    const int per = blockDim.x >> 5, warp = blockIdx.x * per + (threadIdx.x >> 5), nwarp = gridDim.x * per;
+    if (store) store_planes(c, g.mask, g.level, which, warp, nwarp);
+    else load_planes(c, g.mask, g.level, which, warp, nwarp);
+}
+// in, out: the planes that the launch converts itself.
+__global__ void __launch_bounds__(kPassThreads) k_pass1d(Inst1* insts, int inst, Pool P, int op, int bit, int level_id, unsigned in, unsigned out)
 {
     __shared__ Work1 wk;
     Inst1& I = insts[inst];
     const Buffers1 g = pool_buffers(I, P);
     Ctx c = make_ctx(I, g, &wk, P.W);
     if (threadIdx.x < 32) wk.cls[threadIdx.x] = 0;
-    load_planes(c, g.mask, g.level);
+    if (in) load_planes(c, g.mask, g.level, in, threadIdx.x >> 5, blockDim.x >> 5);
     __syncthreads();
     uint32_t* M = c.mask(bit);  // bit kBitTemp is plane kPlTemp
+    auto on = [&](int i) { return (g.mask[i + kGhost] >> bit) & 1u; };
     switch (op) {
         case 0: {  // AddAdjacentZone
             for (int x = threadIdx.x; x < c.nw; x += blockDim.x)
@@ -1408,26 +1527,43 @@ __global__ void k_pass1d(Inst1* insts, int inst, Pool P, int op, int bit, int le
             }
             break;
         }
-        case 3: levels1(c, level_id, M); break;
+        case 3:
+            // a point without any neighbour keeps its level: all ones in the planes keep the byte
+            for (int x = threadIdx.x; x < c.nw; x += blockDim.x) {
+                c.fine(level_id)[x] = 0;
+                for (int b = 0; b < c.nb; ++b) c.slice(level_id, b)[x] = ~0u;
+            }
+            levels1(c, level_id, M);  // word x by the same thread
+            break;
         case 4:
             for (int i = threadIdx.x; i <= c.N1; i += blockDim.x)
-                if (!Ctx::bit(M, i)) c.Q(0, i) = c.Q(1, i) = c.Q(2, i) = 0;
+                if (!on(i)) c.Q(0, i) = c.Q(1, i) = c.Q(2, i) = 0;
             break;
-        case 5:
-            for (int x = threadIdx.x; x < c.nw; x += blockDim.x) M[x] |= band_word(c, x);
+        case 5:  // BadingBoundary
+            if (threadIdx.x < 6) {
+                const int t = (int)threadIdx.x, i = t < 3 ? t : c.N1 - (t - 3);
+                if (t < 3 || i >= 3) g.mask[i + kGhost] |= (uint8_t)(1u << bit);
+            }
             break;
         case 10:
             prepare1(c, I.scheme != kScalarAdvection);
             zero_off1(c, c.plane(3));
             break;
-        case 11: fwt1(c, order_points(c, 0, c.m0)); break;
-        case 12: iwt_any1(c, M); break;
+        case 11:
+            if (c.nx <= kShortLine1) fwt_short1(c);
+            else fwt1(c, order_points(c, 0, c.m0));
+            break;
+        case 12: iwt_any1(c, on); break;
         case 13: interp_any1(c, M, c.mask(level_id)); break;  // InterpolateEuler(from = bit, to = level_id as a bit)
         case 14: bc1(c); break;
         default: break;
     }
     __syncthreads();
-    store_planes(c, g.mask, g.level);
+    if (out) store_planes(c, g.mask, g.level, out, threadIdx.x >> 5, blockDim.x >> 5);
+    else if (c.m0 != c.plane(0)) {
+        // the planes are stored by a launch of their own, which looks for mask0 at its own place
+        for (int x = threadIdx.x; x < c.nw; x += blockDim.x) c.plane(0)[x] = c.m0[x];
+    }
 }
 
 // EULER_EQUATION_1D batch entry points (EULER_EQUATION.h:16-26, 42-47): n states of 3 doubles.
@@ -1688,10 +1824,21 @@ struct Batch1D {
         return kOk;
     }
 
+    // Plane words up to which a single pass converts its planes in its own launch: a launch more costs 3 us,
+    // a CTA alone converts about 100 words in one.  Whole calls in one launch / with launches of their own:
+    // CheckReconstruction of 8193 points 23 / 26 us, of 32769 points 37 / 24; PrepareEuler of 2049 points
+    // 87 / 90, of 4097 points 114 / 108, of 32769 points 585 / 415.
+    static constexpr int kPassWords = 1500;
     int pass(int inst, int op, int bit, int level_id)
     {
         if (inst < 0 || inst >= n) return kErrArg;
-        k_pass1d<<<1, 256, 0, stream>>>(d_inst, inst, P, op, bit, level_id);
+        PassPlanes p = pass_planes(op, bit, level_id), own{};
+        const int nw = plane_words1(host[inst].nx);
+        if (nw * (__builtin_popcount(p.in) + __builtin_popcount(p.out)) <= kPassWords) std::swap(p, own);
+        const int blocks = std::min((nw + 7) / 8, 4 * 148);
+        if (p.in) k_planes1d<<<blocks, 256, 0, stream>>>(d_inst, inst, P, p.in, 0);
+        k_pass1d<<<1, kPassThreads, 0, stream>>>(d_inst, inst, P, op, bit, level_id, own.in, own.out);
+        if (p.out) k_planes1d<<<blocks, 256, 0, stream>>>(d_inst, inst, P, p.out, 1);
         AWCM_CUDA_TRY(cudaGetLastError());
         AWCM_CUDA_TRY(cudaStreamSynchronize(stream));
         return kOk;
