@@ -966,11 +966,14 @@ __global__ void k_aaz(Grid2 g, uint8_t* m, int bit, int src, const StepState* st
     AWCM_SKIP_IF_DONE(st);
     ph_aaz(g, m, bit, src, grid_span());
 }
-__global__ void k_cl(Grid2 g, uint8_t* m, int8_t* lvl, int bit, int copy_to, size_t plane, const StepState* st)
+// live: the level set's plane in Bits2 (null for level3), where every point may now have a level.
+__global__ void k_cl(Grid2 g, uint8_t* m, int8_t* lvl, int bit, size_t plane, uint32_t* live)
 {
     pdl_begin();
-    AWCM_SKIP_IF_DONE(st);
-    ph_cl(g, m, lvl, bit, copy_to, plane, grid_span());
+    const Span sp = grid_span();
+    if (live)
+        for (unsigned w = sp.t0; w < (unsigned)(plane / 32); w += sp.stride) live[w] = ~0u;
+    ph_cl(g, m, lvl, bit, -1, plane, sp);
 }
 __global__ void k_apd(Grid2 g, uint8_t* m, const int8_t* lvl, int bit, int src, const StepState* st)
 {
@@ -3309,8 +3312,7 @@ struct Solver2D {
                 launch(k_apd, pb(words()), 256, g, m, lvl[level_id], b, kBitCopy, nullptr);
                 break;
             case 3:
-                launch(k_cl, pb(words()), 256, g, m, lvl[level_id], b, -1, plane, nullptr);
-                mark_levels();
+                launch(k_cl, pb(words()), 256, g, m, lvl[level_id], b, plane, level_id < 3 ? bits.live[level_id] : nullptr);
                 break;
             case 4: launch(k_remove_residue, pb(words()), 256, g, q, m, b, 0, nullptr); break;
             case 5: launch(k_band_copy, pb(words()), 256, g, m, b, -1, nullptr); break;
