@@ -1936,6 +1936,17 @@ struct StageArgs {
     StepState* dt_st;                         // set: this launch also computes the step's dt
     unsigned coarse;                          // CTAs of the coarse points, the first ones
 };
+// CTAs, of `grid`, for nc coarse points beside nf faces: `least` of them, or more where the points' share of
+// the work is larger (a face counts as five points).  Grids of two or three levels are mostly coarse points:
+// a frozen step of 2049 x 2049 points on two levels, 1,000,000 coarse points and 309,000 faces, takes 616 us with
+// `least` CTAs and 481 so (521 with one launch a kind and direction); with a face as one point 521, but
+// 1597 x 1597 on three levels 198 instead of 185, as three points 479 and 190.
+__device__ __forceinline__ unsigned coarse_ctas(unsigned least, unsigned grid, unsigned nc, unsigned nf)
+{
+    if (!nf) return grid;
+    const unsigned share = (unsigned)((float)grid * ((float)nc / ((float)nc + 5.0f * (float)nf)));
+    return max(least, min(share, grid - 1));
+}
 template <bool CUSTOM, int KIND>
 __global__ void __launch_bounds__(128, AWCM_FACE_MIN_CTAS) k_faces(Grid2 g, const __grid_constant__ StageArgs A)
 {
@@ -1944,16 +1955,16 @@ __global__ void __launch_bounds__(128, AWCM_FACE_MIN_CTAS) k_faces(Grid2 g, cons
     // dt from the CFL speed of the scan before: the faces do not need it, the coarse points take it
     // themselves, the finest points follow in k_update
     if (A.dt_st && blockIdx.x == 0 && threadIdx.x == 0) compute_dt(g, A.dt_st);
-    if (blockIdx.x < A.coarse) {
-        const unsigned n = A.n[1];
+    const unsigned nc = A.n[1], nx = A.n[2], n = nx + A.n[3];
+    const unsigned coarse = coarse_ctas(A.coarse, gridDim.x, nc, n);
+    if (blockIdx.x < coarse) {
         bool clipped;
         const double dt = A.dt_st ? step_dt(g, A.st, clipped) : 0.0;
-        for (unsigned e = gtid(); e < n; e += A.coarse * 128)
+        for (unsigned e = gtid(); e < nc; e += coarse * 128)
             update_crs_point<KIND>(g, A.in, A.inx, A.out, A.qn, A.lvl, A.crs[e], A.st, A.dt_st ? &dt : nullptr);
         return;
     }
-    const unsigned nx = A.n[2], n = nx + A.n[3];
-    for (unsigned e = (blockIdx.x - A.coarse) * 128 + threadIdx.x; e < n; e += (gridDim.x - A.coarse) * 128) {
+    for (unsigned e = (blockIdx.x - coarse) * 128 + threadIdx.x; e < n; e += (gridDim.x - coarse) * 128) {
         const bool y = e >= nx;
         const uint32_t idx = y ? A.yf[e - nx] : A.xf[e];
         const unsigned row = row_of(g, idx);
