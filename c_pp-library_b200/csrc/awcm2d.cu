@@ -1944,6 +1944,9 @@ struct StageArgs {
 __device__ __forceinline__ unsigned coarse_ctas(unsigned least, unsigned grid, unsigned nc, unsigned nf)
 {
     if (!nf) return grid;
+    // a share above `least`, a seventh of the grid, needs nc > 5/6 nf: the common case without a division (computing
+    // it always, a 129 x 129 step takes 134.0 us instead of 133.1)
+    if (nc <= nf - nf / 6) return least;
     const unsigned share = (unsigned)((float)grid * ((float)nc / ((float)nc + 5.0f * (float)nf)));
     return max(least, min(share, grid - 1));
 }
