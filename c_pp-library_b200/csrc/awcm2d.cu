@@ -1790,8 +1790,7 @@ __device__ __forceinline__ void face2(DV& dv, const Field4& f, uint32_t idx, boo
         const long a = (long)idx + (p - 2) * step;
         s[p][0] = f.p[0][a], s[p][1] = f1[a], s[p][2] = f2[a], s[p][3] = f.p[3][a];
     }
-    if (CUSTOM) face_flux_2d(dv, s, y, al, gamma, o, eps, delta);
-    else face_flux_2d(dv, s, y, al, gamma, o);
+    if (!(CUSTOM ? face_flux_2d(dv, s, y, al, gamma, o, eps, delta) : face_flux_2d(dv, s, y, al, gamma, o))) return;
     out.p[0][idx] = o[0];
     (y ? out.p[2] : out.p[1])[idx] = o[1];
     (y ? out.p[1] : out.p[2])[idx] = o[2];

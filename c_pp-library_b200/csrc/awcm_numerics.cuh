@@ -385,8 +385,11 @@ __device__ __forceinline__ void cell_flux2(DV& dv, const double* q, double g, do
 // One code for both directions: a y face passes its cells, and gets its flux, with the momenta exchanged.
 // ComputeFluxY then takes the same operations on the same operands, but for the order in which the Roe
 // velocities' squares are subtracted from H.
+// false, with nothing in out, where the cells, alpha or the speed of sound are outside the range of DV: a state in
+// units that are out of range everywhere then pays for little more than the IEEE divisions (scaled by 2^25, a
+// 2049 x 2049 step takes 860 us; 991 with both ways in full, 949 with IEEE divisions alone).
 template <class DV>
-__device__ __forceinline__ void face_flux_2d(DV& dv, const double (&s)[6][4], bool y, double alpha, double g, double* out,
+__device__ __forceinline__ bool face_flux_2d(DV& dv, const double (&s)[6][4], bool y, double alpha, double g, double* out,
                                              double wz_eps = 1e-40, double wz_delta = 0.0)
 {
     double f[6][4], L[3], R[3];
@@ -400,6 +403,8 @@ __device__ __forceinline__ void face_flux_2d(DV& dv, const double (&s)[6][4], bo
     const double H = dv.quot(sl * L[2] + sr * R[2], den);
     const double c = sqrt(0.4 * (H - 0.5 * (u * u + v * v)));
     dv.range(c, kSafeC, kSafeHi);
+    if constexpr (DV::checked)
+        if (dv.bad) return false;
     const auto c1 = dv.by(c);
     const double kc = dv.quot_pos(dv.quot_pos(0.4, c1), c1);
     const auto c2 = dv.twice(c1);
@@ -431,6 +436,7 @@ __device__ __forceinline__ void face_flux_2d(DV& dv, const double (&s)[6][4], bo
     r1[3] = H - u * c, r2[3] = v, r3[3] = 0.5 * (u * u + v * v), r4[3] = H + u * c;
 #pragma unroll
     for (int k = 0; k < 4; ++k) out[k] = S[0] * r1[k] + S[1] * r2[k] + S[2] * r3[k] + S[3] * r4[k];
+    return true;
 }
 
 }  // namespace awcm
