@@ -208,40 +208,90 @@ __device__ __forceinline__ double reduce_get(const Work1* wk, int slot, int whic
 // Sets of planes: bits 0..4 mask0..mask3 and the previous mask0 (as in a mask byte), bits 8..11 the levels.
 constexpr unsigned kAllPlanes = 0xf1fu;
 __host__ __device__ constexpr unsigned level_plane(int k) { return 0x100u << k; }
-// One warp per word, one point per lane: warp `warp` of `nwarp`, four words at a time, so that the latencies
-// of their loads overlap.
-constexpr int kConvWords = 4;
-__device__ __forceinline__ void load_planes(const Ctx& c, const uint8_t* mb, const int8_t* lb, unsigned which, int warp, int nwarp)
+// One warp per word, one point per lane.
+__device__ void load_planes(const Ctx& c, const uint8_t* mb, const int8_t* lb)
+{
+    const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    for (int x = threadIdx.x >> 5; x < c.nw; x += nwarp) {
+        const int i = 32 * (x - 1) + lane;
+        const bool on = i >= -kGhost && i <= c.N1 + kGhost;
+        const unsigned v = on ? mb[i + kGhost] : 0x1fu;
+        for (int k = 0; k < 5; ++k) {
+            const uint32_t b = __ballot_sync(0xffffffffu, (v >> k) & 1u);
+            if (lane == 0) (k == kPlTemp ? c.plane(kPlTemp) : c.mask(k))[x] = b;
+        }
+        for (int k = 0; k < 4; ++k) {
+            const int l = on && i >= 0 && i <= c.N1 ? lb[k * c.w + i + kGhost] : 0;
+            const int s = l < 0 || l > c.maxl ? c.no_level() : l;
+            const uint32_t f = __ballot_sync(0xffffffffu, s == c.maxl);
+            if (lane == 0) c.fine(k)[x] = f;
+            for (int b = 0; b < c.nb; ++b) {
+                const uint32_t y = __ballot_sync(0xffffffffu, (s >> b) & 1);
+                if (lane == 0) c.slice(k, b)[x] = y;
+            }
+        }
+    }
+}
+// A level outside 0..maxl keeps its byte.
+__device__ void store_planes(const Ctx& c, uint8_t* mb, int8_t* lb)
+{
+    const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    for (int x = threadIdx.x >> 5; x < c.nw; x += nwarp) {
+        const int i = 32 * (x - 1) + lane;
+        if (i < -kGhost || i > c.N1 + kGhost) continue;
+        const bool ghost = i < 0 || i > c.N1;
+        unsigned v = ghost ? 0xe0u : 0u;
+        for (int k = 0; k < 4; ++k) v |= ((c.mask(k)[x] >> lane) & 1u) << k;
+        v |= ((c.plane(kPlTemp)[x] >> lane) & 1u) << kBitTemp;
+        mb[i + kGhost] = (uint8_t)v;
+        if (ghost) continue;
+        for (int k = 0; k < 4; ++k) {
+            int l = 0;
+            for (int b = 0; b < c.nb; ++b) l |= (int)((c.slice(k, b)[x] >> lane) & 1u) << b;
+            if (l != c.no_level()) lb[k * c.w + i + kGhost] = (int8_t)l;
+        }
+    }
+}
+// The planes `which` alone, U words of a warp at a time, so that the latencies of their loads overlap: a single
+// pass's conversions, by warp `warp` of `nwarp`.  (A step, whose launch converts all planes once beside its
+// twenty passes, keeps the short loops above: these cost a 257-point scalar step 41 us instead of 34.)
+// The bits of the planes left out keep their values.
+template <int U>
+__device__ __forceinline__ void load_some(const Ctx& c, const uint8_t* mb, const int8_t* lb, unsigned which, int warp, int nwarp)
 {
     const int lane = threadIdx.x & 31;
-    for (int x0 = warp; x0 < c.nw; x0 += kConvWords * nwarp) {
+    for (int x0 = warp; x0 < c.nw; x0 += U * nwarp) {
         auto word = [&](int u) { return x0 + u * nwarp; };
         auto point = [&](int u) { return 32 * (word(u) - 1) + lane; };
-        if (which & 0x1fu) {
-            unsigned v[kConvWords];
+        bool on[U], in[U];  // on the ghosted line, on the line
 #pragma unroll
-            for (int u = 0; u < kConvWords; ++u)
-                v[u] = point(u) >= -kGhost && point(u) <= c.N1 + kGhost ? mb[point(u) + kGhost] : 0x1fu;
+        for (int u = 0; u < U; ++u) {
+            on[u] = point(u) >= -kGhost && point(u) <= c.N1 + kGhost;
+            in[u] = point(u) >= 0 && point(u) <= c.N1;
+        }
+        if (which & 0x1fu) {
+            unsigned v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = on[u] ? mb[point(u) + kGhost] : 0x1fu;
 #pragma unroll
             for (int k = 0; k < 5; ++k) {
                 if (!((which >> k) & 1u)) continue;
                 uint32_t* P = k == kPlTemp ? c.plane(kPlTemp) : c.mask(k);
 #pragma unroll
-                for (int u = 0; u < kConvWords; ++u) {
+                for (int u = 0; u < U; ++u) {
                     const uint32_t b = __ballot_sync(0xffffffffu, (v[u] >> k) & 1u);
                     if (lane == 0 && word(u) < c.nw) P[word(u)] = b;
                 }
             }
         }
-#pragma unroll
         for (int k = 0; k < 4; ++k) {
             if (!(which & level_plane(k))) continue;
-            int l[kConvWords];
+            int l[U];
 #pragma unroll
-            for (int u = 0; u < kConvWords; ++u)
-                l[u] = point(u) >= 0 && point(u) <= c.N1 ? lb[k * c.w + point(u) + kGhost] : 0;
+            for (int u = 0; u < U; ++u)
+                l[u] = in[u] ? lb[k * c.w + point(u) + kGhost] : 0;
 #pragma unroll
-            for (int u = 0; u < kConvWords; ++u) {
+            for (int u = 0; u < U; ++u) {
                 const int s = l[u] < 0 || l[u] > c.maxl ? c.no_level() : l[u];
                 const bool put = lane == 0 && word(u) < c.nw;
                 const uint32_t f = __ballot_sync(0xffffffffu, s == c.maxl);
@@ -254,47 +304,51 @@ __device__ __forceinline__ void load_planes(const Ctx& c, const uint8_t* mb, con
         }
     }
 }
-// A level outside 0..maxl keeps its byte, and so do the bits of the planes left out.
-__device__ __forceinline__ void store_planes(const Ctx& c, uint8_t* mb, int8_t* lb, unsigned which, int warp, int nwarp)
+template <int U>
+__device__ __forceinline__ void store_some(const Ctx& c, uint8_t* mb, int8_t* lb, unsigned which, int warp, int nwarp)
 {
     const int lane = threadIdx.x & 31;
     const unsigned masks = which & 0x1fu;
-    for (int x0 = warp; x0 < c.nw; x0 += kConvWords * nwarp) {
+    for (int x0 = warp; x0 < c.nw; x0 += U * nwarp) {
         auto word = [&](int u) { return x0 + u * nwarp; };
         auto point = [&](int u) { return 32 * (word(u) - 1) + lane; };
-        auto on = [&](int u, int g) { return point(u) >= -g && point(u) <= c.N1 + g; };
-        if (masks) {
-            unsigned v[kConvWords];
+        bool on[U], in[U];
 #pragma unroll
-            for (int u = 0; u < kConvWords; ++u) {
-                v[u] = on(u, 0) ? 0u : 0xe0u;
-                if (masks != 0x1fu && on(u, kGhost)) v[u] = mb[point(u) + kGhost] & ~masks;
+        for (int u = 0; u < U; ++u) {
+            on[u] = point(u) >= -kGhost && point(u) <= c.N1 + kGhost;
+            in[u] = point(u) >= 0 && point(u) <= c.N1;
+        }
+        if (masks) {
+            unsigned v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                v[u] = in[u] ? 0u : 0xe0u;
+                if (masks != 0x1fu && on[u]) v[u] = mb[point(u) + kGhost] & ~masks;
             }
 #pragma unroll
             for (int k = 0; k < 5; ++k) {
                 if (!((which >> k) & 1u)) continue;
                 const uint32_t* P = k == kPlTemp ? c.plane(kPlTemp) : c.mask(k);
 #pragma unroll
-                for (int u = 0; u < kConvWords; ++u)
-                    if (on(u, kGhost)) v[u] |= ((P[word(u)] >> lane) & 1u) << k;
+                for (int u = 0; u < U; ++u)
+                    if (on[u]) v[u] |= ((P[word(u)] >> lane) & 1u) << k;
             }
 #pragma unroll
-            for (int u = 0; u < kConvWords; ++u)
-                if (on(u, kGhost)) mb[point(u) + kGhost] = (uint8_t)v[u];
+            for (int u = 0; u < U; ++u)
+                if (on[u]) mb[point(u) + kGhost] = (uint8_t)v[u];
         }
-#pragma unroll
         for (int k = 0; k < 4; ++k) {
             if (!(which & level_plane(k))) continue;
-            int l[kConvWords] = {};
+            int l[U] = {};
             for (int b = 0; b < c.nb; ++b) {
                 const uint32_t* P = c.slice(k, b);
 #pragma unroll
-                for (int u = 0; u < kConvWords; ++u)
-                    if (on(u, 0)) l[u] |= (int)((P[word(u)] >> lane) & 1u) << b;
+                for (int u = 0; u < U; ++u)
+                    if (in[u]) l[u] |= (int)((P[word(u)] >> lane) & 1u) << b;
             }
 #pragma unroll
-            for (int u = 0; u < kConvWords; ++u)
-                if (on(u, 0) && l[u] != c.no_level()) lb[k * c.w + point(u) + kGhost] = (int8_t)l[u];
+            for (int u = 0; u < U; ++u)
+                if (in[u] && l[u] != c.no_level()) lb[k * c.w + point(u) + kGhost] = (int8_t)l[u];
         }
     }
 }
@@ -1308,7 +1362,7 @@ __device__ void step_inst(const Buffers1& g, const Weights& W, uint8_t* smem, si
     c.ls = p;
     c.cap = lay.cap;
     if (threadIdx.x < 32) wk->cls[threadIdx.x] = 0;
-    load_planes(c, g.mask, g.level, kAllPlanes, threadIdx.x >> 5, blockDim.x >> 5);
+    load_planes(c, g.mask, g.level);
     __syncthreads();
     // Between steps the field is zero off mask0 (RemoveResidue); a field or masks set from outside
     // need not be, and then the first step removes the residue everywhere.
@@ -1325,7 +1379,7 @@ __device__ void step_inst(const Buffers1& g, const Weights& W, uint8_t* smem, si
         else stages1(I, c, L3, dense);
         dense = false;
     }
-    store_planes(c, g.mask, g.level, kAllPlanes, threadIdx.x >> 5, blockDim.x >> 5);
+    store_planes(c, g.mask, g.level);
     for (int t = threadIdx.x; t < w; t += blockDim.x) {
         if (c.f.m0) g.q[t] = c.f.q0[place(t, kPlaceMask)];
         if (c.f.m12) {
@@ -1491,8 +1545,8 @@ __global__ void k_planes1d(Inst1* insts, int inst, Pool P, unsigned which, int s
     const Buffers1 g = pool_buffers(I, P);
     const Ctx c = make_ctx(I, g, nullptr, P.W);
     const int per = blockDim.x >> 5, warp = blockIdx.x * per + (threadIdx.x >> 5), nwarp = gridDim.x * per;
-    if (store) store_planes(c, g.mask, g.level, which, warp, nwarp);
-    else load_planes(c, g.mask, g.level, which, warp, nwarp);
+    if (store) store_some<4>(c, g.mask, g.level, which, warp, nwarp);
+    else load_some<4>(c, g.mask, g.level, which, warp, nwarp);
 }
 // in, out: the planes that the launch converts itself.
 __global__ void __launch_bounds__(kPassThreads) k_pass1d(Inst1* insts, int inst, Pool P, int op, int bit, int level_id, unsigned in, unsigned out)
@@ -1502,7 +1556,9 @@ __global__ void __launch_bounds__(kPassThreads) k_pass1d(Inst1* insts, int inst,
     const Buffers1 g = pool_buffers(I, P);
     Ctx c = make_ctx(I, g, &wk, P.W);
     if (threadIdx.x < 32) wk.cls[threadIdx.x] = 0;
-    if (in) load_planes(c, g.mask, g.level, in, threadIdx.x >> 5, blockDim.x >> 5);
+    const int warp = threadIdx.x >> 5, nwarp = kPassThreads / 32;
+    if (in && c.nw <= nwarp) load_some<1>(c, g.mask, g.level, in, warp, nwarp);
+    else if (in) load_some<4>(c, g.mask, g.level, in, warp, nwarp);
     __syncthreads();
     uint32_t* M = c.mask(bit);  // bit kBitTemp is plane kPlTemp
     auto on = [&](int i) { return (g.mask[i + kGhost] >> bit) & 1u; };
@@ -1559,7 +1615,8 @@ __global__ void __launch_bounds__(kPassThreads) k_pass1d(Inst1* insts, int inst,
         default: break;
     }
     __syncthreads();
-    if (out) store_planes(c, g.mask, g.level, out, threadIdx.x >> 5, blockDim.x >> 5);
+    if (out && c.nw <= nwarp) store_some<1>(c, g.mask, g.level, out, warp, nwarp);
+    else if (out) store_some<4>(c, g.mask, g.level, out, warp, nwarp);
     else if (c.m0 != c.plane(0)) {
         // the planes are stored by a launch of their own, which looks for mask0 at its own place
         for (int x = threadIdx.x; x < c.nw; x += blockDim.x) c.plane(0)[x] = c.m0[x];
