@@ -432,23 +432,20 @@ __device__ void ph_cr(const Grid2& g, uint8_t* __restrict__ m, int lev, int bit,
 // odd) off the left/right columns, d3 = (odd, odd) -- exactly the sub-band extents of band_of.
 // Rows with parity `rows` (0 even, 1 odd, 2 both) in units of h.
 constexpr int kRowScanMaxH = 2;
-__device__ __forceinline__ unsigned rowscan_n(const Grid2& g, int lev, int rows)
+__device__ __forceinline__ unsigned rowscan_n(const Grid2& g, int lev)
 {
     const unsigned nr = (unsigned)((g.ny - 1) >> (g.maxl - lev - 1)) + 1u;  // rows 0, h, .., NY
-    const unsigned wpr = (unsigned)g.pitch / 4u;
-    return (rows == 2 ? nr : (rows == 0 ? (nr + 1u) / 2u : nr / 2u)) * wpr;
+    return nr * ((unsigned)g.pitch / 4u);
 }
 // Decodes virtual thread t of a row scan into the row j and the word (its first column i0, its
 // mask bits v) ; returns the set of lanes that are points of this level (columns multiple of h in
 // [0, NX]).
-__device__ __forceinline__ unsigned rowscan_word(const Grid2& g, int lev, int rows, unsigned t, int& j, int& i0,
-                                                 unsigned& widx)
+__device__ __forceinline__ unsigned rowscan_word(const Grid2& g, int lev, unsigned t, int& j, int& i0, unsigned& widx)
 {
     const int h = g.D(lev) >> 1;
     const unsigned wpr = (unsigned)g.pitch / 4u;
     const unsigned r = row_of_word(g, t), wi = t - r * wpr;
-    const unsigned rr = rows == 2 ? r : 2u * r + (unsigned)rows;
-    j = (int)rr * h;
+    j = (int)r * h;
     i0 = 4 * (int)wi - kGhost;
     widx = (unsigned)(j + kGhost) * wpr + wi;
     unsigned lanes = lanes_in(i0, 0, g.nx - 1);
@@ -468,7 +465,7 @@ __device__ __forceinline__ int rowscan_band(const Grid2& g, int i, int j, int h)
 __device__ void ph_cr_rows(const Grid2& g, uint8_t* __restrict__ m, int lev, int bit, Span sp)
 {
     const int D = g.D(lev), h = D >> 1;
-    const unsigned n = rowscan_n(g, lev, 2);
+    const unsigned n = rowscan_n(g, lev);
     const unsigned* mp = reinterpret_cast<const unsigned*>(m);
     const unsigned row0 = (unsigned)kGhost * ((unsigned)g.pitch / 4u);
     for (unsigned t = sp.t0; t < n; t += sp.stride) {
@@ -477,7 +474,7 @@ __device__ void ph_cr_rows(const Grid2& g, uint8_t* __restrict__ m, int lev, int
         if (h == 1 && !((mp[row0 + t] >> bit) & kLaneBits)) continue;
         int j, i0;
         unsigned wdx;
-        const unsigned lanes = rowscan_word(g, lev, 2, t, j, i0, wdx);
+        const unsigned lanes = rowscan_word(g, lev, t, j, i0, wdx);
         unsigned hit = (mp[wdx] >> bit) & lane_bits(lanes);
         while (hit) {
             const int L = (__ffs(hit) - 1) >> 3;
@@ -1645,10 +1642,8 @@ constexpr int kNumLists = 4 * kStages;
 
 struct ListArgs {
     uint32_t* list[kNumLists];
-    // optional: LF-speed accumulators of stages 2 and 3 to zero, and the dt computation (both need
-    // only to happen after stage 1's speeds and before their own use)
+    // optional: LF-speed accumulators of stages 2 and 3 to zero (after stage 1's speeds and before their own use)
     double *zx1 = nullptr, *zy1 = nullptr, *zx2 = nullptr, *zy2 = nullptr;
-    int with_dt = 0;
 };
 
 // Stage predicates of the point (i, j) (i from -1, j from -1): per stage s (bits 4s..4s+3):
@@ -1692,7 +1687,6 @@ __global__ void __launch_bounds__(256) k_lists(Grid2 g, const uint8_t* __restric
         const unsigned lin = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
         if (la.zx1 && lin < (unsigned)g.ny) la.zx1[lin] = la.zx2[lin] = 0.0;
         if (la.zy1 && lin < (unsigned)g.nx) la.zy1[lin] = la.zy2[lin] = 0.0;
-        if (la.with_dt && lin == 0) compute_dt(g, st);
     }
     __shared__ unsigned wcnt[8][kNumLists];
     __shared__ unsigned woff[8][kNumLists];
@@ -2596,18 +2590,17 @@ struct Solver2D {
     // Fine levels (point spacing <= kRowScanMaxH) scan mask words row by row and skip empty words;
     // coarser levels enumerate their sub-band points.
     bool row_scan(int lev) const { return (g.D(lev) >> 1) <= kRowScanMaxH; }
-    long rowscan_threads(int lev, int rows) const
+    long rowscan_threads(int lev) const
     {
         const int h = g.D(lev) >> 1;
-        const long nr = (g.ny - 1) / h + 1, wpr = g.pitch / 4;
-        return (rows == 2 ? nr : (rows == 0 ? (nr + 1) / 2 : nr / 2)) * wpr;
+        return (long)((g.ny - 1) / h + 1) * (g.pitch / 4);
     }
 
     void enq_cr(int bit, const StepState* s)
     {
         for (int lev = g.maxl - 1; lev >= 0; --lev) {
             if (row_scan(lev)) {
-                launch(k_cr_rows, pb(rowscan_threads(lev, 2)), 256, g, m, lev, bit, s);
+                launch(k_cr_rows, pb(rowscan_threads(lev)), 256, g, m, lev, bit, s);
                 after("k_cr_rows");
             } else {
                 launch(k_cr, pb(details(lev)), 256, g, m, lev, bit, s);
@@ -2746,9 +2739,8 @@ struct Solver2D {
     // Scalar AWCM instance (Wavelet/main_2d_advect.cpp): plane 0 of q, q2, q1 carries the field.
     bool scalar = false;
 
-    // Worklists of the step's three stages and the mask counts; with_dt also computes dt (from the
-    // CFL speed, so after the stage-1 scan).
-    void enq_lists(int with_dt)
+    // Worklists of the step's three stages and the mask counts.
+    void enq_lists()
     {
         ListArgs la;
         for (int L = 0; L < kNumLists; ++L) la.list[L] = lists[L];
@@ -2756,14 +2748,13 @@ struct Solver2D {
         la.zy1 = ay[1];
         la.zx2 = ax[2];
         la.zy2 = ay[2];
-        la.with_dt = with_dt;
         dim3 grid((g.nx + 1 + 255) / 256, (g.ny + 1 + kListRows - 1) / kListRows);
         launch(k_lists, grid, 256, g, m, lvl[2], lvl[1], lvl[0], la, st);
         after("k_lists");
         launches += 1;
     }
 
-    // Begins the step (k_begin or k_begin_copy) as well.  lists: the step's worklists are built too (without dt),
+    // Begins the step (k_begin or k_begin_copy) as well.  lists: the step's worklists are built too,
     // as soon as the masks and levels are final.
     void enq_prepare(const StepState* s, bool lists = false)
     {
@@ -2796,7 +2787,7 @@ struct Solver2D {
             cudaLaunchKernelEx(&cfg, k_prepare, A);
             after("k_prepare");
             launches += 1;
-            if (lists) enq_lists(0);
+            if (lists) enq_lists();
             return;
         }
         // mask_temp = mask0
@@ -2810,11 +2801,11 @@ struct Solver2D {
         // AWCM_2D::Prepare (the scalar form, Wavelet/AWCM_2D.h:52-79) ends with the inverse transform
         if (scalar) {
             enq_iwt(3, s);
-            if (lists) enq_lists(0);
+            if (lists) enq_lists();
         } else if (!fork_ok()) {
             enq_iwt(3, s, true);
             enq_interp_new(s);
-            if (lists) enq_lists(0);
+            if (lists) enq_lists();
         } else {
             // The inverse transform writes the density only and reads mask3; the interpolation
             // reads mask3 and mask_temp and reads and writes components 1..3; the worklist build
@@ -2827,7 +2818,7 @@ struct Solver2D {
             enq_interp_new(s);
             if (lists) {
                 cur = side2;
-                enq_lists(0);
+                enq_lists();
             }
             cur = nullptr;
             enq_iwt(3, s, true);
@@ -2939,7 +2930,7 @@ struct Solver2D {
         launches = 0;
         mark();
         // the worklists (and the zeroing of stage 2/3's speed accumulators) are built beside the
-        // last PrepareEuler passes; dt is computed by the first stage's y-face launch
+        // last PrepareEuler passes; dt is computed by the first stage's launch
         enq_prepare(st, true);
         mark();
         const bool wt = g.bc_kind == AWCM_BC_WIND_TUNNEL;

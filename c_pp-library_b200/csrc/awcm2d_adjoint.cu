@@ -170,7 +170,7 @@ struct RoeAdj {
     double u, v, H, c, kc, i2c;  // i2c = 1 / (2 c)
 };
 
-// Reverse of inv2<0> (ROE_SOLVER_2D::Inversion_X, ROESOLVER.h:73-96): adds (dx/db)^T xb to
+// Reverse of inv2 (ROE_SOLVER_2D::Inversion_X, ROESOLVER.h:73-96): adds (dx/db)^T xb to
 // bb and the parameter adjoints to P.
 template <class DV>
 __device__ __forceinline__ void inv2_vjp(DV& dv, const RoeAdj& R, const typename DV::Divisor& c1, const double* b,
@@ -265,9 +265,9 @@ __device__ __forceinline__ bool face_flux_2d_vjp(DV& dv, const Cell& cell, const
     for (int p = 0; p < 6; ++p) {
         double s[4], f[4], rq[4], rf[4];
         cell(p, s);
-        cell_flux2<0>(dv, s, g, f, nullptr);
-        inv2<0>(dv, A, R.u, R.v, R.c, R.kc, c2, s, rq);
-        inv2<0>(dv, A, R.u, R.v, R.c, R.kc, c2, f, rf);
+        cell_flux2(dv, s, g, f, nullptr);
+        inv2(dv, A, R.u, R.v, R.c, R.kc, c2, s, rq);
+        inv2(dv, A, R.u, R.v, R.c, R.kc, c2, f, rf);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             RQs(p, k) = rq[k];
@@ -322,7 +322,7 @@ __device__ __forceinline__ bool face_flux_2d_vjp(DV& dv, const Cell& cell, const
         double s[4], go[4] = {0, 0, 0, 0}, f[4], fb[4] = {0, 0, 0, 0}, rqb[4], rfb[4];
         double* gs = p == 2 ? gl : p == 3 ? gr : go;
         cell(p, s);
-        cell_flux2<0>(dv, s, g, f, nullptr);
+        cell_flux2(dv, s, g, f, nullptr);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             rqb[k] = RQs(p, k);

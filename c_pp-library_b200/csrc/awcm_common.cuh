@@ -78,13 +78,6 @@ __device__ __forceinline__ void atomic_max_nonneg(double* addr, double v)
     atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
 }
 
-__device__ __forceinline__ double warp_max(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = maxd(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
 #define AWCM_CUDA_TRY(expr)                                                                        \
     do {                                                                                           \
         cudaError_t _e = (expr);                                                                   \

@@ -332,18 +332,16 @@ __device__ __forceinline__ void speeds2(DV& dv, const double* q, double g, doubl
     sy = absd(dv.quot(q[2], rho)) + c;
 }
 
-// ROE_SOLVER_2D::Inversion_X / Inversion_Y (ROESOLVER.h:73-96); kc = 0.4 / c / c, same value, c2 the
-// divisor 2 c, A = H - u * u - v * v.
-template <int DIR, class DV>
+// ROE_SOLVER_2D::Inversion_X (ROESOLVER.h:73-84; Inversion_Y with the momenta exchanged); kc = 0.4 / c / c, same
+// value, c2 the divisor 2 c, A = H - u * u - v * v.
+template <class DV>
 __device__ __forceinline__ void inv2(DV& dv, double A, double u, double v, double c, double kc,
                                      const typename DV::Divisor& c2, const double* b, double* x)
 {
-    double x3;
-    if (DIR == 0) x3 = A * b[0] + u * b[1] + v * b[2] - b[3];
-    else x3 = A * b[0] + v * b[2] + u * b[1] - b[3];
+    double x3 = A * b[0] + u * b[1] + v * b[2] - b[3];
     x3 *= kc;
-    const double x2 = DIR == 0 ? b[2] - v * b[0] : b[1] - u * b[0];
-    double x4 = DIR == 0 ? b[1] + (c - u) * b[0] - c * x3 : b[2] + (c - v) * b[0] - c * x3;
+    const double x2 = b[2] - v * b[0];
+    double x4 = b[1] + (c - u) * b[0] - c * x3;
     x4 = dv.quot(x4, c2);
     x[0] = b[0] - x3 - x4;
     x[1] = x2;
@@ -351,8 +349,8 @@ __device__ __forceinline__ void inv2(DV& dv, double A, double u, double v, doubl
     x[3] = x4;
 }
 
-// The flux of one cell (flux2) with its total enthalpy, velocities and pressure from one reciprocal.
-template <int DIR, class DV>
+// The x flux of one cell (flux2<0>) with its velocities and total enthalpy from one reciprocal.
+template <class DV>
 __device__ __forceinline__ void cell_flux2(DV& dv, const double* q, double g, double* f, double* prim)
 {
     dv.range(q[0], -kSafeRho, kSafeRho);
@@ -362,17 +360,10 @@ __device__ __forceinline__ void cell_flux2(DV& dv, const double* q, double g, do
     const auto r = dv.by(q[0]);
     const double rho = q[0], u = dv.quot(q[1], r), v = dv.quot(q[2], r), E = q[3];
     const double p = (g - 1) * (q[3] - dv.quot(0.5 * (sqr(q[1]) + sqr(q[2])), r));
-    if (DIR == 0) {
-        f[0] = rho * u;
-        f[1] = rho * u * u + p;
-        f[2] = rho * v * u;
-        f[3] = (E + p) * u;
-    } else {
-        f[0] = rho * v;
-        f[1] = rho * u * v;
-        f[2] = rho * v * v + p;
-        f[3] = (E + p) * v;
-    }
+    f[0] = rho * u;
+    f[1] = rho * u * u + p;
+    f[2] = rho * v * u;
+    f[3] = (E + p) * u;
     if (prim) {
         prim[0] = u;
         prim[1] = v;
@@ -395,7 +386,7 @@ __device__ __forceinline__ bool face_flux_2d(DV& dv, const double (&s)[6][4], bo
     double f[6][4], L[3], R[3];
     dv.range(alpha, kSafeLo, kSafeAlpha);
 #pragma unroll
-    for (int p = 0; p < 6; ++p) cell_flux2<0>(dv, s[p], g, f[p], p == 2 ? L : p == 3 ? R : nullptr);
+    for (int p = 0; p < 6; ++p) cell_flux2(dv, s[p], g, f[p], p == 2 ? L : p == 3 ? R : nullptr);
     const double sl = sqrt(s[2][0]), sr = sqrt(s[3][0]);
     const auto den = dv.by(sl + sr);
     const double u = dv.quot(sl * L[0] + sr * R[0], den);
@@ -414,8 +405,8 @@ __device__ __forceinline__ bool face_flux_2d(DV& dv, const double (&s)[6][4], bo
 #pragma unroll
     for (int p = 0; p < 6; ++p) {
         double RQ[4], RF[4];
-        inv2<0>(dv, A, u, v, c, kc, c2, s[p], RQ);
-        inv2<0>(dv, A, u, v, c, kc, c2, f[p], RF);
+        inv2(dv, A, u, v, c, kc, c2, s[p], RQ);
+        inv2(dv, A, u, v, c, kc, c2, f[p], RF);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             fp[p][k] = 0.5 * (RF[k] + alpha * RQ[k]);

@@ -64,7 +64,7 @@ __device__ void all2(DV& face, DV& point, const double* q, bool y, double alpha,
         for (int k = 0; k < 4; ++k) s[p][k] = q[4 * p + k];
     face_flux_2d(face, s, y, alpha, g, o, eps, delta);
     speeds2(point, s[2], g, o[4], o[5]);
-    cell_flux2<0>(point, s[2], g, o + 6, prim);
+    cell_flux2(point, s[2], g, o + 6, prim);
     for (int k = 0; k < 3; ++k) o[10 + k] = prim[k];
 }
 // out: flux[4], speeds[2], physical flux[4], primitives[3], then the same by IeeeDiv
