@@ -2409,7 +2409,6 @@ struct Solver2D {
         AWCM_CUDA_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(k_fwt_coarse), (int)kCoarseSmem));
         AWCM_CUDA_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(k_iwt_coarse), (int)kCoarseSmem));
         AWCM_CUDA_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(k_interp_coarse), (int)kCoarseSmem));
-        AWCM_CUDA_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(k_bits_all), kBitsSmem));
         for (int s = 0; s < kStages; ++s) {
             AWCM_CUDA_TRY(cudaMalloc(&ax[s], sizeof(double) * g.ny));
             AWCM_CUDA_TRY(cudaMalloc(&ay[s], sizeof(double) * g.nx));
@@ -2687,10 +2686,11 @@ struct Solver2D {
     }
 
     // The mask and level chain on bit planes, from the forward transform's mask0 to mask0..mask3 and
-    // level0..level2.  Grids of up to kBitsOne words a plane (128 x 129 points and the like) in one launch of one
-    // CTA; larger ones a launch per pass.
-    static constexpr long kBitsOne = 4096;
-    static constexpr int kBitsSmem = 200 * 1024;
+    // level0..level2.  Grids of up to kBitsOne words a plane (177 x 177 points and the like) in one launch of one
+    // CTA; larger ones a launch per pass.  Steps in one launch / a launch per pass: 129^2 (675 words) 132.5 / 141 us,
+    // 161^2 (1002 words) 154.3 / 154.0 with 4 levels and 167.6 / 172.6 with 5, 177^2 (1098 words) 175.0 / 176.3,
+    // 193^2 (1393 words) 187 / 179, 257^2 221 / 191, 321^2 274 / 205.
+    static constexpr long kBitsOne = 1100;
     void enq_masks(const StepState* s)
     {
         const long n = (long)bit_words();
