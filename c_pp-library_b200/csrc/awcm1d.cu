@@ -821,11 +821,13 @@ __device__ __forceinline__ void stencil_push(const Ctx& c, uint32_t* P, int x, i
 // ComputeLevel(level_{k-1}, mask_{k-1}), mask_k = mask_{k-1}, AddAdjacentZone(mask_k) (zone) and
 // AddPointForDifferentiation(mask_k, level_{k-1}) in one phase.  All of them read mask_{k-1} only
 // (the zone's points are not in it, so their level is 0), and mask_k (clear before) takes ORs.
-// Lines of up to a few hundred points leave most warps idle at one word per thread.  There a warp takes
+// Lines of up to a few thousand points leave most warps idle at one word per thread.  There a warp takes
 // 32 words and one job at a time -- the points of one distance, the zone, or the level planes -- so that
 // the searches of the levels run side by side; each of them searches the nearer distances again, so
-// with more words a thread goes through its word's distances in turn.
-constexpr int kJobWords1 = 3;  // times 32 words
+// with more words a thread goes through its word's distances in turn.  Steps by jobs / by words: 1025 points (34
+// words) 52.0 / 57.0 us, 2049 64.2 / 68.9, 3073 (98 words) 71.3 / 74.6, 4097 (130) 84.5 / 86.4, 5121 (162) 79.0 / 79.8,
+// 6145 (194) 93.6 / 91.6, 8193 114.4 / 110.8, 15361 193 / 172.
+constexpr int kJobWords1 = 5;  // times 32 words
 __device__ void next_mask1(const Ctx& c, int k, bool zone)
 {
     const uint32_t* A = c.mask(k - 1);
