@@ -646,7 +646,7 @@ def run_b200(args):
     if os.path.exists(tr_path):
         try:
             per_face = json.load(open(tr_path))["dram_bytes_per_face"]
-            traffic = per_face * faces / (len(prof) * 6)
+            traffic = per_face * faces / (len(prof) * 3)
         except Exception:
             traffic = None
 
@@ -766,13 +766,13 @@ def run_capture(k: int):
 
 
 def run_capture_batch(k: int, skip: int = 0):
-    """Small, self-ending run for ncu: the seeded 512-tube batch at 768 threads per CTA, `skip` RK3
+    """Small, self-ending run for ncu: the seeded 512-tube batch at 512 threads per CTA, `skip` RK3
     steps, then k more (each step one k_step1d launch), then its totals and the running instances."""
     import awcm
     from awcm import workloads
 
     b = workloads.make_batch(awcm, workloads.shock_tubes(BATCHED["instances"]))
-    b.set_launch(768, 0)
+    b.set_launch(512, 0)
     b.set_run(BATCHED["tol"], BATCHED["cfl"], 0.0, BATCHED["t_end"])
     if skip:
         b.steps(skip)
